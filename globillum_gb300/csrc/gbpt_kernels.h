@@ -232,7 +232,7 @@ inline void bind_slots(Frame& F, unsigned char* slots, unsigned char* shadow) {
 // Launch-wide parameters of one chunk.
 struct RenderParams {
     int refill;        // refill a warp's lanes once this many are idle (1..32)
-    int tri_mode;      // 0: all pending triangles then a node; 1/2: triangle postponing, one / all triangles;
+    int tri_mode;      // 0: a warp step is a node visit or a triangle test; 1/2: triangle postponing, one / all triangles;
                        // 3: warp-cooperative triangle tests, then a node
     int blocks_per_sm; // resident blocks per SM of the traversal kernels (0 = occupancy limit)
     int sampling_terms; // adjoint: add the derivatives of the sampling decisions (sampling_scores)

@@ -451,8 +451,9 @@ typedef struct {
     int refill;
     int slots;
     int sample_mb;
-    int tri_mode;   /* traversal triangle policy + 1: 1 = every pending triangle then a
-                       node; 2 / 3 = postpone triangle groups when fewer than a fifth of a
+    int tri_mode;   /* traversal triangle policy + 1: 1 (default) = the warp visits a node or
+                       tests one pending triangle per lane, whichever keeps more lanes
+                       busy; 2 / 3 = postpone triangle groups when fewer than a fifth of a
                        warp's active lanes have any, else test one (2) / all (3);
                        4 = the warp tests all lanes' pending triangles together
                        (32 at a time), then every lane visits one node */
