@@ -29,10 +29,6 @@ import numpy as np
 ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
-# DRAM bytes (read + write) k_extend moves per closest-hit ray on the 1M-triangle
-# workload with the default slot pool, from an ncu capture of a whole 16-spp
-# frame with a warm L2 (profiles/k_extend_dram_traffic_icospheres1m_16spp.txt).
-K_EXTEND_DRAM_BYTES_PER_RAY = 1246.3
 METRIC = "Mpaths/s"
 
 
@@ -726,24 +722,20 @@ def run_gbpt(args, rank, world):
     ist = ctx.stats()
     node_b, tri_b = 80, 36
     ext_rays = ist["camera_rays"] + ist["extension_rays"]
-    trav_bytes = ist["closest_node_visits"] * node_b + ist["closest_tri_tests"] * tri_b + ext_rays * 48
-    # the light sample k_extend takes at every hit, and a miss's end of path:
-    # per hit the hit triangle's positions and normals (72 B), the light
-    # record (64 B), one draw of three uniforms (12 B), the shadow ray out
-    # (32 B) and its potential contribution (12 B); per miss the throughput
-    # and accumulation in (24 B) and the sample out (12 B)
+    # k_rays: closest hits (32 B ray in, 16 B hit out) and any hits (32 B ray
+    # in, 1 B out) of one iteration
+    visits = ist["closest_node_visits"] + ist["shadow_node_visits"]
+    tests = ist["closest_tri_tests"] + ist["shadow_tri_tests"]
+    ray_bytes = visits * node_b + tests * tri_b + ext_rays * 48 + ist["shadow_rays"] * 33
     hits = ist["light_samples"]
     misses = ext_rays - hits
-    closest_bytes = trav_bytes + hits * (72 + 64 + 12 + 32 + 12) + misses * 36
-    ext_ms = stage_ms[1]          # per frame
-    ext_launches = stage_n[1]
+    ray_ms, ray_launches = stage_ms[1], stage_n[1]  # per frame
     peak, peak_kind = measured_peaks()
-    achieved = closest_bytes / (ext_ms / 1e3) / 1e9 if ext_ms > 0 else None
-    achieved_trav = trav_bytes / (ext_ms / 1e3) / 1e9 if ext_ms > 0 else None
+    achieved = ray_bytes / (ray_ms / 1e3) / 1e9 if ray_ms > 0 else None
     # FP32 work of the traversal: ~24 flops per child slab test (8 children
     # per node visit), ~30 per triangle test
-    trav_flops = ist["closest_node_visits"] * 8 * 24 + ist["closest_tri_tests"] * 30
-    fp32_tflops = trav_flops / (ext_ms / 1e3) / 1e12 if ext_ms > 0 else None
+    trav_flops = visits * 8 * 24 + tests * 30
+    fp32_tflops = trav_flops / (ray_ms / 1e3) / 1e12 if ray_ms > 0 else None
     rays = ist["camera_rays"] + ist["extension_rays"] + ist["shadow_rays"]
     mrays = rays / (total_ms / args.steps / 1e3) / 1e6
 
@@ -761,27 +753,17 @@ def run_gbpt(args, rank, world):
                                   "closest_tri_tests": ist["closest_tri_tests"] / max(1, ext_rays),
                                   "shadow_node_visits": ist["shadow_node_visits"] / max(1, ist["shadow_rays"]),
                                   "shadow_tri_tests": ist["shadow_tri_tests"] / max(1, ist["shadow_rays"])},
-            "stage_ms_per_frame": {"path_start": stage_ms[0], "closest_hit+light_sample": ext_ms,
-                                   "any_hit+restart_of_misses": stage_ms[2], "shade+restart": stage_ms[3],
-                                   "iteration_end": stage_ms[4],
+            "stage_ms_per_frame": {"path_start": stage_ms[0], "closest_hit+any_hit": ray_ms,
+                                   "light_sample+shade+restart": stage_ms[3],
                                    "moving_average": stage_ms[5], "frame_ms_with_stage_events": stage_frame_ms},
             "stage_launches_per_frame": [int(x) for x in stage_n],
-            "roofline": {"bound": "hbm", "kernel": "k_extend (closest-hit traversal + light sample)",
+            "roofline": {"bound": "hbm", "kernel": "k_rays (closest-hit and any-hit traversal)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None,
-                         "traffic": (K_EXTEND_DRAM_BYTES_PER_RAY * ext_rays / max(1.0, ext_launches)
-                                     if args.workload == "icospheres-1m" else None),
-                         "traffic_source": "ncu dram__bytes_read+write of k_extend per closest-hit ray "
-                                           "(warm L2, whole 16-spp frame of this workload) x rays per launch",
-                         "algorithmic_bytes_per_launch": closest_bytes / max(1.0, ext_launches),
-                         "bytes_model": "per ray: node visits*80 + tri tests*36 + 32 ray in + 16 hit out; per hit "
-                                        "(light sample): 72 hit triangle positions+normals + 64 light + 12 draw + "
-                                        "32 shadow ray out + 12 potential contribution; per miss: 24 in + 12 "
-                                        "sample out (counts from the instrumented render of the same frame)",
-                         "traversal_only": {"achieved": achieved_trav,
-                                            "frac": (achieved_trav / peak) if achieved_trav else None,
-                                            "bytes_per_launch": trav_bytes / max(1.0, ext_launches),
-                                            "bytes_model": "node visits*80 + tri tests*36 + 48 per ray"},
+                         "algorithmic_bytes_per_launch": ray_bytes / max(1.0, ray_launches),
+                         "bytes_model": "node visits*80 + tri tests*36 + per closest-hit ray 32 in + 16 out, per "
+                                        "any-hit ray 32 in + 1 out (counts from the instrumented render of the same "
+                                        "frame)",
                          "closest_hits_per_frame": int(hits), "misses_per_frame": int(misses),
                          "fp32": {"achieved_tflops": fp32_tflops,
                                   "model": "node visits*8*24 + tri tests*30 flops (slab tests of 8 children, "

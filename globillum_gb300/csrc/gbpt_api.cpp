@@ -25,7 +25,7 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
-static const int kSnaps = 16;
+static const int kSnaps = 16, kSnapWords = 3;
 static const size_t kMaxGraphs = 16;
 
 // One scene of a frame as the host sees it.
@@ -97,7 +97,7 @@ struct gb_ctx {
     int mode = MODE_FORWARD;            // render mode of the next chunks
     // frozen-sampling replay and adjoint buffers
     std::vector<void*> adj_allocs;
-    size_t tp0_cap = 0, adj_cap = 0, dimg_cap = 0, grad_cap = 0, gsum_cap = 0;
+    size_t tp0_cap = 0, rdiff_cap = 0, adj_cap = 0, dimg_cap = 0, grad_cap = 0, gsum_cap = 0;
     double* d_gsum = nullptr;
     float* d_eval_mats = nullptr;
     LightRec* d_eval_lights = nullptr;
@@ -247,6 +247,22 @@ cudaError_t ensure_scratch(gb_ctx* ctx, int k, size_t bytes) {
     return e;
 }
 
+// A buffer of the context grown on demand.
+cudaError_t ensure_buf(gb_ctx* ctx, void** p, size_t* cap, size_t bytes) {
+    if (bytes <= *cap) return cudaSuccess;
+    cudaStreamSynchronize(ctx->stream);
+    if (*p) {
+        auto it = std::find(ctx->adj_allocs.begin(), ctx->adj_allocs.end(), *p);
+        if (it != ctx->adj_allocs.end()) ctx->adj_allocs.erase(it);
+        cudaFree(*p);
+    }
+    *p = nullptr;
+    *cap = 0;
+    cudaError_t e = dalloc(ctx->adj_allocs, p, bytes);
+    if (e == cudaSuccess) *cap = bytes;
+    return e;
+}
+
 // Per-slot buffers for `nslots` slots, per-pixel buffers for `n` pixels,
 // sample and jitter buffers of `samples` float4 entries and `nscenes` scene
 // records; grown on demand.
@@ -257,17 +273,14 @@ cudaError_t ensure_frame(gb_ctx* ctx, int n, int nslots, size_t samples, int nsc
         cudaStreamSynchronize(ctx->stream);
         free_all(ctx->slot_allocs);
         ctx->slot_cap = 0;
-        unsigned char *recs = nullptr, *shadow = nullptr;
-        if ((e = dalloc(ctx->slot_allocs, (void**)&recs, kSlotBytes * (size_t)nslots)) != cudaSuccess) return e;
-        if (GB_SHADOW_SPLIT && (e = dalloc(ctx->slot_allocs, (void**)&shadow, 32 * (size_t)nslots)) != cudaSuccess)
-            return e;
-        bind_slots(F, recs, shadow);
-        for (int k = 0; k < 4; ++k)
-            if ((e = dalloc(ctx->slot_allocs, (void**)&F.q[k], 4 * (size_t)nslots)) != cudaSuccess) return e;
+        const size_t cap = ((size_t)nslots + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
+        unsigned char* slots = nullptr;
+        if ((e = dalloc(ctx->slot_allocs, (void**)&slots, kSlotBytes * cap)) != cudaSuccess) return e;
+        bind_slots(F, slots, cap);
         if ((e = dalloc(ctx->slot_allocs, (void**)&F.ctr, 4 * 32)) != cudaSuccess) return e;
         if ((e = dalloc(ctx->slot_allocs, (void**)&F.path_ctr, 4 * 8)) != cudaSuccess) return e;
         if ((e = dalloc(ctx->slot_allocs, (void**)&F.iter, 4 * 8)) != cudaSuccess) return e;
-        ctx->slot_cap = (size_t)nslots;
+        ctx->slot_cap = cap;
     }
     if ((size_t)n > ctx->pixel_cap) {
         cudaStreamSynchronize(ctx->stream);
@@ -374,7 +387,7 @@ int gb_ctx_create(const gb_ctx_desc* desc, gb_ctx** out) {
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_stats, sizeof(unsigned long long) * 16);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_stats, 0, sizeof(unsigned long long) * 16);
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->snap_host, sizeof(uint32_t) * kSnaps, cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->snap_host, sizeof(uint32_t) * kSnaps * kSnapWords, cudaHostAllocDefault);
     for (int k = 0; k < kSnaps && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ctx->snap_ev[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -832,6 +845,11 @@ int begin_frame(gb_ctx* ctx, std::vector<BatchScene>& items) {
     const long long samples = std::min(total_paths, std::max(ntot, sample_budget(ctx)));
     const int nslots = (int)std::max(1ll, std::min<long long>(total_paths, ctx->slots));
     CK(ensure_frame(ctx, (int)ntot, nslots, (size_t)samples, (int)items.size()));
+    for (const BatchScene& b : items)
+        if (b.scene->S.texcoord) {
+            CK(ensure_buf(ctx, (void**)&ctx->F.rdiff, &ctx->rdiff_cap, 3 * sizeof(float4) * ctx->slot_cap));
+            break;
+        }
     ctx->recs.assign(items.size(), SceneRec{});
     uint32_t base = 0;
     for (size_t i = 0; i < items.size(); ++i) {
@@ -875,9 +893,9 @@ int begin_frame(gb_ctx* ctx, std::vector<BatchScene>& items) {
 }
 
 // Slot-pool loop of one chunk driven by the host: every iteration launches
-// extend, shadow, shade, regen and step; the host reads the next queue count
+// rays and shade (and adjoint and regen in adjoint mode); the host reads the next queue count
 // through snapshots and stays at most kLead iterations ahead of the GPU.
-int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters) {
+int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart) {
     const Frame& F = ctx->F;
     CK(cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, ctx->stream));
     CK(stage_mark(ctx, 0, true));
@@ -890,25 +908,24 @@ int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters
     int head = 0, tail = 0;  // pending snapshots [tail, head)
     bool done = false;
     for (int it = 0; !done; ++it) {
-        if (it >= max_iters) return fail(ctx, GB_ERR_TRAVERSAL, "path iteration bound exceeded");
+        if (it > P.max_iters + kLead) return fail(ctx, GB_ERR_TRAVERSAL, "path iteration bound exceeded");
         CK(stage_mark(ctx, 1, true));
-        CK(k_launch_extend(F, P, ctx->instrument, ctx->stream));
+        CK(k_launch_rays(F, P, ctx->instrument, 0, false, ctx->stream));
         CK(stage_mark(ctx, 1, false));
-        CK(stage_mark(ctx, 2, true));
-        CK(k_launch_shadow(F, P, ctx->instrument, ctx->stream));
-        CK(stage_mark(ctx, 2, false));
         CK(stage_mark(ctx, 3, true));
         CK(k_launch_shade(F, P, ctx->stream));
         CK(stage_mark(ctx, 3, false));
-        CK(stage_mark(ctx, 4, true));
-        if (P.mode == MODE_ADJOINT) CK(k_launch_adjoint(F, P, ctx->stream));
-        CK(k_launch_regen(F, P, ctx->stream));
-        CK(k_launch_step(F, P, 0, false, max_iters, ctx->stream));
-        CK(stage_mark(ctx, 4, false));
+        if (P.mode == MODE_ADJOINT) {
+            CK(stage_mark(ctx, 4, true));
+            CK(k_launch_adjoint(F, P, ctx->stream));
+            CK(k_launch_regen(F, P, ctx->stream));
+            CK(stage_mark(ctx, 4, false));
+        }
         if (it % kEvery == kEvery - 1) {
             int k = head % kSnaps;
-            CK(cudaMemcpyAsync(ctx->snap_host + k, F.ctr + 8 * ((it + 1) % 3), sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, ctx->stream));
+            // extension, shadow and pending ended counts of the next iteration
+            CK(cudaMemcpyAsync(ctx->snap_host + kSnapWords * k, F.ctr + 8 * ((it + 1) % 3),
+                               kSnapWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaEventRecord(ctx->snap_ev[k], ctx->stream));
             snap_it[k] = it;
             ++head;
@@ -922,7 +939,8 @@ int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters
                 if (q == cudaErrorNotReady) break;
                 if (q != cudaSuccess) return cuda_fail(ctx, q, "snapshot event");
             }
-            if (ctx->snap_host[k] == 0u) done = true;
+            const uint32_t* c = ctx->snap_host + kSnapWords * k;
+            if ((c[CTR_EXT] | c[CTR_SHADOW] | c[CTR_ENDED]) == 0u) done = true;
             ++tail;
         }
     }
@@ -935,16 +953,17 @@ int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters
 
 // Everything a captured chunk graph depends on: the frame's buffers and
 // sizes, the chunk parameters and the kernel variants.
-std::vector<uint64_t> graph_key(const gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters) {
+std::vector<uint64_t> graph_key(const gb_ctx* ctx, const RenderParams& P, int nstart) {
     const Frame& F = ctx->F;
     std::vector<uint64_t> k;
     k.push_back(((uint64_t)(uint32_t)F.ntot << 32) | (uint32_t)F.nslots);
     k.push_back(((uint64_t)(uint32_t)F.nscenes << 32) | (uint32_t)nstart);
-    k.push_back(((uint64_t)(uint32_t)max_iters << 32) | (ctx->instrument ? 1u : 0u));
-    const void* ptrs[] = {F.scenes, F.slots, F.shadow, F.q[0], F.q[1], F.q[2], F.q[3], F.out,
+    k.push_back(ctx->instrument ? 1u : 0u);
+    const void* ptrs[] = {F.scenes, F.ray, F.rdiff, F.out,
                           F.pristine, F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr,
                           F.iter, F.stats, F.status, F.tp0, F.adj, F.dimg, F.grad};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
+    k.push_back((uint64_t)ctx->slot_cap);
     k.push_back(((uint64_t)(uint32_t)F.grad_stride << 32) | (uint32_t)F.grad_replicas);
     static_assert(sizeof(RenderParams) % 4 == 0, "RenderParams is made of 32-bit words");
     uint32_t w[sizeof(RenderParams) / 4];
@@ -954,10 +973,10 @@ std::vector<uint64_t> graph_key(const gb_ctx* ctx, const RenderParams& P, int ns
 }
 
 // One chunk as a CUDA graph: counter reset, jitter pool and first paths,
-// then a conditional WHILE node whose body (extend, shadow, shade, regen,
-// step) repeats until k_step finds the next extension queue empty, then the
-// moving average.  Captured on the context's second stream.
-int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters, cudaGraphExec_t* out) {
+// then a conditional WHILE node whose body (rays, shade; adjoint and regen in
+// adjoint mode) repeats until k_rays finds its queues empty, then the moving
+// average.  Captured on the context's second stream.
+int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, cudaGraphExec_t* out) {
     const Frame& F = ctx->F;
     cudaStream_t a = ctx->aux;
     cudaGraph_t g = nullptr;
@@ -990,12 +1009,10 @@ int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, int max_it
         cudaGraph_t body = np.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(a, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
         if (e == cudaSuccess) {
-            e = k_launch_extend(F, P, ctx->instrument, a);
-            if (e == cudaSuccess) e = k_launch_shadow(F, P, ctx->instrument, a);
+            e = k_launch_rays(F, P, ctx->instrument, (unsigned long long)h, true, a);
             if (e == cudaSuccess) e = k_launch_shade(F, P, a);
             if (e == cudaSuccess && P.mode == MODE_ADJOINT) e = k_launch_adjoint(F, P, a);
             if (e == cudaSuccess) e = k_launch_regen(F, P, a);
-            if (e == cudaSuccess) e = k_launch_step(F, P, (unsigned long long)h, true, max_iters, a);
             cudaGraph_t body_out = nullptr;
             e2 = cudaStreamEndCapture(a, &body_out);
             if (e == cudaSuccess) e = e2;
@@ -1009,7 +1026,7 @@ int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, int max_it
 
 // The same chunk appended to the capture in progress on stream `a`; the
 // loop body is captured on stream `b` while `a` keeps capturing.
-int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters, cudaStream_t a, cudaStream_t b) {
+int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, cudaStream_t a, cudaStream_t b) {
     const Frame& F = ctx->F;
     cudaError_t e = cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, a);
     if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, a);
@@ -1035,12 +1052,10 @@ int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters, 
         e = cudaStreamBeginCaptureToGraph(b, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                           cudaStreamCaptureModeRelaxed);
         if (e == cudaSuccess) {
-            e = k_launch_extend(F, P, ctx->instrument, b);
-            if (e == cudaSuccess) e = k_launch_shadow(F, P, ctx->instrument, b);
+            e = k_launch_rays(F, P, ctx->instrument, (unsigned long long)h, true, b);
             if (e == cudaSuccess) e = k_launch_shade(F, P, b);
             if (e == cudaSuccess && P.mode == MODE_ADJOINT) e = k_launch_adjoint(F, P, b);
             if (e == cudaSuccess) e = k_launch_regen(F, P, b);
-            if (e == cudaSuccess) e = k_launch_step(F, P, (unsigned long long)h, true, max_iters, b);
             cudaGraph_t body_out = nullptr;
             cudaError_t e2 = cudaStreamEndCapture(b, &body_out);
             if (e == cudaSuccess) e = e2;
@@ -1051,14 +1066,14 @@ int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters, 
     return GB_OK;
 }
 
-int run_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iters) {
-    std::vector<uint64_t> key = graph_key(ctx, P, nstart, max_iters);
+int run_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart) {
+    std::vector<uint64_t> key = graph_key(ctx, P, nstart);
     size_t hit = ctx->graphs.size();
     for (size_t i = 0; i < ctx->graphs.size(); ++i)
         if (ctx->graphs[i].key == key) { hit = i; break; }
     if (hit == ctx->graphs.size()) {
         cudaGraphExec_t ex = nullptr;
-        int rc = build_chunk_graph(ctx, P, nstart, max_iters, &ex);
+        int rc = build_chunk_graph(ctx, P, nstart, &ex);
         if (rc != GB_OK) return rc;
         if (ctx->graphs.size() >= kMaxGraphs) {
             cudaGraphExecDestroy(ctx->graphs.front().exec);
@@ -1074,7 +1089,7 @@ int run_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, int max_iter
 
 // Launch parameters of the chunk of rounds [p0, p1): sets the frame's slot
 // count and returns the paths started first and the iteration bound.
-void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out, int* max_iters_out) {
+void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out) {
     RenderParams P{};
     P.refill = ctx->refill;
     P.tri_mode = ctx->tri_mode;
@@ -1131,24 +1146,25 @@ void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out,
     if (ctx->mode == MODE_ADJOINT) F.nslots = std::min(F.nslots, kAdjMaxSlots);
     const int nstart = (int)std::min<long long>(F.nslots, acc);
     // Every iteration moves each busy slot's path one bounce (at most L + 1
-    // per path), and all slots stay busy until the chunk's last path has
-    // started, so the loop ends within acc (L + 1) / nslots + L + 1
-    // iterations; twice that (plus slack) bounds it.
+    // per path, the last of them for a light sample still pending), and all
+    // slots stay busy until the chunk's last path has started, so the loop
+    // ends within acc (L + 1) / nslots + L + 1 iterations; twice that (plus
+    // slack) bounds it.
     const long long L1 = ctx->max_L + 1;
     const int max_iters =
         (int)std::min<long long>(1ll << 30, 2 * ((acc * L1 + F.nslots - 1) / F.nslots + L1) + 16);
+    P.max_iters = max_iters;
     *out = P;
     *nstart_out = nstart;
-    *max_iters_out = max_iters;
 }
 
 // Rounds [p0, p1) of every pixel that takes them, through the slot pool.
 int run_chunk(gb_ctx* ctx, int p0, int p1) {
     RenderParams P{};
-    int nstart = 0, max_iters = 0;
-    make_chunk(ctx, p0, p1, &P, &nstart, &max_iters);
-    if (ctx->use_graph && !ctx->stage_timing) return run_chunk_graph(ctx, P, nstart, max_iters);
-    return run_chunk_loop(ctx, P, nstart, max_iters);
+    int nstart = 0;
+    make_chunk(ctx, p0, p1, &P, &nstart);
+    if (ctx->use_graph && !ctx->stage_timing) return run_chunk_graph(ctx, P, nstart);
+    return run_chunk_loop(ctx, P, nstart);
 }
 
 int step_frame(gb_ctx* ctx, int paths) {
@@ -1212,8 +1228,8 @@ int finish_frame(gb_ctx* ctx) {
     ctx->stats.shadow_node_visits = st[5];
     ctx->stats.shadow_tri_tests = st[6];
     ctx->stats.light_samples = st[8];
-    // every slot-pool iteration (counted by k_step in st[7]) is 4 launches
-    // (extend, shadow, shade, step), 6 with the adjoint sweep
+    // every slot-pool iteration (counted by k_rays in st[7]) is 2 launches
+    // (rays, shade), 4 with the adjoint sweep
     ctx->stats.kernel_launches = ctx->launches + (uint64_t)k_launches_per_iteration(ctx->mode) * st[7];
     ctx->stats.paths_done = ctx->paths_done;
     for (int k = 0; k < 6; ++k) { ctx->stats.stage_ms[k] = 0.0; ctx->stats.stage_launches[k] = 0; }
@@ -1353,21 +1369,6 @@ bool all_finite(const float* x, int n) {
     for (int i = 0; i < n; ++i)
         if (!std::isfinite(x[i])) return false;
     return true;
-}
-
-cudaError_t ensure_buf(gb_ctx* ctx, void** p, size_t* cap, size_t bytes) {
-    if (bytes <= *cap) return cudaSuccess;
-    cudaStreamSynchronize(ctx->stream);
-    if (*p) {
-        auto it = std::find(ctx->adj_allocs.begin(), ctx->adj_allocs.end(), *p);
-        if (it != ctx->adj_allocs.end()) ctx->adj_allocs.erase(it);
-        cudaFree(*p);
-    }
-    *p = nullptr;
-    *cap = 0;
-    cudaError_t e = dalloc(ctx->adj_allocs, p, bytes);
-    if (e == cudaSuccess) *cap = bytes;
-    return e;
 }
 
 }  // namespace
@@ -1575,7 +1576,7 @@ namespace {
 std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     const Frame& F = ctx->F;
     std::vector<uint64_t> k;
-    const void* ptrs[] = {ctx->d_scenes, F.slots, F.shadow, F.q[0], F.q[1], F.q[2], F.q[3], F.out, F.pristine,
+    const void* ptrs[] = {ctx->d_scenes, F.ray, F.out, F.pristine,
                           F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr, F.iter, F.stats,
                           F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->d_rgb, ctx->fit.d_loss};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
@@ -1696,9 +1697,9 @@ int fit_build(gb_ctx* ctx) {
             long long cp = 0;
             const int p1 = chunk_end(ctx, p0, ctx->max_spp, &cp);
             RenderParams P{};
-            int nstart = 0, max_iters = 0;
-            make_chunk(ctx, p0, p1, &P, &nstart, &max_iters);
-            rc = append_chunk(ctx, P, nstart, max_iters, a, b);
+            int nstart = 0;
+            make_chunk(ctx, p0, p1, &P, &nstart);
+            rc = append_chunk(ctx, P, nstart, a, b);
             p0 = p1;
         }
         if (rc != GB_OK) break;

@@ -4,19 +4,22 @@
 // paths of a chunk (samples p0..p1-1 of every pixel) are handed out to the
 // slots in path order; a slot whose path ends stores the path's sample and
 // takes the next path, so every iteration works on a full queue until the
-// chunk runs dry.  One iteration:
-//   k_extend  closest-hit traversal of the extension queue; misses add
-//             handle_no_hit's contribution (hybrid-pt.cpp:196-206) and end
-//             the path; hits draw the bounce's uniforms and emit the
-//             area-light shadow ray (arealight-sampler-cpu.cpp:25-143)
-//   k_shadow  any-hit traversal of the shadow queue
-//   k_shade   BRDF sample/eval, NEE accumulation, throughput and next ray of
-//             compute_path_contribution_and_bounce (hybrid-pt.cpp:450-584)
+// chunk runs dry.  One iteration is two launches:
+//   k_rays   traces the extension rays (closest hit) and the shadow rays of
+//            the previous vertices (any hit) in one persistent grid
+//   k_shade  adds the previous vertex's light sample if its shadow ray was
+//            free; a miss adds handle_no_hit's contribution
+//            (hybrid-pt.cpp:196-206) and ends the path; a hit draws the
+//            bounce's uniforms, takes the area-light sample
+//            (arealight-sampler-cpu.cpp:25-143), the BRDF sample and eval,
+//            throughput and next ray of
+//            compute_path_contribution_and_bounce (hybrid-pt.cpp:450-584)
 // then k_combine folds the chunk's samples into the image with new_path's
 // moving average (util-kernels.cu:17-25), in path order per pixel, so the
 // image equals the reference's pixel-sequential one bit for bit.
-// Queues are compacted with one warp ballot + one atomic per warp; traversal
-// kernels run persistent warps that refill idle lanes from the queue.
+// Tracing both ray kinds together halves the launches that end in a tail of
+// a few long rays, and a traced ray leaves only its hit behind, so the
+// traversal kernel carries no shading code (registers, refill cost).
 //
 // Traversal: compressed 8-wide BVH (80 B nodes, 8-bit quantised child
 // boxes), node-group stack of 32 entries, octant-ordered child visits,
@@ -44,31 +47,18 @@ constexpr int kStack = 32;
 constexpr int kIterLimit = 1 << 22;
 // Experimental build options, each off by default (measured in the design
 // notes): traversal stack entries kept in shared memory, L2 prefetch of hit
-// child nodes, light samples in a kernel of their own, register budgets and
-// grid of the streaming kernels.
+// child nodes, register budgets.
 #ifndef GB_SMEM_STACK
 #define GB_SMEM_STACK 0
 #endif
 #ifndef GB_PREFETCH
 #define GB_PREFETCH 0
 #endif
-#ifndef GB_SPLIT_NEE
-#define GB_SPLIT_NEE 0
-#endif
 #ifndef GB_SHADE_MIN_BLOCKS
 #define GB_SHADE_MIN_BLOCKS 5  // resident k_shade blocks per SM (register budget 102)
 #endif
-#ifndef GB_STREAM_MIN_BLOCKS
-#define GB_STREAM_MIN_BLOCKS 1
-#endif
 #ifndef GB_NODE_FOLD
 #define GB_NODE_FOLD 0  // 1: plane bias folded into the per-node origin term
-#endif
-#ifndef GB_FUSED_RESTART
-#define GB_FUSED_RESTART 1  // paths ended by a miss restart in k_shadow's warps
-#endif
-#ifndef GB_WIDE_STREAM_GRIDS
-#define GB_WIDE_STREAM_GRIDS 0
 #endif
 constexpr int kSmemStack = GB_SMEM_STACK;
 
@@ -115,12 +105,6 @@ __device__ __forceinline__ RayInv make_ray(v3 o, v3 d) {
 // Read-only 16-byte loads of the tree with cache hints: triangles without L1
 // allocation (GB_TRI_NOALLOC), nodes with a 128-byte L2 fetch (GB_NODE_L2_128);
 // plain __ldg otherwise.
-#ifndef GB_SHADOW_MIN_BLOCKS
-#define GB_SHADOW_MIN_BLOCKS 8  // resident any-hit blocks per SM (register budget)
-#endif
-#ifndef GB_SHADOW_REFILL
-#define GB_SHADOW_REFILL 12  // refill threshold of the any-hit kernel (0: the frame's refill)
-#endif
 #ifndef GB_TRI_NOALLOC
 #define GB_TRI_NOALLOC 0
 #endif
@@ -133,20 +117,6 @@ __device__ __forceinline__ float4 ld_tri(const float4* p) {
     asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(__cvta_generic_to_global(p)));
     return v;
-#else
-    return __ldg(p);
-#endif
-}
-// The hit triangle's shading record (positions and normals for the hit
-// point), read once per hit with little reuse across a frame: with
-// GB_SHADE_EVICT_FIRST the load is marked evict-first (ld.global.cs), so
-// that the 98 MB array streaming past does not push the tree out of L2.
-#ifndef GB_SHADE_EVICT_FIRST
-#define GB_SHADE_EVICT_FIRST 0
-#endif
-__device__ __forceinline__ float4 ld_shade(const float4* p) {
-#if GB_SHADE_EVICT_FIRST
-    return __ldcs(p);
 #else
     return __ldg(p);
 #endif
@@ -316,12 +286,15 @@ struct Trav {
     uint32_t best_id;
 };
 
-__device__ __forceinline__ void trav_init(Trav& s, const RayInv& r) {
+// best_t starts at t_max (at most FLT_MAX, so that an infinite distance is
+// never a hit): a hit at t_max exactly is taken, as closer() prefers any id to
+// none, and one test serves both limits.
+__device__ __forceinline__ void trav_init(Trav& s, const RayInv& r, float tmax) {
     s.ng = make_uint2(0u, 0x80000000u | (1u << (r.oxor ^ 7u)));
     s.tg = make_uint2(0u, 0u);
     s.nt = make_uint2(0u, 0u);
     s.sp = 0;
-    s.best_t = FLT_MAX;
+    s.best_t = fminf(tmax, FLT_MAX);
     s.best_id = 0xffffffffu;
     s.bb = 0.0f;
     s.bg = 0.0f;
@@ -332,8 +305,8 @@ __device__ __forceinline__ void trav_init(Trav& s, const RayInv& r) {
 //
 // tri_step: one triangle of the current triangle group.  Returns true when
 // an any-hit query has found its hit.
-template <bool ANY, bool INSTR>
-__device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const RayInv& r, float tmax, Trav& s,
+template <bool INSTR>
+__device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const RayInv& r, bool any, Trav& s,
                                          uint32_t* ntri) {
     int b = __ffs(s.tg.y) - 1;
     s.tg.y &= s.tg.y - 1u;
@@ -341,10 +314,12 @@ __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const 
     float4 a0 = ld_tri(tp + 0), a1 = ld_tri(tp + 1), a2 = ld_tri(tp + 2);
     if (INSTR) ++*ntri;
     float t, u, v;
-    if (intersect_tri(r.o, r.d, ld3(a0), ld3(a1), ld3(a2), &t, &u, &v) && t <= tmax) {
+    if (intersect_tri(r.o, r.d, ld3(a0), ld3(a1), ld3(a2), &t, &u, &v)) {
         uint32_t id = __float_as_uint(a0.w);
-        if (ANY) { s.best_t = t; s.best_id = id; return true; }
-        if (closer(t, id, s.best_t, s.best_id)) { s.best_t = t; s.best_id = id; s.bb = u; s.bg = v; }
+        if (closer(t, id, s.best_t, s.best_id)) {
+            s.best_t = t; s.best_id = id; s.bb = u; s.bg = v;
+            return any;
+        }
     }
     return false;
 }
@@ -352,7 +327,7 @@ __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const 
 // visit_node: the next node of the current node group (not empty).  Returns
 // true when the stack overflows.
 template <bool INSTR, int STACK = kStack>
-__device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, const RayInv& r, float tmax, Trav& s,
+__device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
                                            const StackRef& stack, uint32_t* status, uint32_t* nvis, uint2* tg) {
     const uint32_t k = 31u - (uint32_t)__clz(s.ng.y);
     s.ng.y &= ~(1u << k);
@@ -364,7 +339,7 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
         stack_put(stack, s.sp++, s.ng);
     }
     if (INSTR) ++*nvis;
-    intersect_node(nodes, child, r, fminf(s.best_t, tmax), &s.ng, tg);
+    intersect_node(nodes, child, r, s.best_t, &s.ng, tg);
     return false;
 }
 
@@ -372,10 +347,10 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
 // group, or a stack pop.  Returns true when the ray is finished; the result
 // is the (t, id)-minimum in s (any-hit: best_id != none when found).
 template <bool INSTR, int STACK = kStack>
-__device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, float tmax, Trav& s,
-                                          const StackRef& stack, uint32_t* status, uint32_t* nvis) {
+__device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, Trav& s, const StackRef& stack,
+                                          uint32_t* status, uint32_t* nvis) {
     if (s.ng.y > 0x00ffffffu)
-        return visit_node<INSTR, STACK>(nodes, r, tmax, s, stack, status, nvis, &s.tg);
+        return visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &s.tg);
     if (s.sp > 0) {
         uint2 g = stack_get(stack, --s.sp);
         if (g.y > 0x00ffffffu) s.ng = g;
@@ -401,9 +376,9 @@ __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, cons
 #ifndef GB_TRI_RATIO
 #define GB_TRI_RATIO 2
 #endif
-template <bool ANY, bool INSTR, int STACK>
+template <bool INSTR, int STACK>
 __device__ __forceinline__ bool warp_step(bool act, const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                          const RayInv& r, float tmax, Trav& s, const StackRef& stack,
+                                          const RayInv& r, bool any, Trav& s, const StackRef& stack,
                                           uint32_t* status, uint32_t* nvis, uint32_t* ntri) {
     const bool tri = act && s.tg.y != 0u;
     const bool node = act && s.nt.y == 0u && (s.ng.y > 0x00ffffffu || s.sp > 0);
@@ -411,7 +386,7 @@ __device__ __forceinline__ bool warp_step(bool act, const float4* __restrict__ n
     bool done = false;
     if (lt * GB_TRI_RATIO >= ln) {
         if (tri) {
-            done = tri_step<ANY, INSTR>(tris, r, tmax, s, ntri);
+            done = tri_step<INSTR>(tris, r, any, s, ntri);
             if (s.tg.y == 0u) {
                 s.tg = s.nt;
                 s.nt.y = 0u;
@@ -420,7 +395,7 @@ __device__ __forceinline__ bool warp_step(bool act, const float4* __restrict__ n
     } else if (node) {
         if (s.ng.y <= 0x00ffffffu) s.ng = stack_get(stack, --s.sp);
         uint2 tg = make_uint2(0u, 0u);
-        done = visit_node<INSTR, STACK>(nodes, r, tmax, s, stack, status, nvis, &tg);
+        done = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg);
         if (s.tg.y == 0u) s.tg = tg;
         else s.nt = tg;
     }
@@ -428,13 +403,13 @@ __device__ __forceinline__ bool warp_step(bool act, const float4* __restrict__ n
 }
 
 // Whole traversal of one ray without warp cooperation.
-template <bool ANY, bool INSTR, int STACK = kStack>
+template <bool ANY>
 __device__ __forceinline__ bool trav_step(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                          const RayInv& r, float tmax, Trav& s, const StackRef& stack, uint32_t* status,
-                                          uint32_t* nvis, uint32_t* ntri) {
+                                          const RayInv& r, Trav& s, const StackRef& stack, uint32_t* status) {
+    uint32_t nvis = 0, ntri = 0;
     while (s.tg.y != 0u)
-        if (tri_step<ANY, INSTR>(tris, r, tmax, s, ntri)) return true;
-    return node_step<INSTR, STACK>(nodes, r, tmax, s, stack, status, nvis);
+        if (tri_step<false>(tris, r, ANY, s, &ntri)) return true;
+    return node_step<false>(nodes, r, s, stack, status, &nvis);
 }
 
 struct TraceOut {
@@ -447,52 +422,22 @@ template <bool ANY>
 __device__ __forceinline__ bool traverse(const DevScene& S, const RayInv& r, float tmax, TraceOut* out,
                                          uint32_t* status) {
     Trav s;
-    trav_init(s, r);
+    trav_init(s, r, tmax);
     uint2 lstack[kStack];
     const StackRef stack{lstack, lstack + kSmemStack, 1};
-    uint32_t nv = 0, nt = 0;
     int iters = 0;
-    while (!trav_step<ANY, false>(S.nodes, S.tris, r, tmax, s, stack, status, &nv, &nt)) {
+    while (!trav_step<ANY>(S.nodes, S.tris, r, s, stack, status)) {
         if (++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); break; }
     }
-    if (out) { out->t = s.best_t; out->beta = s.bb; out->gamma = s.bg; out->id = s.best_id; }
+    if (out) { out->t = s.best_id != 0xffffffffu ? s.best_t : FLT_MAX; out->beta = s.bb; out->gamma = s.bg; out->id = s.best_id; }
     return s.best_id != 0xffffffffu;
 }
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
-// Warp-aggregated append of `id` (when pred) to queue q with counter c.
-__device__ __forceinline__ void push(bool pred, uint32_t id, uint32_t* q, uint32_t* c) {
-    uint32_t mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0u) return;
-    uint32_t leader = (uint32_t)__ffs(mask) - 1u;
-    uint32_t base = 0u;
-    if (lane_id() == leader) base = atomicAdd(c, (uint32_t)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, (int)leader);
-    if (pred) q[base + (uint32_t)__popc(mask & ((1u << lane_id()) - 1u))] = id;
-}
-
-// Warp-aggregated counter increment: the lane's index among the warp's
-// increments, counted from the counter's value (0 where pred is false).
-__device__ __forceinline__ uint32_t warp_inc(bool pred, uint32_t* c) {
-    uint32_t mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0u) return 0u;
-    uint32_t leader = (uint32_t)__ffs(mask) - 1u;
-    uint32_t base = 0u;
-    if (lane_id() == leader) base = atomicAdd(c, (uint32_t)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, (int)leader);
-    return base + (uint32_t)__popc(mask & ((1u << lane_id()) - 1u));
-}
-
 __device__ __forceinline__ void add_stats(unsigned long long* s, uint32_t v) {
     uint32_t w = __reduce_add_sync(0xffffffffu, v);
     if (lane_id() == 0u && w) atomicAdd(s, (unsigned long long)w);
-}
-
-// One count from a (possibly divergent) lane.
-__device__ __forceinline__ void add_stats_lane(unsigned long long* s) {
-    uint32_t m = __activemask();
-    if (lane_id() == (uint32_t)__ffs(m) - 1u) atomicAdd(s, (unsigned long long)__popc(m));
 }
 
 // ----------------------------------------------------------------- kernels
@@ -553,21 +498,6 @@ __device__ __forceinline__ void st_mrg(MrgState* base, size_t i, const MrgState&
     rec_st(q, make_uint2(m.s1[0], m.s1[1]));
     rec_st(q + 1, make_uint2(m.s1[2], m.s2[0]));
     rec_st(q + 2, make_uint2(m.s2[1], m.s2[2]));
-}
-// the same for the stream of a slot record, stored as its whole 32-byte
-// sector (the state and 8 zero bytes)
-__device__ __forceinline__ MrgState ld_mrg(const SlotField<MrgState>& f, size_t slot) { return ld_mrg(&f[slot], 0); }
-__device__ __forceinline__ void st_mrg(const SlotField<MrgState>& f, size_t slot, const MrgState& m,
-                                       bool hit_line = false) {
-    uint4* q = reinterpret_cast<uint4*>(&f[slot]);
-    const uint4 a = make_uint4(m.s1[0], m.s1[1], m.s1[2], m.s2[0]), b = make_uint4(m.s2[1], m.s2[2], 0u, 0u);
-    if (GB_HIT_LINE_KEEP && hit_line) {
-        q[0] = a;
-        q[1] = b;
-    } else {
-        rec_st(q, a);
-        rec_st(q + 1, b);
-    }
 }
 __device__ __forceinline__ v3 draw3(MrgState* m) {
     curandStateMRG32k3a st = mrg_expand(*m);
@@ -675,7 +605,8 @@ __global__ void k_jitter_pool(Frame F, RenderParams P) {
 
 // Ray differentials of a slot, 12 floats in 3 planes of nslots float4.
 __device__ __forceinline__ RayDiff ld_rdiff(const Frame& F, uint32_t slot) {
-    const float4 a = F.rdiff[0][slot], b = F.rdiff[1][slot], c = F.rdiff[2][slot];
+    const size_t n = (size_t)F.nslots;
+    const float4 a = F.rdiff[slot], b = F.rdiff[n + slot], c = F.rdiff[2 * n + slot];
     RayDiff r;
     r.uo = mk(a.x, a.y, a.z);
     r.ud = mk(a.w, b.x, b.y);
@@ -684,9 +615,24 @@ __device__ __forceinline__ RayDiff ld_rdiff(const Frame& F, uint32_t slot) {
     return r;
 }
 __device__ __forceinline__ void st_rdiff(const Frame& F, uint32_t slot, const RayDiff& r) {
-    F.rdiff[0][slot] = make_float4(r.uo.x, r.uo.y, r.uo.z, r.ud.x);
-    F.rdiff[1][slot] = make_float4(r.ud.y, r.ud.z, r.ro.x, r.ro.y);
-    F.rdiff[2][slot] = make_float4(r.ro.z, r.rd.x, r.rd.y, r.rd.z);
+    const size_t n = (size_t)F.nslots;
+    F.rdiff[slot] = make_float4(r.uo.x, r.uo.y, r.uo.z, r.ud.x);
+    F.rdiff[n + slot] = make_float4(r.ud.y, r.ud.z, r.ro.x, r.ro.y);
+    F.rdiff[2 * n + slot] = make_float4(r.ro.z, r.rd.x, r.rd.y, r.rd.z);
+}
+
+__device__ __forceinline__ Sector pack_sector(v3 a, v3 b, uint32_t c, uint32_t d) {
+    return Sector{{__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(b.x),
+                   __float_as_uint(b.y), __float_as_uint(b.z), c, d}};
+}
+__device__ __forceinline__ v3 sec3(const Sector& s, int k) {
+    return mk(__uint_as_float(s.w[k]), __uint_as_float(s.w[k + 1]), __uint_as_float(s.w[k + 2]));
+}
+// The `path` and `strm` sectors of a slot: throughput, accumulation, stream
+// and pending light sample.
+__device__ __forceinline__ void st_path(const Frame& F, uint32_t slot, v3 tp, v3 acc, const MrgState& m, v3 pend) {
+    rec_st(&F.path[slot], pack_sector(tp, acc, __float_as_uint(pend.x), __float_as_uint(pend.y)));
+    rec_st(&F.strm[slot], Sector{{m.s1[0], m.s1[1], m.s1[2], m.s2[0], m.s2[1], m.s2[2], __float_as_uint(pend.z), 0u}});
 }
 
 __device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t l) {
@@ -708,140 +654,68 @@ __device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P
         lx = lj.z - 0.5f;
         ly = lj.y - 0.5f;
     }
-    st_mrg(F.rng, slot, ld_mrg(F.spool, l));
+    const int x = (int)(lp % (uint32_t)R.w), y = (int)(lp / (uint32_t)R.w);
     v3 o, d;
-    camera_ray(R.cam, (int)(lp % (uint32_t)R.w), (int)(lp / (uint32_t)R.w), j.x, j.y, lx, ly, &o, &d);
-    F.ray_o.st(slot, make_float4(o.x, o.y, o.z, FLT_MAX));
-    F.ray_d.st(slot, make_float4(d.x, d.y, d.z, __uint_as_float(((uint32_t)P.p0 + (uint32_t)lo) << 10)));  // w: pb
-    F.tp.st(slot, make_float4(1.0f, 1.0f, 1.0f, 0.0f));
+    camera_ray(R.cam, x, y, j.x, j.y, lx, ly, &o, &d);
+    rec_st(&F.ray[slot], pack_sector(o, d, ((uint32_t)P.p0 + (uint32_t)lo) << 10, gpix));
+    st_path(F, slot, mk(1.0f, 1.0f, 1.0f), mk(0.0f, 0.0f, 0.0f), ld_mrg(F.spool, l), mk(0.0f, 0.0f, 0.0f));
     if (P.mode == MODE_FROZEN) F.tp0[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    F.accum.st(slot, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    F.pixw.st(slot, make_uint4(gpix, sc, 0u, 0u));
-    if (R.S.texcoord) st_rdiff(F, slot, camera_diff(R.cam, (int)(lp % (uint32_t)R.w), (int)(lp / (uint32_t)R.w)));
-    else F.rdiff[0][slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // completes the sector of pix / ps
+    if (P.textured && R.S.texcoord) st_rdiff(F, slot, camera_diff(R.cam, x, y));
 }
 
-// The scene record of a slot's path; a frame of one scene needs no load of
-// the slot's scene word.
-__device__ __forceinline__ const SceneRec& scene_of(const Frame& F, uint32_t slot) {
-    return F.scenes[F.nscenes == 1 ? 0u : F.ps.ld(slot)];
-}
+// The scene of a pixel's paths; a frame of one scene needs no load.
+__device__ __forceinline__ uint32_t scene_of(const Frame& F, uint32_t pix) { return F.nscenes == 1 ? 0u : F.pscene[pix]; }
 
-// Counter set of iteration `it`: [0] queue count, [1] extension head,
-// [2] shadow count, [3] shadow head, [4] ended paths (free queue count).
 // The iteration index lives in F.iter (device), so an iteration's launches
 // are the same every time (graph-capturable).
 __device__ __forceinline__ uint32_t* ctr_set(const Frame& F, int it) { return F.ctr + 8 * (it % 3); }
 
 // The sample of a path that ended (new_path's input to the moving average):
 // path p's colour at sample index round_start[p - p0] + pixel.
-__device__ __forceinline__ void store_sample(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t pbv,
-                                             float4 acc) {
-    rec_st(&F.samples[P.round_start[(pbv >> 10) - (uint32_t)P.p0] + F.pix.ld(slot)], acc);
+__device__ __forceinline__ void store_sample(const Frame& F, const RenderParams& P, uint32_t pix, uint32_t pbv, v3 acc) {
+    rec_st(&F.samples[P.round_start[(pbv >> 10) - (uint32_t)P.p0] + pix], make_float4(acc.x, acc.y, acc.z, 0.0f));
 }
 
-// Slots whose path ended go to the free queue; k_regen starts the next
-// paths on them.
-__device__ __forceinline__ void end_paths(const Frame& F, bool ended, uint32_t slot, uint32_t* cn) {
-    push(ended, slot, F.q[3], cn + 4);
-}
-
-// Stores the sample of every ended path (new_path's input to the moving
-// average) and starts the next paths of the chunk on the freed slots,
-// appending them to the next extension queue.
-__global__ void __launch_bounds__(kBlock, GB_STREAM_MIN_BLOCKS) k_regen(Frame F, RenderParams P) {
-    const int it = *F.iter;
-    const uint32_t* cn = ctr_set(F, it + 1);
-    // free-queue entries before cn[5] were restarted by k_shadow (cn[7]
-    // paths started); the rest are the paths k_shade ended (all of them
-    // when k_shadow restarted none)
-    const uint32_t first = cn[5];
-    const uint32_t count = cn[4] - first;
-    const uint32_t next0 = cn[0];   // paths already queued for the next iteration
-    const uint32_t l0 = *F.path_ctr + cn[7];
-    const uint32_t avail = l0 < P.chunk_paths ? P.chunk_paths - l0 : 0u;
-    uint32_t* qout = F.q[(it + 1) & 1];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    // free-queue entry first + qi takes path l0 + qi and next-queue entry
-    // next0 + qi: no counter round trip; k_step advances both counters
-    // afterwards.  The ended paths' samples were stored where they ended
-    // (store_sample).
-    const uint32_t nstart = min(count, avail);
-    for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < nstart; qi += stride) {
-        const uint32_t slot = F.q[3][first + qi];
-        start_path(F, P, slot, l0 + qi);
-        qout[next0 + qi] = slot;
-    }
-}
-
-// Restart of the paths k_extend ended (misses), run by the warps of
-// k_shadow once the shadow queue has no rays left for them, so that it
-// fills the tail of the any-hit launch.  Free-queue entry qi < nA takes
-// path l0 + qi and next-queue entry qi; k_shade appends the continuing
-// paths after them, k_regen restarts the paths k_shade ends.  Not in the
-// adjoint mode, whose sweep reads the ended paths' records first.
-__device__ __forceinline__ void restart_misses(const Frame& F, const RenderParams& P) {
-    const int it = *F.iter;
-    uint32_t* cn = ctr_set(F, it + 1);
-    const uint32_t count = cn[4];  // misses of k_extend (k_shade has not run)
-    const uint32_t l0 = *F.path_ctr;
-    const uint32_t avail = l0 < P.chunk_paths ? P.chunk_paths - l0 : 0u;
-    const uint32_t nA = min(count, avail);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cn[0] = nA;     // next-queue entries taken (k_shade appends after them)
-        cn[5] = count;  // free-queue entries consumed
-        cn[7] = nA;     // paths started
-    }
-    uint32_t* qout = F.q[(it + 1) & 1];
-    const uint32_t lane = lane_id();
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0u) base = atomicAdd(&cn[6], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= nA) break;
-        const uint32_t qi = base + lane;
-        if (qi < nA) {
-            const uint32_t slot = F.q[3][qi];
-            start_path(F, P, slot, l0 + qi);
-            qout[qi] = slot;
+// Adjoint mode: starts the next paths of the chunk on the slots whose paths
+// k_adjoint has swept, appending them to the next extension queue.
+__global__ void __launch_bounds__(kBlock) k_regen(Frame F, RenderParams P) {
+    uint32_t* cn = ctr_set(F, F.iter[1] + 1);
+    const uint32_t count = cn[CTR_DONE];
+    uint32_t* qout = F.q[(F.iter[1] + 1) & 1];
+    __shared__ uint32_t s_l, s_q;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock) {
+        if (threadIdx.x == 0) {
+            const uint32_t n = min(count - base, (uint32_t)kBlock);
+            const uint32_t l = atomicAdd(F.path_ctr, n);
+            const uint32_t go = l < P.chunk_paths ? min(n, P.chunk_paths - l) : 0u;
+            s_l = l;
+            s_q = go ? atomicAdd(&cn[CTR_EXT], go) : 0u;
+            if (go) atomicAdd(&cn[CTR_STARTED], go);
         }
+        __syncthreads();
+        const uint32_t i = base + threadIdx.x, l = s_l + threadIdx.x;
+        if (i < count && l < P.chunk_paths) {
+            const uint32_t slot = F.q[5][i];
+            start_path(F, P, slot, l);
+            qout[s_q + threadIdx.x] = slot;
+        }
+        __syncthreads();
     }
 }
 
-// First paths of a chunk: slot s takes path s.  Resets the iteration index.
+// First paths of a chunk: slot s takes path s.  Sets the queue of iteration 0
+// (the counters are zero) and the iteration index.
 __global__ void __launch_bounds__(kBlock) k_start(Frame F, RenderParams P, int nstart) {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) { *F.path_ctr = (uint32_t)nstart; *F.iter = 0; }
-    bool go = s < (uint32_t)nstart;
-    if (go) start_path(F, P, s, s);
-    add_stats(&F.stats[0], go ? 1u : 0u);
-    push(go, s, F.q[0], F.ctr + 0);  // queue of iteration 0
-}
-
-// End of an iteration: accounts the paths k_regen started (path counter,
-// next queue count, camera rays), clears the counter set two iterations
-// ahead, moves the iteration index, counts the iteration (stats[7]) and
-// tells the graph's loop (when there is one) whether the next extension
-// queue has work.
-__global__ void k_step(Frame F, RenderParams P, unsigned long long cond, int has_cond, int max_iters) {
-    const int it = *F.iter;
-    uint32_t* cn = ctr_set(F, it + 1);
-    const uint32_t l0 = *F.path_ctr;
-    const uint32_t avail = l0 < P.chunk_paths ? P.chunk_paths - l0 : 0u;
-    // restarts in k_shadow and k_shade (cn[7] attempts, already queued), or
-    // in k_regen (the free queue, queued at cn[0] + qi)
-    const bool fused = GB_FUSED_RESTART && P.mode != MODE_ADJOINT;
-    const uint32_t started = fused ? min(cn[7], avail) : min(cn[4], avail);
-    *F.path_ctr = l0 + started;
-    if (!fused) cn[0] += started;
-    F.stats[0] += (unsigned long long)started;
-    uint32_t* c2 = ctr_set(F, it + 2);
-    for (int k = 0; k < 8; ++k) c2[k] = 0u;
-    const uint32_t next = cn[0];
-    *F.iter = it + 1;
-    F.stats[7] += 1ull;
-    if (next != 0u && it + 1 >= max_iters) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
-    if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, (next != 0u && it + 1 < max_iters) ? 1u : 0u);
+    if (s == 0) {
+        *F.path_ctr = (uint32_t)nstart;
+        F.iter[0] = 0;
+        F.ctr[CTR_EXT] = (uint32_t)nstart;
+        F.ctr[CTR_STARTED] = (uint32_t)nstart;
+    }
+    if (s >= (uint32_t)nstart) return;
+    start_path(F, P, s, s);
+    F.q[0][s] = s;
 }
 
 // (t, canonical id) as one 64-bit key whose unsigned order is the
@@ -860,9 +734,9 @@ __device__ __forceinline__ unsigned long long hit_key(float t, uint32_t id) {
 // closest hit's barycentrics are recomputed by its owner from the shading
 // record with the same (v0, v1 - v0, v2 - v0) arithmetic as the triangle
 // layout, so they are bit-identical too.  All 32 lanes must call this.
-template <bool ANY, bool INSTR>
+template <bool INSTR>
 __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, const float4* shade, const RayInv& r,
-                                               float tmax, Trav& s, unsigned long long* skey, uint32_t* ntri) {
+                                               bool any, Trav& s, unsigned long long* skey, uint32_t* ntri) {
     const uint32_t lane = lane_id();
     const uint32_t cnt = act ? (uint32_t)__popc(s.tg.y) : 0u;
     uint32_t incl = cnt;
@@ -892,7 +766,6 @@ __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, con
                          __shfl_sync(0xffffffffu, r.o.z, (int)o));
         const v3 rd = mk(__shfl_sync(0xffffffffu, r.d.x, (int)o), __shfl_sync(0xffffffffu, r.d.y, (int)o),
                          __shfl_sync(0xffffffffu, r.d.z, (int)o));
-        const float otmax = __shfl_sync(0xffffffffu, tmax, (int)o);
         const float4* otris = (const float4*)__shfl_sync(0xffffffffu, (unsigned long long)tris, (int)o);
         if (g < total) {
             const uint32_t bit = __fns(om, 0u, (int)(g - oe) + 1);
@@ -901,7 +774,7 @@ __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, con
                 float4 a0 = ld_tri(tp + 0), a1 = ld_tri(tp + 1), a2 = ld_tri(tp + 2);
                 if (INSTR) ++*ntri;
                 float t, u, v;
-                if (intersect_tri(ro, rd, ld3(a0), ld3(a1), ld3(a2), &t, &u, &v) && t <= otmax)
+                if (intersect_tri(ro, rd, ld3(a0), ld3(a1), ld3(a2), &t, &u, &v))
                     atomicMin(skey + o, hit_key(t, __float_as_uint(a0.w)));
             }
         }
@@ -917,7 +790,7 @@ __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, con
             s.best_t = t;
             s.best_id = id;
             found = true;
-            if (!ANY) {
+            if (!any) {
                 const float4* sh = shade + 6 * (size_t)id;
                 const v3 a = ld3(__ldg(sh + 0)), b = ld3(__ldg(sh + 1)), c = ld3(__ldg(sh + 2));
                 float tt, u, v;
@@ -929,16 +802,18 @@ __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, con
     return found;
 }
 
-// Persistent-warp ray loop shared by the traversal kernels: lanes whose ray
-// has finished run `finish` together, idle lanes are refilled from the queue
-// as soon as `refill` lanes are idle (all lanes once the queue is
-// exhausted), and traversal resumes where each lane stopped.  The first
-// wave is assigned by warp index (warp w takes entries [32w, 32w+32)); later
-// fetches take one atomic per warp on `head`.  Each lane carries the
-// geometry of its own scene.  fetch(q, &handle, ...) loads queue entry q's
-// ray and sets the handle that finish(fin, handle, trav, t_max) gets back
-// when the ray is done.
-template <bool ANY, bool INSTR, int MODE, int STACK, int BT, typename Fetch, typename Finish>
+// Persistent-warp ray loop of the traversal kernels: lanes whose ray has
+// finished run `finish` together, idle lanes are refilled from the queue as
+// soon as `refill` lanes are idle (all lanes once the queue is exhausted),
+// and traversal resumes where each lane stopped.  The first wave is assigned
+// by warp index (warp w takes entries [32w, 32w+32)); later fetches take one
+// atomic per warp on `head`.  Each lane carries the geometry of its own
+// scene.  fetch(q, &handle, ...) loads queue entry q's ray; bit 31 of the
+// handle says any-hit; finish(handle, trav) gets it back when the ray is
+// done.  A warp that makes kIterLimit steps without a refill gives up.
+constexpr uint32_t kAnyHit = 0x80000000u;
+
+template <bool INSTR, int MODE, int STACK, int BT, typename Fetch, typename Finish>
 __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int refill, uint32_t* status, Fetch fetch,
                                          Finish finish, uint32_t* nvis, uint32_t* ntri) {
     const uint32_t lane = lane_id();
@@ -946,10 +821,8 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
     const uint32_t dyn0 = nwarps * 32u;
     const uint32_t gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     bool act = false, fin = false, exhausted = false, first = true;
-    uint32_t qi = 0;  // the lane's handle for finish, as fetch sets it
-    int iters = 0;
+    uint32_t hd = 0;  // the lane's handle for finish, as fetch sets it
     RayInv r;
-    float tmax = 0.0f;
     Trav s;
     __shared__ uint2 s_stack[kSmemStack > 0 ? kSmemStack * BT : 1];
     uint2 deep[STACK - kSmemStack];
@@ -960,7 +833,7 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
     __shared__ unsigned long long s_key[MODE == 3 ? BT : 1];
     unsigned long long* skey = s_key + (MODE == 3 ? (threadIdx.x & ~31u) : 0u);
     while (true) {
-        finish(fin, qi, s, tmax);
+        if (fin) finish(hd, s);
         fin = false;
         uint32_t idle = __ballot_sync(0xffffffffu, !act);
         if (!exhausted && idle) {
@@ -981,34 +854,26 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
                 uint32_t q = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
                 if (q < count) {
                     v3 o, d;
-                    if (fetch(q, &qi, &o, &d, &tmax, &nodes, &tris, &shade)) {
-                        r = make_ray(o, d);
-                        trav_init(s, r);
-                        iters = 0;
-                        act = true;
-                    } else {
-                        trav_init(s, make_ray(o, d));
-                        fin = true;  // nothing to trace (e.g. no light): finish directly
-                    }
+                    float tmax;
+                    fetch(q, &hd, &o, &d, &tmax, &nodes, &tris, &shade);
+                    r = make_ray(o, d);
+                    trav_init(s, r, tmax);
+                    act = true;
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, act || fin)) break;
+        if (!__any_sync(0xffffffffu, act)) break;
+        const bool any = (hd & kAnyHit) != 0u;
+        int steps = 0;
         while (true) {
+            bool done = false;
             if (MODE == 3) {
                 // the warp tests every lane's pending triangles together, then
                 // each lane visits one node
-                bool hit = coop_triangles<ANY, INSTR>(act, tris, shade, r, tmax, s, skey, ntri);
-                if (ANY && act && hit) { act = false; fin = true; }
-                if (act) {
-                    bool done = node_step<INSTR, STACK>(nodes, r, tmax, s, stack, status, nvis);
-                    if (!done && ++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); done = true; }
-                    if (done) { act = false; fin = true; }
-                }
+                const bool hit = coop_triangles<INSTR>(act, tris, shade, r, any, s, skey, ntri);
+                if (act) done = (any && hit) || node_step<INSTR, STACK>(nodes, r, s, stack, status, nvis);
             } else if (MODE == 0) {
-                bool done = warp_step<ANY, INSTR, STACK>(act, nodes, tris, r, tmax, s, stack, status, nvis, ntri);
-                if (act && !done && ++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); done = true; }
-                if (done) { act = false; fin = true; }
+                done = warp_step<INSTR, STACK>(act, nodes, tris, r, any, s, stack, status, nvis, ntri);
             } else {
                 // triangle postponing: when fewer than a fifth of the active
                 // lanes have triangles pending, those lanes stack their
@@ -1025,177 +890,94 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
                     do_tri = false;
                 }
                 if (act) {
-                    bool done = false;
                     if (do_tri) {
-                        if (MODE == 1) done = tri_step<ANY, INSTR>(tris, r, tmax, s, ntri);
+                        if (MODE == 1) done = tri_step<INSTR>(tris, r, any, s, ntri);
                         else
-                            while (s.tg.y != 0u && !done) done = tri_step<ANY, INSTR>(tris, r, tmax, s, ntri);
+                            while (s.tg.y != 0u && !done) done = tri_step<INSTR>(tris, r, any, s, ntri);
                     } else {
-                        done = node_step<INSTR, STACK>(nodes, r, tmax, s, stack, status, nvis);
+                        done = node_step<INSTR, STACK>(nodes, r, s, stack, status, nvis);
                     }
-                    if (!done && ++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); done = true; }
-                    if (done) { act = false; fin = true; }
                 }
             }
+            if (++steps > kIterLimit) {
+                if (act) atomicOr(status, ST_ITER_LIMIT);
+                done = act;
+            }
+            if (done) { act = false; fin = true; }
             uint32_t nidle = (uint32_t)__popc(__ballot_sync(0xffffffffu, !act));
             if (nidle == 32u || (!exhausted && nidle >= (uint32_t)refill)) break;
         }
     }
 }
 
-// Closest hit of the extension queue.  Misses add handle_no_hit's
-// contribution and end their path; hits draw the bounce's uniforms and emit
-// the area-light shadow ray (arealight-sampler-cpu.cpp:25-143).
-// The light sample of a hit (generate_arealight_sample,
-// arealight-sampler-cpu.cpp:25-143) on the path's light draw: shadow ray,
-// potential_sample_contribution and the path draw of this bounce.
-// skip_dark: a sample whose potential contribution is exactly zero (the
-// surface or the light faces away) gets no shadow ray (max_t = -1, read as
-// occluded).  Its visibility cannot change the path: shading adds
-// bl * (tp * psc) = +-0 when unoccluded (or nothing, when that is NaN), and
-// the accumulation is never -0, so the sum is the same bits either way.
-__device__ __forceinline__ void nee_at_hit(const Frame& F, const SceneRec& R, uint32_t slot, v3 Pp, v3 Nr,
-                                           bool skip_dark) {
-    const DevScene& S = R.S;
-    MrgState st = ld_mrg(F.rng, slot);
-    v3 rnd = draw3(&st);
-    st_mrg(F.rng, slot, st, true);
-    v3 lr = rnd;
-    if (R.rng_mode == 1) {
-        int pid = (int)(F.pix.ld(slot) - R.pixel_base) + 1;
-        float hy = halton(pid, 3);
-        lr = mk(halton(pid, 2), hy, hy);
-    }
-    v3 so = mk(0.0f, 0.0f, 0.0f), sd = mk(0.0f, 0.0f, 0.0f), psc = mk(0.0f, 0.0f, 0.0f);
-    float smax = -1.0f, scale = 0.0f;
-    if (S.n_lights > 0) {
-        int l = pick_light(S.lights, S.n_lights, S.overall_power, lr.z);
-        LightRec L = S.lights[l];
-        if (L.type == 1)
-            sky_light_sample(S.sky, L.power, S.overall_power, Pp, Nr, lr.x, lr.y, R.sp.shadow_offset, &so, &sd,
-                             &smax, &psc);
-        else
-            rect_light_sample(L, S.lights_eval[l].col, S.overall_power, Pp, Nr, lr.x, lr.y, R.sp.shadow_offset,
-                              &so, &sd, &smax, &psc, &scale);
-    }
-    if (skip_dark && psc.x == 0.0f && psc.y == 0.0f && psc.z == 0.0f) smax = -1.0f;
-    F.sh_o.st_hit(slot, make_float4(so.x, so.y, so.z, smax));
-    F.sh_d.st_hit(slot, make_float4(sd.x, sd.y, sd.z, 0.0f));
-    F.psc.st_hit(slot, make_float4(psc.x, psc.y, psc.z, scale));
-    F.rnd.st_hit(slot, make_float4(rnd.x, rnd.y, rnd.z, 0.0f));
-}
-
-// STACK: traversal stack entries; BT: threads per block (the register
-// budget stays that of GB_TRAV_MIN_BLOCKS blocks of 128 threads).
+// The rays of one iteration: the closest hit of every extension ray (to
+// F.hit), then whether anything blocks every shadow ray (to F.occl).  Block 0
+// keeps the loop: it hands the iteration index to the kernels after it,
+// clears the counter set after next (nobody reads it now), accounts the rays
+// and paths of this iteration and tells the graph's loop (when there is one)
+// to go on, so the loop ends with one iteration on empty queues.
+// STACK: traversal stack entries; BT: threads per block (the register budget
+// is that of GB_TRAV_MIN_BLOCKS blocks of 128 threads).
 template <bool INSTR, int MODE, int STACK, int BT>
-__global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_extend(Frame F, RenderParams P) {
-    const int it = *F.iter;
+__global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Frame F, RenderParams P,
+                                                                            unsigned long long cond, int has_cond) {
+    const int it = F.iter[0];
     uint32_t* cs = ctr_set(F, it);
-    uint32_t* cn = ctr_set(F, it + 1);
-    const uint32_t count = cs[0];
-    const uint32_t* qin = F.q[it & 1];
-    uint32_t* qsh = F.q[2];
-    uint32_t nvis = 0, ntri = 0, nhit = 0;
-    // the handle finish gets back is the queue entry: re-reading the slot
-    // there costs less than keeping it live through the traversal
+    const uint32_t next = cs[CTR_EXT], nsh = cs[CTR_SHADOW];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t work = next | nsh | cs[CTR_ENDED], started = cs[CTR_STARTED];
+        F.iter[1] = it;
+        uint32_t* c2 = ctr_set(F, it + 2);
+        for (int k = 0; k < 8; ++k) c2[k] = 0u;
+        F.stats[0] += started;
+        F.stats[1] += next - started;
+        F.stats[2] += nsh;
+        if (work) F.stats[7] += 1ull;
+        if (work && it >= P.max_iters) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
+        if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, work && it < P.max_iters ? 1u : 0u);
+    }
+    const uint32_t *qe = F.q[it & 1], *qs = F.q[2];
+    uint32_t nvis = 0, ntri = 0, nvis_any = 0, ntri_any = 0;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
                      const float4** tris, const float4** shade) {
-        const uint32_t slot = qin[q];
-        *handle = q;
-        float4 ro = F.ray_o.ld(slot), rd = F.ray_d.ld(slot);
-        const SceneRec& R = scene_of(F, slot);
+        Sector r;
+        uint32_t sc;
+        if (q < next) {
+            const uint32_t slot = qe[q];
+            *handle = slot;
+            r = rec_ld(&F.ray[slot]);
+            *tmax = FLT_MAX;
+            sc = scene_of(F, r.w[7]);
+        } else {
+            const uint32_t slot = qs[q - next];
+            *handle = slot | kAnyHit;
+            r = rec_ld(&F.shray[slot]);
+            *tmax = __uint_as_float(r.w[6]);
+            sc = r.w[7];
+        }
+        const SceneRec& R = F.scenes[sc];
         *nodes = R.S.nodes;
         *tris = R.S.tris;
         *shade = R.S.shade;
-        *o = ld3(ro); *d = ld3(rd); *tmax = ro.w;
-        return true;
+        *o = sec3(r, 0);
+        *d = sec3(r, 3);
     };
-    auto finish = [&](bool fin, uint32_t q, const Trav& h, float) {
-        bool hit = false, ended = false;
-        uint32_t slot = 0;
-        if (fin) {
-            slot = qin[q];
-            hit = h.best_id != 0xffffffffu;
-            const SceneRec& R = scene_of(F, slot);
-            uint32_t pbv = F.pb.ld(slot);
-            if ((pbv & 1023u) > 0u) add_stats_lane(&F.stats[1]);
-            if (!hit) {
-                float4 tp4 = F.tp.ld(slot);
-                float4 acc = F.accum.ld(slot);
-                v3 add = miss_contribution(ld3(tp4), ld3(F.ray_d.ld(slot)), R.sp, &R.S.sky);
-                store_sample(F, P, slot, pbv, make_float4(acc.x + add.x, acc.y + add.y, acc.z + add.z, 0.0f));
-                ended = true;
-            } else {
-                const DevScene& S = R.S;
-                if (INSTR) ++nhit;
-                const float4* sh = S.shade + 6 * (size_t)h.best_id;
-                float4 a = ld_shade(sh + 0), b = ld_shade(sh + 1), c = ld_shade(sh + 2);
-                float4 na = ld_shade(sh + 3), nb = ld_shade(sh + 4), nc = ld_shade(sh + 5);
-                v3 Pp = bary(h.bb, h.bg, ld3(a), ld3(b), ld3(c));
-                v3 Nr = bary(h.bb, h.bg, ld3(na), ld3(nb), ld3(nc));
-                if (!GB_SPLIT_NEE) nee_at_hit(F, R, slot, Pp, Nr, P.mode != MODE_ADJOINT);
-                F.hit_p.st_hit(slot, make_float4(Pp.x, Pp.y, Pp.z, a.w));
-                F.hit_n.st_hit(slot, make_float4(Nr.x, Nr.y, Nr.z, __uint_as_float(h.best_id)));
-            }
+    auto finish = [&](uint32_t handle, const Trav& h) {
+        const uint32_t slot = handle & ~kAnyHit;
+        if (handle & kAnyHit) F.occl[slot] = h.best_id != 0xffffffffu ? 1 : 0;
+        else rec_st(&F.hit[slot], make_float4(h.bb, h.bg, __uint_as_float(h.best_id), 0.0f));
+        if (INSTR) {
+            if (handle & kAnyHit) { nvis_any += nvis; ntri_any += ntri; }
+            else { atomicAdd(&F.stats[3], (unsigned long long)nvis); atomicAdd(&F.stats[4], (unsigned long long)ntri); }
+            nvis = 0;
+            ntri = 0;
         }
-        push(fin && hit, slot, qsh, cs + 2);
-        end_paths(F, ended, slot, cn);
     };
-    ray_loop<false, INSTR, MODE, STACK, BT>(count, cs + 1, P.refill, F.status, fetch, finish, &nvis, &ntri);
+    ray_loop<INSTR, MODE, STACK, BT>(next + nsh, cs + CTR_HEAD, P.refill, F.status, fetch, finish, &nvis, &ntri);
     if (INSTR) {
-        add_stats(&F.stats[3], nvis);
-        add_stats(&F.stats[4], ntri);
-        add_stats(&F.stats[8], nhit);
+        add_stats(&F.stats[5], nvis_any);
+        add_stats(&F.stats[6], ntri_any);
     }
-}
-
-// Light samples of every hit of the iteration (shadow queue), when they are
-// not taken inside k_extend (GB_SPLIT_NEE).
-__global__ void __launch_bounds__(kBlock) k_nee(Frame F, int mode) {
-    const uint32_t* cs = ctr_set(F, *F.iter);
-    const uint32_t count = cs[2];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        const uint32_t slot = F.q[2][i];
-        const SceneRec& R = scene_of(F, slot);
-        nee_at_hit(F, R, slot, ld3(F.hit_p.ld(slot)), ld3(F.hit_n.ld(slot)), mode != MODE_ADJOINT);
-    }
-}
-
-// Any-hit of the shadow queue; the result goes to sh_d.w (1 = occluded).
-template <bool INSTR, int MODE, int STACK, int BT>
-__global__ void __launch_bounds__(BT, GB_SHADOW_MIN_BLOCKS * 128 / BT) k_shadow(Frame F, RenderParams P) {
-    const int it = *F.iter;
-    uint32_t* cs = ctr_set(F, it);
-    const uint32_t count = cs[2];
-    const uint32_t* qsh = F.q[2];
-    uint32_t nvis = 0, ntri = 0;
-    // the handle finish gets back is the slot
-    auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
-                     const float4** tris, const float4** shade) {
-        const uint32_t slot = qsh[q];
-        *handle = slot;
-        float4 so = F.sh_o.ld(slot), sd = F.sh_d.ld(slot);
-        const SceneRec& R = scene_of(F, slot);
-        *nodes = R.S.nodes;
-        *tris = R.S.tris;
-        *shade = R.S.shade;
-        *o = ld3(so); *d = ld3(sd); *tmax = so.w;
-        const bool traced = so.w >= 0.0f;
-        if (traced) add_stats_lane(&F.stats[2]);  // shadow rays traced
-        return traced;
-    };
-    // smax: the shadow ray's max_t (negative: a dark sample, not traced)
-    auto finish = [&](bool fin, uint32_t slot, const Trav& h, float smax) {
-        if (fin) {
-            bool occl = smax < 0.0f || h.best_id != 0xffffffffu;
-            rec_st(reinterpret_cast<float*>(&F.sh_d[slot]) + 3, occl ? 1.0f : 0.0f);
-        }
-    };
-    ray_loop<true, INSTR, MODE, STACK, BT>(count, cs + 3, GB_SHADOW_REFILL > 0 ? GB_SHADOW_REFILL : P.refill,
-                                           F.status, fetch, finish, &nvis, &ntri);
-    if (INSTR) { add_stats(&F.stats[5], nvis); add_stats(&F.stats[6], ntri); }
-    if (GB_FUSED_RESTART && P.mode != MODE_ADJOINT) restart_misses(F, P);
 }
 
 // Material record of index mi; the texture fields (last float4) only when
@@ -1213,126 +995,240 @@ __device__ __forceinline__ MaterialRec load_material(const float* mats, uint32_t
     return unpack_material(mf);
 }
 
-// Light the NEE of a hit picked (arealight-sampler-cpu.cpp:32-39 on the
-// light draw of k_extend).
-__device__ __forceinline__ int nee_light(const Frame& F, const SceneRec& R, uint32_t slot, v3 rnd) {
-    if (R.S.n_lights <= 0) return 0;
-    float lz = rnd.z;
-    if (R.rng_mode == 1) lz = halton((int)(F.pix.ld(slot) - R.pixel_base) + 1, 3);
-    return pick_light(R.S.lights, R.S.n_lights, R.S.overall_power, lz);
-}
-
 // Hit of a path in a textured scene: the ray differentials move to the hit
 // (computeRayDiffs, hybrid-pt.cpp:518-519) and a diffuse texture scales the
-// material's base colour.  The hit's barycentrics are recomputed with the
-// traversal's own triangle test (same operands, same bits).
-__device__ __noinline__ void texture_hit(const Frame& F, const SceneRec& R, uint32_t slot, float4 hn,
-                                         MaterialRec* m) {
-    const uint32_t tid = __float_as_uint(hn.w);
+// material's base colour.
+__device__ __noinline__ void texture_hit(const Frame& F, const SceneRec& R, uint32_t slot, uint32_t tid, float bb,
+                                         float bg, v3 Nr, MaterialRec* m) {
     const float4* sh = R.S.shade + 6 * (size_t)tid;
     const v3 a = ld3(__ldg(sh)), b = ld3(__ldg(sh + 1)), c = ld3(__ldg(sh + 2));
-    float t, bb = 0.0f, bg = 0.0f;
-    intersect_tri(ld3(F.ray_o.ld(slot)), ld3(F.ray_d.ld(slot)), a, b - a, c - a, &t, &bb, &bg);
     const float* tcs = R.S.texcoord + 6 * (size_t)tid;
     float ts, tt;
     bary2(bb, bg, tcs, &ts, &tt);
     RayDiff df = ld_rdiff(F, slot);
-    const float diff = ray_diff_hit(&df, a, b, c, tcs, ts, tt, normalize_div(ld3(hn)));
+    const float diff = ray_diff_hit(&df, a, b, c, tcs, ts, tt, normalize_div(Nr));
     st_rdiff(F, slot, df);
     if (m->dtex >= 0 && m->dtex < R.S.n_tex)
         *m = textured_material(*m, tex_sample_bilin_lod(R.S.tex[m->dtex], ts, tt, diff));
 }
 
-// BRDF sample/eval, NEE accumulation and next ray for every shadow-queue
-// entry (compute_path_contribution_and_bounce for the hits); paths that end
-// go to the free queue.  MODE_FROZEN evaluates the BRDF with the scene's
-// eval records and carries the sampling throughput in tp0; MODE_ADJOINT
-// writes the vertex record of the path-replay adjoint.  Every path leaves
-// with pb's bounce field = the number of vertices it shaded.
+// The light sample of a hit (generate_arealight_sample,
+// arealight-sampler-cpu.cpp:25-143) on the bounce's light draw.
+struct LightSample {
+    v3 so, sd, psc;      // shadow ray (to_light), potential_sample_contribution
+    float smax, scale;   // max_t (negative: no light), geometry term over the pick probability
+    int light;
+};
+__device__ __forceinline__ LightSample light_sample(const SceneRec& R, uint32_t pix, v3 Pp, v3 Nr, v3 rnd) {
+    const DevScene& S = R.S;
+    v3 lr = rnd;
+    if (R.rng_mode == 1) {
+        int pid = (int)(pix - R.pixel_base) + 1;
+        float hy = halton(pid, 3);
+        lr = mk(halton(pid, 2), hy, hy);
+    }
+    LightSample s;
+    s.so = s.sd = s.psc = mk(0.0f, 0.0f, 0.0f);
+    s.smax = -1.0f;
+    s.scale = 0.0f;
+    s.light = 0;
+    if (S.n_lights > 0) {
+        s.light = pick_light(S.lights, S.n_lights, S.overall_power, lr.z);
+        LightRec L = S.lights[s.light];
+        if (L.type == 1)
+            sky_light_sample(S.sky, L.power, S.overall_power, Pp, Nr, lr.x, lr.y, R.sp.shadow_offset, &s.so, &s.sd,
+                             &s.smax, &s.psc);
+        else
+            rect_light_sample(L, S.lights_eval[s.light].col, S.overall_power, Pp, Nr, lr.x, lr.y,
+                              R.sp.shadow_offset, &s.so, &s.sd, &s.smax, &s.psc, &s.scale);
+    }
+    return s;
+}
+
+// Shading of every traced path (compute_path_contribution_and_bounce for the
+// hits, handle_no_hit for the misses).  The block first permutes its 128
+// queue entries: hits first, then paths that end here (misses, and ended
+// paths whose last shadow ray has now been traced), so that at most one warp
+// holds both kinds.  A path that ends stores its sample and restarts on its
+// slot with the chunk's next path; in MODE_ADJOINT it goes to the done queue
+// instead, for k_adjoint and k_regen.
+//
+// A vertex's light sample adds bl * (tp * psc) to the accumulation if its
+// shadow ray is free.  The contribution is formed here and kept pending; the
+// next iteration's k_rays traces the ray and the next k_shade adds it before
+// anything else, so the sums and their order are those of the reference.  No
+// ray is traced for a contribution of exactly zero (the light or the surface
+// faces away, no lobe towards the light): adding +-0 to an accumulation that
+// is never -0 leaves its bits as they are.  The adjoint traces those too: its
+// vertex records carry the visibility.
+//
+// MODE_FROZEN evaluates the BRDF with the scene's eval records and carries
+// the sampling throughput in tp0; MODE_ADJOINT writes the vertex record of
+// the path-replay adjoint and leaves pb's bounce field = the number of
+// vertices the path shaded.
 template <int MODE, bool TEX>
 __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, RenderParams P) {
-    const int it = *F.iter;
-    uint32_t* cs = ctr_set(F, it);
-    uint32_t* cn = ctr_set(F, it + 1);
-    const uint32_t count = cs[2];
-    const uint32_t* qsh = F.q[2];
-    uint32_t* qout = F.q[(it + 1) & 1];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t l0 = *F.path_ctr;
-    const uint32_t avail = l0 < P.chunk_paths ? P.chunk_paths - l0 : 0u;
-    for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < count; i0 += stride) {
-        uint32_t qi = i0 + lane_id();
-        bool valid = qi < count;
-        uint32_t slot = 0;
-        bool cont = false, ended = false;
-        if (valid) {
-            slot = qsh[qi];
-            const SceneRec& R = scene_of(F, slot);
-            float4 sd = F.sh_d.ld(slot);
-            float4 hp = F.hit_p.ld(slot), hn = F.hit_n.ld(slot);
-            uint32_t mi = __float_as_uint(hp.w);
-            const bool textured = TEX && R.S.texcoord != nullptr;
-            MaterialRec m = load_material(R.S.mats, mi, textured);
-            if (textured) texture_hit(F, R, slot, hn, &m);
-            uint32_t pbv = F.pb.ld(slot);
-            int bounce = (int)(pbv & 1023u);
-            uint32_t path = pbv >> 10;
-            float4 rd = F.ray_d.ld(slot), tp4 = F.tp.ld(slot), rn = F.rnd.ld(slot),
-                   ps = F.psc.ld(slot);
-            float4 acc = F.accum.ld(slot);
-            ShadeOut o;
-            if (MODE == MODE_FROZEN) {
-                MaterialRec me = load_material(R.S.mats_eval, mi);
-                v3 t0 = ld3(F.tp0[slot]);
-                o = shade_hit(m, ld3(hp), ld3(hn), ld3(rd), ld3(tp4), ld3(rn), sd.w == 0.0f, ld3(sd), ld3(ps), R.sp,
-                              F.pix.ld(slot) - R.pixel_base, path, bounce, &me, &t0);
-                F.tp0[slot] = make_float4(t0.x, t0.y, t0.z, 0.0f);
-            } else if (MODE == MODE_ADJOINT) {
-                ShadeTrace tr;
-                o = shade_hit(m, ld3(hp), ld3(hn), ld3(rd), ld3(tp4), ld3(rn), sd.w == 0.0f, ld3(sd), ld3(ps), R.sp,
-                              F.pix.ld(slot) - R.pixel_base, path, bounce, nullptr, nullptr, &tr);
-                int light = nee_light(F, R, slot, ld3(rn));
-                uint32_t info = (uint32_t)light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
-                                (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
-                float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
-                rec[0] = make_float4(tp4.x, tp4.y, tp4.z, tr.pdf);
-                rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
-                rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ps.w : 0.0f);
-                rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(mi));
-                rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
+    __shared__ uint32_t s_cnt[4][kBlock / 32], s_base[4];
+    __shared__ uint32_t s_slot[kBlock];
+    __shared__ float4 s_hit[kBlock];
+    const int it = F.iter[1];
+    const uint32_t *cs = ctr_set(F, it), *qe = F.q[it & 1], *qc = F.q[3 + (it & 1)];
+    uint32_t *cn = ctr_set(F, it + 1), *qout = F.q[(it + 1) & 1], *qcout = F.q[3 + ((it + 1) & 1)];
+    const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
+    const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, lt = (1u << lane) - 1u;
+    if (blockIdx.x == 0 && tid == 0) F.iter[0] = it + 1;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock) {
+        // entries of the tile, hits first
+        const uint32_t n = min(count - base, (uint32_t)kBlock);
+        uint32_t slot = 0u;
+        float4 hit = make_float4(0.0f, 0.0f, __uint_as_float(0xffffffffu), 0.0f);
+        const uint32_t i = base + tid;
+        if (i < ne) {
+            slot = qe[i];
+            hit = rec_ld(&F.hit[slot]);
+        } else if (i < count) {
+            slot = qc[i - ne] | kAnyHit;  // marks an ended path
+        }
+        const bool ishit = __float_as_uint(hit.z) != 0xffffffffu;
+        const uint32_t mh = __ballot_sync(0xffffffffu, ishit);
+        if (lane == 0) s_cnt[0][wid] = (uint32_t)__popc(mh);
+        __syncthreads();
+        uint32_t nh = 0, before = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kBlock / 32; ++w) {
+            if (w < wid) before += s_cnt[0][w];
+            nh += s_cnt[0][w];
+        }
+        const uint32_t rank = before + (uint32_t)__popc(mh & lt);  // hits before this thread's entry
+        const uint32_t pos = ishit ? rank : nh + (tid - rank);
+        s_slot[pos] = slot;
+        s_hit[pos] = hit;
+        __syncthreads();
+        slot = s_slot[tid];
+        hit = s_hit[tid];
+        const bool dead = (slot & kAnyHit) != 0u;
+        slot &= ~kAnyHit;
+
+        bool cont = false, fin = false, shadow = false, ended = false;
+        if (tid < n) {
+            const Sector rs = rec_ld(&F.ray[slot]), ps = rec_ld(&F.path[slot]), ss = rec_ld(&F.strm[slot]);
+            const uint32_t pbv = rs.w[6], pix = rs.w[7];
+            const int bounce = (int)(pbv & 1023u);
+            v3 acc = sec3(ps, 3);
+            const v3 tp = sec3(ps, 0), rd = sec3(rs, 3);
+            const bool occl = F.occl[slot] != 0;
+            if (!occl)
+                acc = acc + mk(__uint_as_float(ps.w[6]), __uint_as_float(ps.w[7]), __uint_as_float(ss.w[6]));
+            else if (MODE == MODE_ADJOINT && bounce > 0)  // the last vertex's light sample did not count
+                atomicAnd(reinterpret_cast<uint32_t*>(
+                              F.adj + ((size_t)(bounce - 1) * kAdjPlanes + 4) * F.nslots + slot) + 3, ~(1u << 23));
+            const uint32_t sc = scene_of(F, pix);
+            const SceneRec& R = F.scenes[sc];
+            if (tid < nh) {
+                MrgState st{{ss.w[0], ss.w[1], ss.w[2]}, {ss.w[3], ss.w[4], ss.w[5]}};
+                const v3 rnd = draw3(&st);
+                const uint32_t id = __float_as_uint(hit.z);
+                const float4* sh = R.S.shade + 6 * (size_t)id;
+                const float4 a = __ldg(sh), b = __ldg(sh + 1), c = __ldg(sh + 2);
+                const v3 Pp = bary(hit.x, hit.y, ld3(a), ld3(b), ld3(c));
+                const v3 Nr = bary(hit.x, hit.y, ld3(__ldg(sh + 3)), ld3(__ldg(sh + 4)), ld3(__ldg(sh + 5)));
+                const LightSample ls = light_sample(R, pix, Pp, Nr, rnd);
+                const uint32_t mi = __float_as_uint(a.w);
+                const bool textured = TEX && R.S.texcoord != nullptr;
+                MaterialRec m = load_material(R.S.mats, mi, textured);
+                if (textured) texture_hit(F, R, slot, id, hit.x, hit.y, Nr, &m);
+                const uint32_t path = pbv >> 10, lp = pix - R.pixel_base;
+                ShadeOut o;
+                if (MODE == MODE_FROZEN) {
+                    MaterialRec me = load_material(R.S.mats_eval, mi);
+                    v3 t0 = ld3(F.tp0[slot]);
+                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce, &me,
+                                  &t0);
+                    F.tp0[slot] = make_float4(t0.x, t0.y, t0.z, 0.0f);
+                } else if (MODE == MODE_ADJOINT) {
+                    ShadeTrace tr;
+                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
+                                  nullptr, nullptr, &tr);
+                    uint32_t info = (uint32_t)ls.light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
+                                    (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
+                    float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
+                    rec[0] = make_float4(tp.x, tp.y, tp.z, tr.pdf);
+                    rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
+                    rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ls.scale : 0.0f);
+                    rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(mi));
+                    rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
+                    shadow = tr.nee;
+                } else {
+                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce);
+                }
+                const v3 pend = o.accum_add;
+                if (MODE != MODE_ADJOINT) shadow = pend.x != 0.0f || pend.y != 0.0f || pend.z != 0.0f;
+                if (shadow) rec_st(&F.shray[slot], pack_sector(ls.so, ls.sd, __float_as_uint(ls.smax), sc));
+                cont = o.alive && bounce + 1 < R.L;
+                if (cont) rec_st(&F.ray[slot], pack_sector(o.org, o.dir, pbv + 1u, pix));
+                else if (MODE == MODE_ADJOINT) F.ray[slot].w[6] = pbv + 1u;  // the path's vertices, for k_adjoint
+                ended = !cont && shadow;
+                fin = !cont && !shadow;
+                if (!fin) st_path(F, slot, o.tp, acc, st, pend);
             } else {
-                o = shade_hit(m, ld3(hp), ld3(hn), ld3(rd), ld3(tp4), ld3(rn), sd.w == 0.0f, ld3(sd), ld3(ps), R.sp,
-                              F.pix.ld(slot) - R.pixel_base, path, bounce);
+                if (!dead) acc = acc + miss_contribution(tp, rd, R.sp, &R.S.sky);
+                fin = true;
             }
-            acc = make_float4(acc.x + o.accum_add.x, acc.y + o.accum_add.y, acc.z + o.accum_add.z, 0.0f);
-            cont = o.alive && bounce + 1 < R.L;
-            ended = !cont;
-            const float pbw = __uint_as_float(pbv + 1u);  // ray_d.w
-            if (cont) {
-                F.tp.st(slot, make_float4(o.tp.x, o.tp.y, o.tp.z, 0.0f));
-                F.accum.st(slot, acc);
-                F.ray_o.st(slot, make_float4(o.org.x, o.org.y, o.org.z, FLT_MAX));
-                F.ray_d.st(slot, make_float4(o.dir.x, o.dir.y, o.dir.z, pbw));
-            } else {
-                store_sample(F, P, slot, pbv, acc);
-                if (MODE == MODE_ADJOINT) F.ray_d.st(slot, make_float4(rd.x, rd.y, rd.z, pbw));  // bounces for k_adjoint
+            if (fin) store_sample(F, P, pix, pbv, acc);
+        }
+        // queue places: continuing paths, shadow rays, pending ended paths, finished paths
+        const uint32_t m0 = __ballot_sync(0xffffffffu, cont), m1 = __ballot_sync(0xffffffffu, shadow),
+                       m2 = __ballot_sync(0xffffffffu, ended), m3 = __ballot_sync(0xffffffffu, fin);
+        if (lane == 0) {
+            s_cnt[0][wid] = (uint32_t)__popc(m0);
+            s_cnt[1][wid] = (uint32_t)__popc(m1);
+            s_cnt[2][wid] = (uint32_t)__popc(m2);
+            s_cnt[3][wid] = (uint32_t)__popc(m3);
+        }
+        __syncthreads();
+        uint32_t tot[4], off[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            tot[k] = off[k] = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < kBlock / 32; ++w) {
+                if (w < wid) off[k] += s_cnt[k][w];
+                tot[k] += s_cnt[k][w];
             }
         }
-        if (GB_FUSED_RESTART && MODE != MODE_ADJOINT) {
-            // a path that shading ends restarts on its slot at once: path
-            // l0 + j, j counted on from k_shadow's restarts (cn[7])
-            const uint32_t j = warp_inc(ended, &cn[7]);
-            const bool restart = ended && j < avail;
-            if (restart) start_path(F, P, slot, l0 + j);
-            push(cont || restart, slot, qout, cn);
-        } else {
-            push(cont, slot, qout, cn);
-            end_paths(F, ended, slot, cn);
+        if (tid == 0) {
+            uint32_t go = 0;
+            if (MODE == MODE_ADJOINT) {
+                s_base[3] = tot[3] ? atomicAdd(&cn[CTR_DONE], tot[3]) : 0u;
+            } else if (tot[3]) {
+                // finished paths take the chunk's next paths and queue places after the continuing ones
+                const uint32_t l = atomicAdd(F.path_ctr, tot[3]);
+                s_base[3] = l;
+                go = l < P.chunk_paths ? min(tot[3], P.chunk_paths - l) : 0u;
+                if (go) atomicAdd(&cn[CTR_STARTED], go);
+            }
+            if (tot[0] + go) s_base[0] = atomicAdd(&cn[CTR_EXT], tot[0] + go);
+        }
+        if (tid == 32 && tot[1]) s_base[1] = atomicAdd(&cn[CTR_SHADOW], tot[1]);
+        if (tid == 64 && tot[2]) s_base[2] = atomicAdd(&cn[CTR_ENDED], tot[2]);
+        if (tid == 96 && nh) atomicAdd(&F.stats[8], (unsigned long long)nh);
+        __syncthreads();
+        if (cont) qout[s_base[0] + off[0] + (uint32_t)__popc(m0 & lt)] = slot;
+        if (shadow) F.q[2][s_base[1] + off[1] + (uint32_t)__popc(m1 & lt)] = slot;
+        if (ended) qcout[s_base[2] + off[2] + (uint32_t)__popc(m2 & lt)] = slot;
+        if (fin) {
+            const uint32_t j = off[3] + (uint32_t)__popc(m3 & lt);
+            if (MODE == MODE_ADJOINT) {
+                F.q[5][s_base[3] + j] = slot;
+            } else if (s_base[3] + j < P.chunk_paths) {
+                start_path(F, P, slot, s_base[3] + j);
+                qout[s_base[0] + tot[0] + j] = slot;
+            }
         }
     }
 }
 
-// Path-replay adjoint of every path that ended this iteration (free queue,
+// Path-replay adjoint of every path that finished this iteration (done queue,
 // before k_regen reuses the slots).  The path's value is
 //   C = sum_k T_k * bl_k * col_l(k) * s_k,  T_{k+1} = clamp1(T_k * brdf_k / pdf_k) / q_k
 // with pdf, q, the clamp pattern and all directions held at their recorded
@@ -1340,17 +1236,16 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 // the BRDF vector-Jacobian products and the emission gradient to this
 // block's gradient replica.  g = dLoss/dI(pixel) / spp.
 __global__ void __launch_bounds__(kBlock) k_adjoint(Frame F, RenderParams P) {
-    const int it = *F.iter;
-    uint32_t* cn = ctr_set(F, it + 1);
-    const uint32_t count = cn[4];
+    const uint32_t count = ctr_set(F, F.iter[1] + 1)[CTR_DONE];
     float* grad = F.grad + (size_t)(blockIdx.x % (uint32_t)F.grad_replicas) * (size_t)F.grad_stride;
     const size_t ns = (size_t)F.nslots;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t slot = F.q[3][i];
-        const int K = (int)(F.pb.ld(slot) & 1023u);
-        const float4 g4 = F.dimg[F.pix.ld(slot)];
+        const uint32_t slot = F.q[5][i];
+        const uint32_t pbv = F.ray[slot].w[6], pix = F.ray[slot].w[7];
+        const int K = (int)(pbv & 1023u);
+        const float4 g4 = F.dimg[pix];
         if (K == 0 || (g4.x == 0.0f && g4.y == 0.0f && g4.z == 0.0f)) continue;
-        const SceneRec& R = scene_of(F, slot);
+        const SceneRec& R = F.scenes[scene_of(F, pix)];
         const v3 g = ld3(g4);
         float* gm_base = grad + R.grad_base;
         float* gl_base = gm_base + (size_t)kMatGradFloats * (size_t)R.n_mats;
@@ -1430,8 +1325,7 @@ __global__ void __launch_bounds__(kBlock) k_adjoint(Frame F, RenderParams P) {
             // the path's final miss (the white background a throughput of
             // (1, 1, 1) adds, hybrid-pt.cpp:567-572): its sample minus the
             // light-sample terms; below rounding of the sum it is none
-            const uint32_t pbv = F.pb.ld(slot);
-            const float4 sv = F.samples[P.round_start[(pbv >> 10) - (uint32_t)P.p0] + F.pix.ld(slot)];
+            const float4 sv = F.samples[P.round_start[(pbv >> 10) - (uint32_t)P.p0] + pix];
             const float gtot = dot(g, ld3(sv));
             const float gmiss = gtot - gsuf;
             if (fabsf(gmiss) > 1e-4f * fabsf(gtot)) {
@@ -1834,10 +1728,10 @@ cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cu
 // array) the launch carries it as an access-policy attribute: node lines
 // persist in the L2 set-aside, so that the per-iteration state streaming
 // past does not evict them.
-template <typename K>
-void launch_traversal(K kernel, dim3 grid, int block, const Frame& F, const RenderParams& P, cudaStream_t st) {
+template <typename K, typename... Args>
+void launch_traversal(K kernel, dim3 grid, int block, const RenderParams& P, cudaStream_t st, Args... args) {
     if (P.l2_nodes_bytes == 0) {
-        kernel<<<grid, block, 0, st>>>(F, P);
+        kernel<<<grid, block, 0, st>>>(args...);
         return;
     }
     cudaLaunchAttribute at[1];
@@ -1854,67 +1748,39 @@ void launch_traversal(K kernel, dim3 grid, int block, const Frame& F, const Rend
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, F, P);
+    cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <bool INSTR, int MODE, int STACK, int BT>
-void launch_extend_v(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    static Grid g = persistent_grid(k_extend<INSTR, MODE, STACK, BT>, BT);
-    launch_traversal(k_extend<INSTR, MODE, STACK, BT>, traversal_grid(g, P.blocks_per_sm, BT), BT, F, P, st);
+void launch_rays_v(const Frame& F, const RenderParams& P, unsigned long long cond, bool has_cond, cudaStream_t st) {
+    static Grid g = persistent_grid(k_rays<INSTR, MODE, STACK, BT>, BT);
+    launch_traversal(k_rays<INSTR, MODE, STACK, BT>, traversal_grid(g, P.blocks_per_sm, BT), BT, P, st, F, P, cond,
+                     has_cond ? 1 : 0);
 }
 
 // The default triangle policy has variants for two stack depths and two
 // block shapes (RenderParams::trav_variant), the other policies one each.
 template <bool INSTR, int MODE>
-void launch_extend_t(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    if (MODE == 0 && P.trav_variant == 1) launch_extend_v<INSTR, MODE, 24, 128>(F, P, st);
-    else if (MODE == 0 && P.trav_variant == 2) launch_extend_v<INSTR, MODE, 32, 64>(F, P, st);
-    else if (MODE == 0 && P.trav_variant == 3) launch_extend_v<INSTR, MODE, 24, 64>(F, P, st);
-    else launch_extend_v<INSTR, MODE, kStack, kBlock>(F, P, st);
-    if (GB_SPLIT_NEE) {
-        static int gn = persistent_blocks(k_nee);
-        k_nee<<<gn, kBlock, 0, st>>>(F, P.mode);
+void launch_rays_t(const Frame& F, const RenderParams& P, unsigned long long c, bool h, cudaStream_t st) {
+    if constexpr (MODE == 0) {
+        if (P.trav_variant == 1) return launch_rays_v<INSTR, MODE, 24, 128>(F, P, c, h, st);
+        if (P.trav_variant == 2) return launch_rays_v<INSTR, MODE, 32, 64>(F, P, c, h, st);
+        if (P.trav_variant == 3) return launch_rays_v<INSTR, MODE, 24, 64>(F, P, c, h, st);
     }
+    launch_rays_v<INSTR, MODE, kStack, kBlock>(F, P, c, h, st);
 }
 
-template <bool INSTR, int MODE, int STACK, int BT>
-void launch_shadow_v(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    static Grid g = persistent_grid(k_shadow<INSTR, MODE, STACK, BT>, BT);
-    launch_traversal(k_shadow<INSTR, MODE, STACK, BT>, traversal_grid(g, P.blocks_per_sm, BT), BT, F, P, st);
-}
-
-template <bool INSTR, int MODE>
-void launch_shadow_t(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    if (MODE == 0 && P.trav_variant == 1) launch_shadow_v<INSTR, MODE, 24, 128>(F, P, st);
-    else if (MODE == 0 && P.trav_variant == 2) launch_shadow_v<INSTR, MODE, 32, 64>(F, P, st);
-    else if (MODE == 0 && P.trav_variant == 3) launch_shadow_v<INSTR, MODE, 24, 64>(F, P, st);
-    else launch_shadow_v<INSTR, MODE, kStack, kBlock>(F, P, st);
-}
-
-cudaError_t k_launch_extend(const Frame& F, const RenderParams& P, bool instrument, cudaStream_t st) {
+cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument, unsigned long long c, bool h,
+                          cudaStream_t st) {
     switch (P.tri_mode * 2 + (instrument ? 1 : 0)) {
-        case 0: launch_extend_t<false, 0>(F, P, st); break;
-        case 1: launch_extend_t<true, 0>(F, P, st); break;
-        case 2: launch_extend_t<false, 1>(F, P, st); break;
-        case 3: launch_extend_t<true, 1>(F, P, st); break;
-        case 4: launch_extend_t<false, 2>(F, P, st); break;
-        case 5: launch_extend_t<true, 2>(F, P, st); break;
-        case 6: launch_extend_t<false, 3>(F, P, st); break;
-        default: launch_extend_t<true, 3>(F, P, st); break;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t k_launch_shadow(const Frame& F, const RenderParams& P, bool instrument, cudaStream_t st) {
-    switch (P.tri_mode * 2 + (instrument ? 1 : 0)) {
-        case 0: launch_shadow_t<false, 0>(F, P, st); break;
-        case 1: launch_shadow_t<true, 0>(F, P, st); break;
-        case 2: launch_shadow_t<false, 1>(F, P, st); break;
-        case 3: launch_shadow_t<true, 1>(F, P, st); break;
-        case 4: launch_shadow_t<false, 2>(F, P, st); break;
-        case 5: launch_shadow_t<true, 2>(F, P, st); break;
-        case 6: launch_shadow_t<false, 3>(F, P, st); break;
-        default: launch_shadow_t<true, 3>(F, P, st); break;
+        case 0: launch_rays_t<false, 0>(F, P, c, h, st); break;
+        case 1: launch_rays_t<true, 0>(F, P, c, h, st); break;
+        case 2: launch_rays_t<false, 1>(F, P, c, h, st); break;
+        case 3: launch_rays_t<true, 1>(F, P, c, h, st); break;
+        case 4: launch_rays_t<false, 2>(F, P, c, h, st); break;
+        case 5: launch_rays_t<true, 2>(F, P, c, h, st); break;
+        case 6: launch_rays_t<false, 3>(F, P, c, h, st); break;
+        default: launch_rays_t<true, 3>(F, P, c, h, st); break;
     }
     return cudaGetLastError();
 }
@@ -1932,8 +1798,7 @@ cudaError_t k_launch_shadow(const Frame& F, const RenderParams& P, bool instrume
 #define GB_WIDE_GRID_DIV 4  // the wide grid has nslots / GB_WIDE_GRID_DIV threads
 #endif
 inline int stream_grid(int persistent, int nslots) {
-    return (GB_WIDE_STREAM_GRIDS || nslots > (1 << 20)) ? std::max(1, blocks_for(nslots / GB_WIDE_GRID_DIV))
-                                                          : persistent;
+    return nslots > (1 << 20) ? std::max(1, blocks_for(nslots / GB_WIDE_GRID_DIV)) : persistent;
 }
 
 template <int MODE, bool TEX>
@@ -1999,20 +1864,13 @@ cudaError_t k_launch_grad_reduce(const float* grad, int replicas, int stride, do
 }
 
 int k_launches_per_iteration(int mode) {
-    if (mode == MODE_ADJOINT) return 6;   // extend, shadow, shade, adjoint, regen, step
-    return GB_FUSED_RESTART ? 4 : 5;      // restarts inside shadow and shade
+    return mode == MODE_ADJOINT ? 4 : 2;  // rays, shade; adjoint, regen
 }
 
 cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    if (GB_FUSED_RESTART && P.mode != MODE_ADJOINT) return cudaSuccess;  // restarted in k_shadow / k_shade
+    if (P.mode != MODE_ADJOINT) return cudaSuccess;  // paths restart in k_shade
     static int g0 = persistent_blocks(k_regen);
     k_regen<<<stream_grid(g0, F.nslots), kBlock, 0, st>>>(F, P);
-    return cudaGetLastError();
-}
-
-cudaError_t k_launch_step(const Frame& F, const RenderParams& P, unsigned long long cond, bool has_cond,
-                          int max_iters, cudaStream_t st) {
-    k_step<<<1, 1, 0, st>>>(F, P, cond, has_cond ? 1 : 0, max_iters);
     return cudaGetLastError();
 }
 

@@ -64,33 +64,24 @@ constexpr int kAdjMaxSlots = 1 << 22;  // slots of an adjoint chunk (vertex reco
 
 constexpr int kMaxRounds = 64;  // path samples per chunk
 
-// Per-slot state of the wavefront: one 256-byte record per path slot.
-// Slots are visited in queue order, which is not slot order, so every field
-// access of a slot is a scattered access.  A record keeps what one stage
-// reads or writes together in one 128-byte line, so that a stage touches a
-// few whole 32-byte sectors of a slot instead of one partly used sector per
-// field, and the kernels write whole sectors (a partly written sector costs
-// DRAM a read-modify-write when it leaves the L2):
-//   line 0 (path state: written by path start and by shading)
-//     0 ray_o, 16 ray_d (w: pb), 32 tp, 48 accum, 64 pix, 68 ps, 72 zero,
-//     80 rdiff[0..2] (ray differentials of textured scenes; rdiff[0] is
-//     zeroed at path start otherwise)
-//   line 1 (hit record: written by the closest-hit kernel)
-//     128 hit_p, 144 hit_n, 160 sh_o, 176 sh_d, 192 psc, 208 rnd,
-//     224 rng (+ 8 zero bytes)
-constexpr size_t kSlotBytes = 256;
-// GB_SHADOW_SPLIT: shadow rays (sh_o, sh_d) in their own 32-byte-per-slot
-// array instead of the hit line
-#ifndef GB_SHADOW_SPLIT
-#define GB_SHADOW_SPLIT 0
-#endif
-constexpr size_t kShadowStride = GB_SHADOW_SPLIT ? 32 : kSlotBytes;
-enum : size_t {
-    kSlotRayO = 0, kSlotRayD = 16, kSlotPb = 28, kSlotTp = 32, kSlotAccum = 48, kSlotPix = 64, kSlotPs = 68,
-    kSlotRdiff = 80, kSlotHitP = 128, kSlotHitN = 144, kSlotShO = 160, kSlotShD = 176, kSlotPsc = 192,
-    kSlotRnd = 208, kSlotRng = 224
-};
-static_assert(kSlotRdiff + 48 <= 128 && kSlotRng + 24 <= kSlotBytes, "slot record layout");
+// Per-slot state of the wavefront: arrays of 32-byte sectors, one entry per
+// path slot, each moved by one 256-bit access.  A sector holds what a stage
+// reads or writes together, so that no access moves part of a sector (a
+// partly written sector costs DRAM a read-modify-write when it leaves the
+// L2), and queue order stays close to slot order (paths restart on their own
+// slot, queues are filled block by block), so that neighbouring lanes touch
+// neighbouring sectors.
+//   ray    origin 3, direction 3, path index << 10 | bounce, global pixel
+//   path   throughput 3, col_accum 3, pending light sample x, y
+//   strm   light/path stream of the path (MrgState), pending z, 0
+//   shray  shadow ray: origin 3, direction 3, max_t, scene
+// The pending light sample is the contribution of the last vertex's light
+// sample; it is added once its shadow ray is known to be free.  `hit` (16
+// bytes: beta, gamma, triangle id) and `occl` (1 byte) are what a traced
+// extension / shadow ray returns.
+struct alignas(32) Sector { uint32_t w[8]; };
+constexpr size_t kSlotBytes = 4 * sizeof(Sector) + 16 + 1 + 6 * 4;  // sectors, hit, occl, six queue entries
+constexpr size_t kSlotAlign = 256;  // slot counts of an allocation are multiples of this
 
 // Loads and stores of the per-iteration state stream (slot records, samples,
 // jitter pool, stream cursors) carry the cache-streaming hint (ld.cs /
@@ -100,9 +91,6 @@ static_assert(kSlotRdiff + 48 <= 128 && kSlotRng + 24 <= kSlotBytes, "slot recor
 // plain accesses.
 #ifndef GB_REC_EVICT_FIRST
 #define GB_REC_EVICT_FIRST 1
-#endif
-#ifndef GB_HIT_LINE_KEEP
-#define GB_HIT_LINE_KEEP 0
 #endif
 #ifdef __CUDACC__
 template <class T>
@@ -123,61 +111,46 @@ __device__ __forceinline__ void rec_st(T* p, const T& v) {
 }
 #endif
 
-// One field of the slot records: f[slot] is that field of record `slot`;
-// f.ld(slot) / f.st(slot, v) are the stream accesses (rec_ld / rec_st).
-template <class T, size_t Stride = kSlotBytes>
-struct SlotField {
-    unsigned char* base = nullptr;  // the field in record 0
 #ifdef __CUDACC__
-    __host__ __device__
-#endif
-    inline T& operator[](size_t slot) const {
-        return *reinterpret_cast<T*>(base + slot * Stride);
-    }
-#ifdef __CUDACC__
-    __device__ inline T ld(size_t slot) const { return rec_ld(reinterpret_cast<const T*>(base + slot * Stride)); }
-    __device__ inline void st(size_t slot, const T& v) const {
-        rec_st(reinterpret_cast<T*>(base + slot * Stride), v);
-    }
-    // the hit line the closest-hit kernel writes and the any-hit and
-    // shading kernels of the same iteration read back (GB_HIT_LINE_KEEP:
-    // with normal L2 priority instead of evict-first)
-    __device__ inline void st_hit(size_t slot, const T& v) const {
-#if GB_HIT_LINE_KEEP
-        *reinterpret_cast<T*>(base + slot * Stride) = v;
+__device__ __forceinline__ Sector rec_ld(const Sector* p) {
+    Sector r;
+#if GB_REC_EVICT_FIRST
+    asm volatile("ld.global.cs.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
 #else
-        rec_st(reinterpret_cast<T*>(base + slot * Stride), v);
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
 #endif
-    }
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
+                   "=r"(r.w[7])
+                 : "l"(__cvta_generic_to_global(p))
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void rec_st(Sector* p, const Sector& r) {
+#if GB_REC_EVICT_FIRST
+    asm volatile("st.global.cs.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+#else
+    asm volatile("st.global.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
 #endif
-};
+                 :
+                 : "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]),
+                   "r"(r.w[7]), "l"(__cvta_generic_to_global(p))
+                 : "memory");
+}
+#endif
 
-// Wavefront state: per path slot (records above) and per global pixel.
+// Wavefront state: per path slot (sectors above) and per global pixel.
 struct Frame {
     int ntot;          // pixels of all scenes
     int nslots;        // path slots in flight
     const SceneRec* scenes;  // device array
     int nscenes;
-    // per slot: nslots records of kSlotBytes at `slots`, viewed field by field
-    unsigned char* slots;
-    SlotField<float4> ray_o;     // origin xyz, t_max
-    SlotField<float4> ray_d;     // direction xyz
-    SlotField<float4> tp;        // throughput
-    SlotField<float4> accum;     // col_accum of the slot's path
-    SlotField<float4, kShadowStride> sh_o;  // shadow origin xyz, max_t
-    SlotField<float4, kShadowStride> sh_d;  // shadow direction xyz (to_light), w = occluded
-    unsigned char* shadow;       // the shadow-ray array (GB_SHADOW_SPLIT), else null
-    SlotField<float4> psc;       // potential_sample_contribution
-    SlotField<float4> rnd;       // path draw of this bounce
-    SlotField<float4> hit_p;     // hit point xyz | material index bits
-    SlotField<float4> hit_n;     // interpolated (unnormalised) normal | hit triangle id bits
-    SlotField<float4> rdiff[3];  // ray differentials of textured scenes (RayDiff packed)
-    SlotField<MrgState> rng;     // light/path stream of the slot's path
-    SlotField<uint32_t> pix;     // global pixel of the slot's path
-    SlotField<uint32_t> ps;      // scene of the slot's path
-    SlotField<uint32_t> pb;      // path index << 10 | bounce (the bits of ray_d.w)
-    SlotField<uint4> pixw;       // (pix, ps, 0, 0) as one 16-byte word
-    uint32_t* q[4];    // queues: extension (ping/pong), shadow, ended paths; nslots entries each
+    // per slot (bind_slots): the sectors, what traced rays return, and the queues
+    Sector *ray, *path, *strm, *shray;
+    float4* hit;         // beta, gamma, triangle id bits (0xffffffff: miss), 0
+    uint8_t* occl;       // 1 = the slot's shadow ray was blocked
+    uint32_t* q[6];      // extension rays (0 / 1, by iteration), shadow rays (2), ended paths whose light sample
+                         // is still pending (3 / 4), finished paths of the adjoint (5)
+    float4* rdiff;       // ray differentials of textured frames: 3 planes of nslots
     // per global pixel
     float4* out;       // output_color (moving average)
     MrgState* pristine;  // stream after curand_init(seed, pixel, 0)
@@ -188,9 +161,10 @@ struct Frame {
     float4* jpool;     // camera jitter of path l of the chunk
     MrgState* spool;   // light/path stream state at the start of path l of the chunk
     // control
-    uint32_t* ctr;     // 3 sets of 8 (by iteration % 3): count, ext head, shadow count, shadow head, ended
+    uint32_t* ctr;     // 3 sets of 8 (by iteration % 3), see CTR_*
     uint32_t* path_ctr;  // next path of the chunk to start
-    int* iter;         // iteration index of the chunk's slot-pool loop
+    int* iter;         // iteration index of the chunk's slot-pool loop: [0] as k_rays reads it (k_shade moves it
+                       // on), [1] as the kernels after it read it (k_rays copies it there)
     unsigned long long* stats;  // 0 camera, 1 ext, 2 shadow rays; 3/4 closest, 5/6 shadow node visits / tri tests;
                                 // 7 iterations; 8 closest hits (light samples); 16 words
     uint32_t* status;
@@ -205,28 +179,21 @@ struct Frame {
     int grad_replicas;
 };
 
-// Points the slot fields of F at the records at `slots` (kSlotBytes-aligned)
-// and, with GB_SHADOW_SPLIT, the shadow rays at `shadow` (nslots * 32 bytes).
-inline void bind_slots(Frame& F, unsigned char* slots, unsigned char* shadow) {
-    F.slots = slots;
-    auto at = [slots](size_t off) { return slots ? slots + off : nullptr; };
-    F.ray_o.base = at(kSlotRayO);
-    F.ray_d.base = at(kSlotRayD);
-    F.tp.base = at(kSlotTp);
-    F.accum.base = at(kSlotAccum);
-    F.pix.base = at(kSlotPix);
-    F.ps.base = at(kSlotPs);
-    F.pb.base = at(kSlotPb);
-    F.pixw.base = at(kSlotPix);
-    for (int k = 0; k < 3; ++k) F.rdiff[k].base = at(kSlotRdiff + 16 * (size_t)k);
-    F.hit_p.base = at(kSlotHitP);
-    F.hit_n.base = at(kSlotHitN);
-    F.shadow = GB_SHADOW_SPLIT ? shadow : nullptr;
-    F.sh_o.base = GB_SHADOW_SPLIT ? shadow : at(kSlotShO);
-    F.sh_d.base = GB_SHADOW_SPLIT ? (shadow ? shadow + 16 : nullptr) : at(kSlotShD);
-    F.psc.base = at(kSlotPsc);
-    F.rnd.base = at(kSlotRnd);
-    F.rng.base = at(kSlotRng);
+// Counter set of an iteration: extension rays, shadow rays and pending ended
+// paths queued for it, head of its ray queue, finished paths of the adjoint,
+// closest hits found, paths started.
+enum { CTR_EXT = 0, CTR_SHADOW = 1, CTR_ENDED = 2, CTR_HEAD = 3, CTR_DONE = 4, CTR_HITS = 5, CTR_STARTED = 6 };
+
+// Points the per-slot arrays of F at `base` (kSlotBytes * cap bytes, cap a
+// multiple of kSlotAlign).
+inline void bind_slots(Frame& F, unsigned char* base, size_t cap) {
+    F.ray = (Sector*)base;
+    F.path = F.ray + cap;
+    F.strm = F.path + cap;
+    F.shray = F.strm + cap;
+    F.hit = (float4*)(F.shray + cap);
+    for (int k = 0; k < 6; ++k) F.q[k] = (uint32_t*)(F.hit + cap) + (size_t)k * cap;
+    F.occl = (uint8_t*)(F.q[5] + cap);
 }
 
 // Launch-wide parameters of one chunk.
@@ -239,8 +206,9 @@ struct RenderParams {
     int trav_variant;  // traversal kernels of the default triangle policy: stack entries / threads per
                        // block 0: 32 / 128, 1: 24 / 128, 2: 32 / 64, 3: 24 / 64
     int mode;          // MODE_*
-    int textured;      // some scene of the frame has textures (k_shade's texture variant)
+    int textured;      // some scene of the frame has textures (k_shade's texture variant, Frame::rdiff)
     int p0, rounds;    // path samples p0 .. p0+rounds-1
+    int max_iters;     // iteration bound of the chunk's loop
     // L2 window of the traversal launches (GB_NODE_L2_PERSIST, frames of one
     // scene): the scene's node array, accessed as persisting
     const void* l2_nodes;
@@ -254,12 +222,10 @@ cudaError_t k_launch_trace(const DevScene& S, int n, const float* orig, const fl
                            float4* hits, uint8_t* occluded, bool any, uint32_t* status, cudaStream_t st);
 cudaError_t k_launch_frame_init(const Frame& F, bool rng, cudaStream_t st);
 cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cudaStream_t st);
-cudaError_t k_launch_extend(const Frame& F, const RenderParams& P, bool instrument, cudaStream_t st);
-cudaError_t k_launch_shadow(const Frame& F, const RenderParams& P, bool instrument, cudaStream_t st);
+cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument, unsigned long long cond,
+                          bool has_cond, cudaStream_t st);
 cudaError_t k_launch_shade(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t st);
-cudaError_t k_launch_step(const Frame& F, const RenderParams& P, unsigned long long cond, bool has_cond,
-                          int max_iters, cudaStream_t st);
 cudaError_t k_launch_jitter_pool(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_combine(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_pack_rgb(const float4* src, int n, float* dst, cudaStream_t st);

@@ -51,20 +51,20 @@ constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 constexpr size_t kV4 = align_up(sizeof(float4) * (size_t)kNoAllocMaxPixels);  // one float4 per slot / pixel
 constexpr size_t kRng = align_up(sizeof(MrgState) * (size_t)kNoAllocMaxPixels);  // MRG32k3a words per slot / pixel
-constexpr size_t kU32 = align_up(4 * (size_t)kNoAllocMaxPixels);              // one 32-bit word per slot
+constexpr size_t kU32 = align_up(4 * (size_t)kNoAllocMaxPixels);              // one 32-bit word per pixel
 constexpr size_t kCtr = align_up(4 * 32);
 constexpr size_t kStats = align_up(16 * 8);
 constexpr size_t kStatus = align_up(4);
 constexpr size_t kRec = align_up(sizeof(SceneRec));
-constexpr size_t kSlots = kSlotBytes * (size_t)kNoAllocMaxPixels;  // slot records
-constexpr size_t kShadow = GB_SHADOW_SPLIT ? 32 * (size_t)kNoAllocMaxPixels : 0;  // shadow rays
-// One slot per pixel and one path sample per pass: the slot records and
-// 4 queues; per pixel the image, the
+constexpr size_t kSlots = align_up(kSlotBytes * (size_t)kNoAllocMaxPixels);  // per-slot state and queues
+static_assert(kNoAllocMaxPixels % kSlotAlign == 0, "bind_slots alignment");
+// One slot per pixel and one path sample per pass: the per-slot state and
+// queues; per pixel the image, the
 // initial RNG states, the two stream cursors, the scene word, one sample,
 // one stream state and
 // one jitter value; counters, path counter, iteration, stats, status and the
 // scene record.
-constexpr size_t kScratchBytes = kSlots + kShadow + 4 * kU32 + kV4 + 4 * kRng + kU32 + 2 * kV4 + kCtr +
+constexpr size_t kScratchBytes = kSlots + kV4 + 4 * kRng + kU32 + 2 * kV4 + kCtr +
                                  kCtr + kCtr + kStats + kStatus + kRec;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -91,8 +91,7 @@ Frame carve(unsigned char* base, int n, SceneRec** rec) {
     F.nslots = n;
     F.nscenes = 1;
     size_t off = 0;
-    bind_slots(F, base + off, base + off + kSlots); off += kSlots + kShadow;
-    for (int k = 0; k < 4; ++k) { F.q[k] = (uint32_t*)(base + off); off += kU32; }
+    bind_slots(F, base + off, kNoAllocMaxPixels); off += kSlots;
     F.out = (float4*)(base + off); off += kV4;
     F.pristine = (MrgState*)(base + off); off += kRng;
     F.cursor = (MrgState*)(base + off); off += kRng;
@@ -202,11 +201,13 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     if (e == cudaSuccess) e = cudaMemcpyAsync(F.cursor, F.pristine, sizeof(MrgState) * (size_t)n, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(F.jcursor, F.pristine, sizeof(MrgState) * (size_t)n, cudaMemcpyDeviceToDevice, st);
     // one path sample of every pixel per pass, one slot per pixel: a path
-    // has at most max_bounces segments, so the queue is empty after
-    // max_bounces + 1 iterations; the host checks the queue count every 8
-    // iterations and the device flags a queue still non-empty after
-    // max_bounces + 2 iterations (ST_ITER_LIMIT)
+    // has at most max_bounces segments and its last light sample is settled
+    // one iteration later, so the queues are empty after max_bounces + 1
+    // iterations; the host checks the queue counts every 8 iterations and the
+    // device flags queues still non-empty after max_bounces + 2 iterations
+    // (ST_ITER_LIMIT)
     const int max_iters = d->max_bounces + 2;
+    P.max_iters = max_iters;
     uint32_t left = 0;
     for (int p = 0; p < d->spp && e == cudaSuccess; ++p) {
         P.p0 = p;
@@ -215,14 +216,13 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
         if (e == cudaSuccess) e = k_launch_start(F, P, n, st);
         left = 1;
         for (int it = 0; e == cudaSuccess && left != 0u && it < max_iters; ++it) {
-            e = k_launch_extend(F, P, false, st);
-            if (e == cudaSuccess) e = k_launch_shadow(F, P, false, st);
+            e = k_launch_rays(F, P, false, 0, false, st);
             if (e == cudaSuccess) e = k_launch_shade(F, P, st);
-            if (e == cudaSuccess) e = k_launch_regen(F, P, st);
-            if (e == cudaSuccess) e = k_launch_step(F, P, 0, false, max_iters, st);
             if (e == cudaSuccess && (it % 8 == 7 || it == d->max_bounces || it == max_iters - 1)) {
-                e = cudaMemcpyAsync(&left, F.ctr + 8 * ((it + 1) % 3), sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+                uint32_t c[3] = {0, 0, 0};  // extension, shadow and pending ended counts of the next iteration
+                e = cudaMemcpyAsync(c, F.ctr + 8 * ((it + 1) % 3), sizeof(c), cudaMemcpyDeviceToHost, st);
                 if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                left = c[CTR_EXT] | c[CTR_SHADOW] | c[CTR_ENDED];
             }
         }
         if (e == cudaSuccess && left != 0u) break;  // paths still queued: reported below

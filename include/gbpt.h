@@ -430,20 +430,20 @@ typedef struct {
     uint64_t kernel_launches;                           /* launches of the last render */
     double render_ms;                                   /* device time, begin -> last step */
     /* per-stage device time when stage timing is on (gb_ctx_set_stage_timing):
-     * 0 path start, 1 closest-hit + light sample, 2 any-hit, 3 shade,
-     * 4 path end + restart, 5 moving average                                   */
+     * 0 path start, 1 traversal (closest-hit and any-hit rays together),
+     * 2 unused, 3 shade + light sample + restart, 4 adjoint sweep + its
+     * restarts, 5 moving average                                               */
     double stage_ms[6];
     uint64_t stage_launches[6];
     int paths_done;
-    uint64_t light_samples;  /* closest hits, each with its light sample; only
-                              * counted by gb_render_instrumented          */
+    uint64_t light_samples;  /* closest hits, each with its light sample */
 } gb_stats;
 
 /* Knobs of the wavefront (chosen by the autotuner); 0 keeps a value:
  *   refill    idle lanes (1..32) at which a closest-hit traversal warp
  *             fetches new rays, default 20 (any-hit warps refill at 12)
  *   slots     paths in flight (queue capacity), default 2^24 (a frame
- *             allocates min(its paths, slots); 256 B of path state per slot;
+ *             allocates min(its paths, slots); 169 B of path state and queues per slot;
  *             the adjoint replay uses at most 2^22)
  *   sample_mb budget of the per-path sample buffer, which bounds how many
  *             path samples per pixel one pass of the slot pool covers */
@@ -560,7 +560,7 @@ int gb_render_instrumented(gb_ctx* ctx, gb_scene* scene, const gb_camera* cam,
  * The scene is created beforehand (gb_scene_create allocates); this call
  * renders the same frame as gb_render into the caller's device buffer
  * `out_rgb` (w*h*3 floats) on `stream` (NULL = legacy default stream), with
- * its wavefront state in one fixed file-scope device array (about 27 MB,
+ * its wavefront state in one fixed file-scope device array (about 21 MB,
  * held by every GPU that loads the library until exit) instead of cudaMalloc.
  * Limits: w*h <= 65536 pixels and max_bounces <= 64, else GB_ERR_INVALID;
  * scenes with texture coordinates return GB_ERR_UNSUPPORTED (use gb_render).

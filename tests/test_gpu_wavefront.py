@@ -1,0 +1,73 @@
+"""The slot-pool loop at the sizes where its queues can go wrong: path counts
+around the shading tile (128) and a warp, pools far smaller than the frame,
+one-bounce paths (every path ends with its light sample still pending), a
+scene without lights, and every lobe of the principled room.  Frames and
+gradients equal those of the oracle / of another pool size."""
+import numpy as np
+import pytest
+
+from globillum_gb300 import gbpt, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _against_oracle(ctx, sc, rd):
+    from oracle import oracle
+    s = ctx.scene(sc)
+    img = s.render(sc.camera, rd)
+    st = ctx.stats()
+    s.close()
+    n = rd["width"] * rd["height"]
+    pool = ctx.mrg_pool(n, rd["spp"] * rd["max_bounces"], seed=rd.get("seed", 0))
+    ref = oracle.OracleScene(sc, use_bvh=False).render(sc.camera, rd, pool)
+    assert np.array_equal(img, ref.astype(np.float32)), np.abs(img - ref).max()
+    assert st["camera_rays"] == n * rd["spp"]
+    return st
+
+
+@pytest.mark.parametrize("w,h,spp,slots", [(1, 1, 1, 1), (31, 1, 1, 0), (127, 1, 1, 0), (43, 3, 1, 0), (16, 16, 3, 129),
+                                           (33, 31, 5, 100), (64, 65, 2, 4097)])
+@pytest.mark.parametrize("bounces", [1, 2, 7])
+def test_path_counts_and_pools(gpu_ctx, w, h, spp, slots, bounces):
+    sc = scenes.principled_room(width=w, height=h, spp=spp, max_bounces=bounces, rr_start=3)
+    old = gpu_ctx.get_tuning()
+    try:
+        if slots:
+            gpu_ctx.set_tuning(slots=slots)
+        _against_oracle(gpu_ctx, sc, sc.render)
+    finally:
+        gpu_ctx.set_tuning(slots=old["slots"])
+
+
+def test_no_lights_and_dark_light(gpu_ctx):
+    sc = scenes.cornell(width=40, height=30, spp=2, max_bounces=4)
+    rd = dict(sc.render, rng_mode=gbpt.GB_RNG_MRG32K3A_POOL)
+    dark = scenes.SceneData(**{**sc.__dict__, "lights": []})
+    assert _against_oracle(gpu_ctx, dark, rd)["shadow_rays"] == 0
+    # the light faces away from all but the ceiling above it: most light
+    # samples are exactly zero and trace no shadow ray
+    away = scenes.SceneData(**{**sc.__dict__, "lights": [dict(sc.lights[0], dir=(0.0, 1.0, 0.0))]})
+    st = _against_oracle(gpu_ctx, away, rd)
+    assert 0 < st["shadow_rays"] < st["light_samples"] // 2
+
+
+@pytest.mark.parametrize("slots", [97, 1024])
+def test_adjoint_pool_size_does_not_matter(gpu_ctx, slots):
+    """The visibility of a vertex's light sample reaches its record one
+    iteration after the vertex: the gradient with a small pool (paths restart
+    many times on a slot) equals the one with every path in flight, up to the
+    order of the float atomics (1e-5 of the largest entry)."""
+    sc = scenes.principled_room(width=29, height=23, spp=4, max_bounces=5, rr_start=2)
+    sc.materials[5] = dict(sc.materials[4])  # the adjoint room without glass
+    s = gpu_ctx.scene(sc)
+    g = np.random.default_rng(3).normal(size=(23, 29, 3)).astype(np.float32)
+    ref = s.backward(sc.camera, sc.render, g)
+    old = gpu_ctx.get_tuning()
+    try:
+        gpu_ctx.set_tuning(slots=slots)
+        got = s.backward(sc.camera, sc.render, g)
+    finally:
+        gpu_ctx.set_tuning(slots=old["slots"])
+    s.close()
+    assert np.abs(ref).max() > 0
+    assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
