@@ -130,6 +130,8 @@ struct gb_ctx {
     // scratch for API calls with host pointers
     DevBuf scratch[4];
     float* d_rgb = nullptr;
+    float2* d_halton = nullptr;         // Frame::halton's buffer, grown on demand
+    size_t halton_cap = 0;
     size_t rgb_cap = 0;
     // fitting steps: the loop bodies of the step graph are captured on fit_aux
     cudaStream_t fit_aux = nullptr;
@@ -804,10 +806,11 @@ int enqueue_frame_setup(gb_ctx* ctx, cudaStream_t st, const SceneRec* recs, bool
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), st));
     if (record_start) CK(cudaEventRecord(ctx->ev0, st));
     CK(cudaMemcpyAsync(ctx->d_scenes, recs, sizeof(SceneRec) * ctx->recs.size(), cudaMemcpyHostToDevice, st));
-    // F.pscene and the initial RNG states depend on the pixel counts, their
-    // order and the seeds only
+    // F.pscene, F.halton and the initial RNG states depend on the pixel counts,
+    // their order and the seeds only
     std::vector<uint64_t> key;
     key.push_back((uint64_t)F.ntot);
+    key.push_back((uint64_t)(uintptr_t)F.halton);
     for (const BatchScene& b : ctx->items) key.push_back(((uint64_t)b.desc.seed << 32) | (uint32_t)b.n);
     if (key != ctx->pristine_key) {
         CK(k_launch_frame_init(F, true, st));
@@ -845,6 +848,13 @@ int begin_frame(gb_ctx* ctx, std::vector<BatchScene>& items) {
     const long long samples = std::min(total_paths, std::max(ntot, sample_budget(ctx)));
     const int nslots = (int)std::max(1ll, std::min<long long>(total_paths, ctx->slots));
     CK(ensure_frame(ctx, (int)ntot, nslots, (size_t)samples, (int)items.size()));
+    ctx->F.halton = nullptr;
+    for (const BatchScene& b : items)
+        if (b.desc.rng_mode == GB_RNG_HALTON_LIGHT) {
+            CK(ensure_buf(ctx, (void**)&ctx->d_halton, &ctx->halton_cap, sizeof(float2) * (size_t)ntot));
+            ctx->F.halton = ctx->d_halton;
+            break;
+        }
     for (const BatchScene& b : items)
         if (b.scene->S.texcoord) {
             CK(ensure_buf(ctx, (void**)&ctx->F.rdiff, &ctx->rdiff_cap, 3 * sizeof(float4) * ctx->slot_cap));
@@ -959,7 +969,7 @@ std::vector<uint64_t> graph_key(const gb_ctx* ctx, const RenderParams& P, int ns
     k.push_back(((uint64_t)(uint32_t)F.ntot << 32) | (uint32_t)F.nslots);
     k.push_back(((uint64_t)(uint32_t)F.nscenes << 32) | (uint32_t)nstart);
     k.push_back(ctx->instrument ? 1u : 0u);
-    const void* ptrs[] = {F.scenes, F.ray, F.rdiff, F.out,
+    const void* ptrs[] = {F.scenes, F.ray, F.rdiff, F.halton, F.out,
                           F.pristine, F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr,
                           F.iter, F.stats, F.status, F.tp0, F.adj, F.dimg, F.grad};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
@@ -1576,7 +1586,7 @@ namespace {
 std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     const Frame& F = ctx->F;
     std::vector<uint64_t> k;
-    const void* ptrs[] = {ctx->d_scenes, F.ray, F.out, F.pristine,
+    const void* ptrs[] = {ctx->d_scenes, F.ray, F.halton, F.out, F.pristine,
                           F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr, F.iter, F.stats,
                           F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->d_rgb, ctx->fit.d_loss};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);

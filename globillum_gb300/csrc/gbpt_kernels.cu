@@ -55,7 +55,7 @@ constexpr int kIterLimit = 1 << 22;
 #define GB_PREFETCH 0
 #endif
 #ifndef GB_SHADE_MIN_BLOCKS
-#define GB_SHADE_MIN_BLOCKS 5  // resident k_shade blocks per SM (register budget 102)
+#define GB_SHADE_MIN_BLOCKS 7  // resident k_shade blocks per SM (72 registers)
 #endif
 #ifndef GB_NODE_FOLD
 #define GB_NODE_FOLD 0  // 1: plane bias folded into the per-node origin term
@@ -347,8 +347,8 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
 // group, or a stack pop.  Returns true when the ray is finished; the result
 // is the (t, id)-minimum in s (any-hit: best_id != none when found).
 template <bool INSTR, int STACK = kStack>
-__device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, Trav& s, const StackRef& stack,
-                                          uint32_t* status, uint32_t* nvis) {
+__device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
+                                          const StackRef& stack, uint32_t* status, uint32_t* nvis) {
     if (s.ng.y > 0x00ffffffu)
         return visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &s.tg);
     if (s.sp > 0) {
@@ -429,7 +429,12 @@ __device__ __forceinline__ bool traverse(const DevScene& S, const RayInv& r, flo
     while (!trav_step<ANY>(S.nodes, S.tris, r, s, stack, status)) {
         if (++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); break; }
     }
-    if (out) { out->t = s.best_id != 0xffffffffu ? s.best_t : FLT_MAX; out->beta = s.bb; out->gamma = s.bg; out->id = s.best_id; }
+    if (out) {
+        out->t = s.best_id != 0xffffffffu ? s.best_t : FLT_MAX;
+        out->beta = s.bb;
+        out->gamma = s.bg;
+        out->id = s.best_id;
+    }
     return s.best_id != 0xffffffffu;
 }
 
@@ -548,7 +553,7 @@ __global__ void k_mrg_states(const MrgSubseqTable T, uint32_t seed, const uint32
     for (int k = 0; k < 3; ++k) { out[6 * i + k] = m.s1[k]; out[6 * i + 3 + k] = m.s2[k]; }
 }
 
-// Scene of every global pixel.
+// Scene and Halton light draw of every global pixel.
 __global__ void k_fill_pscene(Frame F) {
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= F.ntot) return;
@@ -559,6 +564,14 @@ __global__ void k_fill_pscene(Frame F) {
         else hi = mid - 1;
     }
     F.pscene[g] = (uint32_t)lo;
+    // the pixel's light draw of GB_RNG_HALTON_LIGHT, the same for all its
+    // paths and bounces: about 650 instructions of digit loops and divisions,
+    // against 1100 for the rest of a hit's shading (256x256 room at 16 spp:
+    // 1.045 -> 1.007 ms)
+    if (F.halton) {
+        const int pid = g - (int)F.scenes[lo].pixel_base + 1;
+        F.halton[g] = make_float2(halton(pid, 2), halton(pid, 3));
+    }
 }
 
 // ------------------------------------------------------------ path slots --
@@ -664,7 +677,9 @@ __device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P
 }
 
 // The scene of a pixel's paths; a frame of one scene needs no load.
-__device__ __forceinline__ uint32_t scene_of(const Frame& F, uint32_t pix) { return F.nscenes == 1 ? 0u : F.pscene[pix]; }
+__device__ __forceinline__ uint32_t scene_of(const Frame& F, uint32_t pix) {
+    return F.nscenes == 1 ? 0u : F.pscene[pix];
+}
 
 // The iteration index lives in F.iter (device), so an iteration's launches
 // are the same every time (graph-capturable).
@@ -672,7 +687,8 @@ __device__ __forceinline__ uint32_t* ctr_set(const Frame& F, int it) { return F.
 
 // The sample of a path that ended (new_path's input to the moving average):
 // path p's colour at sample index round_start[p - p0] + pixel.
-__device__ __forceinline__ void store_sample(const Frame& F, const RenderParams& P, uint32_t pix, uint32_t pbv, v3 acc) {
+__device__ __forceinline__ void store_sample(const Frame& F, const RenderParams& P, uint32_t pix, uint32_t pbv,
+                                             v3 acc) {
     rec_st(&F.samples[P.round_start[(pbv >> 10) - (uint32_t)P.p0] + pix], make_float4(acc.x, acc.y, acc.z, 0.0f));
 }
 
@@ -1019,13 +1035,13 @@ struct LightSample {
     float smax, scale;   // max_t (negative: no light), geometry term over the pick probability
     int light;
 };
-__device__ __forceinline__ LightSample light_sample(const SceneRec& R, uint32_t pix, v3 Pp, v3 Nr, v3 rnd) {
+__device__ __forceinline__ LightSample light_sample(const Frame& F, const SceneRec& R, uint32_t pix, v3 Pp, v3 Nr,
+                                                    v3 rnd) {
     const DevScene& S = R.S;
     v3 lr = rnd;
     if (R.rng_mode == 1) {
-        int pid = (int)(pix - R.pixel_base) + 1;
-        float hy = halton(pid, 3);
-        lr = mk(halton(pid, 2), hy, hy);
+        const float2 h = __ldg(&F.halton[pix]);
+        lr = mk(h.x, h.y, h.y);
     }
     LightSample s;
     s.so = s.sd = s.psc = mk(0.0f, 0.0f, 0.0f);
@@ -1046,12 +1062,26 @@ __device__ __forceinline__ LightSample light_sample(const SceneRec& R, uint32_t 
 }
 
 // Shading of every traced path (compute_path_contribution_and_bounce for the
-// hits, handle_no_hit for the misses).  The block first permutes its 128
-// queue entries: hits first, then paths that end here (misses, and ended
-// paths whose last shadow ray has now been traced), so that at most one warp
-// holds both kinds.  A path that ends stores its sample and restarts on its
+// hits, handle_no_hit for the misses).  A block takes tiles of kShadeTile queue
+// entries, sorts each into hits and paths that end here (misses, and ended
+// paths whose last shadow ray has now been traced) and works on them in rounds
+// of 32 of one kind, one round per warp at a time.  The outcome is gathered in
+// lists in shared memory, which take their places in the global queues with
+// one atomic per list.  A path that ends stores its sample and restarts on its
 // slot with the chunk's next path; in MODE_ADJOINT it goes to the done queue
 // instead, for k_adjoint and k_regen.
+//
+// What bounds it: latency of the scattered sector, triangle and material loads
+// and of the ~1100 dependent instructions of a hit, at 28 warps per SM.
+// Measured on the 1M-triangle 64-spp frame / 1 spp / 256x256 room: tiles of one
+// entry per thread sorted by a block scan 45.8 / 1.37 / 1.02 ms; a warp on its
+// own with tiles of 128 44.6 / 1.39 / 1.05; of 32..64 49.6 / 1.41 / 1.05
+// (rounds half empty); this form with tiles of 256 / 512 / 1024 at 5 blocks per
+// SM 44.8 / 43.3 / 43.5; 512 at 6 / 7 / 8 / 10 blocks (80 / 72 / 64 / 48
+// registers) 43.0 / 42.3 / 42.6 / 43.9, 1.36 / 1.34 / 1.35 / 1.39 and 1.05 /
+// 1.01 / 1.02 / 1.08: more warps are worth the spills up to 7 blocks.  Fetching
+// a tile's sectors to L2 ahead changes nothing, triangles as well slows small
+// scenes by a quarter.
 //
 // A vertex's light sample adds bl * (tp * psc) to the accumulation if its
 // shadow ray is free.  The contribution is formed here and kept pending; the
@@ -1066,165 +1096,190 @@ __device__ __forceinline__ LightSample light_sample(const SceneRec& R, uint32_t 
 // the sampling throughput in tp0; MODE_ADJOINT writes the vertex record of
 // the path-replay adjoint and leaves pb's bounce field = the number of
 // vertices the path shaded.
+// Shared memory of a shading block: the tile's entries and what became of
+// them.
+#ifndef GB_SHADE_TILE
+#define GB_SHADE_TILE 512
+#endif
+constexpr uint32_t kShadeTile = GB_SHADE_TILE;
+enum { L_CONT = 0, L_SHADOW = 1, L_ENDED = 2, L_FIN = 3, L_HIT = 4, L_END = 5 };
+struct ShadeTile {
+    float4 entry[kShadeTile];  // beta, gamma, triangle id, slot: hits from the front, the others from the back
+    uint32_t list[4][kShadeTile];
+    uint32_t n[6];             // entries of the lists, hits, others
+    uint32_t base[4];          // places taken in the global queues
+};
+
+// Tile of a launch with `count` entries: whole kShadeTile entries, or as few
+// as give every block one (at least one per thread).
+__device__ __forceinline__ uint32_t shade_tile(uint32_t count) {
+    const uint32_t per = (count / gridDim.x + 127u) & ~127u;
+    return min(max(per, (uint32_t)kBlock), kShadeTile);
+}
+
+// Appends `v` of the flagged lanes to a list of the block.
+__device__ __forceinline__ void append(bool pred, uint32_t v, ShadeTile& T, int k) {
+    const uint32_t m = __ballot_sync(0xffffffffu, pred);
+    if (m == 0u) return;
+    uint32_t b = 0;
+    if (lane_id() == 0u) b = atomicAdd(&T.n[k], (uint32_t)__popc(m));
+    b = __shfl_sync(0xffffffffu, b, 0);
+    if (pred) T.list[k][b + (uint32_t)__popc(m & ((1u << lane_id()) - 1u))] = v;
+}
+
 template <int MODE, bool TEX>
 __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, RenderParams P) {
-    __shared__ uint32_t s_cnt[4][kBlock / 32], s_base[4];
-    __shared__ uint32_t s_slot[kBlock];
-    __shared__ float4 s_hit[kBlock];
+    __shared__ ShadeTile T;
     const int it = F.iter[1];
     const uint32_t *cs = ctr_set(F, it), *qe = F.q[it & 1], *qc = F.q[3 + (it & 1)];
     uint32_t *cn = ctr_set(F, it + 1), *qout = F.q[(it + 1) & 1], *qcout = F.q[3 + ((it + 1) & 1)];
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
-    const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, lt = (1u << lane) - 1u;
+    const uint32_t tid = threadIdx.x, lane = lane_id(), lt = (1u << lane) - 1u;
+    const uint32_t tile = shade_tile(count);
     if (blockIdx.x == 0 && tid == 0) F.iter[0] = it + 1;
-    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock) {
-        // entries of the tile, hits first
-        const uint32_t n = min(count - base, (uint32_t)kBlock);
-        uint32_t slot = 0u;
-        float4 hit = make_float4(0.0f, 0.0f, __uint_as_float(0xffffffffu), 0.0f);
-        const uint32_t i = base + tid;
-        if (i < ne) {
-            slot = qe[i];
-            hit = rec_ld(&F.hit[slot]);
-        } else if (i < count) {
-            slot = qc[i - ne] | kAnyHit;  // marks an ended path
-        }
-        const bool ishit = __float_as_uint(hit.z) != 0xffffffffu;
-        const uint32_t mh = __ballot_sync(0xffffffffu, ishit);
-        if (lane == 0) s_cnt[0][wid] = (uint32_t)__popc(mh);
+    for (uint32_t base = blockIdx.x * tile; base < count; base += gridDim.x * tile) {
+        if (tid < 6) T.n[tid] = 0;
         __syncthreads();
-        uint32_t nh = 0, before = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < kBlock / 32; ++w) {
-            if (w < wid) before += s_cnt[0][w];
-            nh += s_cnt[0][w];
+        const uint32_t n = min(count - base, tile);
+        for (uint32_t k = tid & ~31u; k < n; k += kBlock) {
+            const uint32_t i = base + k + lane;
+            const bool valid = k + lane < n;
+            uint32_t slot = 0u;
+            float4 hit = make_float4(0.0f, 0.0f, __uint_as_float(0xffffffffu), 0.0f);
+            if (valid && i < ne) {
+                slot = qe[i];
+                hit = rec_ld(&F.hit[slot]);
+            } else if (valid) {
+                slot = qc[i - ne] | kAnyHit;  // marks an ended path
+            }
+            const bool ishit = __float_as_uint(hit.z) != 0xffffffffu;
+            const uint32_t mh = __ballot_sync(0xffffffffu, ishit), md = __ballot_sync(0xffffffffu, valid && !ishit);
+            uint32_t b = 0;
+            if (lane < 2) b = atomicAdd(&T.n[L_HIT + lane], (uint32_t)__popc(lane ? md : mh));
+            const uint32_t bh = __shfl_sync(0xffffffffu, b, 0), bd = __shfl_sync(0xffffffffu, b, 1);
+            if (valid) {
+                hit.w = __uint_as_float(slot);
+                T.entry[ishit ? bh + (uint32_t)__popc(mh & lt) : n - 1u - bd - (uint32_t)__popc(md & lt)] = hit;
+            }
         }
-        const uint32_t rank = before + (uint32_t)__popc(mh & lt);  // hits before this thread's entry
-        const uint32_t pos = ishit ? rank : nh + (tid - rank);
-        s_slot[pos] = slot;
-        s_hit[pos] = hit;
         __syncthreads();
-        slot = s_slot[tid];
-        hit = s_hit[tid];
-        const bool dead = (slot & kAnyHit) != 0u;
-        slot &= ~kAnyHit;
+        const uint32_t nh = T.n[L_HIT], rounds = ((nh + 31u) >> 5) + ((n - nh + 31u) >> 5);
+        for (uint32_t round = tid >> 5; round < rounds; round += kBlock / 32) {
+            const bool hits = round < ((nh + 31u) >> 5);  // this round shades hits
+            const uint32_t e = (hits ? 0u : nh) + (round - (hits ? 0u : (nh + 31u) >> 5)) * 32u + lane;
+            const bool valid = e < (hits ? nh : n);
+            float4 hit = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (valid) hit = T.entry[e];
+            uint32_t slot = __float_as_uint(hit.w);
+            const bool dead = (slot & kAnyHit) != 0u;
+            slot &= ~kAnyHit;
 
-        bool cont = false, fin = false, shadow = false, ended = false;
-        if (tid < n) {
-            const Sector rs = rec_ld(&F.ray[slot]), ps = rec_ld(&F.path[slot]), ss = rec_ld(&F.strm[slot]);
-            const uint32_t pbv = rs.w[6], pix = rs.w[7];
-            const int bounce = (int)(pbv & 1023u);
-            v3 acc = sec3(ps, 3);
-            const v3 tp = sec3(ps, 0), rd = sec3(rs, 3);
-            const bool occl = F.occl[slot] != 0;
-            if (!occl)
-                acc = acc + mk(__uint_as_float(ps.w[6]), __uint_as_float(ps.w[7]), __uint_as_float(ss.w[6]));
-            else if (MODE == MODE_ADJOINT && bounce > 0)  // the last vertex's light sample did not count
-                atomicAnd(reinterpret_cast<uint32_t*>(
-                              F.adj + ((size_t)(bounce - 1) * kAdjPlanes + 4) * F.nslots + slot) + 3, ~(1u << 23));
-            const uint32_t sc = scene_of(F, pix);
-            const SceneRec& R = F.scenes[sc];
-            if (tid < nh) {
-                MrgState st{{ss.w[0], ss.w[1], ss.w[2]}, {ss.w[3], ss.w[4], ss.w[5]}};
-                const v3 rnd = draw3(&st);
-                const uint32_t id = __float_as_uint(hit.z);
-                const float4* sh = R.S.shade + 6 * (size_t)id;
-                const float4 a = __ldg(sh), b = __ldg(sh + 1), c = __ldg(sh + 2);
-                const v3 Pp = bary(hit.x, hit.y, ld3(a), ld3(b), ld3(c));
-                const v3 Nr = bary(hit.x, hit.y, ld3(__ldg(sh + 3)), ld3(__ldg(sh + 4)), ld3(__ldg(sh + 5)));
-                const LightSample ls = light_sample(R, pix, Pp, Nr, rnd);
-                const uint32_t mi = __float_as_uint(a.w);
-                const bool textured = TEX && R.S.texcoord != nullptr;
-                MaterialRec m = load_material(R.S.mats, mi, textured);
-                if (textured) texture_hit(F, R, slot, id, hit.x, hit.y, Nr, &m);
-                const uint32_t path = pbv >> 10, lp = pix - R.pixel_base;
-                ShadeOut o;
-                if (MODE == MODE_FROZEN) {
-                    MaterialRec me = load_material(R.S.mats_eval, mi);
-                    v3 t0 = ld3(F.tp0[slot]);
-                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce, &me,
-                                  &t0);
-                    F.tp0[slot] = make_float4(t0.x, t0.y, t0.z, 0.0f);
-                } else if (MODE == MODE_ADJOINT) {
-                    ShadeTrace tr;
-                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
-                                  nullptr, nullptr, &tr);
-                    uint32_t info = (uint32_t)ls.light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
-                                    (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
-                    float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
-                    rec[0] = make_float4(tp.x, tp.y, tp.z, tr.pdf);
-                    rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
-                    rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ls.scale : 0.0f);
-                    rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(mi));
-                    rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
-                    shadow = tr.nee;
+            bool cont = false, fin = false, shadow = false, ended = false;
+            if (valid) {
+                const Sector rs = rec_ld(&F.ray[slot]), ps = rec_ld(&F.path[slot]), ss = rec_ld(&F.strm[slot]);
+                const uint32_t pbv = rs.w[6], pix = rs.w[7];
+                const int bounce = (int)(pbv & 1023u);
+                v3 acc = sec3(ps, 3);
+                const v3 tp = sec3(ps, 0), rd = sec3(rs, 3);
+                const bool occl = F.occl[slot] != 0;
+                if (!occl)
+                    acc = acc + mk(__uint_as_float(ps.w[6]), __uint_as_float(ps.w[7]), __uint_as_float(ss.w[6]));
+                else if (MODE == MODE_ADJOINT && bounce > 0)  // the last vertex's light sample did not count
+                    atomicAnd(reinterpret_cast<uint32_t*>(
+                                  F.adj + ((size_t)(bounce - 1) * kAdjPlanes + 4) * F.nslots + slot) + 3, ~(1u << 23));
+                const uint32_t sc = scene_of(F, pix);
+                const SceneRec& R = F.scenes[sc];
+                if (hits) {
+                    MrgState st{{ss.w[0], ss.w[1], ss.w[2]}, {ss.w[3], ss.w[4], ss.w[5]}};
+                    const v3 rnd = draw3(&st);
+                    const uint32_t id = __float_as_uint(hit.z);
+                    const float4* sh = R.S.shade + 6 * (size_t)id;
+                    const float4 a = __ldg(sh), b = __ldg(sh + 1), c = __ldg(sh + 2);
+                    const v3 Pp = bary(hit.x, hit.y, ld3(a), ld3(b), ld3(c));
+                    const v3 Nr = bary(hit.x, hit.y, ld3(__ldg(sh + 3)), ld3(__ldg(sh + 4)), ld3(__ldg(sh + 5)));
+                    const LightSample ls = light_sample(F, R, pix, Pp, Nr, rnd);
+                    const uint32_t mi = __float_as_uint(a.w);
+                    const bool textured = TEX && R.S.texcoord != nullptr;
+                    MaterialRec m = load_material(R.S.mats, mi, textured);
+                    if (textured) texture_hit(F, R, slot, id, hit.x, hit.y, Nr, &m);
+                    const uint32_t path = pbv >> 10, lp = pix - R.pixel_base;
+                    ShadeOut o;
+                    if (MODE == MODE_FROZEN) {
+                        MaterialRec me = load_material(R.S.mats_eval, mi);
+                        v3 t0 = ld3(F.tp0[slot]);
+                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
+                                      &me, &t0);
+                        F.tp0[slot] = make_float4(t0.x, t0.y, t0.z, 0.0f);
+                    } else if (MODE == MODE_ADJOINT) {
+                        ShadeTrace tr;
+                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
+                                      nullptr, nullptr, &tr);
+                        uint32_t info = (uint32_t)ls.light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
+                                        (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
+                        float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
+                        rec[0] = make_float4(tp.x, tp.y, tp.z, tr.pdf);
+                        rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
+                        rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ls.scale : 0.0f);
+                        rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(mi));
+                        rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
+                        shadow = tr.nee;
+                    } else {
+                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce);
+                    }
+                    const v3 pend = o.accum_add;
+                    if (MODE != MODE_ADJOINT) shadow = pend.x != 0.0f || pend.y != 0.0f || pend.z != 0.0f;
+                    if (shadow) rec_st(&F.shray[slot], pack_sector(ls.so, ls.sd, __float_as_uint(ls.smax), sc));
+                    cont = o.alive && bounce + 1 < R.L;
+                    if (cont) rec_st(&F.ray[slot], pack_sector(o.org, o.dir, pbv + 1u, pix));
+                    else if (MODE == MODE_ADJOINT) F.ray[slot].w[6] = pbv + 1u;  // the path's vertices, for k_adjoint
+                    ended = !cont && shadow;
+                    fin = !cont && !shadow;
+                    if (!fin) st_path(F, slot, o.tp, acc, st, pend);
                 } else {
-                    o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce);
+                    if (!dead) acc = acc + miss_contribution(tp, rd, R.sp, &R.S.sky);
+                    fin = true;
                 }
-                const v3 pend = o.accum_add;
-                if (MODE != MODE_ADJOINT) shadow = pend.x != 0.0f || pend.y != 0.0f || pend.z != 0.0f;
-                if (shadow) rec_st(&F.shray[slot], pack_sector(ls.so, ls.sd, __float_as_uint(ls.smax), sc));
-                cont = o.alive && bounce + 1 < R.L;
-                if (cont) rec_st(&F.ray[slot], pack_sector(o.org, o.dir, pbv + 1u, pix));
-                else if (MODE == MODE_ADJOINT) F.ray[slot].w[6] = pbv + 1u;  // the path's vertices, for k_adjoint
-                ended = !cont && shadow;
-                fin = !cont && !shadow;
-                if (!fin) st_path(F, slot, o.tp, acc, st, pend);
-            } else {
-                if (!dead) acc = acc + miss_contribution(tp, rd, R.sp, &R.S.sky);
-                fin = true;
+                if (fin) store_sample(F, P, pix, pbv, acc);
             }
-            if (fin) store_sample(F, P, pix, pbv, acc);
-        }
-        // queue places: continuing paths, shadow rays, pending ended paths, finished paths
-        const uint32_t m0 = __ballot_sync(0xffffffffu, cont), m1 = __ballot_sync(0xffffffffu, shadow),
-                       m2 = __ballot_sync(0xffffffffu, ended), m3 = __ballot_sync(0xffffffffu, fin);
-        if (lane == 0) {
-            s_cnt[0][wid] = (uint32_t)__popc(m0);
-            s_cnt[1][wid] = (uint32_t)__popc(m1);
-            s_cnt[2][wid] = (uint32_t)__popc(m2);
-            s_cnt[3][wid] = (uint32_t)__popc(m3);
+            append(cont, slot, T, L_CONT);
+            append(shadow, slot, T, L_SHADOW);
+            append(ended, slot, T, L_ENDED);
+            append(fin, slot, T, L_FIN);
         }
         __syncthreads();
-        uint32_t tot[4], off[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            tot[k] = off[k] = 0;
-#pragma unroll
-            for (uint32_t w = 0; w < kBlock / 32; ++w) {
-                if (w < wid) off[k] += s_cnt[k][w];
-                tot[k] += s_cnt[k][w];
-            }
-        }
+        // places in the queues; finished paths take the chunk's next paths and
+        // queue places after the continuing ones
+        const uint32_t n_cont = T.n[L_CONT], n_shadow = T.n[L_SHADOW], n_ended = T.n[L_ENDED], n_fin = T.n[L_FIN];
         if (tid == 0) {
             uint32_t go = 0;
             if (MODE == MODE_ADJOINT) {
-                s_base[3] = tot[3] ? atomicAdd(&cn[CTR_DONE], tot[3]) : 0u;
-            } else if (tot[3]) {
-                // finished paths take the chunk's next paths and queue places after the continuing ones
-                const uint32_t l = atomicAdd(F.path_ctr, tot[3]);
-                s_base[3] = l;
-                go = l < P.chunk_paths ? min(tot[3], P.chunk_paths - l) : 0u;
+                if (n_fin) T.base[L_FIN] = atomicAdd(&cn[CTR_DONE], n_fin);
+            } else if (n_fin) {
+                const uint32_t l = atomicAdd(F.path_ctr, n_fin);
+                T.base[L_FIN] = l;
+                go = l < P.chunk_paths ? min(n_fin, P.chunk_paths - l) : 0u;
                 if (go) atomicAdd(&cn[CTR_STARTED], go);
             }
-            if (tot[0] + go) s_base[0] = atomicAdd(&cn[CTR_EXT], tot[0] + go);
+            if (n_cont + go) T.base[L_CONT] = atomicAdd(&cn[CTR_EXT], n_cont + go);
         }
-        if (tid == 32 && tot[1]) s_base[1] = atomicAdd(&cn[CTR_SHADOW], tot[1]);
-        if (tid == 64 && tot[2]) s_base[2] = atomicAdd(&cn[CTR_ENDED], tot[2]);
+        if (tid == 32 && n_shadow) T.base[L_SHADOW] = atomicAdd(&cn[CTR_SHADOW], n_shadow);
+        if (tid == 64 && n_ended) T.base[L_ENDED] = atomicAdd(&cn[CTR_ENDED], n_ended);
         if (tid == 96 && nh) atomicAdd(&F.stats[8], (unsigned long long)nh);
         __syncthreads();
-        if (cont) qout[s_base[0] + off[0] + (uint32_t)__popc(m0 & lt)] = slot;
-        if (shadow) F.q[2][s_base[1] + off[1] + (uint32_t)__popc(m1 & lt)] = slot;
-        if (ended) qcout[s_base[2] + off[2] + (uint32_t)__popc(m2 & lt)] = slot;
-        if (fin) {
-            const uint32_t j = off[3] + (uint32_t)__popc(m3 & lt);
+        const uint32_t b0 = T.base[L_CONT], b1 = T.base[L_SHADOW], b2 = T.base[L_ENDED], b3 = T.base[L_FIN];
+        for (uint32_t j = tid; j < n_cont; j += kBlock) qout[b0 + j] = T.list[L_CONT][j];
+        for (uint32_t j = tid; j < n_shadow; j += kBlock) F.q[2][b1 + j] = T.list[L_SHADOW][j];
+        for (uint32_t j = tid; j < n_ended; j += kBlock) qcout[b2 + j] = T.list[L_ENDED][j];
+        for (uint32_t j = tid; j < n_fin; j += kBlock) {
+            const uint32_t slot = T.list[L_FIN][j];
             if (MODE == MODE_ADJOINT) {
-                F.q[5][s_base[3] + j] = slot;
-            } else if (s_base[3] + j < P.chunk_paths) {
-                start_path(F, P, slot, s_base[3] + j);
-                qout[s_base[0] + tot[0] + j] = slot;
+                F.q[5][b3 + j] = slot;
+            } else if (b3 + j < P.chunk_paths) {
+                start_path(F, P, slot, b3 + j);
+                qout[b0 + n_cont + j] = slot;
             }
         }
+        __syncthreads();
     }
 }
 

@@ -157,6 +157,7 @@ struct Frame {
     MrgState* cursor;    // light/path stream at the pixel's next chunk
     MrgState* jcursor;   // camera-jitter stream at the pixel's next chunk
     uint32_t* pscene;  // scene of each pixel
+    float2* halton;    // Halton light draw of each pixel (null when no scene of the frame uses it)
     float4* samples;   // sample of path l of the chunk (l = round_start[r] + pixel)
     float4* jpool;     // camera jitter of path l of the chunk
     MrgState* spool;   // light/path stream state at the start of path l of the chunk

@@ -52,6 +52,7 @@ constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign;
 constexpr size_t kV4 = align_up(sizeof(float4) * (size_t)kNoAllocMaxPixels);  // one float4 per slot / pixel
 constexpr size_t kRng = align_up(sizeof(MrgState) * (size_t)kNoAllocMaxPixels);  // MRG32k3a words per slot / pixel
 constexpr size_t kU32 = align_up(4 * (size_t)kNoAllocMaxPixels);              // one 32-bit word per pixel
+constexpr size_t kF2 = align_up(sizeof(float2) * (size_t)kNoAllocMaxPixels);  // one float2 per pixel
 constexpr size_t kCtr = align_up(4 * 32);
 constexpr size_t kStats = align_up(16 * 8);
 constexpr size_t kStatus = align_up(4);
@@ -60,11 +61,11 @@ constexpr size_t kSlots = align_up(kSlotBytes * (size_t)kNoAllocMaxPixels);  // 
 static_assert(kNoAllocMaxPixels % kSlotAlign == 0, "bind_slots alignment");
 // One slot per pixel and one path sample per pass: the per-slot state and
 // queues; per pixel the image, the
-// initial RNG states, the two stream cursors, the scene word, one sample,
+// initial RNG states, the two stream cursors, the scene word, the Halton draw, one sample,
 // one stream state and
 // one jitter value; counters, path counter, iteration, stats, status and the
 // scene record.
-constexpr size_t kScratchBytes = kSlots + kV4 + 4 * kRng + kU32 + 2 * kV4 + kCtr +
+constexpr size_t kScratchBytes = kSlots + kV4 + 4 * kRng + kU32 + kF2 + 2 * kV4 + kCtr +
                                  kCtr + kCtr + kStats + kStatus + kRec;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -98,6 +99,7 @@ Frame carve(unsigned char* base, int n, SceneRec** rec) {
     F.spool = (MrgState*)(base + off); off += kRng;
     F.jcursor = (MrgState*)(base + off); off += kRng;
     F.pscene = (uint32_t*)(base + off); off += kU32;
+    F.halton = (float2*)(base + off); off += kF2;
     F.samples = (float4*)(base + off); off += kV4;
     F.jpool = (float4*)(base + off); off += kV4;
     F.ctr = (uint32_t*)(base + off); off += kCtr;
