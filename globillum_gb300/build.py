@@ -72,7 +72,7 @@ def build_lib(force: bool = False, verbose_ptxas: bool = False) -> Path:
     # the library records the build-time defines it was made with
     # experimental compile options (GBPT_<name> in the environment -> -DGB_<name>)
     knobs = ("TRAV_MIN_BLOCKS", "SMEM_STACK", "PREFETCH", "SHADE_MIN_BLOCKS", "TRI_NOALLOC", "NODE_L2_128",
-             "REC_EVICT_FIRST", "NODE_FOLD", "NODE_L2_PERSIST", "TREE_WINDOW", "WIDE_GRID_DIV", "TRI_RATIO")
+             "REC_EVICT_FIRST", "NODE_L2_PERSIST", "TREE_WINDOW", "WIDE_GRID_DIV", "TRI_RATIO")
     flags = " ".join(f"GB_{k}={os.environ.get('GBPT_' + k, '')}" for k in knobs)
     stamp = LIB.with_suffix(".flags")
     if not stamp.exists() or stamp.read_text() != flags:

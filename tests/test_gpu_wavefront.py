@@ -71,3 +71,39 @@ def test_adjoint_pool_size_does_not_matter(gpu_ctx, slots):
     s.close()
     assert np.abs(ref).max() > 0
     assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("scale", [1e-4, 1.0, 3e7, 2e12])
+def test_axis_parallel_and_scaled_rays(gpu_ctx, scale):
+    """Node tests at the ends of their range: rays parallel to one or two axes
+    (inverse directions of 2^80), tiny and huge scenes, rays starting on a
+    node's plane; closest and any hits equal the oracle's brute force."""
+    from oracle import oracle
+    sc = scenes.icospheres(n_spheres=6, level=2, box=8.0, width=8, height=8, spp=1, max_bounces=1, n_lights=1)
+    sc.positions = (sc.positions.astype(np.float64) * scale).astype(np.float32)
+    rng = np.random.default_rng(5)
+    n = 6000
+    p = sc.positions.reshape(-1, 3)
+    tgt = p[rng.integers(0, p.shape[0], n)].astype(np.float64)
+    d = rng.normal(size=(n, 3))
+    k = rng.integers(0, 3, n)
+    r = np.arange(n)
+    d[r[: n // 2], k[: n // 2]] = 0.0                      # parallel to a plane
+    axis = np.zeros((n, 3))
+    axis[r, k] = rng.choice([-1.0, 1.0], n)
+    d[n // 2: 3 * n // 4] = axis[n // 2: 3 * n // 4]       # parallel to an axis
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = tgt - d * scale * rng.choice([0.0, 3.0, 40.0], n)[:, None]
+    o[:, 0] += rng.normal(size=n) * scale * 1e-3
+    o, d = o.astype(np.float32), d.astype(np.float32)
+    t = np.where(rng.uniform(size=n) < 0.5, 3.4e38, 10.0 * scale).astype(np.float32)
+    orc = oracle.OracleScene(sc, use_bvh=False)
+    s = gpu_ctx.scene(sc)
+    a, b = s.trace_closest(o, d, t), orc.trace_closest(o, d, t)
+    assert np.array_equal(a["ref"], b["ref"])
+    hit = b["ref"] != 0xFFFFFFFF
+    assert hit.mean() > 0.2
+    for f in ("t", "beta", "gamma"):
+        assert np.array_equal(a[f][hit].view(np.uint32), b[f][hit].view(np.uint32))
+    assert np.array_equal(s.trace_any(o, d, t) != 0, orc.trace_any(o, d, t) != 0)
+    s.close()
