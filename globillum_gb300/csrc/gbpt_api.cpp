@@ -149,7 +149,6 @@ struct gb_scene {
     std::vector<gb_light> lights;
     // device-built tree (GB_BVH_DEVICE_PLOC) and what a refit rewrites
     GpuBvh gbvh;
-    std::vector<int> material_index;
     void* shade_buf = nullptr;
     size_t tree_bytes = 0;  // host-built tree: nodes then triangles in one allocation at S.nodes
     std::vector<int> mat_dtex;  // diffuse texture of each material (-1 = none)
@@ -608,7 +607,6 @@ int gb_scene_create_ex(gb_ctx* ctx, const gb_scene_desc* d, const gb_build_optio
         pt = sc->gbvh.tris;
         bn = sc->gbvh.device_bytes;
         bt = 0;
-        sc->material_index.assign(d->material_index, d->material_index + n);
     }
     // a host-built tree is one allocation (nodes, then triangles at a
     // 256-byte boundary), so that one L2 access-policy window can cover it
@@ -744,21 +742,21 @@ int gb_scene_refit(gb_scene* scene, const float* positions, const float* normals
     if (scene->info.builder != GB_BVH_DEVICE_PLOC)
         return fail(ctx, GB_ERR_UNSUPPORTED, "refit needs a scene built with GB_BVH_DEVICE_PLOC");
     CK(cudaSetDevice(ctx->device));
-    CK(cudaStreamSynchronize(ctx->stream));  // frames in flight still read the old tree
-    const int n = scene->gbvh.n;
-    SceneAllocator SA(scene->allocs);
-    float* dpos = nullptr;
+    const int n = scene->gbvh.n;  // frames in flight read the old tree: the refit follows them on the stream
+    const size_t bytes = sizeof(float) * 9 * (size_t)n;
+    CK(ensure_scratch(ctx, 0, bytes));
+    CK(ensure_scratch(ctx, 1, normals ? bytes : 16));
+    CK(ensure_scratch(ctx, 2, refit_scratch_bytes(scene->gbvh)));
+    CK(cudaMemcpyAsync(ctx->scratch[0].p, positions, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (normals) CK(cudaMemcpyAsync(ctx->scratch[1].p, normals, bytes, cudaMemcpyHostToDevice, ctx->stream));
     std::string err;
-    cudaError_t e = SA.alloc((void**)&dpos, sizeof(float) * 9 * (size_t)n, false);
-    if (e == cudaSuccess) e = cudaMemcpy(dpos, positions, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = gpu_refit_cwbvh(dpos, SA, &scene->gbvh, &err, ctx->stream);
+    cudaError_t e = gpu_refit_cwbvh((const float*)ctx->scratch[0].p,
+                                    normals ? (const float*)ctx->scratch[1].p : nullptr, (float4*)scene->shade_buf,
+                                    ctx->scratch[2].p, &scene->gbvh, &err, ctx->stream);
     if (e != cudaSuccess) {
         if (e == cudaErrorInvalidValue && !err.empty()) return fail(ctx, GB_ERR_INVALID, "refit: " + err);
         return cuda_fail(ctx, e, "refit");
     }
-    std::vector<float> shade;
-    make_shade_records(positions, normals, scene->material_index.data(), n, &shade);
-    CK(cudaMemcpy(scene->shade_buf, shade.data(), sizeof(float) * shade.size(), cudaMemcpyHostToDevice));
     return GB_OK;
 }
 

@@ -63,8 +63,13 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
                             std::string* err, cudaStream_t st, bool sah_collapse = false, float prim_cost = 1.2f);
 
 // Recomputes the boxes of a built tree for moved vertices (same triangle
-// count and order) and rewrites nodes and triangle records in place.
-cudaError_t gpu_refit_cwbvh(const float* d_pos, DevAllocator& A, GpuBvh* bvh, std::string* err,
-                            cudaStream_t st);
+// count and order; d_pos 9 floats each) and rewrites nodes, triangle records
+// and shading records (d_shade, 6 float4 per triangle; d_nrm: 9 floats each, or
+// null for face normals) in place.  scratch: refit_scratch_bytes of device
+// memory.  Nothing is written when a vertex is not finite.  The stream is
+// synchronised on return.
+size_t refit_scratch_bytes(const GpuBvh& bvh);
+cudaError_t gpu_refit_cwbvh(const float* d_pos, const float* d_nrm, float4* d_shade, void* scratch, GpuBvh* bvh,
+                            std::string* err, cudaStream_t st);
 
 }  // namespace gb
