@@ -104,7 +104,7 @@ struct gb_ctx {
     size_t eval_mats_cap = 0, eval_lights_cap = 0;
     std::vector<ChunkGraph> graphs;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    uint32_t* d_status = nullptr;
+    uint32_t* d_status = nullptr;       // kernel status, then the queue head of gb_trace_*
     unsigned long long* d_stats = nullptr;
     gb_stats stats{};
     uint64_t launches = 0;              // launches outside the slot-pool iterations
@@ -384,7 +384,7 @@ int gb_ctx_create(const gb_ctx_desc* desc, gb_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_stats, sizeof(unsigned long long) * 16);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_stats, 0, sizeof(unsigned long long) * 16);
@@ -2078,7 +2078,7 @@ static int trace_common(gb_ctx* ctx, gb_scene* scene, int n, const float* orig, 
         d_h = (float4*)ctx->scratch[3].p;
         d_oc = (uint8_t*)ctx->scratch[3].p;
     }
-    CK(k_launch_trace(scene->S, n, d_o, d_d, d_t, d_h, d_oc, any, ctx->d_status, ctx->stream));
+    CK(k_launch_trace(scene->S, n, d_o, d_d, d_t, d_h, d_oc, any, ctx->d_status + 1, ctx->d_status, ctx->stream));
     if (!device_ptrs) {
         if (any) CK(cudaMemcpyAsync(occl, d_oc, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
         else CK(cudaMemcpyAsync(hits, d_h, sizeof(gb_hit) * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));

@@ -427,26 +427,6 @@ __device__ __forceinline__ void add_stats(unsigned long long* s, uint32_t v) {
 
 // ----------------------------------------------------------------- kernels
 
-__global__ void __launch_bounds__(kBlock) k_trace(DevScene S, int n, const float* __restrict__ orig,
-                                                  const float* __restrict__ dir, const float* __restrict__ tmaxv,
-                                                  float4* hits, uint8_t* occluded, int any, uint32_t* status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    v3 o = mk(orig[3 * i], orig[3 * i + 1], orig[3 * i + 2]);
-    v3 d = mk(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
-    float tmax = tmaxv[i];
-    RayInv r = make_ray(o, d);
-    if (any) {
-        bool f = (tmax >= 0.0f) && traverse<true>(S, r, tmax, nullptr, status);
-        occluded[i] = f ? 1 : 0;
-    } else {
-        TraceOut h;
-        if (tmax >= 0.0f) traverse<false>(S, r, tmax, &h, status);
-        else { h.t = FLT_MAX; h.beta = 0.0f; h.gamma = 0.0f; h.id = 0xffffffffu; }
-        hits[i] = make_float4(h.t, h.beta, h.gamma, __uint_as_float(h.id));
-    }
-}
-
 __device__ __forceinline__ v3 draw3(curandStateMRG32k3a* s) {
     float x = curand_uniform(s);
     float y = curand_uniform(s);
@@ -904,6 +884,41 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
             if (nidle == 32u || (!exhausted && nidle >= (uint32_t)refill)) break;
         }
     }
+}
+
+// gb_trace_closest / gb_trace_any: the caller's rays through the persistent
+// ray loop.  head: the queue head (zero), read only when there are more rays
+// than lanes in the grid.  A negative or NaN max_t traces nothing.
+#ifndef GB_TRACE_REFILL
+#define GB_TRACE_REFILL 12
+#endif
+__global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S, uint32_t n,
+                                                                      const float* __restrict__ orig,
+                                                                      const float* __restrict__ dir,
+                                                                      const float* __restrict__ tmaxv, float4* hits,
+                                                                      uint8_t* occluded, int any, uint32_t* head,
+                                                                      uint32_t* status) {
+    uint32_t nvis = 0, ntri = 0;
+    const uint32_t flag = any ? kAnyHit : 0u;
+    auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
+                     const float4** tris, const float4** shade) {
+        *handle = q | flag;
+        const float *po = orig + 3 * (size_t)q, *pd = dir + 3 * (size_t)q;
+        *o = mk(po[0], po[1], po[2]);
+        *d = mk(pd[0], pd[1], pd[2]);
+        const float t = tmaxv[q];
+        *tmax = t >= 0.0f ? t : -1.0f;
+        *nodes = S.nodes;
+        *tris = S.tris;
+        *shade = S.shade;
+    };
+    auto finish = [&](uint32_t handle, const Trav& h) {
+        const uint32_t i = handle & ~kAnyHit;
+        const bool hit = h.best_id != 0xffffffffu;
+        if (any) occluded[i] = hit ? 1 : 0;
+        else hits[i] = make_float4(hit ? h.best_t : FLT_MAX, h.bb, h.bg, __uint_as_float(h.best_id));
+    };
+    ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, fetch, finish, &nvis, &ntri);
 }
 
 // The rays of one iteration: the closest hit of every extension ray (to
@@ -1732,9 +1747,16 @@ inline int traversal_grid(const Grid& g, int blocks_per_sm, int bt = kBlock) {
 }  // namespace
 
 cudaError_t k_launch_trace(const DevScene& S, int n, const float* orig, const float* dir, const float* tmax,
-                           float4* hits, uint8_t* occluded, bool any, uint32_t* status, cudaStream_t st) {
+                           float4* hits, uint8_t* occluded, bool any, uint32_t* head, uint32_t* status,
+                           cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_trace<<<blocks_for(n), kBlock, 0, st>>>(S, n, orig, dir, tmax, hits, occluded, any ? 1 : 0, status);
+    static int g = persistent_blocks(k_trace);
+    if (n > g * kBlock) {
+        cudaError_t e = cudaMemsetAsync(head, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return e;
+    }
+    k_trace<<<std::min(g, blocks_for(n)), kBlock, 0, st>>>(S, (uint32_t)n, orig, dir, tmax, hits, occluded,
+                                                           any ? 1 : 0, head, status);
     return cudaGetLastError();
 }
 

@@ -220,7 +220,8 @@ struct RenderParams {
 };
 
 cudaError_t k_launch_trace(const DevScene& S, int n, const float* orig, const float* dir, const float* tmax,
-                           float4* hits, uint8_t* occluded, bool any, uint32_t* status, cudaStream_t st);
+                           float4* hits, uint8_t* occluded, bool any, uint32_t* head, uint32_t* status,
+                           cudaStream_t st);
 cudaError_t k_launch_frame_init(const Frame& F, bool rng, cudaStream_t st);
 cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cudaStream_t st);
 cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument, unsigned long long cond,
