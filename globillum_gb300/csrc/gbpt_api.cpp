@@ -28,6 +28,10 @@ struct DevBuf {
 static const int kSnaps = 16, kSnapWords = 3;
 static const size_t kMaxGraphs = 16;
 
+// Chunks of at most kPathsMax paths run in k_paths, the last kFinishMax paths of
+// larger ones in k_finish (measured at follow_paths).
+static const int kPathsMax = 1 << 18, kFinishMax = 1 << 16;
+
 // One scene of a frame as the host sees it.
 struct BatchScene {
     gb_scene* scene = nullptr;
@@ -1010,6 +1014,7 @@ int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, cudaGraphE
         e = cudaGraphAddNode(&loop, cg, deps, nullptr, nd, &np);
     }
     if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(a, &loop, nullptr, 1, cudaStreamSetCaptureDependencies);
+    if (e == cudaSuccess) e = k_launch_finish(F, P, a);
     if (e == cudaSuccess) e = k_launch_combine(F, P, a);
     cudaError_t e2 = cudaStreamEndCapture(a, &g);
     if (e == cudaSuccess) e = e2;
@@ -1069,6 +1074,7 @@ int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, cudaStream_t a,
             if (e == cudaSuccess) e = e2;
         }
     }
+    if (e == cudaSuccess) e = k_launch_finish(F, P, a);
     if (e == cudaSuccess) e = k_launch_combine(F, P, a);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "step graph chunk");
     return GB_OK;
@@ -1091,7 +1097,7 @@ int run_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart) {
         hit = ctx->graphs.size() - 1;
     }
     CK(cudaGraphLaunch(ctx->graphs[hit].exec, ctx->stream));
-    ctx->launches += 3;
+    ctx->launches += P.finish_max > 0 ? 4 : 3;
     return GB_OK;
 }
 
@@ -1162,6 +1168,11 @@ void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out)
     const int max_iters =
         (int)std::min<long long>(1ll << 30, 2 * ((acc * L1 + F.nslots - 1) / F.nslots + L1) + 16);
     P.max_iters = max_iters;
+    // whole paths by one thread each (k_paths, k_finish): forward frames with
+    // the default traversal, whose loop the device drives
+    if (ctx->mode == MODE_FORWARD && ctx->use_graph && !ctx->stage_timing && !ctx->instrument && P.tri_mode == 0 &&
+        ctx->stack_depth == 32)
+        P.finish_max = kFinishMax;
     *out = P;
     *nstart_out = nstart;
 }
@@ -1171,6 +1182,13 @@ int run_chunk(gb_ctx* ctx, int p0, int p1) {
     RenderParams P{};
     int nstart = 0;
     make_chunk(ctx, p0, p1, &P, &nstart);
+    if (P.finish_max > 0 && P.chunk_paths <= (uint32_t)kPathsMax) {
+        CK(k_launch_jitter_pool(ctx->F, P, ctx->stream));
+        CK(k_launch_paths(ctx->F, P, ctx->stream));
+        CK(k_launch_combine(ctx->F, P, ctx->stream));
+        ctx->launches += 3;
+        return GB_OK;
+    }
     if (ctx->use_graph && !ctx->stage_timing) return run_chunk_graph(ctx, P, nstart);
     return run_chunk_loop(ctx, P, nstart);
 }

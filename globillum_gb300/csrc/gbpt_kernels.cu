@@ -608,32 +608,45 @@ __device__ __forceinline__ void st_path(const Frame& F, uint32_t slot, v3 tp, v3
     rec_st(&F.strm[slot], Sector{{m.s1[0], m.s1[1], m.s1[2], m.s2[0], m.s2[1], m.s2[2], __float_as_uint(pend.z), 0u}});
 }
 
-__device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t l) {
+// Path l of the chunk: its pixel, scene, sample index and camera ray.
+struct PathStart {
+    uint32_t pix, sc, path;
+    int x, y;
+    v3 o, d;
+};
+__device__ __forceinline__ PathStart path_start(const Frame& F, const RenderParams& P, uint32_t l) {
     int lo = 0, hi = P.rounds - 1;
     while (lo < hi) {  // round holding path l
         int mid = (lo + hi + 1) >> 1;
         if (P.round_start[mid] <= l) lo = mid;
         else hi = mid - 1;
     }
-    const uint32_t gpix = l - P.round_start[lo];
-    const uint32_t sc = F.nscenes == 1 ? 0u : F.pscene[gpix];
-    const SceneRec& R = F.scenes[sc];
-    const uint32_t lp = gpix - R.pixel_base;
+    PathStart s;
+    s.pix = l - P.round_start[lo];
+    s.sc = F.nscenes == 1 ? 0u : F.pscene[s.pix];
+    s.path = (uint32_t)P.p0 + (uint32_t)lo;
+    const SceneRec& R = F.scenes[s.sc];
+    const uint32_t lp = s.pix - R.pixel_base;
     const float4* jp = F.jpool + P.round_start[lo];
-    float4 j = rec_ld(&jp[gpix]);
+    float4 j = rec_ld(&jp[s.pix]);
     float lx = 0.0f, ly = 0.0f;
     if (R.cam.aperture != 0.0f) {
         float4 lj = rec_ld(&jp[R.pixel_base + (lp + 17u) % (uint32_t)R.n]);
         lx = lj.z - 0.5f;
         ly = lj.y - 0.5f;
     }
-    const int x = (int)(lp % (uint32_t)R.w), y = (int)(lp / (uint32_t)R.w);
-    v3 o, d;
-    camera_ray(R.cam, x, y, j.x, j.y, lx, ly, &o, &d);
-    rec_st(&F.ray[slot], pack_sector(o, d, ((uint32_t)P.p0 + (uint32_t)lo) << 10, gpix));
+    s.x = (int)(lp % (uint32_t)R.w);
+    s.y = (int)(lp / (uint32_t)R.w);
+    camera_ray(R.cam, s.x, s.y, j.x, j.y, lx, ly, &s.o, &s.d);
+    return s;
+}
+
+__device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t l) {
+    const PathStart s = path_start(F, P, l);
+    rec_st(&F.ray[slot], pack_sector(s.o, s.d, s.path << 10, s.pix));
     st_path(F, slot, mk(1.0f, 1.0f, 1.0f), mk(0.0f, 0.0f, 0.0f), ld_mrg(F.spool, l), mk(0.0f, 0.0f, 0.0f));
     if (P.mode == MODE_FROZEN) F.tp0[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    if (P.textured && R.S.texcoord) st_rdiff(F, slot, camera_diff(R.cam, x, y));
+    if (P.textured && F.scenes[s.sc].S.texcoord) st_rdiff(F, slot, camera_diff(F.scenes[s.sc].cam, s.x, s.y));
 }
 
 // The scene of a pixel's paths; a frame of one scene needs no load.
@@ -921,6 +934,14 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
     ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, fetch, finish, &nvis, &ntri);
 }
 
+// Whether the chunk's loop stops before iteration `it` and leaves its queues
+// to k_finish: every path has started and few are alive.  k_rays decides and
+// notes it in F.iter[2]: path_ctr moves while k_shade runs.
+__device__ __forceinline__ bool left_to_finish(const Frame& F, const RenderParams& P, const uint32_t* cs) {
+    return P.finish_max > 0 && *F.path_ctr >= P.chunk_paths &&
+           cs[CTR_EXT] + cs[CTR_ENDED] <= (uint32_t)P.finish_max;
+}
+
 // The rays of one iteration: the closest hit of every extension ray (to
 // F.hit), then whether anything blocks every shadow ray (to F.occl).  Block 0
 // keeps the loop: it hands the iteration index to the kernels after it,
@@ -935,18 +956,25 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
     const int it = F.iter[0];
     uint32_t* cs = ctr_set(F, it);
     const uint32_t next = cs[CTR_EXT], nsh = cs[CTR_SHADOW];
+    const bool leave = left_to_finish(F, P, cs);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t work = next | nsh | cs[CTR_ENDED], started = cs[CTR_STARTED];
         F.iter[1] = it;
+        F.iter[2] = leave ? 1 : 0;
         uint32_t* c2 = ctr_set(F, it + 2);
         for (int k = 0; k < 8; ++k) c2[k] = 0u;
         F.stats[0] += started;
         F.stats[1] += next - started;
         F.stats[2] += nsh;
+        if (leave) {
+            if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
+            return;
+        }
         if (work) F.stats[7] += 1ull;
         if (work && it >= P.max_iters) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
         if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, work && it < P.max_iters ? 1u : 0u);
     }
+    if (leave) return;
     const uint32_t *qe = F.q[it & 1], *qs = F.q[2];
     uint32_t nvis = 0, ntri = 0, nvis_any = 0, ntri_any = 0;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
@@ -1009,16 +1037,14 @@ __device__ __forceinline__ MaterialRec load_material(const float* mats, uint32_t
 // Hit of a path in a textured scene: the ray differentials move to the hit
 // (computeRayDiffs, hybrid-pt.cpp:518-519) and a diffuse texture scales the
 // material's base colour.
-__device__ __noinline__ void texture_hit(const Frame& F, const SceneRec& R, uint32_t slot, uint32_t tid, float bb,
-                                         float bg, v3 Nr, MaterialRec* m) {
+__device__ __noinline__ void texture_hit(const SceneRec& R, uint32_t tid, float bb, float bg, v3 Nr, RayDiff* df,
+                                         MaterialRec* m) {
     const float4* sh = R.S.shade + 6 * (size_t)tid;
     const v3 a = ld3(__ldg(sh)), b = ld3(__ldg(sh + 1)), c = ld3(__ldg(sh + 2));
     const float* tcs = R.S.texcoord + 6 * (size_t)tid;
     float ts, tt;
     bary2(bb, bg, tcs, &ts, &tt);
-    RayDiff df = ld_rdiff(F, slot);
-    const float diff = ray_diff_hit(&df, a, b, c, tcs, ts, tt, normalize_div(Nr));
-    st_rdiff(F, slot, df);
+    const float diff = ray_diff_hit(df, a, b, c, tcs, ts, tt, normalize_div(Nr));
     if (m->dtex >= 0 && m->dtex < R.S.n_tex)
         *m = textured_material(*m, tex_sample_bilin_lod(R.S.tex[m->dtex], ts, tt, diff));
 }
@@ -1091,6 +1117,33 @@ __device__ __forceinline__ LightSample light_sample(const Frame& F, const SceneR
 // the sampling throughput in tp0; MODE_ADJOINT writes the vertex record of
 // the path-replay adjoint and leaves pb's bounce field = the number of
 // vertices the path shaded.
+// What shading a hit needs beside the path's state.
+struct Vertex {
+    v3 P, N;          // hit point, interpolated (unnormalised) normal
+    uint32_t mi;      // material
+    MaterialRec m;
+    LightSample ls;
+    v3 rnd;           // the bounce's draw
+};
+// Loads a hit's triangle, draws the bounce's uniforms, takes its light sample
+// and loads its material (df: the path's ray differentials, TEX only).
+template <bool TEX>
+__device__ __forceinline__ Vertex make_vertex(const Frame& F, const SceneRec& R, uint32_t pix, float bb, float bg,
+                                              uint32_t id, MrgState& st, RayDiff* df) {
+    Vertex v;
+    v.rnd = draw3(&st);
+    const float4* sh = R.S.shade + 6 * (size_t)id;
+    const float4 a = __ldg(sh), b = __ldg(sh + 1), c = __ldg(sh + 2);
+    v.P = bary(bb, bg, ld3(a), ld3(b), ld3(c));
+    v.N = bary(bb, bg, ld3(__ldg(sh + 3)), ld3(__ldg(sh + 4)), ld3(__ldg(sh + 5)));
+    v.ls = light_sample(F, R, pix, v.P, v.N, v.rnd);
+    v.mi = __float_as_uint(a.w);
+    const bool textured = TEX && R.S.texcoord != nullptr;
+    v.m = load_material(R.S.mats, v.mi, textured);
+    if (textured) texture_hit(R, id, bb, bg, v.N, df, &v.m);
+    return v;
+}
+
 // Shared memory of a shading block: the tile's entries and what became of
 // them.
 #ifndef GB_SHADE_TILE
@@ -1131,6 +1184,7 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
     const uint32_t tid = threadIdx.x, lane = lane_id(), lt = (1u << lane) - 1u;
     const uint32_t tile = shade_tile(count);
+    if (F.iter[2]) return;  // the loop is over: k_finish takes the queues
     if (blockIdx.x == 0 && tid == 0) F.iter[0] = it + 1;
     for (uint32_t base = blockIdx.x * tile; base < count; base += gridDim.x * tile) {
         if (tid < 6) T.n[tid] = 0;
@@ -1186,40 +1240,36 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
                 const SceneRec& R = F.scenes[sc];
                 if (hits) {
                     MrgState st{{ss.w[0], ss.w[1], ss.w[2]}, {ss.w[3], ss.w[4], ss.w[5]}};
-                    const v3 rnd = draw3(&st);
-                    const uint32_t id = __float_as_uint(hit.z);
-                    const float4* sh = R.S.shade + 6 * (size_t)id;
-                    const float4 a = __ldg(sh), b = __ldg(sh + 1), c = __ldg(sh + 2);
-                    const v3 Pp = bary(hit.x, hit.y, ld3(a), ld3(b), ld3(c));
-                    const v3 Nr = bary(hit.x, hit.y, ld3(__ldg(sh + 3)), ld3(__ldg(sh + 4)), ld3(__ldg(sh + 5)));
-                    const LightSample ls = light_sample(F, R, pix, Pp, Nr, rnd);
-                    const uint32_t mi = __float_as_uint(a.w);
+                    RayDiff df;
                     const bool textured = TEX && R.S.texcoord != nullptr;
-                    MaterialRec m = load_material(R.S.mats, mi, textured);
-                    if (textured) texture_hit(F, R, slot, id, hit.x, hit.y, Nr, &m);
+                    if (textured) df = ld_rdiff(F, slot);
+                    const Vertex v = make_vertex<TEX>(F, R, pix, hit.x, hit.y, __float_as_uint(hit.z), st, &df);
+                    if (textured) st_rdiff(F, slot, df);
+                    const LightSample& ls = v.ls;
                     const uint32_t path = pbv >> 10, lp = pix - R.pixel_base;
                     ShadeOut o;
                     if (MODE == MODE_FROZEN) {
-                        MaterialRec me = load_material(R.S.mats_eval, mi);
+                        MaterialRec me = load_material(R.S.mats_eval, v.mi);
                         v3 t0 = ld3(F.tp0[slot]);
-                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
-                                      &me, &t0);
+                        o = shade_hit(v.m, v.P, v.N, rd, tp, v.rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path,
+                                      bounce, &me, &t0);
                         F.tp0[slot] = make_float4(t0.x, t0.y, t0.z, 0.0f);
                     } else if (MODE == MODE_ADJOINT) {
                         ShadeTrace tr;
-                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce,
-                                      nullptr, nullptr, &tr);
+                        o = shade_hit(v.m, v.P, v.N, rd, tp, v.rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path,
+                                      bounce, nullptr, nullptr, &tr);
                         uint32_t info = (uint32_t)ls.light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
                                         (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
                         float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
                         rec[0] = make_float4(tp.x, tp.y, tp.z, tr.pdf);
                         rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
                         rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ls.scale : 0.0f);
-                        rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(mi));
+                        rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(v.mi));
                         rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
                         shadow = tr.nee;
                     } else {
-                        o = shade_hit(m, Pp, Nr, rd, tp, rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path, bounce);
+                        o = shade_hit(v.m, v.P, v.N, rd, tp, v.rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path,
+                                      bounce);
                     }
                     const v3 pend = o.accum_add;
                     if (MODE != MODE_ADJOINT) shadow = pend.x != 0.0f || pend.y != 0.0f || pend.z != 0.0f;
@@ -1276,6 +1326,165 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
         }
         __syncthreads();
     }
+}
+
+// ---------------------------------------------------------- whole paths --
+// Paths followed to their end by one thread each, with the operations of the
+// slot-pool loop in the same order per path: k_paths takes a small chunk from
+// the camera on, k_finish the paths a chunk has left when few are alive.
+// After a vertex the warp traces the lanes' shadow rays and next extension
+// rays together (a lane goes on to its extension ray as soon as its shadow ray
+// is done) and meets again to shade.
+//
+// A queue that does not fill the chip is bound by latency: each bounce costs
+// the loop two launches, a tail of long rays and a round trip of the path
+// state, whatever the work: 250 us for the 64x64 room at 1 and at 4 spp.
+// Wall time of a frame, loop against k_paths (us, paths in thousands):
+//   room      4K 249 / 153   48K 269 / 169   128K 312 / 267   256K 393 / 368   512K 569 / 628
+//   64 K tri  6K 393 / 215   48K 434 / 247   144K 493 / 336   250K 539 / 431
+//   512 K tri               48K 485 / 287   144K 536 / 440   225K 618 / 526
+// hence k_paths up to 2^18 paths.  The last paths of a chunk at 0 / 2^14 /
+// 2^15 / 2^16 / 2^17 / 2^18 alive: 1 spp of the 1M-triangle frame 1303 / 1187
+// / 1187 / 1097 / 1149 / 1146, textured sky 1231 / 1195 / 1113 / 1140 / 1131 /
+// 1151, 12 mixed scenes 3692 / 3635 / 3628 / 3632 / 3634 / 3594: 2^16.
+// 10 blocks of 64 per SM (102 registers): 1-3 % slower than with as many
+// registers as it likes below 64 K paths, up to 20 % faster above.
+#ifndef GB_PATHS_BLOCK
+#define GB_PATHS_BLOCK 64
+#endif
+#ifndef GB_PATHS_MIN
+#define GB_PATHS_MIN 10
+#endif
+struct PathState {
+    v3 o, d, tp, acc, pend;  // extension ray, throughput, accumulation, pending light sample
+    v3 so, sd;               // shadow ray of the pending light sample
+    float smax;
+    bool ext, shadow;        // rays to trace
+    int bounce;
+    uint32_t path, pix;
+    MrgState st;
+};
+
+// All 32 lanes call this; `alive` lanes have a path.  The sample goes to
+// *sample.
+template <bool TEX>
+__device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, bool alive, PathState& p, RayDiff& df,
+                                             float4* sample) {
+    uint32_t n_ext = 0, n_shadow = 0, n_hit = 0, nvis = 0, ntri = 0;
+    uint2 deep[kStack];
+    const StackRef stack{deep, deep, 1};
+    RayInv r;
+    Trav s;
+    while (__any_sync(0xffffffffu, alive)) {
+        bool act = alive, any = p.shadow, occl = false;
+        if (act) {
+            r = any ? make_ray(p.so, p.sd) : make_ray(p.o, p.d);
+            trav_init(s, r, any ? p.smax : FLT_MAX);
+        }
+        int steps = 0;
+        while (__any_sync(0xffffffffu, act)) {
+            bool done = warp_step<false, kStack>(act, R.S.nodes, R.S.tris, r, any, s, stack, F.status, &nvis, &ntri);
+            if (++steps > kIterLimit) {
+                if (act) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
+                done = act;
+            }
+            if (done && any) {
+                occl = s.best_id != 0xffffffffu;
+                any = false;
+                act = p.ext;
+                if (act) {
+                    r = make_ray(p.o, p.d);
+                    trav_init(s, r, FLT_MAX);
+                }
+            } else if (done) {
+                act = false;
+            }
+        }
+        if (alive) {
+            if (p.shadow && !occl) p.acc = p.acc + p.pend;
+            p.shadow = false;
+            bool end = true;
+            if (p.ext && s.best_id != 0xffffffffu) {
+                ++n_hit;
+                const Vertex v = make_vertex<TEX>(F, R, p.pix, s.bb, s.bg, s.best_id, p.st, &df);
+                const ShadeOut o = shade_hit(v.m, v.P, v.N, p.d, p.tp, v.rnd, v.ls.smax >= 0.0f, v.ls.sd, v.ls.psc,
+                                             R.sp, p.pix - R.pixel_base, p.path, p.bounce);
+                p.pend = o.accum_add;
+                p.shadow = p.pend.x != 0.0f || p.pend.y != 0.0f || p.pend.z != 0.0f;
+                p.so = v.ls.so;
+                p.sd = v.ls.sd;
+                p.smax = v.ls.smax;
+                p.ext = o.alive && p.bounce + 1 < R.L;
+                p.o = o.org;
+                p.d = o.dir;
+                p.tp = o.tp;
+                ++p.bounce;
+                n_ext += p.ext ? 1u : 0u;
+                n_shadow += p.shadow ? 1u : 0u;
+                end = !p.ext && !p.shadow;
+            } else if (p.ext) {
+                p.acc = p.acc + miss_contribution(p.tp, p.d, R.sp, &R.S.sky);
+            }
+            if (end) {
+                rec_st(sample, make_float4(p.acc.x, p.acc.y, p.acc.z, 0.0f));
+                alive = false;
+                p.ext = false;
+            }
+        }
+    }
+    add_stats(&F.stats[1], n_ext);
+    add_stats(&F.stats[2], n_shadow);
+    add_stats(&F.stats[8], n_hit);
+}
+
+template <bool TEX>
+__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P) {
+    const uint32_t l = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
+    const bool alive = l < P.chunk_paths;
+    const PathStart ps = path_start(F, P, alive ? l : 0u);
+    const SceneRec& R = F.scenes[ps.sc];
+    const v3 z = mk(0.0f, 0.0f, 0.0f);
+    PathState p{ps.o, ps.d, mk(1.0f, 1.0f, 1.0f), z, z, z, z, 0.0f, alive, false, 0, ps.path, ps.pix,
+                ld_mrg(F.spool, alive ? l : 0u)};
+    RayDiff df;
+    if (TEX && R.S.texcoord) df = camera_diff(R.cam, ps.x, ps.y);
+    add_stats(&F.stats[0], alive ? 1u : 0u);
+    follow_paths<TEX>(F, R, alive, p, df, F.samples + l);
+}
+
+template <bool TEX>
+__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F, RenderParams P) {
+    const int it = F.iter[0];
+    const uint32_t* cs = ctr_set(F, it);
+    const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
+    const uint32_t i = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
+    if ((i & ~31u) >= count) return;
+    const bool alive = i < count;
+    const uint32_t k = alive ? i : 0u;
+    const uint32_t slot = k < ne ? F.q[it & 1][k] : F.q[3 + (it & 1)][k - ne];
+    const Sector rs = rec_ld(&F.ray[slot]), ps = rec_ld(&F.path[slot]), ss = rec_ld(&F.strm[slot]);
+    const SceneRec& R = F.scenes[scene_of(F, rs.w[7])];
+    PathState p;
+    p.o = sec3(rs, 0);
+    p.d = sec3(rs, 3);
+    p.tp = sec3(ps, 0);
+    p.acc = sec3(ps, 3);
+    p.pend = mk(__uint_as_float(ps.w[6]), __uint_as_float(ps.w[7]), __uint_as_float(ss.w[6]));
+    p.ext = alive && k < ne;
+    p.shadow = alive && (p.pend.x != 0.0f || p.pend.y != 0.0f || p.pend.z != 0.0f);
+    p.bounce = (int)(rs.w[6] & 1023u);
+    p.path = rs.w[6] >> 10;
+    p.pix = rs.w[7];
+    p.st = MrgState{{ss.w[0], ss.w[1], ss.w[2]}, {ss.w[3], ss.w[4], ss.w[5]}};
+    if (p.shadow) {
+        const Sector sh = rec_ld(&F.shray[slot]);
+        p.so = sec3(sh, 0);
+        p.sd = sec3(sh, 3);
+        p.smax = __uint_as_float(sh.w[6]);
+    }
+    RayDiff df;
+    if (TEX && R.S.texcoord) df = ld_rdiff(F, slot);
+    follow_paths<TEX>(F, R, alive, p, df, F.samples + P.round_start[p.path - (uint32_t)P.p0] + p.pix);
 }
 
 // Path-replay adjoint of every path that finished this iteration (done queue,
@@ -1928,6 +2137,21 @@ cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t s
     if (P.mode != MODE_ADJOINT) return cudaSuccess;  // paths restart in k_shade
     static int g0 = persistent_blocks(k_regen);
     k_regen<<<stream_grid(g0, F.nslots), kBlock, 0, st>>>(F, P);
+    return cudaGetLastError();
+}
+
+cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t st) {
+    const unsigned grid = (P.chunk_paths + GB_PATHS_BLOCK - 1) / GB_PATHS_BLOCK;
+    if (P.textured) k_paths<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
+    else k_paths<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
+    return cudaGetLastError();
+}
+
+cudaError_t k_launch_finish(const Frame& F, const RenderParams& P, cudaStream_t st) {
+    if (P.finish_max <= 0) return cudaSuccess;
+    const unsigned grid = ((unsigned)std::min(P.finish_max, F.nslots) + GB_PATHS_BLOCK - 1) / GB_PATHS_BLOCK;
+    if (P.textured) k_finish<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
+    else k_finish<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
     return cudaGetLastError();
 }
 

@@ -165,7 +165,8 @@ struct Frame {
     uint32_t* ctr;     // 3 sets of 8 (by iteration % 3), see CTR_*
     uint32_t* path_ctr;  // next path of the chunk to start
     int* iter;         // iteration index of the chunk's slot-pool loop: [0] as k_rays reads it (k_shade moves it
-                       // on), [1] as the kernels after it read it (k_rays copies it there)
+                       // on), [1] as the kernels after it read it (k_rays copies it there); [2] 1 = the loop has stopped
+                       // for k_finish
     unsigned long long* stats;  // 0 camera, 1 ext, 2 shadow rays; 3/4 closest, 5/6 shadow node visits / tri tests;
                                 // 7 iterations; 8 closest hits (light samples); 16 words
     uint32_t* status;
@@ -210,6 +211,7 @@ struct RenderParams {
     int textured;      // some scene of the frame has textures (k_shade's texture variant, Frame::rdiff)
     int p0, rounds;    // path samples p0 .. p0+rounds-1
     int max_iters;     // iteration bound of the chunk's loop
+    int finish_max;    // the loop leaves the chunk's last paths to k_finish once at most this many are alive (0: never)
     // L2 window of the traversal launches (GB_NODE_L2_PERSIST, frames of one
     // scene): the scene's node array, accessed as persisting
     const void* l2_nodes;
@@ -227,6 +229,8 @@ cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cu
 cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument, unsigned long long cond,
                           bool has_cond, cudaStream_t st);
 cudaError_t k_launch_shade(const Frame& F, const RenderParams& P, cudaStream_t st);
+cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t st);
+cudaError_t k_launch_finish(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_jitter_pool(const Frame& F, const RenderParams& P, cudaStream_t st);
 cudaError_t k_launch_combine(const Frame& F, const RenderParams& P, cudaStream_t st);

@@ -1,8 +1,10 @@
-"""The slot-pool loop at the sizes where its queues can go wrong: path counts
-around the shading tile (128) and a warp, pools far smaller than the frame,
+"""The slot-pool loop (host-driven, graph = 1) and the kernels that follow whole
+paths (k_paths for small chunks, k_finish for the last paths of a chunk's
+graph, graph = 2) at the sizes where they can go wrong: path counts around a
+warp, a block and the shading tile, pools far smaller than the frame,
 one-bounce paths (every path ends with its light sample still pending), a
-scene without lights, and every lobe of the principled room.  Frames and
-gradients equal those of the oracle / of another pool size."""
+scene without lights, every lobe of the principled room, textures with a sky.
+Frames and gradients equal those of the oracle / of the other driver."""
 import numpy as np
 import pytest
 
@@ -28,15 +30,47 @@ def _against_oracle(ctx, sc, rd):
 @pytest.mark.parametrize("w,h,spp,slots", [(1, 1, 1, 1), (31, 1, 1, 0), (127, 1, 1, 0), (43, 3, 1, 0), (16, 16, 3, 129),
                                            (33, 31, 5, 100), (64, 65, 2, 4097)])
 @pytest.mark.parametrize("bounces", [1, 2, 7])
-def test_path_counts_and_pools(gpu_ctx, w, h, spp, slots, bounces):
+@pytest.mark.parametrize("graph", [1, 2])
+def test_path_counts_and_pools(gpu_ctx, w, h, spp, slots, bounces, graph):
     sc = scenes.principled_room(width=w, height=h, spp=spp, max_bounces=bounces, rr_start=3)
     old = gpu_ctx.get_tuning()
     try:
+        gpu_ctx.set_tuning(graph=graph)
         if slots:
             gpu_ctx.set_tuning(slots=slots)
         _against_oracle(gpu_ctx, sc, sc.render)
     finally:
-        gpu_ctx.set_tuning(slots=old["slots"])
+        gpu_ctx.set_tuning(slots=old["slots"], graph=old["graph"])
+
+
+@pytest.mark.parametrize("w,h,spp,slots", [(512, 512, 1, 0), (513, 512, 1, 0), (300, 310, 3, 5000), (257, 129, 16, 0)])
+@pytest.mark.parametrize("kind", ["room", "textured"])
+def test_finish_of_a_chunk(gpu_ctx, w, h, spp, slots, kind):
+    """Chunks at and above the 2^18 paths of k_paths: the graph's loop leaves
+    its last paths to k_finish; the host-driven loop does not.  Same frames,
+    same ray counts."""
+    if kind == "room":
+        sc = scenes.principled_room(width=w, height=h, spp=spp, max_bounces=5, rr_start=1)
+    else:
+        sc = scenes.with_textures(scenes.icospheres(n_spheres=30, level=2, box=12.0, width=w, height=h, spp=spp,
+                                                    max_bounces=4, n_lights=1), scale=0.2)
+        sc.lights.append({"type": gbpt.GB_LIGHT_SKY, "map": scenes.procedural_sky(32, 16), "scale": 0.5,
+                          "diameter": 30.0, "power": -1.0})
+        sc.camera.update(aperture=0.2, focus_distance=8.0)
+    s = gpu_ctx.scene(sc)
+    old = gpu_ctx.get_tuning()
+    out = []
+    try:
+        for graph in (1, 2):
+            gpu_ctx.set_tuning(graph=graph, **({"slots": slots} if slots else {}))
+            img = s.render(sc.camera, sc.render)
+            st = gpu_ctx.stats()
+            out.append((img, [st[k] for k in ("camera_rays", "extension_rays", "shadow_rays", "light_samples")]))
+    finally:
+        gpu_ctx.set_tuning(graph=old["graph"], slots=old["slots"])
+        s.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert out[0][1] == out[1][1] and out[0][1][0] == w * h * spp
 
 
 def test_no_lights_and_dark_light(gpu_ctx):
