@@ -704,6 +704,37 @@ GB_HD double pow22(double x) {
     return ldexp(q, (int)kf);
 }
 
+#ifdef __CUDACC__
+// (float)pow22((double)x) on the device.  pow22 is some 280 double operations,
+// of which an SM does 2 a clock, for each of a texture sample's three
+// channels.  Here x^2.2 = x^2 * x^(1/5) in pairs of floats: the fifth root
+// starts from exp2(log2(x) / 5) (relative error below 2^-19), its residual
+// x - y^5 is formed exactly enough by fmaf and the series of (1 + r)^(1/5) to
+// r^2 corrects it, so the product (h, l) is within 2^-40 of x^2.2.  If
+// moving it by 2^-39 either way rounds to the same float, that is the float
+// pow22 rounds to as well (pow22 is within 2^-46); else, and outside
+// [2^-20, 2^20], pow22 itself decides (Ziv 1991, "Fast evaluation of elementary
+// mathematical functions with correctly rounded last bit").  Equal to
+// (float)pow22 for every float of that range.
+static __device__ __noinline__ float pow22_slow(float x) { return (float)pow22((double)x); }
+__device__ __forceinline__ float pow22_float(float x) {
+    if (x == 0.0f) return 0.0f;
+    if (!(x >= 9.5367431640625e-07f && x <= 1048576.0f)) return pow22_slow(x);
+    const float y = exp2f(0.2f * log2f(x));
+    const float h2 = y * y, l2 = fmaf(y, y, -h2);
+    const float h4 = h2 * h2, l4 = fmaf(h2, h2, -h4) + 2.0f * (h2 * l2);
+    const float h5 = h4 * y, l5 = fmaf(h4, y, -h5) + l4 * y;
+    const float r = ((x - h5) - l5) / h5;            // x / y^5 - 1
+    const float t = 0.2f * r * (1.0f - 0.4f * r);    // (1 + r)^(1/5) - 1
+    const float xh = x * x, xl = fmaf(x, x, -xh);
+    const float h = xh * y;
+    const float l = fmaf(xh, y, -h) + (xh * (y * t) + xl * y);
+    const float e = h * 1.8189894035458565e-12f;     // 2^-39
+    const float a = h + (l - e), b = h + (l + e);
+    return a == b ? a : pow22_slow(x);
+}
+#endif
+
 enum { MAT_LAMBERT = 0, MAT_PRINCIPLED = 1 };
 struct MaterialRec {
     int kind;
@@ -743,7 +774,7 @@ GB_HD void material_colour_terms(MaterialRec* r, const float* c, bool own_pow) {
     for (int k = 0; k < 3; ++k) {
         r->diffuse[k] = c[k];
 #ifdef __CUDA_ARCH__
-        cdlin[k] = (float)pow22((double)c[k]);
+        cdlin[k] = pow22_float(c[k]);
         (void)own_pow;
 #else
         cdlin[k] = own_pow ? (float)pow22((double)c[k]) : (float)pow((double)c[k], 2.2);
