@@ -427,24 +427,6 @@ __device__ __forceinline__ void add_stats(unsigned long long* s, uint32_t v) {
 
 // ----------------------------------------------------------------- kernels
 
-__device__ __forceinline__ v3 draw3(curandStateMRG32k3a* s) {
-    float x = curand_uniform(s);
-    float y = curand_uniform(s);
-    float z = curand_uniform(s);
-    return mk(x, y, z);
-}
-
-// MrgState <-> curandStateMRG32k3a (the Box-Muller caches are unused by
-// uniform draws and start cleared, as after curand_init).
-__device__ __forceinline__ curandStateMRG32k3a mrg_expand(const MrgState& m) {
-    curandStateMRG32k3a st;
-    for (int k = 0; k < 3; ++k) { st.s1[k] = m.s1[k]; st.s2[k] = m.s2[k]; }
-    st.boxmuller_flag = 0;
-    st.boxmuller_flag_double = 0;
-    st.boxmuller_extra = 0.0f;
-    st.boxmuller_extra_double = 0.0;
-    return st;
-}
 __device__ __forceinline__ MrgState mrg_pack(const curandStateMRG32k3a& st) {
     MrgState m;
     for (int k = 0; k < 3; ++k) { m.s1[k] = st.s1[k]; m.s2[k] = st.s2[k]; }
@@ -464,11 +446,17 @@ __device__ __forceinline__ void st_mrg(MrgState* base, size_t i, const MrgState&
     rec_st(q + 1, make_uint2(m.s1[2], m.s2[0]));
     rec_st(q + 2, make_uint2(m.s2[1], m.s2[2]));
 }
+// Three uniforms of a stream: the numbers curand_uniform gives (equal for all
+// 2^32 - 209 values of z and for four draws from each of 2^30 pseudo-random
+// states), with the recurrences in integers and three double operations a
+// draw (an SM does two double operations a clock): k_jitter_pool of the 256x256
+// 16-spp room 43 -> 25 us (with mrg_apply reducing rows), of 12 mixed scenes
+// 262 -> 163 us.
 __device__ __forceinline__ v3 draw3(MrgState* m) {
-    curandStateMRG32k3a st = mrg_expand(*m);
-    v3 r = draw3(&st);
-    *m = mrg_pack(st);
-    return r;
+    const float x = mrg_uniform(mrg_next(m->s1, m->s2));
+    const float y = mrg_uniform(mrg_next(m->s1, m->s2));
+    const float z = mrg_uniform(mrg_next(m->s1, m->s2));
+    return mk(x, y, z);
 }
 
 // The state curand_init(seed, sub, 0) leaves: curand_init of subsequence 0
@@ -1637,7 +1625,7 @@ __global__ void __launch_bounds__(kBlock) k_direct(DevScene S, CameraRec cam, in
             mcol = mcol * tex_sample_bilin_lod(S.tex[dtex], ts, tt, diff);
         }
     }
-    curandStateMRG32k3a st = mrg_expand(mrg_stream(T, seed, (uint32_t)g));
+    MrgState st = mrg_stream(T, seed, (uint32_t)g);
     v3 rnd = draw3(&st);
     v3 buf_dir = d;
     v3 acc = mk(0.0f, 0.0f, 0.0f);
@@ -1689,9 +1677,9 @@ __global__ void __launch_bounds__(kBlock) k_direct_hybrid(DevScene S, CameraRec 
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= w * h) return;
     const int px = g % w, py = g / w;
-    curandStateMRG32k3a js = mrg_expand(mrg_stream(T, seed, (uint32_t)g)), ls = js, lens;
+    MrgState js = mrg_stream(T, seed, (uint32_t)g), ls = js, lens;
     const bool aperture = cam.aperture != 0.0f;
-    if (aperture) lens = mrg_expand(mrg_stream(T, seed, (uint32_t)((g + 17) % (w * h))));
+    if (aperture) lens = mrg_stream(T, seed, (uint32_t)((g + 17) % (w * h)));
     const int L = light_samples;
     v3 acc = mk(0.0f, 0.0f, 0.0f);
     for (int c = 0; c < cam_samples; ++c) {
@@ -1829,11 +1817,10 @@ __global__ void k_mrg_pool(int pixel0, int npix, uint32_t seed, int first_update
     if (i >= npix) return;
     curandStateMRG32k3a s;
     curand_init((unsigned long long)seed, (unsigned long long)(uint32_t)(pixel0 + i), 0ull, &s);
-    for (int u = 0; u < first_update; ++u) (void)draw3(&s);
+    for (int u = 0; u < 3 * first_update; ++u) (void)curand_uniform(&s);
     for (int u = 0; u < num_updates; ++u) {
-        v3 r = draw3(&s);
         size_t o = ((size_t)u * npix + i) * 3;
-        out[o] = r.x; out[o + 1] = r.y; out[o + 2] = r.z;
+        for (int k = 0; k < 3; ++k) out[o + k] = curand_uniform(&s);
     }
 }
 

@@ -225,12 +225,20 @@ GB_HD uint32_t mrg_reduce(uint64_t x, uint32_t c, uint32_t m) {
     return (uint32_t)x;
 }
 
+// s = J s mod m.  The three products of a row are summed to 66 bits and
+// reduced once (2^32 = c, 2^64 = c^2 mod m): hi c + lo + carry c^2 < 2^48, one
+// more fold leaves less than 2^32 + 2^31 < 2 m.  Reducing every product by
+// itself, each with a loop of subtractions, was 60 % of k_jitter_pool.
 GB_HD void mrg_apply(uint32_t s[3], const uint32_t* J, uint32_t c, uint32_t m) {
     uint32_t r[3];
     for (int i = 0; i < 3; ++i) {
-        uint64_t acc = 0;
-        for (int j = 0; j < 3; ++j) acc += mrg_reduce((uint64_t)J[3 * i + j] * s[j], c, m);
-        r[i] = mrg_reduce(acc, c, m);  // acc < 3 m
+        const uint64_t p0 = (uint64_t)J[3 * i] * s[0], p1 = (uint64_t)J[3 * i + 1] * s[1],
+                       p2 = (uint64_t)J[3 * i + 2] * s[2];
+        const uint64_t a = p0 + p1, b = a + p2;
+        const uint32_t carry = (a < p0 ? 1u : 0u) + (b < p2 ? 1u : 0u);
+        uint64_t x = (b >> 32) * c + (uint32_t)b + (uint64_t)(carry * (c * c));
+        x = (x >> 32) * c + (uint32_t)x;
+        r[i] = (uint32_t)(x >= m ? x - m : x);
     }
     s[0] = r[0]; s[1] = r[1]; s[2] = r[2];
 }
@@ -294,6 +302,26 @@ GB_HD void mrg_jump(uint32_t s1[3], uint32_t s2[3], const uint32_t* J1, const ui
     mrg_apply(s1, J1, 209u, kMrgM1);
     mrg_apply(s2, J2, 22853u, kMrgM2);
 }
+
+// One step of both recurrences and the combined value z = (x_n - y_n) mod m1
+// in 1 .. m1 (L'Ecuyer 1999), in 64-bit integers: -a x is taken as a (m - x),
+// so the sums stay below 2^54, and 2^32 = c (mod m) folds the high word in
+// (once for m1: 2214308 * 209 < 2^29; twice for m2), leaving less than 2 m.
+GB_HD uint32_t mrg_next(uint32_t s1[3], uint32_t s2[3]) {
+    uint64_t x = 1403580ull * s1[1] + 810728ull * (kMrgM1 - s1[0]);
+    x = (x >> 32) * 209u + (uint32_t)x;
+    const uint32_t p1 = (uint32_t)(x >= kMrgM1 ? x - kMrgM1 : x);
+    uint64_t y = 527612ull * s2[2] + 1370589ull * (kMrgM2 - s2[0]);
+    y = (y >> 32) * 22853u + (uint32_t)y;
+    y = (y >> 32) * 22853u + (uint32_t)y;
+    const uint32_t p2 = (uint32_t)(y >= kMrgM2 ? y - kMrgM2 : y);
+    s1[0] = s1[1]; s1[1] = s1[2]; s1[2] = p1;
+    s2[0] = s2[1]; s2[1] = s2[2]; s2[2] = p2;
+    return p1 > p2 ? p1 - p2 : p1 - p2 + kMrgM1;
+}
+
+// z / m1 in (0, 1].
+GB_HD float mrg_uniform(uint32_t z) { return (float)((double)z * (1.0 / 4294967087.0)); }
 
 // ----------------------------------------------------------------- camera --
 // Per-frame constants of setup_jittered_dof_shirley (raygen.cu:61-118); the
