@@ -36,12 +36,11 @@ namespace gb {
 namespace {
 
 constexpr int kBlock = 128;
-// Resident 128-thread blocks per SM the traversal kernels are compiled for:
-// 7 (72 registers, 28 warps per SM) measured fastest on the 1 M-triangle
-// frame (8 blocks spill more; the compiler's own choice of 80 registers
-// gives 6 blocks).
+// Resident 128-thread blocks per SM the traversal kernels are compiled for: 8
+// (64 registers).  1M-triangle frame, 64 spp, at 7 / 8 / 9 blocks: 37.6 / 37.1 /
+// 38.2 ms; 2 M shadow rays 333 / 321 / 348 us.
 #ifndef GB_TRAV_MIN_BLOCKS
-#define GB_TRAV_MIN_BLOCKS 7
+#define GB_TRAV_MIN_BLOCKS 8
 #endif
 constexpr int kStack = 32;
 constexpr int kIterLimit = 1 << 22;
@@ -148,12 +147,30 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     return d;
 }
 
+// The visit order of a node's hit children is a permutation of its 8-bit hit
+// mask by the ray's octant: a 2 KB table in shared memory (2 instructions)
+// instead of three conditional swaps (15): 38.0 -> 37.1 ms on the 1M-triangle
+// 64-spp frame, 333 -> 321 us on 2 M shadow rays.
+__device__ __forceinline__ uint8_t* order_table() {
+    __shared__ __align__(4) uint8_t t[2048];  // [octant][mask]
+    return t;
+}
 // Bits of an 8-bit mask moved from position i to i ^ x (x in 0..7).
 __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t x) {
     if (x & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
     if (x & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
     if (x & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
     return m;
+}
+
+// Fills order_table: all threads of the block call it before they traverse.
+__device__ __forceinline__ void fill_order_table() {
+    uint32_t* t = reinterpret_cast<uint32_t*>(order_table());
+    for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) {
+        const uint32_t x = i >> 6, m = (i & 63u) << 2, w = xor_permute8(m, x), b0 = 1u << x, b1 = 1u << (x ^ 1u);
+        t[i] = w | (w | b0) << 8 | (w | b1) << 16 | (w | b0 | b1) << 24;
+    }
+    __syncthreads();
 }
 
 // Intersects the 8 children of node `ni`; returns the node group (child
@@ -253,7 +270,7 @@ __device__ __forceinline__ void intersect_node(const float4* __restrict__ nodes,
         asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(cp + 4)));
     }
 #endif
-    *ng = make_uint2(__float_as_uint(n1.x), (xor_permute8(inner, r.oxor) << 24) | imask);
+    *ng = make_uint2(__float_as_uint(n1.x), ((uint32_t)order_table()[(r.oxor << 8) | inner] << 24) | imask);
     *tg = make_uint2(__float_as_uint(n1.y), hits_t);
 }
 
@@ -293,13 +310,20 @@ __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const 
     const float4* tp = tris + 3 * (size_t)(s.tg.x + (uint32_t)b);
     float4 a0 = ld_tri(tp + 0), a1 = ld_tri(tp + 1), a2 = ld_tri(tp + 2);
     if (INSTR) ++*ntri;
-    float t, u, v;
-    if (intersect_tri(r.o, r.d, ld3(a0), ld3(a1), ld3(a2), &t, &u, &v)) {
-        uint32_t id = __float_as_uint(a0.w);
-        if (closer(t, id, s.best_t, s.best_id)) {
-            s.best_t = t; s.best_id = id; s.bb = u; s.bg = v;
-            return any;
-        }
+    // intersect_tri with its conditions joined at the end (the same operations;
+    // det = 0 gives u = inf or NaN, which is no hit either): no branch to
+    // reconverge between the steps, 38.4 -> 37.8 ms on the 1M-triangle frame
+    const v3 e1 = ld3(a1), e2 = ld3(a2);
+    const v3 p = fcross(r.d, e2);
+    const float inv = 1.0f / fdot(e1, p);
+    const v3 w = r.o - ld3(a0);
+    const float u = fdot(w, p) * inv;
+    const v3 q = fcross(w, e1);
+    const float v = fdot(r.d, q) * inv, t = fdot(e2, q) * inv;
+    const uint32_t id = __float_as_uint(a0.w);
+    if (u >= 0.0f && u <= 1.0f && v >= 0.0f && u + v <= 1.0f && t > 0.0f && closer(t, id, s.best_t, s.best_id)) {
+        s.best_t = t; s.best_id = id; s.bb = u; s.bg = v;
+        return any;
     }
     return false;
 }
@@ -352,34 +376,40 @@ __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, cons
 // tests triangles) on the 1M-triangle 64-spp frame: 51.0 / 50.0 / 50.0 /
 // 50.1 / 50.5 ms for 1 / 2 / 3 / 4 / 6, 1.84 / 1.82 / 1.84 / 1.85 / 1.89 ms
 // at 1 spp; every pending triangle after each visit, with pops as steps of
-// their own: 55.4 and 2.05 ms.  Returns true when the lane's ray is finished.
+// their own: 55.4 and 2.05 ms.  A lane is finished when it has neither, so the
+// two votes of the step also tell which lanes are idle.
 #ifndef GB_TRI_RATIO
 #define GB_TRI_RATIO 2
 #endif
+__device__ __forceinline__ bool has_tri(const Trav& s) { return s.tg.y != 0u; }
+__device__ __forceinline__ bool has_node(const Trav& s) { return s.nt.y == 0u && (s.ng.y > 0x00ffffffu || s.sp > 0); }
+// A lane without a ray, or whose any-hit query is answered, has neither.
+__device__ __forceinline__ void trav_stop(Trav& s) {
+    s.tg.y = s.nt.y = s.ng.y = 0u;
+    s.sp = 0;
+}
 template <bool INSTR, int STACK>
-__device__ __forceinline__ bool warp_step(bool act, const float4* __restrict__ nodes, const float4* __restrict__ tris,
+__device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint32_t mn,
+                                          const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                           const RayInv& r, bool any, Trav& s, const StackRef& stack,
                                           uint32_t* status, uint32_t* nvis, uint32_t* ntri) {
-    const bool tri = act && s.tg.y != 0u;
-    const bool node = act && s.nt.y == 0u && (s.ng.y > 0x00ffffffu || s.sp > 0);
-    const int lt = __popc(__ballot_sync(0xffffffffu, tri)), ln = __popc(__ballot_sync(0xffffffffu, node));
-    bool done = false;
-    if (lt * GB_TRI_RATIO >= ln) {
+    if (__popc(mt) * GB_TRI_RATIO >= __popc(mn)) {
         if (tri) {
-            done = tri_step<INSTR>(tris, r, any, s, ntri);
+            const bool found = tri_step<INSTR>(tris, r, any, s, ntri);
             if (s.tg.y == 0u) {
                 s.tg = s.nt;
                 s.nt.y = 0u;
             }
+            if (found) trav_stop(s);
         }
     } else if (node) {
         if (s.ng.y <= 0x00ffffffu) s.ng = stack_get(stack, --s.sp);
         uint2 tg = make_uint2(0u, 0u);
-        done = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg);
+        const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg);
         if (s.tg.y == 0u) s.tg = tg;
         else s.nt = tg;
+        if (over) trav_stop(s);
     }
-    return done || (act && s.tg.y == 0u && s.ng.y <= 0x00ffffffu && s.sp == 0);
 }
 
 // Whole traversal of one ray without warp cooperation.
@@ -801,6 +831,7 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
     uint32_t hd = 0;  // the lane's handle for finish, as fetch sets it
     RayInv r;
     Trav s;
+    trav_stop(s);
     __shared__ uint2 s_stack[kSmemStack > 0 ? kSmemStack * BT : 1];
     uint2 deep[STACK - kSmemStack];
     const StackRef stack{s_stack + threadIdx.x, deep, BT};
@@ -842,6 +873,25 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
         if (!__any_sync(0xffffffffu, act)) break;
         const bool any = (hd & kAnyHit) != 0u;
         int steps = 0;
+        if (MODE == 0) {
+            bool tri, node;
+            while (true) {
+                tri = has_tri(s);
+                node = has_node(s);
+                const uint32_t mt = __ballot_sync(0xffffffffu, tri), mn = __ballot_sync(0xffffffffu, node);
+                const int live = __popc(mt | mn);
+                if (live == 0 || (!exhausted && live <= 32 - refill)) break;
+                if (++steps > kIterLimit) {
+                    if (act) atomicOr(status, ST_ITER_LIMIT);
+                    trav_stop(s);
+                    continue;
+                }
+                warp_step<INSTR, STACK>(tri, node, mt, mn, nodes, tris, r, any, s, stack, status, nvis, ntri);
+            }
+            fin = act && !tri && !node;
+            act = tri || node;
+            continue;
+        }
         while (true) {
             bool done = false;
             if (MODE == 3) {
@@ -849,8 +899,6 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
                 // each lane visits one node
                 const bool hit = coop_triangles<INSTR>(act, tris, shade, r, any, s, skey, ntri);
                 if (act) done = (any && hit) || node_step<INSTR, STACK>(nodes, r, s, stack, status, nvis);
-            } else if (MODE == 0) {
-                done = warp_step<INSTR, STACK>(act, nodes, tris, r, any, s, stack, status, nvis, ntri);
             } else {
                 // triangle postponing: when fewer than a fifth of the active
                 // lanes have triangles pending, those lanes stack their
@@ -899,6 +947,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
                                                                       const float* __restrict__ tmaxv, float4* hits,
                                                                       uint8_t* occluded, int any, uint32_t* head,
                                                                       uint32_t* status) {
+    fill_order_table();
     uint32_t nvis = 0, ntri = 0;
     const uint32_t flag = any ? kAnyHit : 0u;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
@@ -963,6 +1012,7 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
         if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, work && it < P.max_iters ? 1u : 0u);
     }
     if (leave) return;
+    fill_order_table();
     const uint32_t *qe = F.q[it & 1], *qs = F.q[2];
     uint32_t nvis = 0, ntri = 0, nvis_any = 0, ntri_any = 0;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
@@ -1364,29 +1414,34 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
     RayInv r;
     Trav s;
     while (__any_sync(0xffffffffu, alive)) {
-        bool act = alive, any = p.shadow, occl = false;
-        if (act) {
+        bool any = alive && p.shadow, occl = false;
+        if (alive) {
             r = any ? make_ray(p.so, p.sd) : make_ray(p.o, p.d);
             trav_init(s, r, any ? p.smax : FLT_MAX);
         }
+        else trav_stop(s);
         int steps = 0;
-        while (__any_sync(0xffffffffu, act)) {
-            bool done = warp_step<false, kStack>(act, R.S.nodes, R.S.tris, r, any, s, stack, F.status, &nvis, &ntri);
-            if (++steps > kIterLimit) {
-                if (act) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
-                done = act;
-            }
-            if (done && any) {
+        while (true) {
+            const bool tri = has_tri(s);
+            bool node = has_node(s);
+            if (any && !tri && !node) {  // the shadow ray is done
                 occl = s.best_id != 0xffffffffu;
                 any = false;
-                act = p.ext;
-                if (act) {
+                if (p.ext) {
                     r = make_ray(p.o, p.d);
                     trav_init(s, r, FLT_MAX);
+                    node = true;
                 }
-            } else if (done) {
-                act = false;
             }
+            const uint32_t mt = __ballot_sync(0xffffffffu, tri), mn = __ballot_sync(0xffffffffu, node);
+            if ((mt | mn) == 0u) break;
+            if (++steps > kIterLimit) {
+                if (tri || node) atomicOr(F.status, (uint32_t)ST_ITER_LIMIT);
+                any = false;
+                trav_stop(s);
+                continue;
+            }
+            warp_step<false, kStack>(tri, node, mt, mn, R.S.nodes, R.S.tris, r, any, s, stack, F.status, &nvis, &ntri);
         }
         if (alive) {
             if (p.shadow && !occl) p.acc = p.acc + p.pend;
@@ -1427,6 +1482,7 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
 
 template <bool TEX>
 __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P) {
+    fill_order_table();
     const uint32_t l = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
     const bool alive = l < P.chunk_paths;
     const PathStart ps = path_start(F, P, alive ? l : 0u);
@@ -1445,6 +1501,8 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F
     const int it = F.iter[0];
     const uint32_t* cs = ctr_set(F, it);
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
+    if (blockIdx.x * GB_PATHS_BLOCK >= count) return;
+    fill_order_table();
     const uint32_t i = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
     if ((i & ~31u) >= count) return;
     const bool alive = i < count;
@@ -1600,6 +1658,7 @@ __global__ void __launch_bounds__(kBlock) k_adjoint(Frame F, RenderParams P) {
 __global__ void __launch_bounds__(kBlock) k_direct(DevScene S, CameraRec cam, int w, int h, int samples,
                                                    uint32_t seed, float shadow_offset, v3 background, float* out,
                                                    uint32_t* status, const MrgSubseqTable T) {
+    fill_order_table();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= w * h) return;
     v3 o, d;
@@ -1674,6 +1733,7 @@ __global__ void __launch_bounds__(kBlock) k_direct_hybrid(DevScene S, CameraRec 
                                                           int light_samples, uint32_t seed, float shadow_offset,
                                                           v3 background, float* out, uint32_t* status,
                                                           const MrgSubseqTable T) {
+    fill_order_table();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= w * h) return;
     const int px = g % w, py = g / w;
