@@ -26,7 +26,7 @@ struct DevBuf {
 };
 
 static const int kSnaps = 16, kSnapWords = 3;
-static const size_t kMaxGraphs = 16;
+static const size_t kMaxGraphs = 16, kStatWords = 16;
 
 // Chunks of at most kPathsMax paths run in k_paths, the last kFinishMax paths of
 // larger ones in k_finish (measured at follow_paths).
@@ -108,8 +108,9 @@ struct gb_ctx {
     size_t eval_mats_cap = 0, eval_lights_cap = 0;
     std::vector<ChunkGraph> graphs;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    unsigned long long* d_stats = nullptr;  // kernel counters (kStatWords), then d_status
     uint32_t* d_status = nullptr;       // kernel status, then the queue head of gb_trace_*
-    unsigned long long* d_stats = nullptr;
+    unsigned long long* h_stats = nullptr;  // pinned copy of both (kStatWords + 1 words)
     gb_stats stats{};
     uint64_t launches = 0;              // launches outside the slot-pool iterations
     bool stage_timing = false;
@@ -332,10 +333,13 @@ int check_render_desc(gb_ctx* ctx, const gb_camera* cam, const gb_render_desc* d
     return GB_OK;
 }
 
+// Waits for the stream and reports the kernels' status; the counters arrive in
+// ctx->h_stats with the same copy.
 int check_status(gb_ctx* ctx) {
-    uint32_t st = 0;
-    CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(unsigned long long) * (kStatWords + 1),
+                       cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const uint32_t st = (uint32_t)ctx->h_stats[kStatWords];
     if (st) {
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
         return fail(ctx, GB_ERR_TRAVERSAL,
@@ -388,10 +392,11 @@ int gb_ctx_create(const gb_ctx_desc* desc, gb_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, 2 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_stats, sizeof(unsigned long long) * 16);
-    if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(ctx->d_stats, 0, sizeof(unsigned long long) * 16);
+    const size_t stat_bytes = sizeof(unsigned long long) * (kStatWords + 1);
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_stats, stat_bytes);
+    if (e == cudaSuccess) e = cudaMemset(ctx->d_stats, 0, stat_bytes);
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->h_stats, stat_bytes, cudaHostAllocDefault);
+    if (ctx->d_stats) ctx->d_status = (uint32_t*)(ctx->d_stats + kStatWords);
     if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->snap_host, sizeof(uint32_t) * kSnaps * kSnapWords, cudaHostAllocDefault);
     for (int k = 0; k < kSnaps && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ctx->snap_ev[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -425,7 +430,7 @@ void gb_ctx_destroy(gb_ctx* ctx) {
     if (ctx->snap_host) cudaFreeHost(ctx->snap_host);
     for (int k = 0; k < kSnaps; ++k) if (ctx->snap_ev[k]) cudaEventDestroy(ctx->snap_ev[k]);
     if (ctx->d_rgb) cudaFree(ctx->d_rgb);
-    if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
     if (ctx->d_stats) cudaFree(ctx->d_stats);
     if (ctx->l2_persist) {
         // give back the persisting L2 set-aside this context asked for
@@ -800,12 +805,11 @@ int chunk_end(const gb_ctx* ctx, int p0, int end, long long* paths) {
 
 // The device part of starting a frame, on stream `st`: counters, the scene
 // records (copied from `recs`, ctx->recs.size() of them), the layout's
-// initial RNG states when the layout changed, and both stream cursors of
-// every pixel reset to them.  Captured into the fitting graph as well.
+// initial RNG states when the layout changed (k_jitter_pool starts a frame's
+// streams from them).  Captured into the fitting graph as well.
 int enqueue_frame_setup(gb_ctx* ctx, cudaStream_t st, const SceneRec* recs, bool record_start) {
     const Frame& F = ctx->F;
-    CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(unsigned long long) * 16, st));
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), st));
+    CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(unsigned long long) * (kStatWords + 1), st));  // counters and status
     if (record_start) CK(cudaEventRecord(ctx->ev0, st));
     CK(cudaMemcpyAsync(ctx->d_scenes, recs, sizeof(SceneRec) * ctx->recs.size(), cudaMemcpyHostToDevice, st));
     // F.pscene, F.halton and the initial RNG states depend on the pixel counts,
@@ -819,9 +823,6 @@ int enqueue_frame_setup(gb_ctx* ctx, cudaStream_t st, const SceneRec* recs, bool
         ctx->launches += 2;
         ctx->pristine_key = key;
     }
-    // both streams of every pixel restart at curand_init(seed, pixel, 0)
-    CK(cudaMemcpyAsync(F.cursor, F.pristine, sizeof(MrgState) * (size_t)F.ntot, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(F.jcursor, F.pristine, sizeof(MrgState) * (size_t)F.ntot, cudaMemcpyDeviceToDevice, st));
     return GB_OK;
 }
 
@@ -1224,12 +1225,13 @@ int ensure_rgb(gb_ctx* ctx) {
     return GB_OK;
 }
 
-// Packs the frame's colours into RGB triples (device scratch of 3 * ntot floats).
-int pack_frame(gb_ctx* ctx) {
-    int rc = ensure_rgb(ctx);
+// Packs the frame's colours into RGB triples: at `dst`, or in the device
+// scratch of 3 * ntot floats.
+int pack_frame(gb_ctx* ctx, float* dst = nullptr) {
+    int rc = dst ? GB_OK : ensure_rgb(ctx);
     if (rc != GB_OK) return rc;
     if (ctx->paths_done == 0) CK(cudaMemsetAsync(ctx->F.out, 0, sizeof(float4) * (size_t)ctx->F.ntot, ctx->stream));
-    CK(k_launch_pack_rgb(ctx->F.out, ctx->F.ntot, ctx->d_rgb, ctx->stream));
+    CK(k_launch_pack_rgb(ctx->F.out, ctx->F.ntot, dst ? dst : ctx->d_rgb, ctx->stream));
     ctx->launches += 1;
     return GB_OK;
 }
@@ -1243,9 +1245,9 @@ int copy_scene(gb_ctx* ctx, const BatchScene& b, float* out, int out_is_device) 
 
 // Waits for the frame, gathers its statistics and reports kernel status.
 int finish_frame(gb_ctx* ctx) {
-    CK(cudaStreamSynchronize(ctx->stream));
-    unsigned long long st[16];
-    CK(cudaMemcpy(st, ctx->d_stats, sizeof(st), cudaMemcpyDeviceToHost));
+    const int rc = check_status(ctx);
+    if (rc != GB_OK && rc != GB_ERR_TRAVERSAL) return rc;
+    const unsigned long long* st = ctx->h_stats;
     ctx->stats.camera_rays = st[0];
     ctx->stats.extension_rays = st[1];
     ctx->stats.shadow_rays = st[2];
@@ -1269,7 +1271,7 @@ int finish_frame(gb_ctx* ctx) {
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) ctx->stats.render_ms = ms;
     cudaGetLastError();
-    return check_status(ctx);
+    return rc;
 }
 
 }  // namespace
@@ -1297,8 +1299,14 @@ int gb_render_read(gb_ctx* ctx, float* out_rgb, int out_is_device) {
     if (!out_rgb) return fail(ctx, GB_ERR_INVALID, "null output");
     if (ctx->items.size() != 1) return fail(ctx, GB_ERR_INVALID, "gb_render_read reads single-scene renders");
     CK(cudaSetDevice(ctx->device));
-    int rc = pack_frame(ctx);
-    if (rc == GB_OK) rc = copy_scene(ctx, ctx->items[0], out_rgb, out_is_device);
+    // an image in this device's memory is packed in place; any other pointer
+    // that a copy can reach is copied to
+    cudaPointerAttributes at{};
+    const bool here = out_is_device && cudaPointerGetAttributes(&at, out_rgb) == cudaSuccess &&
+                      at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+    cudaGetLastError();
+    int rc = pack_frame(ctx, here ? out_rgb : nullptr);
+    if (rc == GB_OK && !here) rc = copy_scene(ctx, ctx->items[0], out_rgb, out_is_device);
     if (rc != GB_OK) return rc;
     return finish_frame(ctx);
 }
@@ -1712,11 +1720,7 @@ int fit_build(gb_ctx* ctx) {
     for (int pass = 0; pass < 2 && rc == GB_OK; ++pass) {
         ctx->mode = pass == 0 ? MODE_FORWARD : MODE_ADJOINT;
         if (pass == 1) {
-            // the adjoint replays the same paths: both streams of every pixel restart
-            e = cudaMemcpyAsync(F.cursor, F.pristine, sizeof(MrgState) * (size_t)F.ntot, cudaMemcpyDeviceToDevice, a);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(F.jcursor, F.pristine, sizeof(MrgState) * (size_t)F.ntot, cudaMemcpyDeviceToDevice, a);
-            if (e == cudaSuccess) e = cudaMemsetAsync(F.grad, 0, sizeof(float) * (size_t)f.replicas * (size_t)f.stride, a);
+            e = cudaMemsetAsync(F.grad, 0, sizeof(float) * (size_t)f.replicas * (size_t)f.stride, a);
             if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "step graph adjoint set-up"); break; }
         }
         for (int p0 = 0; p0 < ctx->max_spp && rc == GB_OK;) {

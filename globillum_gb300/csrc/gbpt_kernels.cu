@@ -580,8 +580,9 @@ __global__ void k_jitter_pool(Frame F, RenderParams P) {
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= F.ntot) return;
     const SceneRec& R = F.scenes[F.nscenes == 1 ? 0u : F.pscene[g]];
-    MrgState s = ld_mrg(F.jcursor, (size_t)g);
-    MrgState c = ld_mrg(F.cursor, (size_t)g);
+    // a frame starts at curand_init(seed, pixel, 0), a later chunk where the last one ended
+    MrgState s = ld_mrg(P.p0 == 0 ? F.pristine : F.jcursor, (size_t)g);
+    MrgState c = ld_mrg(P.p0 == 0 ? F.pristine : F.cursor, (size_t)g);
     const int pe = min(P.p0 + P.rounds, R.spp);
     for (int p = P.p0; p < pe; ++p) {
         const uint32_t l = P.round_start[p - P.p0] + (uint32_t)g;

@@ -200,8 +200,6 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     if (e == cudaSuccess) e = cudaMemsetAsync(F.stats, 0, 16 * 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(F.status, 0, 4, st);
     if (e == cudaSuccess) e = k_launch_frame_init(F, true, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(F.cursor, F.pristine, sizeof(MrgState) * (size_t)n, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(F.jcursor, F.pristine, sizeof(MrgState) * (size_t)n, cudaMemcpyDeviceToDevice, st);
     // one path sample of every pixel per pass, one slot per pixel: a path
     // has at most max_bounces segments and its last light sample is settled
     // one iteration later, so the queues are empty after max_bounces + 1
