@@ -412,42 +412,6 @@ __device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint
     }
 }
 
-// Whole traversal of one ray without warp cooperation.
-template <bool ANY>
-__device__ __forceinline__ bool trav_step(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                          const RayInv& r, Trav& s, const StackRef& stack, uint32_t* status) {
-    uint32_t nvis = 0, ntri = 0;
-    while (s.tg.y != 0u)
-        if (tri_step<false>(tris, r, ANY, s, &ntri)) return true;
-    return node_step<false>(nodes, r, s, stack, status, &nvis);
-}
-
-struct TraceOut {
-    float t, beta, gamma;
-    uint32_t id;
-};
-
-// Whole traversal of one ray (API tracing kernel).
-template <bool ANY>
-__device__ __forceinline__ bool traverse(const DevScene& S, const RayInv& r, float tmax, TraceOut* out,
-                                         uint32_t* status) {
-    Trav s;
-    trav_init(s, r, tmax);
-    uint2 lstack[kStack];
-    const StackRef stack{lstack, lstack + kSmemStack, 1};
-    int iters = 0;
-    while (!trav_step<ANY>(S.nodes, S.tris, r, s, stack, status)) {
-        if (++iters > kIterLimit) { atomicOr(status, ST_ITER_LIMIT); break; }
-    }
-    if (out) {
-        out->t = s.best_id != 0xffffffffu ? s.best_t : FLT_MAX;
-        out->beta = s.bb;
-        out->gamma = s.bg;
-        out->id = s.best_id;
-    }
-    return s.best_id != 0xffffffffu;
-}
-
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ void add_stats(unsigned long long* s, uint32_t v) {
@@ -1656,68 +1620,7 @@ __global__ void __launch_bounds__(kBlock) k_adjoint(Frame F, RenderParams P) {
 // (the pool advances after the second sample is set up).  A missed pixel's
 // psc is the scaled sky texel of the direction its ray buffer holds: the
 // camera ray's for the first sample, (0, 0, 0) afterwards.
-__global__ void __launch_bounds__(kBlock) k_direct(DevScene S, CameraRec cam, int w, int h, int samples,
-                                                   uint32_t seed, float shadow_offset, v3 background, float* out,
-                                                   uint32_t* status, const MrgSubseqTable T) {
-    fill_order_table();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= w * h) return;
-    v3 o, d;
-    camera_ray(cam, g % w, g / w, 0.5f, 0.5f, 0.0f, 0.0f, &o, &d);
-    TraceOut hit;
-    const bool is_hit = traverse<false>(S, make_ray(o, d), FLT_MAX, &hit, status);
-    v3 P = mk(0.0f, 0.0f, 0.0f), N = P, mcol = background;
-    if (is_hit) {
-        const float4* sh = S.shade + 6 * (size_t)hit.id;
-        const float4 a = sh[0];
-        P = bary(hit.beta, hit.gamma, ld3(a), ld3(sh[1]), ld3(sh[2]));
-        N = bary(hit.beta, hit.gamma, ld3(sh[3]), ld3(sh[4]), ld3(sh[5]));
-        const float* mf = S.mats + (size_t)kMaterialFloats * __float_as_uint(a.w);
-        mcol = mk(mf[25], mf[26], mf[27]);
-        const int dtex = (int)mf[31];
-        if (S.texcoord && dtex >= 0 && dtex < S.n_tex) {
-            // pixel_evaluate_material_bilin_lod_cpu (material-cpu.cpp:36-77)
-            const float* tcs = S.texcoord + 6 * (size_t)hit.id;
-            float ts, tt;
-            bary2(hit.beta, hit.gamma, tcs, &ts, &tt);
-            RayDiff df = camera_diff(cam, g % w, g / w);
-            const float diff = ray_diff_hit(&df, ld3(a), ld3(sh[1]), ld3(sh[2]), tcs, ts, tt, N);
-            mcol = mcol * tex_sample_bilin_lod(S.tex[dtex], ts, tt, diff);
-        }
-    }
-    MrgState st = mrg_stream(T, seed, (uint32_t)g);
-    v3 rnd = draw3(&st);
-    v3 buf_dir = d;
-    v3 acc = mk(0.0f, 0.0f, 0.0f);
-    for (int k = 0; k < samples; ++k) {
-        if (k >= 2) rnd = draw3(&st);
-        v3 weight = mk(0.0f, 0.0f, 0.0f);
-        bool occluded = false;
-        if (is_hit && S.n_lights > 0) {
-            const int l = pick_light(S.lights, S.n_lights, S.overall_power, rnd.z);
-            const LightRec L = S.lights[l];
-            v3 so, sd;
-            float smax;
-            if (L.type == 1)
-                sky_light_sample_uniform(S.sky, L.power, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so,
-                                         &sd, &smax, &weight);
-            else
-                rect_light_sample(L, L.col, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so, &sd, &smax,
-                                  &weight, nullptr, false);
-            buf_dir = sd;
-            occluded = smax >= 0.0f && traverse<true>(S, make_ray(so, sd), smax, nullptr, status);
-        } else {
-            if (S.sky.light >= 0) weight = S.sky.scale * sky_eval(S.sky, buf_dir);
-            buf_dir = mk(0.0f, 0.0f, 0.0f);
-        }
-        const v3 mat = occluded ? mk(0.0f, 0.0f, 0.0f) : mcol;
-        acc = (float(k) * acc + weight * mat) / (float(k) + 1.0f);
-    }
-    out[3 * g] = acc.x;
-    out[3 * g + 1] = acc.y;
-    out[3 * g + 2] = acc.z;
-}
-
+//
 // hybrid_area_lights (direct-lighting.cpp:203-316, direct-lighting.h:137-215):
 // per pixel `cam_samples` jittered camera rays (jittered lens generator,
 // jitter pool update c), the material colour of each camera hit
@@ -1730,78 +1633,160 @@ __global__ void __launch_bounds__(kBlock) k_direct(DevScene S, CameraRec cam, in
 // L-th update of each camera sample goes unused.  All pools are seeded
 // alike in the reference (curand_init(0, pixel, 0), util-kernels.cu:276-285),
 // so the jitter and light draws are one stream read twice.
-__global__ void __launch_bounds__(kBlock) k_direct_hybrid(DevScene S, CameraRec cam, int w, int h, int cam_samples,
-                                                          int light_samples, uint32_t seed, float shadow_offset,
-                                                          v3 background, float* out, uint32_t* status,
-                                                          const MrgSubseqTable T) {
+//
+// Both (HYBRID: the second): a thread per pixel.  Light samples are taken
+// kDirectGroup at a time: all their shadow rays are set up together, each lane
+// traces its own one after the other while the warp steps together
+// (warp_step), and the samples are then averaged in order, so that the warp
+// waits for its slowest lane once a group and not once a ray.  A sample whose
+// weight is exactly zero traces nothing (its term is zero either way while the
+// colour is finite).  641x359, 64 K triangles, hybrid 2 x 8 / 2 x 2; 1280x720,
+// 384 K triangles, 16 samples (us with the image to the host): a ray at a time
+// per thread 1446 / 642 / 4594; groups of 4 / 8 / 16 at 10 blocks of 64 per SM
+// 962 476 3522 / 952 482 3470 / 950 479 5225; of 8 at 12 / 14 / 16 blocks 926
+// 471 3267 / 923 470 3275 / 906 468 3210, but 200x150 frames 172 / 161 / 173.
+// The loops over a group stay rolled: unrolled, the code leaves the
+// instruction cache (1190 us).
+#ifndef GB_DIRECT_GROUP
+#define GB_DIRECT_GROUP 8
+#endif
+#ifndef GB_DIRECT_BLOCK
+#define GB_DIRECT_BLOCK 64
+#endif
+#ifndef GB_DIRECT_MIN
+#define GB_DIRECT_MIN 14
+#endif
+constexpr int kDirectGroup = GB_DIRECT_GROUP;
+template <bool HYBRID>
+__global__ void __launch_bounds__(GB_DIRECT_BLOCK, GB_DIRECT_MIN) k_direct(
+    DevScene S, CameraRec cam, int w, int h, int cam_samples, int light_samples, uint32_t seed, float shadow_offset,
+    v3 background, float* out, uint32_t* status, const MrgSubseqTable T) {
     fill_order_table();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= w * h) return;
+    const int g0 = blockIdx.x * GB_DIRECT_BLOCK + threadIdx.x;
+    const bool mine = g0 < w * h;
+    const int g = mine ? g0 : 0;  // idle threads of the last block trace nothing
     const int px = g % w, py = g / w;
-    MrgState js = mrg_stream(T, seed, (uint32_t)g), ls = js, lens;
-    const bool aperture = cam.aperture != 0.0f;
+    MrgState js = mrg_stream(T, seed, (uint32_t)g), ls = js, lens = js;
+    const bool aperture = HYBRID && cam.aperture != 0.0f;
     if (aperture) lens = mrg_stream(T, seed, (uint32_t)((g + 17) % (w * h)));
     const int L = light_samples;
+    uint2 deep[kStack];
+    const StackRef stack{deep, deep, 1};
+    Trav t;
+    RayInv r;
+    uint32_t nvis = 0, ntri = 0;
     v3 acc = mk(0.0f, 0.0f, 0.0f);
     for (int c = 0; c < cam_samples; ++c) {
-        const v3 j = draw3(&js);
-        float lx = 0.0f, ly = 0.0f;
-        if (aperture) {
-            const v3 lj = draw3(&lens);
-            lx = lj.z - 0.5f;
-            ly = lj.y - 0.5f;
-        }
         v3 o, d;
-        camera_ray(cam, px, py, j.x, j.y, lx, ly, &o, &d);
-        TraceOut hit;
-        const bool is_hit = traverse<false>(S, make_ray(o, d), FLT_MAX, &hit, status);
+        if (HYBRID) {
+            const v3 j = draw3(&js);
+            float lx = 0.0f, ly = 0.0f;
+            if (aperture) {
+                const v3 lj = draw3(&lens);
+                lx = lj.z - 0.5f;
+                ly = lj.y - 0.5f;
+            }
+            camera_ray(cam, px, py, j.x, j.y, lx, ly, &o, &d);
+        } else {
+            camera_ray(cam, px, py, 0.5f, 0.5f, 0.0f, 0.0f, &o, &d);
+        }
+        r = make_ray(o, d);
+        trav_init(t, r, FLT_MAX);
+        if (!mine) trav_stop(t);
+        for (int steps = 0;;) {
+            const bool tri = has_tri(t), node = has_node(t);
+            const uint32_t mt = __ballot_sync(0xffffffffu, tri), mn = __ballot_sync(0xffffffffu, node);
+            if ((mt | mn) == 0u) break;
+            if (++steps > kIterLimit) { atomicOr(status, (uint32_t)ST_ITER_LIMIT); trav_stop(t); continue; }
+            warp_step<false, kStack>(tri, node, mt, mn, S.nodes, S.tris, r, false, t, stack, status, &nvis, &ntri);
+        }
+        const bool is_hit = mine && t.best_id != 0xffffffffu;
         v3 P = mk(0.0f, 0.0f, 0.0f), N = P, mcol = background;
         if (is_hit) {
-            const float4* sh = S.shade + 6 * (size_t)hit.id;
+            const float4* sh = S.shade + 6 * (size_t)t.best_id;
             const float4 a = sh[0];
-            P = bary(hit.beta, hit.gamma, ld3(a), ld3(sh[1]), ld3(sh[2]));
-            N = bary(hit.beta, hit.gamma, ld3(sh[3]), ld3(sh[4]), ld3(sh[5]));
+            P = bary(t.bb, t.bg, ld3(a), ld3(sh[1]), ld3(sh[2]));
+            N = bary(t.bb, t.bg, ld3(sh[3]), ld3(sh[4]), ld3(sh[5]));
             const float* mf = S.mats + (size_t)kMaterialFloats * __float_as_uint(a.w);
             mcol = mk(mf[25], mf[26], mf[27]);
             const int dtex = (int)mf[31];
             if (S.texcoord && dtex >= 0 && dtex < S.n_tex) {
-                const float* tcs = S.texcoord + 6 * (size_t)hit.id;
+                // pixel_evaluate_material_bilin_lod_cpu (material-cpu.cpp:36-77)
+                const float* tcs = S.texcoord + 6 * (size_t)t.best_id;
                 float ts, tt;
-                bary2(hit.beta, hit.gamma, tcs, &ts, &tt);
+                bary2(t.bb, t.bg, tcs, &ts, &tt);
                 RayDiff df = camera_diff(cam, px, py);
                 const float diff = ray_diff_hit(&df, ld3(a), ld3(sh[1]), ld3(sh[2]), tcs, ts, tt, N);
                 mcol = mcol * tex_sample_bilin_lod(S.tex[dtex], ts, tt, diff);
             }
         }
+        const bool finite = isfinite(mcol.x) && isfinite(mcol.y) && isfinite(mcol.z);
         v3 buf_dir = d;
         v3 rnd = draw3(&ls);
-        for (int k = 0; k < L; ++k) {
-            if (k >= 2) rnd = draw3(&ls);
-            v3 weight = mk(0.0f, 0.0f, 0.0f);
-            bool occluded = false;
-            if (is_hit && S.n_lights > 0) {
-                const int l = pick_light(S.lights, S.n_lights, S.overall_power, rnd.z);
-                const LightRec Lr = S.lights[l];
-                v3 so, sd;
-                float smax;
-                if (Lr.type == 1)
-                    sky_light_sample(S.sky, Lr.power, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so, &sd,
-                                     &smax, &weight);
-                else
-                    rect_light_sample(Lr, Lr.col, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so, &sd,
-                                      &smax, &weight);
-                buf_dir = sd;
-                occluded = smax >= 0.0f && traverse<true>(S, make_ray(so, sd), smax, nullptr, status);
-            } else {
-                if (S.sky.light >= 0) weight = S.sky.scale * sky_eval(S.sky, buf_dir);
-                buf_dir = mk(0.0f, 0.0f, 0.0f);
+        for (int k0 = 0; k0 < L; k0 += kDirectGroup) {
+            const int n = min(kDirectGroup, L - k0);
+            v3 so[kDirectGroup], sd[kDirectGroup], weight[kDirectGroup];
+            float smax[kDirectGroup];
+            uint32_t rays = 0, occluded = 0;  // by sample of the group
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+                if (k0 + i >= 2) rnd = draw3(&ls);
+                weight[i] = mk(0.0f, 0.0f, 0.0f);
+                if (is_hit && S.n_lights > 0) {
+                    const int l = pick_light(S.lights, S.n_lights, S.overall_power, rnd.z);
+                    const LightRec Lr = S.lights[l];
+                    if (Lr.type == 1 && HYBRID)
+                        sky_light_sample(S.sky, Lr.power, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so[i],
+                                         &sd[i], &smax[i], &weight[i]);
+                    else if (Lr.type == 1)
+                        sky_light_sample_uniform(S.sky, Lr.power, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset,
+                                                 &so[i], &sd[i], &smax[i], &weight[i]);
+                    else
+                        rect_light_sample(Lr, Lr.col, S.overall_power, P, N, rnd.x, rnd.y, shadow_offset, &so[i],
+                                          &sd[i], &smax[i], &weight[i], nullptr, HYBRID);
+                    buf_dir = sd[i];
+                    const bool zero = finite && weight[i].x == 0.0f && weight[i].y == 0.0f && weight[i].z == 0.0f;
+                    if (smax[i] >= 0.0f && !zero) rays |= 1u << i;
+                } else {
+                    if (S.sky.light >= 0) weight[i] = S.sky.scale * sky_eval(S.sky, buf_dir);
+                    buf_dir = mk(0.0f, 0.0f, 0.0f);
+                }
             }
-            const v3 mat = occluded ? mk(0.0f, 0.0f, 0.0f) : mcol;
-            const float s = float(c * L + k);
-            acc = (s * acc + weight * mat) / (s + 1.0f);
+            int cur = -1;
+            trav_stop(t);
+            for (int steps = 0;;) {
+                const bool tri = has_tri(t);
+                bool node = has_node(t);
+                if (!tri && !node) {  // the ray of sample `cur` is done: on to the lane's next one
+                    if (cur >= 0 && t.best_id != 0xffffffffu) occluded |= 1u << cur;
+                    cur = __ffs(rays) - 1;
+                    if (cur >= 0) {
+                        rays &= rays - 1u;
+                        r = make_ray(so[cur], sd[cur]);
+                        trav_init(t, r, smax[cur]);
+                        node = true;
+                    }
+                }
+                const uint32_t mt = __ballot_sync(0xffffffffu, tri), mn = __ballot_sync(0xffffffffu, node);
+                if ((mt | mn) == 0u) break;
+                if (++steps > kIterLimit) {
+                    atomicOr(status, (uint32_t)ST_ITER_LIMIT);
+                    trav_stop(t);
+                    rays = 0;
+                    continue;
+                }
+                warp_step<false, kStack>(tri, node, mt, mn, S.nodes, S.tris, r, true, t, stack, status, &nvis, &ntri);
+            }
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+                const v3 mat = (occluded >> i) & 1u ? mk(0.0f, 0.0f, 0.0f) : mcol;
+                const float s = float(c * L + k0 + i);
+                acc = (s * acc + weight[i] * mat) / (s + 1.0f);
+            }
         }
-        if (L >= 2) draw3(&ls);
+        if (HYBRID && L >= 2) draw3(&ls);
     }
+    if (!mine) return;
     out[3 * g] = acc.x;
     out[3 * g + 1] = acc.y;
     out[3 * g + 2] = acc.z;
@@ -2144,8 +2129,8 @@ cudaError_t k_launch_adjoint(const Frame& F, const RenderParams& P, cudaStream_t
 cudaError_t k_launch_direct(const DevScene& S, const CameraRec& cam, int w, int h, int samples, uint32_t seed,
                             float shadow_offset, v3 background, float* out, uint32_t* status, cudaStream_t st) {
     if (w * h <= 0) return cudaSuccess;
-    k_direct<<<blocks_for(w * h), kBlock, 0, st>>>(S, cam, w, h, samples, seed, shadow_offset, background, out, status,
-                                                   subseq_table());
+    k_direct<false><<<(w * h + GB_DIRECT_BLOCK - 1) / GB_DIRECT_BLOCK, GB_DIRECT_BLOCK, 0, st>>>(
+        S, cam, w, h, 1, samples, seed, shadow_offset, background, out, status, subseq_table());
     return cudaGetLastError();
 }
 
@@ -2153,8 +2138,8 @@ cudaError_t k_launch_direct_hybrid(const DevScene& S, const CameraRec& cam, int 
                                    int light_samples, uint32_t seed, float shadow_offset, v3 background, float* out,
                                    uint32_t* status, cudaStream_t st) {
     if (w * h <= 0) return cudaSuccess;
-    k_direct_hybrid<<<blocks_for(w * h), kBlock, 0, st>>>(S, cam, w, h, cam_samples, light_samples, seed,
-                                                          shadow_offset, background, out, status, subseq_table());
+    k_direct<true><<<(w * h + GB_DIRECT_BLOCK - 1) / GB_DIRECT_BLOCK, GB_DIRECT_BLOCK, 0, st>>>(
+        S, cam, w, h, cam_samples, light_samples, seed, shadow_offset, background, out, status, subseq_table());
     return cudaGetLastError();
 }
 

@@ -141,3 +141,25 @@ def test_axis_parallel_and_scaled_rays(gpu_ctx, scale):
         assert np.array_equal(a[f][hit].view(np.uint32), b[f][hit].view(np.uint32))
     assert np.array_equal(s.trace_any(o, d, t) != 0, orc.trace_any(o, d, t) != 0)
     s.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (33, 31), (64, 3)])
+@pytest.mark.parametrize("cams,lights", [(1, 8), (3, 9), (2, 17)])
+@pytest.mark.parametrize("sky", [False, True])
+def test_direct_light_sample_groups(gpu_ctx, w, h, cams, lights, sky):
+    """Light-sample counts around the groups the direct integrators trace
+    together, image sizes around a warp and a block, with and without a sky:
+    bit-equal to the oracle, sample by sample."""
+    from oracle import oracle
+    sc = scenes.icospheres(n_spheres=12, level=2, box=8.0, width=w, height=h, n_lights=2)
+    if sky:
+        sc.lights.append({"type": gbpt.GB_LIGHT_SKY, "map": scenes.procedural_sky(16, 8), "scale": 0.3,
+                          "diameter": 20.0, "power": -1.0})
+    rd = dict(sc.render, shadow_offset=0.01, seed=2)
+    s = gpu_ctx.scene(sc)
+    orc = oracle.OracleScene(sc, use_bvh=True)
+    pool = gpu_ctx.mrg_pool(w * h, cams * lights + 1, seed=2)
+    assert np.array_equal(s.render_direct(sc.camera, rd, lights), orc.render_direct(sc.camera, rd, lights, pool))
+    assert np.array_equal(s.render_hybrid_direct(sc.camera, rd, cams, lights),
+                          orc.render_hybrid_direct(sc.camera, rd, cams, lights, pool))
+    s.close()
