@@ -74,7 +74,8 @@ struct FitState {
     LightRec* h_lights = nullptr;       // light records of every scene
     std::vector<size_t> mat_off, light_off;
     double* h_out = nullptr;            // gradient sums (stride), then one loss per scene
-    double* d_loss = nullptr;
+    double* d_loss = nullptr;           // one loss per scene, then kLossBlocks partial sums per scene
+    FitLossItem* d_items = nullptr;
     int stride = 0, replicas = 0;
     size_t mats_total = 0, lights_total = 0;
 };
@@ -422,6 +423,7 @@ void gb_ctx_destroy(gb_ctx* ctx) {
     if (ctx->fit.h_lights) cudaFreeHost(ctx->fit.h_lights);
     if (ctx->fit.h_out) cudaFreeHost(ctx->fit.h_out);
     if (ctx->fit.d_loss) cudaFree(ctx->fit.d_loss);
+    if (ctx->fit.d_items) cudaFree(ctx->fit.d_items);
     if (ctx->fit_aux) cudaStreamDestroy(ctx->fit_aux);
     free_all(ctx->adj_allocs);
     if (ctx->d_scenes) cudaFree(ctx->d_scenes);
@@ -1612,7 +1614,7 @@ std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     std::vector<uint64_t> k;
     const void* ptrs[] = {ctx->d_scenes, F.ray, F.halton, F.out, F.pristine,
                           F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr, F.iter, F.stats,
-                          F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->d_rgb, ctx->fit.d_loss};
+                          F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->fit.d_loss};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
     k.push_back(((uint64_t)ctx->slot_cap << 32) ^ (uint64_t)ctx->sample_cap);
     k.push_back(((uint64_t)(uint32_t)ctx->slots << 32) | (uint32_t)ctx->sample_mb);
@@ -1673,11 +1675,17 @@ int fit_build(gb_ctx* ctx) {
         e = ensure_buf(ctx, (void**)&F.grad, &ctx->grad_cap, sizeof(float) * (size_t)f.replicas * (size_t)f.stride);
     if (e == cudaSuccess) e = ensure_buf(ctx, (void**)&ctx->d_gsum, &ctx->gsum_cap, sizeof(double) * (size_t)f.stride);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fitting buffers");
-    rc = ensure_rgb(ctx);
-    if (rc != GB_OK) return rc;
     if (f.d_loss) { cudaFree(f.d_loss); f.d_loss = nullptr; }
+    if (f.d_items) { cudaFree(f.d_items); f.d_items = nullptr; }
     std::vector<void*> tmp;
-    CK(dalloc(tmp, (void**)&f.d_loss, sizeof(double) * ns));
+    CK(dalloc(tmp, (void**)&f.d_loss, sizeof(double) * ns * (1 + kLossBlocks)));
+    CK(dalloc(tmp, (void**)&f.d_items, sizeof(FitLossItem) * ns));
+    std::vector<FitLossItem> loss_items(ns);
+    for (size_t k = 0; k < ns; ++k) {
+        const BatchScene& it = f.items[k];
+        loss_items[k] = FitLossItem{it.target, it.image, it.base, it.n, 1.0f / (float)it.desc.spp};
+    }
+    CK(cudaMemcpy(f.d_items, loss_items.data(), sizeof(FitLossItem) * ns, cudaMemcpyHostToDevice));
     f.mat_off.assign(ns, 0);
     f.light_off.assign(ns, 0);
     f.mats_total = f.lights_total = 0;
@@ -1734,14 +1742,7 @@ int fit_build(gb_ctx* ctx) {
         }
         if (rc != GB_OK) break;
         if (pass == 0) {
-            e = k_launch_pack_rgb(F.out, F.ntot, ctx->d_rgb, a);
-            for (size_t k = 0; k < ns && e == cudaSuccess; ++k) {
-                const BatchScene& it = f.items[k];
-                const float* img = ctx->d_rgb + 3 * (size_t)it.base;
-                e = k_launch_l2_loss(img, it.target, it.n, 1.0f / (float)it.desc.spp, F.dimg + it.base, f.d_loss + k, a);
-                if (e == cudaSuccess && it.image)
-                    e = cudaMemcpyAsync(it.image, img, sizeof(float) * 3 * (size_t)it.n, cudaMemcpyDeviceToDevice, a);
-            }
+            e = k_launch_l2_loss(f.d_items, (int)ns, F.out, F.dimg, f.d_loss + ns, f.d_loss, a);
         } else {
             e = k_launch_grad_reduce(F.grad, f.replicas, f.stride, ctx->d_gsum, a);
             if (e == cudaSuccess)
