@@ -1534,8 +1534,8 @@ int gb_backward_batch(gb_ctx* ctx, int n, const gb_adjoint_item* items, int dimg
     int rc = begin_frame(ctx, v);
     if (rc != GB_OK) return rc;
     Frame& F = ctx->F;
-    const int replicas = k_adjoint_grid();
     const int stride = (int)std::max<uint32_t>(1, gtot);
+    const int replicas = k_adjoint_replicas(stride);
     cudaError_t e = ensure_buf(ctx, (void**)&F.adj, &ctx->adj_cap,
                                sizeof(float4) * kAdjPlanes * (size_t)ctx->max_L *
                                    std::min(ctx->slot_cap, (size_t)kAdjMaxSlots));
@@ -1664,8 +1664,8 @@ int fit_build(gb_ctx* ctx) {
     if (rc != GB_OK) return rc;
     f.items = ctx->items;
     Frame& F = ctx->F;
-    f.replicas = k_adjoint_grid();
     f.stride = (int)std::max<uint32_t>(1, gtot);
+    f.replicas = k_adjoint_replicas(f.stride);
     const size_t ns = f.items.size();
     cudaError_t e = ensure_buf(ctx, (void**)&F.adj, &ctx->adj_cap,
                                sizeof(float4) * kAdjPlanes * (size_t)ctx->max_L *

@@ -1113,8 +1113,8 @@ __device__ __forceinline__ LightSample light_sample(const Frame& F, const SceneR
 // anything else, so the sums and their order are those of the reference.  No
 // ray is traced for a contribution of exactly zero (the light or the surface
 // faces away, no lobe towards the light): adding +-0 to an accumulation that
-// is never -0 leaves its bits as they are.  The adjoint traces those too: its
-// vertex records carry the visibility.
+// is never -0 leaves its bits as they are.  The adjoint leaves out samples of
+// scale zero only: a black light still has a gradient.
 //
 // MODE_FROZEN evaluates the BRDF with the scene's eval records and carries
 // the sampling throughput in tp0; MODE_ADJOINT writes the vertex record of
@@ -1261,15 +1261,16 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
                         ShadeTrace tr;
                         o = shade_hit(v.m, v.P, v.N, rd, tp, v.rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path,
                                       bounce, nullptr, nullptr, &tr);
+                        // a sample of scale zero adds nothing to the value or the gradient: it counts as blocked
+                        shadow = tr.nee && ls.scale != 0.0f;
                         uint32_t info = (uint32_t)ls.light | ((uint32_t)tr.lobe << 16) | (tr.clamp_mask << 20) |
-                                        (tr.nee ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
+                                        (shadow ? (1u << 23) : 0u) | ((tr.flags & 7u) << 24);
                         float4* rec = F.adj + (size_t)bounce * kAdjPlanes * F.nslots + slot;
                         rec[0] = make_float4(tp.x, tp.y, tp.z, tr.pdf);
                         rec[(size_t)F.nslots] = make_float4(tr.wo.x, tr.wo.y, tr.wo.z, tr.q);
-                        rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, tr.nee ? ls.scale : 0.0f);
+                        rec[2 * (size_t)F.nslots] = make_float4(tr.wi.x, tr.wi.y, tr.wi.z, ls.scale);
                         rec[3 * (size_t)F.nslots] = make_float4(tr.N.x, tr.N.y, tr.N.z, __uint_as_float(v.mi));
                         rec[4 * (size_t)F.nslots] = make_float4(tr.ld.x, tr.ld.y, tr.ld.z, __uint_as_float(info));
-                        shadow = tr.nee;
                     } else {
                         o = shade_hit(v.m, v.P, v.N, rd, tp, v.rnd, ls.smax >= 0.0f, ls.sd, ls.psc, R.sp, lp, path,
                                       bounce);
@@ -2144,6 +2145,14 @@ cudaError_t k_launch_shade(const Frame& F, const RenderParams& P, cudaStream_t s
 int k_adjoint_grid() {
     static int g = persistent_blocks(k_adjoint);
     return g;
+}
+// A copy per block while they take no more than 16 MB, else fewer, down to one
+// for five blocks: clearing and summing them costs more than the contention
+// then (8 scenes of 3.6 K floats: 4.15 -> 4.09 ms per fitting step with a fifth
+// of the copies; one scene's gradient 2.94 -> 3.03 ms).
+int k_adjoint_replicas(int stride) {
+    const int g = k_adjoint_grid();
+    return std::max(std::max(1, g / 5), std::min(g, (4 << 20) / std::max(1, stride)));
 }
 
 cudaError_t k_launch_adjoint(const Frame& F, const RenderParams& P, cudaStream_t st) {
