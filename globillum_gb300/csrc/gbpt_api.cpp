@@ -881,7 +881,8 @@ int begin_frame(gb_ctx* ctx, std::vector<BatchScene>& items) {
         R.rng_mode = b.desc.rng_mode;
         R.pixel_base = base;
         R.seed = b.desc.seed;
-        mrg_jump_matrices(3ull * (uint64_t)R.L, R.jump1, R.jump2);
+        if (i > 0 && ctx->recs[i - 1].L == R.L) R.jump = ctx->recs[i - 1].jump;
+        else mrg_powers(3ull * (uint64_t)R.L, &R.jump);
         if (b.mats_eval) R.S.mats_eval = b.mats_eval;
         if (b.lights_eval) R.S.lights_eval = b.lights_eval;
         R.n_mats = (int)b.scene->mats.size();
@@ -914,8 +915,8 @@ int run_chunk_loop(gb_ctx* ctx, const RenderParams& P, int nstart) {
     const Frame& F = ctx->F;
     CK(cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, ctx->stream));
     CK(stage_mark(ctx, 0, true));
-    CK(k_launch_jitter_pool(F, P, ctx->stream));
     CK(k_launch_start(F, P, nstart, ctx->stream));
+    CK(k_launch_jitter_pool(F, P, ctx->stream));
     CK(stage_mark(ctx, 0, false));
     ctx->launches += 2;
     const int kEvery = 2, kLead = 12;
@@ -999,8 +1000,8 @@ int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, cudaGraphE
     if (e != cudaSuccess) return cuda_fail(ctx, e, "graph capture");
     cudaGraphNodeParams np{};
     if (e == cudaSuccess) e = cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, a);
-    if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, a);
     if (e == cudaSuccess) e = k_launch_start(F, P, nstart, a);
+    if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, a);
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1045,8 +1046,8 @@ int build_chunk_graph(gb_ctx* ctx, const RenderParams& P, int nstart, cudaGraphE
 int append_chunk(gb_ctx* ctx, const RenderParams& P, int nstart, cudaStream_t a, cudaStream_t b) {
     const Frame& F = ctx->F;
     cudaError_t e = cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, a);
-    if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, a);
     if (e == cudaSuccess) e = k_launch_start(F, P, nstart, a);
+    if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, a);
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1162,6 +1163,9 @@ void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out)
     // the adjoint's vertex records take 80 B x bounces per slot
     if (ctx->mode == MODE_ADJOINT) F.nslots = std::min(F.nslots, kAdjMaxSlots);
     const int nstart = (int)std::min<long long>(F.nslots, acc);
+    P.pool_round = 0;  // first round with paths that do not start at once
+    while (P.pool_round < P.rounds && P.round_start[P.pool_round + 1] <= (uint32_t)nstart) ++P.pool_round;
+    P.more = p1 < ctx->max_spp ? 1 : 0;
     // Every iteration moves each busy slot's path one bounce (at most L + 1
     // per path, the last of them for a light sample still pending), and all
     // slots stay busy until the chunk's last path has started, so the loop
@@ -1186,10 +1190,11 @@ int run_chunk(gb_ctx* ctx, int p0, int p1) {
     int nstart = 0;
     make_chunk(ctx, p0, p1, &P, &nstart);
     if (P.finish_max > 0 && P.chunk_paths <= (uint32_t)kPathsMax) {
-        CK(k_launch_jitter_pool(ctx->F, P, ctx->stream));
+        P.pool_round = P.rounds;
         CK(k_launch_paths(ctx->F, P, ctx->stream));
+        CK(k_launch_jitter_pool(ctx->F, P, ctx->stream));
         CK(k_launch_combine(ctx->F, P, ctx->stream));
-        ctx->launches += 3;
+        ctx->launches += P.more ? 3 : 2;
         return GB_OK;
     }
     if (ctx->use_graph && !ctx->stage_timing) return run_chunk_graph(ctx, P, nstart);

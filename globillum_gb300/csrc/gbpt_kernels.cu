@@ -534,29 +534,52 @@ __global__ void k_fill_pscene(Frame F) {
 //                    in the chunk's stream pool.
 // A path's stream therefore depends only on (pixel, p): a launch may start
 // several paths of one pixel, in any order, on any slots.
-// Per pixel at the start of a chunk, for every path p of the pixel in the
-// chunk (path l = round_start[p - p0] + pixel): its camera jitter (update p
-// of the pixel's jitter stream) and the state of its light/path stream
-// (L updates per path: one jump of 3 L generator steps from the previous
-// path's).  Paths then start from their own pool entries, in any order and
-// several per pixel at once.
-__global__ void k_jitter_pool(Frame F, RenderParams P) {
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
+// The state n jumps on.
+__device__ __forceinline__ MrgState mrg_skip(MrgState s, const MrgPowers& T, uint32_t n) {
+    for (int k = 0; n != 0u; ++k, n >>= 1)
+        if (n & 1u) mrg_jump(s.s1, s.s2, T.j1[k], T.j2[k]);
+    return s;
+}
+// A pixel's camera-jitter and light/path streams `r` paths after the chunk's
+// start: a frame starts at curand_init(seed, pixel, 0), a later chunk where the
+// last one ended.  J: jumps by the three draws of a jitter update.
+__device__ __forceinline__ MrgState jitter_stream(const Frame& F, const RenderParams& P, const MrgPowers& J,
+                                                  uint32_t pix, uint32_t r) {
+    return mrg_skip(ld_mrg(P.p0 == 0 ? F.pristine : F.jcursor, (size_t)pix), J, r);
+}
+__device__ __forceinline__ MrgState path_stream(const Frame& F, const RenderParams& P, const SceneRec& R,
+                                                uint32_t pix, uint32_t r) {
+    return mrg_skip(ld_mrg(P.p0 == 0 ? F.pristine : F.cursor, (size_t)pix), R.jump, r);
+}
+
+// Per pixel, for the paths p of the pixel in the chunk from round pool_round
+// on (path l = round_start[p - p0] + pixel): its camera jitter (update p of the
+// pixel's jitter stream) and the state of its light/path stream (L updates per
+// path: one jump of 3 L generator steps from the previous path's).  Paths that
+// restart on a slot take these entries, in any order and several per pixel at
+// once; the first paths (k_start, k_paths) jump to their own states instead,
+// which saves 80 B of pool traffic per path and most of this kernel.  Both
+// streams' cursors then move on to the next chunk.
+__global__ void k_jitter_pool(Frame F, RenderParams P, const MrgPowers J) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= F.ntot) return;
     const SceneRec& R = F.scenes[F.nscenes == 1 ? 0u : F.pscene[g]];
-    // a frame starts at curand_init(seed, pixel, 0), a later chunk where the last one ended
-    MrgState s = ld_mrg(P.p0 == 0 ? F.pristine : F.jcursor, (size_t)g);
-    MrgState c = ld_mrg(P.p0 == 0 ? F.pristine : F.cursor, (size_t)g);
-    const int pe = min(P.p0 + P.rounds, R.spp);
-    for (int p = P.p0; p < pe; ++p) {
-        const uint32_t l = P.round_start[p - P.p0] + (uint32_t)g;
+    const int rounds = min(P.rounds, R.spp - P.p0);
+    const int r0 = min(P.pool_round, rounds);
+    if (rounds <= 0) return;
+    MrgState s = jitter_stream(F, P, J, (uint32_t)g, (uint32_t)r0);
+    MrgState c = path_stream(F, P, R, (uint32_t)g, (uint32_t)r0);
+    for (int r = r0; r < rounds; ++r) {
+        const uint32_t l = P.round_start[r] + (uint32_t)g;
         v3 j = draw3(&s);
         rec_st(&F.jpool[l], make_float4(j.x, j.y, j.z, 0.0f));
         st_mrg(F.spool, l, c);
-        mrg_jump(c.s1, c.s2, R.jump1, R.jump2);  // = L draw3 calls
+        mrg_jump(c.s1, c.s2, R.jump.j1[0], R.jump.j2[0]);  // = L draw3 calls
     }
-    st_mrg(F.jcursor, (size_t)g, s);
-    st_mrg(F.cursor, (size_t)g, c);
+    if (P.more) {
+        st_mrg(F.jcursor, (size_t)g, s);
+        st_mrg(F.cursor, (size_t)g, c);
+    }
 }
 
 // Ray differentials of a slot, 12 floats in 3 planes of nslots float4.
@@ -591,13 +614,16 @@ __device__ __forceinline__ void st_path(const Frame& F, uint32_t slot, v3 tp, v3
     rec_st(&F.strm[slot], Sector{{m.s1[0], m.s1[1], m.s1[2], m.s2[0], m.s2[1], m.s2[2], __float_as_uint(pend.z), 0u}});
 }
 
-// Path l of the chunk: its pixel, scene, sample index and camera ray.
+// Path l of the chunk: its pixel, scene, sample index, camera ray and stream.
 struct PathStart {
     uint32_t pix, sc, path;
     int x, y;
     v3 o, d;
+    MrgState st;
 };
-__device__ __forceinline__ PathStart path_start(const Frame& F, const RenderParams& P, uint32_t l) {
+// J: jump to the path's streams; null: they are in the chunk's pool.
+__device__ __forceinline__ PathStart path_start(const Frame& F, const RenderParams& P, uint32_t l,
+                                                const MrgPowers* J) {
     int lo = 0, hi = P.rounds - 1;
     while (lo < hi) {  // round holding path l
         int mid = (lo + hi + 1) >> 1;
@@ -609,27 +635,40 @@ __device__ __forceinline__ PathStart path_start(const Frame& F, const RenderPara
     s.sc = F.nscenes == 1 ? 0u : F.pscene[s.pix];
     s.path = (uint32_t)P.p0 + (uint32_t)lo;
     const SceneRec& R = F.scenes[s.sc];
-    const uint32_t lp = s.pix - R.pixel_base;
-    const float4* jp = F.jpool + P.round_start[lo];
-    float4 j = rec_ld(&jp[s.pix]);
-    float lx = 0.0f, ly = 0.0f;
-    if (R.cam.aperture != 0.0f) {
-        float4 lj = rec_ld(&jp[R.pixel_base + (lp + 17u) % (uint32_t)R.n]);
-        lx = lj.z - 0.5f;
-        ly = lj.y - 0.5f;
+    const uint32_t lp = s.pix - R.pixel_base, lens = R.pixel_base + (lp + 17u) % (uint32_t)R.n;
+    const bool aperture = R.cam.aperture != 0.0f;
+    v3 j, lj = mk(0.0f, 0.5f, 0.5f);
+    if (J) {
+        MrgState js = jitter_stream(F, P, *J, s.pix, (uint32_t)lo);
+        j = draw3(&js);
+        if (aperture) {
+            js = jitter_stream(F, P, *J, lens, (uint32_t)lo);
+            lj = draw3(&js);
+        }
+        s.st = path_stream(F, P, R, s.pix, (uint32_t)lo);
+    } else {
+        const float4* jp = F.jpool + P.round_start[lo];
+        j = ld3(rec_ld(&jp[s.pix]));
+        if (aperture) lj = ld3(rec_ld(&jp[lens]));
+        s.st = ld_mrg(F.spool, l);
     }
+    const float lx = aperture ? lj.z - 0.5f : 0.0f, ly = aperture ? lj.y - 0.5f : 0.0f;
     s.x = (int)(lp % (uint32_t)R.w);
     s.y = (int)(lp / (uint32_t)R.w);
     camera_ray(R.cam, s.x, s.y, j.x, j.y, lx, ly, &s.o, &s.d);
     return s;
 }
 
-__device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t l) {
-    const PathStart s = path_start(F, P, l);
+// Path s on a slot.
+__device__ __forceinline__ void put_path(const Frame& F, const RenderParams& P, uint32_t slot, const PathStart& s) {
     rec_st(&F.ray[slot], pack_sector(s.o, s.d, s.path << 10, s.pix));
-    st_path(F, slot, mk(1.0f, 1.0f, 1.0f), mk(0.0f, 0.0f, 0.0f), ld_mrg(F.spool, l), mk(0.0f, 0.0f, 0.0f));
+    st_path(F, slot, mk(1.0f, 1.0f, 1.0f), mk(0.0f, 0.0f, 0.0f), s.st, mk(0.0f, 0.0f, 0.0f));
     if (P.mode == MODE_FROZEN) F.tp0[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     if (P.textured && F.scenes[s.sc].S.texcoord) st_rdiff(F, slot, camera_diff(F.scenes[s.sc].cam, s.x, s.y));
+}
+// Path l of the chunk, from the pool, on a slot.
+__device__ __forceinline__ void start_path(const Frame& F, const RenderParams& P, uint32_t slot, uint32_t l) {
+    put_path(F, P, slot, path_start(F, P, l, nullptr));
 }
 
 // The scene of a pixel's paths; a frame of one scene needs no load.
@@ -675,19 +714,49 @@ __global__ void __launch_bounds__(kBlock) k_regen(Frame F, RenderParams P) {
     }
 }
 
-// First paths of a chunk: slot s takes path s.  Sets the queue of iteration 0
-// (the counters are zero) and the iteration index.
-__global__ void __launch_bounds__(kBlock) k_start(Frame F, RenderParams P, int nstart) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) {
+// First paths of a chunk: slot s takes path s.  A thread starts the paths of
+// one pixel in `group` rounds one after the other, from where the pixel's
+// streams are then.  Sets the queue of iteration 0 (the counters are zero) and
+// the iteration index.
+__global__ void __launch_bounds__(kBlock) k_start(Frame F, RenderParams P, int nstart, int group, const MrgPowers J) {
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r0 = (int)blockIdx.y * group;
+    if (g == 0 && r0 == 0) {
         *F.path_ctr = (uint32_t)nstart;
         F.iter[0] = 0;
         F.ctr[CTR_EXT] = (uint32_t)nstart;
         F.ctr[CTR_STARTED] = (uint32_t)nstart;
     }
-    if (s >= (uint32_t)nstart) return;
-    start_path(F, P, s, s);
-    F.q[0][s] = s;
+    if (g >= (uint32_t)F.ntot || P.round_start[r0] + g >= (uint32_t)nstart) return;
+    PathStart s;
+    s.pix = g;
+    s.sc = F.nscenes == 1 ? 0u : F.pscene[g];
+    const SceneRec& R = F.scenes[s.sc];
+    const int r1 = min(min(r0 + group, P.rounds), R.spp - P.p0);
+    if (r0 >= r1) return;
+    const uint32_t lp = g - R.pixel_base;
+    s.x = (int)(lp % (uint32_t)R.w);
+    s.y = (int)(lp / (uint32_t)R.w);
+    const bool aperture = R.cam.aperture != 0.0f;
+    MrgState js = jitter_stream(F, P, J, g, (uint32_t)r0), ls = js;
+    if (aperture) ls = jitter_stream(F, P, J, R.pixel_base + (lp + 17u) % (uint32_t)R.n, (uint32_t)r0);
+    s.st = path_stream(F, P, R, g, (uint32_t)r0);
+    for (int r = r0; r < r1; ++r) {
+        const uint32_t l = P.round_start[r] + g;
+        if (l >= (uint32_t)nstart) break;
+        const v3 j = draw3(&js);
+        float lx = 0.0f, ly = 0.0f;
+        if (aperture) {
+            const v3 lj = draw3(&ls);
+            lx = lj.z - 0.5f;
+            ly = lj.y - 0.5f;
+        }
+        s.path = (uint32_t)(P.p0 + r);
+        camera_ray(R.cam, s.x, s.y, j.x, j.y, lx, ly, &s.o, &s.d);
+        put_path(F, P, l, s);
+        F.q[0][l] = l;
+        mrg_jump(s.st.s1, s.st.s2, R.jump.j1[0], R.jump.j2[0]);  // = L draw3 calls
+    }
 }
 
 // (t, canonical id) as one 64-bit key whose unsigned order is the
@@ -1447,15 +1516,15 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
 }
 
 template <bool TEX>
-__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P) {
+__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P, const MrgPowers J) {
     fill_order_table();
     const uint32_t l = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
     const bool alive = l < P.chunk_paths;
-    const PathStart ps = path_start(F, P, alive ? l : 0u);
+    const PathStart ps = path_start(F, P, alive ? l : 0u, &J);
     const SceneRec& R = F.scenes[ps.sc];
     const v3 z = mk(0.0f, 0.0f, 0.0f);
     PathState p{ps.o, ps.d, mk(1.0f, 1.0f, 1.0f), z, z, z, z, 0.0f, alive, false, 0, ps.path, ps.pix,
-                ld_mrg(F.spool, alive ? l : 0u)};
+                ps.st};
     RayDiff df;
     if (TEX && R.S.texcoord) df = camera_diff(R.cam, ps.x, ps.y);
     add_stats(&F.stats[0], alive ? 1u : 0u);
@@ -2044,8 +2113,28 @@ cudaError_t k_launch_frame_init(const Frame& F, bool rng, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// Jumps by the three draws of a camera-jitter update, computed once per process.
+const MrgPowers& jitter_powers() {
+    static const MrgPowers T = [] {
+        MrgPowers t;
+        mrg_powers(3, &t);
+        return t;
+    }();
+    return T;
+}
+
+#ifndef GB_START_THREADS
+#define GB_START_THREADS (1 << 17)
+#endif
 cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cudaStream_t st) {
-    k_start<<<blocks_for(std::max(nstart, 1)), kBlock, 0, st>>>(F, P, nstart);
+    // enough threads to fill the chip, at most 8 paths each (12 mixed scenes 3.43 ms with the pool for every path,
+    // 3.52 with a thread per path, 3.25 so; 256x256 room 0.935 / 0.921 / 0.907); rounds beyond the first nstart
+    // paths have no blocks
+    const int group = std::min(8, std::max(1, nstart / GB_START_THREADS));
+    int rounds = 1;
+    while (rounds < P.rounds && P.round_start[rounds] < (uint32_t)nstart) ++rounds;
+    const dim3 grid((unsigned)blocks_for(F.ntot), (unsigned)((rounds + group - 1) / group));
+    k_start<<<grid, kBlock, 0, st>>>(F, P, nstart, group, jitter_powers());
     return cudaGetLastError();
 }
 
@@ -2210,8 +2299,8 @@ cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t s
 
 cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t st) {
     const unsigned grid = (P.chunk_paths + GB_PATHS_BLOCK - 1) / GB_PATHS_BLOCK;
-    if (P.textured) k_paths<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
-    else k_paths<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
+    if (P.textured) k_paths<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
+    else k_paths<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
     return cudaGetLastError();
 }
 
@@ -2223,8 +2312,10 @@ cudaError_t k_launch_finish(const Frame& F, const RenderParams& P, cudaStream_t 
     return cudaGetLastError();
 }
 
+// After k_start / k_paths, which start from the cursors this moves on.
 cudaError_t k_launch_jitter_pool(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    k_jitter_pool<<<blocks_for(F.ntot), kBlock, 0, st>>>(F, P);
+    if (P.pool_round >= P.rounds && !P.more) return cudaSuccess;
+    k_jitter_pool<<<blocks_for(F.ntot), kBlock, 0, st>>>(F, P, jitter_powers());
     return cudaGetLastError();
 }
 

@@ -51,7 +51,7 @@ struct SceneRec {
     int spp, L, rng_mode;
     uint32_t pixel_base;  // first global pixel of the scene
     uint32_t seed;
-    uint32_t jump1[9], jump2[9];  // MRG32k3a jump by the 3 L draws of one path
+    MrgPowers jump;       // MRG32k3a jumps by the 3 L draws of a path
     int n_mats;
     uint32_t grad_base;   // first record-gradient float of the scene (adjoint)
 };
@@ -159,8 +159,8 @@ struct Frame {
     uint32_t* pscene;  // scene of each pixel
     float2* halton;    // Halton light draw of each pixel (null when no scene of the frame uses it)
     float4* samples;   // sample of path l of the chunk (l = round_start[r] + pixel)
-    float4* jpool;     // camera jitter of path l of the chunk
-    MrgState* spool;   // light/path stream state at the start of path l of the chunk
+    float4* jpool;     // camera jitter of path l of the chunk (rounds from RenderParams::pool_round on)
+    MrgState* spool;   // light/path stream state at the start of path l of the chunk (the same rounds)
     // control
     uint32_t* ctr;     // 3 sets of 8 (by iteration % 3), see CTR_*
     uint32_t* path_ctr;  // next path of the chunk to start
@@ -210,6 +210,9 @@ struct RenderParams {
     int mode;          // MODE_*
     int textured;      // some scene of the frame has textures (k_shade's texture variant, Frame::rdiff)
     int p0, rounds;    // path samples p0 .. p0+rounds-1
+    int pool_round;    // first round of the chunk that k_start does not start whole (rounds: none)
+    int more;          // chunks of the frame follow: the pixels' stream cursors move on
+    int pad_;
     int max_iters;     // iteration bound of the chunk's loop
     int finish_max;    // the loop leaves the chunk's last paths to k_finish once at most this many are alive (0: never)
     // L2 window of the traversal launches (GB_NODE_L2_PERSIST, frames of one

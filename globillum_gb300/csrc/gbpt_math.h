@@ -297,6 +297,20 @@ static inline void mrg_subsequence_table(MrgSubseqTable* T) {
     }
 }
 
+// Jumps by steps 2^k, k = 0 .. 6: any number of jumps up to 127 is the product
+// of those its bits select.
+struct MrgPowers {
+    uint32_t j1[7][9], j2[7][9];
+};
+static inline void mrg_powers(uint64_t steps, MrgPowers* T) {
+    mrg_power(kMrgA1, steps, T->j1[0], 209u, kMrgM1);
+    mrg_power(kMrgA2, steps, T->j2[0], 22853u, kMrgM2);
+    for (int k = 1; k < 7; ++k) {
+        mrg_matmul(T->j1[k - 1], T->j1[k - 1], T->j1[k], 209u, kMrgM1);
+        mrg_matmul(T->j2[k - 1], T->j2[k - 1], T->j2[k], 22853u, kMrgM2);
+    }
+}
+
 // Advances a state (s1, s2) by the steps J1 = A1^k, J2 = A2^k stand for.
 GB_HD void mrg_jump(uint32_t s1[3], uint32_t s2[3], const uint32_t* J1, const uint32_t* J2) {
     mrg_apply(s1, J1, 209u, kMrgM1);

@@ -187,12 +187,13 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     R.rng_mode = d->rng_mode;
     R.pixel_base = 0;
     R.seed = d->seed;
-    mrg_jump_matrices(3ull * (uint64_t)R.L, R.jump1, R.jump2);
+    mrg_powers(3ull * (uint64_t)R.L, &R.jump);
     RenderParams P{};
     P.refill = 16;
     P.tri_mode = 0;
     P.blocks_per_sm = 0;
     P.rounds = 1;
+    P.pool_round = 1;
     P.round_start[0] = 0;
     P.round_start[1] = (uint32_t)n;
     P.chunk_paths = (uint32_t)n;
@@ -212,8 +213,9 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     for (int p = 0; p < d->spp && e == cudaSuccess; ++p) {
         P.p0 = p;
         e = cudaMemsetAsync(F.ctr, 0, sizeof(uint32_t) * 24, st);
-        if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, st);
+        P.more = p + 1 < d->spp ? 1 : 0;
         if (e == cudaSuccess) e = k_launch_start(F, P, n, st);
+        if (e == cudaSuccess) e = k_launch_jitter_pool(F, P, st);
         left = 1;
         for (int it = 0; e == cudaSuccess && left != 0u && it < max_iters; ++it) {
             e = k_launch_rays(F, P, false, 0, false, st);
