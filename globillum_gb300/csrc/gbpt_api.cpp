@@ -1118,6 +1118,10 @@ void make_chunk(gb_ctx* ctx, int p0, int p1, RenderParams* out, int* nstart_out)
     P.textured = 0;
     for (const BatchScene& b : ctx->items)
         if (b.scene->S.texcoord) P.textured = 1;
+    if (ctx->items.size() == 1) {
+        P.nodes = ctx->items[0].scene->S.nodes;
+        P.tris = ctx->items[0].scene->S.tris;
+    }
     P.p0 = p0;
     P.rounds = p1 - p0;
 #if GB_NODE_L2_PERSIST

@@ -18,7 +18,7 @@ namespace {
 
 const int kBuildBlock = 256;
 const int kMaxRadius = 32;
-const int kLeafMax = 3;  // triangles per leaf (the node meta holds 3 bits of them)
+const int kLeafMax = 3;  // triangles per leaf (a node holds 3 bits per slot for them)
 
 // Float order as unsigned order, for atomicMin / atomicMax of bounds.
 __device__ __forceinline__ unsigned f2ord(float f) {
@@ -534,7 +534,7 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
         sc[a] = ldexpf(1.0f, ex[a]);
         rsc[a] = 1.0 / (double)sc[a];
     }
-    uint8_t meta[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t leaves = 0;  // 3 bits per slot: a leaf's triangles in unary
     uint8_t qv[6][8];
     uint32_t imask = 0;
     int k_inner = 0, tri_off = 0;
@@ -555,7 +555,6 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
         }
         if (!bleaf[c]) {
             imask |= 1u << s;
-            meta[s] = 0x20;
             int child = base_child + k_inner;
             if (child >= node_cap) { atomicExch(bad, 3); return; }
             if (!refit) q_next[child - next_base] = c;
@@ -582,7 +581,7 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
                 st[sp++] = xc.x;
             }
         }
-        meta[s] = (uint8_t)((((1u << cnt) - 1u) << 5) | (uint32_t)tri_off);
+        leaves |= ((1u << cnt) - 1u) << (3 * s);
         tri_off += cnt;
     }
     uint32_t w[20];
@@ -592,8 +591,8 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
     w[3] = (uint32_t)(ex[0] + 127) | ((uint32_t)(ex[1] + 127) << 8) | ((uint32_t)(ex[2] + 127) << 16) | (imask << 24);
     w[4] = (uint32_t)base_child;
     w[5] = (uint32_t)base_tri;
-    w[6] = pack4(meta);
-    w[7] = pack4(meta + 4);
+    w[6] = leaves;
+    w[7] = 0;
     for (int a = 0; a < 3; ++a) {
         w[8 + 2 * a] = pack4(qv[a]);
         w[9 + 2 * a] = pack4(qv[a] + 4);

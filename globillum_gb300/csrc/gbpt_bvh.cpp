@@ -293,7 +293,7 @@ struct Collapser {
         for (int s = 0; s < 8; ++s)
             if (child_at[s] >= 0 && !is_leaf[child_at[s]]) imask |= 1u << s;
         w[3] = (uint32_t)(ex[0] + 127) | ((uint32_t)(ex[1] + 127) << 8) | ((uint32_t)(ex[2] + 127) << 16) | (imask << 24);
-        uint8_t meta[8] = {0};
+        uint32_t leaves = 0;  // 3 bits per slot: a leaf's triangles in unary
         uint8_t q[6][8] = {{0}};
         // inner children: contiguous block in slot order
         int n_inner = __builtin_popcount(imask);
@@ -302,7 +302,6 @@ struct Collapser {
         out.nodes.resize((size_t)out.n_nodes * kNodeWords);
         w = &out.nodes[(size_t)ci * kNodeWords];
         int base_tri = (int)(out.tris.size() / kTriWords);
-        int tri_off = 0;
         std::vector<std::pair<int, int>> todo;  // (cw index, binary node)
         int k_inner = 0;
         for (int s = 0; s < 8; ++s) {
@@ -319,22 +318,22 @@ struct Collapser {
                 q[a][s] = (uint8_t)ql; q[3 + a][s] = (uint8_t)qh;
             }
             if (!is_leaf[i]) {
-                meta[s] = 0x20;
                 todo.push_back(std::make_pair(base_child + k_inner, c));
                 ++k_inner;
             } else {
                 std::vector<int> tl;
                 subtree_tris(c, &tl);
                 int cnt = (int)tl.size();
-                meta[s] = (uint8_t)((((1u << cnt) - 1u) << 5) | (uint32_t)tri_off);
+                leaves |= ((1u << cnt) - 1u) << (3 * s);
                 for (int t : tl) emit_tri(t);
-                tri_off += cnt;
+
             }
         }
         w = &out.nodes[(size_t)ci * kNodeWords];
         w[4] = (uint32_t)base_child;
         w[5] = (uint32_t)base_tri;
-        std::memcpy(&w[6], meta, 8);
+        w[6] = leaves;
+        w[7] = 0;
         for (int a = 0; a < 3; ++a) {
             std::memcpy(&w[8 + 2 * a], q[a], 8);
             std::memcpy(&w[14 + 2 * a], q[3 + a], 8);
@@ -394,7 +393,8 @@ bool validate_cwbvh(const CwBvh& b, std::string* err) {
         const uint32_t* w = &b.nodes[(size_t)i * kNodeWords];
         uint32_t imask = w[3] >> 24;
         uint32_t base_child = w[4], base_tri = w[5];
-        uint8_t meta[8]; std::memcpy(meta, &w[6], 8);
+        if (w[6] >> 24) { *err = "bad leaf bits"; return false; }
+        uint32_t off = 0;
         int n_inner = __builtin_popcount(imask);
         if (n_inner > 0 && (uint64_t)base_child + n_inner > (uint64_t)b.n_nodes) { *err = "child index out of range"; return false; }
         for (int k = 0; k < n_inner; ++k) {
@@ -403,13 +403,12 @@ bool validate_cwbvh(const CwBvh& b, std::string* err) {
         }
         for (int s = 0; s < 8; ++s) {
             bool inner = (imask >> s) & 1;
-            if (inner) { if (meta[s] == 0) { *err = "inner child without meta"; return false; } continue; }
-            if (meta[s] == 0) continue;
-            uint32_t bits = meta[s] >> 5, off = meta[s] & 31;
-            int cnt = bits == 1 ? 1 : bits == 3 ? 2 : bits == 7 ? 3 : -1;
-            if (cnt < 0 || off + cnt > 24) { *err = "bad leaf meta"; return false; }
-            for (int j = 0; j < cnt; ++j) {
-                uint64_t t = (uint64_t)base_tri + off + j;
+            uint32_t bits = (w[6] >> (3 * s)) & 7u;
+            if (inner) { if (bits) { *err = "inner child with leaf bits"; return false; } continue; }
+            int cnt = bits == 0 ? 0 : bits == 1 ? 1 : bits == 3 ? 2 : bits == 7 ? 3 : -1;
+            if (cnt < 0) { *err = "bad leaf bits"; return false; }
+            for (int j = 0; j < cnt; ++j, ++off) {
+                uint64_t t = (uint64_t)base_tri + off;
                 if (t >= (uint64_t)b.n_tris) { *err = "triangle index out of range"; return false; }
                 if (seen[t]) { *err = "triangle referenced twice"; return false; }
                 seen[t] = 1;

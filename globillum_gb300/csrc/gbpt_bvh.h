@@ -18,7 +18,9 @@ namespace gb {
 // Node layout (20 x 32-bit words):
 //  w0-2  origin p (float)            w3  bytes: ex, ey, ez (biased exp), imask
 //  w4    base child node index       w5  base triangle index
-//  w6-7  meta[8] (0 = empty; leaf: unary(count)<<5 | tri offset; inner: 0x20)
+//  w6    leaf bits: slot s's triangles in unary at bits 3s .. 3s+2 (0 for
+//        inner and empty slots); a node's triangles follow its base triangle
+//        in the order of these bits      w7  0
 //  w8-9  qlo_x[8]  w10-11 qlo_y[8]  w12-13 qlo_z[8]
 //  w14-15 qhi_x[8] w16-17 qhi_y[8]  w18-19 qhi_z[8]
 static const int kNodeWords = 20;

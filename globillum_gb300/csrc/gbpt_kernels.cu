@@ -36,11 +36,12 @@ namespace gb {
 namespace {
 
 constexpr int kBlock = 128;
-// Resident 128-thread blocks per SM the traversal kernels are compiled for: 8
-// (64 registers).  1M-triangle frame, 64 spp, at 7 / 8 / 9 blocks: 37.6 / 37.1 /
-// 38.2 ms; 2 M shadow rays 333 / 321 / 348 us.
+// Resident 128-thread blocks per SM the traversal kernels are compiled for: 7
+// (72 registers, no spills).  1M-triangle frame, 64 spp, at 6 / 7 / 8 blocks:
+// 36.7 / 35.3 / 35.2 ms; 12 mixed scenes 3.26 / 3.17 / 3.22 ms; 262 K closest
+// hits 95 / 96 / 102 us; 2 M shadow rays 320 / 306 / 304 us.
 #ifndef GB_TRAV_MIN_BLOCKS
-#define GB_TRAV_MIN_BLOCKS 8
+#define GB_TRAV_MIN_BLOCKS 7
 #endif
 constexpr int kStack = 32;
 constexpr int kIterLimit = 1 << 22;
@@ -80,13 +81,19 @@ struct RayInv {
     uint32_t oxor;
 };
 
+__device__ __forceinline__ float fast_rcp(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ RayInv make_ray(v3 o, v3 d) {
     RayInv r;
     r.o = o; r.d = d;
     const float ooeps = 8.271806125530277e-25f;  // 2^-80 (tracers.cu:48-51)
-    r.idir.x = 1.0f / (fabsf(d.x) > ooeps ? d.x : copysignf(ooeps, d.x));
-    r.idir.y = 1.0f / (fabsf(d.y) > ooeps ? d.y : copysignf(ooeps, d.y));
-    r.idir.z = 1.0f / (fabsf(d.z) > ooeps ? d.z : copysignf(ooeps, d.z));
+    // one ulp off at most: only the slab tests use it, whose slack is 2e-5
+    r.idir.x = fast_rcp(fabsf(d.x) > ooeps ? d.x : copysignf(ooeps, d.x));
+    r.idir.y = fast_rcp(fabsf(d.y) > ooeps ? d.y : copysignf(ooeps, d.y));
+    r.idir.z = fast_rcp(fabsf(d.z) > ooeps ? d.z : copysignf(ooeps, d.z));
     uint32_t oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
     r.oxor = oct ^ 7u;
     return r;
@@ -155,6 +162,15 @@ __device__ __forceinline__ uint8_t* order_table() {
     __shared__ __align__(4) uint8_t t[2048];  // [octant][mask]
     return t;
 }
+// Every bit of an 8-bit mask three times over: a hit leaf's triangles are
+// those of the node's leaf bits that survive this mask.  Taken from a table
+// and without asking which hit children are leaves, instead of a loop over the
+// hit leaves (about 30 of a visit's 200 instructions): 36.7 -> 35.5 ms on the
+// 1M-triangle 64-spp frame, 3.25 -> 3.18 ms on 12 mixed scenes.
+__device__ __forceinline__ uint32_t* leaf_table() {
+    __shared__ uint32_t t[256];
+    return t;
+}
 // Bits of an 8-bit mask moved from position i to i ^ x (x in 0..7).
 __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t x) {
     if (x & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
@@ -163,8 +179,13 @@ __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t x) {
     return m;
 }
 
-// Fills order_table: all threads of the block call it before they traverse.
-__device__ __forceinline__ void fill_order_table() {
+// Fills the tables: all threads of the block call it before they traverse.
+__device__ __forceinline__ void fill_tables() {
+    for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
+        uint32_t x = (i | (i << 8)) & 0x00f00fu;
+        x = (x | (x << 4)) & 0x0c30c3u;
+        leaf_table()[i] = ((x | (x << 2)) & 0x249249u) * 7u;
+    }
     uint32_t* t = reinterpret_cast<uint32_t*>(order_table());
     for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) {
         const uint32_t x = i >> 6, m = (i & 63u) << 2, w = xor_permute8(m, x), b0 = 1u << x, b1 = 1u << (x ^ 1u);
@@ -180,7 +201,7 @@ __device__ __forceinline__ void fill_order_table() {
 // equals taking min/max of the two plane distances per child); children are
 // tested two at a time with packed FP32.  The test is conservative: a child
 // is hit when lo * (1 - 2e-5) <= min(hi, bound), on top of outward-rounded
-// boxes.  Empty slots (meta 0, imask bit 0) may test positive; they add
+// boxes.  Empty slots (no leaf bits, imask bit 0) may test positive; they add
 // neither a node nor a triangle.
 //
 // The ALU pipe (byte permutes, min/max, compares, selects; half rate) bounds
@@ -204,7 +225,7 @@ __device__ __forceinline__ uint64_t half_pair(uint32_t h) {
     return r;
 }
 __device__ __forceinline__ void intersect_node(const float4* __restrict__ nodes, uint32_t ni, const RayInv& r,
-                                               float bound, uint2* ng, uint2* tg) {
+                                               float bound, uint2* ng, uint2* tg, uint32_t* tv) {
     const float4* n = nodes + 5 * (size_t)ni;
     float4 n0 = ld_node(n + 0), n1 = ld_node(n + 1), n2 = ld_node(n + 2), n3 = ld_node(n + 3), n4 = ld_node(n + 4);
     const bool fx = r.idir.x < 0.0f, fy = r.idir.y < 0.0f, fz = r.idir.z < 0.0f;
@@ -252,15 +273,6 @@ __device__ __forceinline__ void intersect_node(const float4* __restrict__ nodes,
     }
     hm = ~hm & 0xffu;
     const uint32_t inner = hm & imask;
-    uint32_t leaf = hm & ~imask;
-    uint32_t hits_t = 0;
-    const uint32_t meta_lo = __float_as_uint(n1.z), meta_hi = __float_as_uint(n1.w);
-    while (leaf) {
-        uint32_t slot = (uint32_t)__ffs(leaf) - 1u;
-        leaf &= leaf - 1u;
-        uint32_t meta = __byte_perm(slot < 4u ? meta_lo : meta_hi, 0u, 0x4440u | (slot & 3u));
-        hits_t |= (meta >> 5) << (meta & 31u);
-    }
 #if GB_PREFETCH
     // the hit inner children will be visited: start their fetch into L2 now
     for (uint32_t m = inner; m; m &= m - 1u) {
@@ -271,13 +283,19 @@ __device__ __forceinline__ void intersect_node(const float4* __restrict__ nodes,
     }
 #endif
     *ng = make_uint2(__float_as_uint(n1.x), ((uint32_t)order_table()[(r.oxor << 8) | inner] << 24) | imask);
-    *tg = make_uint2(__float_as_uint(n1.y), hits_t);
+    // the triangles of the hit leaves, and what all their bits are counted
+    // against (n1.z, zero for inner and empty slots)
+    *tg = make_uint2(__float_as_uint(n1.y), leaf_table()[hm] & __float_as_uint(n1.z));
+    *tv = __float_as_uint(n1.z);
 }
 
 // Resumable traversal state of one ray (the node-group stack lives beside it).
 struct Trav {
-    uint2 ng, tg;
-    uint2 nt;  // second pending triangle group (policy 0)
+    uint2 ng;
+    uint2 tg;         // pending triangles: the node's first, and leaf bits still to test
+    uint32_t tv;      // the node's leaf bits: triangle of bit b = first + bits of tv below b
+    uint2 nt;         // second pending group (policy 0)
+    uint32_t nv;
     int sp;
     float best_t, bb, bg;
     uint32_t best_id;
@@ -305,9 +323,9 @@ __device__ __forceinline__ void trav_init(Trav& s, const RayInv& r, float tmax) 
 template <bool INSTR>
 __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const RayInv& r, bool any, Trav& s,
                                          uint32_t* ntri) {
-    int b = __ffs(s.tg.y) - 1;
-    s.tg.y &= s.tg.y - 1u;
-    const float4* tp = tris + 3 * (size_t)(s.tg.x + (uint32_t)b);
+    const uint32_t below = s.tg.y - 1u;  // bits below the lowest one, and the others less it
+    const float4* tp = tris + 3 * (size_t)(s.tg.x + (uint32_t)__popc(s.tv & below & ~s.tg.y));
+    s.tg.y &= below;
     float4 a0 = ld_tri(tp + 0), a1 = ld_tri(tp + 1), a2 = ld_tri(tp + 2);
     if (INSTR) ++*ntri;
     // intersect_tri with its conditions joined at the end (the same operations;
@@ -332,7 +350,8 @@ __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const 
 // true when the stack overflows.
 template <bool INSTR, int STACK = kStack>
 __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
-                                           const StackRef& stack, uint32_t* status, uint32_t* nvis, uint2* tg) {
+                                           const StackRef& stack, uint32_t* status, uint32_t* nvis, uint2* tg,
+                                           uint32_t* tv) {
     const uint32_t k = 31u - (uint32_t)__clz(s.ng.y);
     s.ng.y &= ~(1u << k);
     const uint32_t slot = (k - 24u) ^ r.oxor;
@@ -343,7 +362,7 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
         stack_put(stack, s.sp++, s.ng);
     }
     if (INSTR) ++*nvis;
-    intersect_node(nodes, child, r, s.best_t, &s.ng, tg);
+    intersect_node(nodes, child, r, s.best_t, &s.ng, tg, tv);
     return false;
 }
 
@@ -353,8 +372,15 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
 template <bool INSTR, int STACK = kStack>
 __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
                                           const StackRef& stack, uint32_t* status, uint32_t* nvis) {
-    if (s.ng.y > 0x00ffffffu)
-        return visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &s.tg);
+    if (s.ng.y > 0x00ffffffu) {
+        const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &s.tg, &s.tv);
+        // these policies stack groups and hand them to other lanes: bits without gaps, for any tv
+        uint32_t m = 0;
+        for (uint32_t left = s.tg.y; left; left &= left - 1u) m |= 1u << __popc(s.tv & (left - 1u) & ~left);
+        s.tg.y = m;
+        s.tv = 0xffffffffu;
+        return over;
+    }
     if (s.sp > 0) {
         uint2 g = stack_get(stack, --s.sp);
         if (g.y > 0x00ffffffu) s.ng = g;
@@ -398,6 +424,7 @@ __device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint
             const bool found = tri_step<INSTR>(tris, r, any, s, ntri);
             if (s.tg.y == 0u) {
                 s.tg = s.nt;
+                s.tv = s.nv;
                 s.nt.y = 0u;
             }
             if (found) trav_stop(s);
@@ -405,9 +432,15 @@ __device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint
     } else if (node) {
         if (s.ng.y <= 0x00ffffffu) s.ng = stack_get(stack, --s.sp);
         uint2 tg = make_uint2(0u, 0u);
-        const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg);
-        if (s.tg.y == 0u) s.tg = tg;
-        else s.nt = tg;
+        uint32_t tv = 0u;
+        const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg, &tv);
+        if (s.tg.y == 0u) {
+            s.tg = tg;
+            s.tv = tv;
+        } else {
+            s.nt = tg;
+            s.nv = tv;
+        }
         if (over) trav_stop(s);
     }
 }
@@ -854,9 +887,11 @@ __device__ __forceinline__ bool coop_triangles(bool act, const float4* tris, con
 // done.  A warp that makes kIterLimit steps without a refill gives up.
 constexpr uint32_t kAnyHit = 0x80000000u;
 
+// nodes0, tris0: the tree every lane starts with (fetch may change it).
 template <bool INSTR, int MODE, int STACK, int BT, typename Fetch, typename Finish>
-__device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int refill, uint32_t* status, Fetch fetch,
-                                         Finish finish, uint32_t* nvis, uint32_t* ntri) {
+__device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int refill, uint32_t* status,
+                                         const float4* nodes0, const float4* tris0, Fetch fetch, Finish finish,
+                                         uint32_t* nvis, uint32_t* ntri) {
     const uint32_t lane = lane_id();
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     const uint32_t dyn0 = nwarps * 32u;
@@ -869,8 +904,8 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
     __shared__ uint2 s_stack[kSmemStack > 0 ? kSmemStack * BT : 1];
     uint2 deep[STACK - kSmemStack];
     const StackRef stack{s_stack + threadIdx.x, deep, BT};
-    const float4* nodes = nullptr;
-    const float4* tris = nullptr;
+    const float4* nodes = nodes0;
+    const float4* tris = tris0;
     const float4* shade = nullptr;
     __shared__ unsigned long long s_key[MODE == 3 ? BT : 1];
     unsigned long long* skey = s_key + (MODE == 3 ? (threadIdx.x & ~31u) : 0u);
@@ -981,7 +1016,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
                                                                       const float* __restrict__ tmaxv, float4* hits,
                                                                       uint8_t* occluded, int any, uint32_t* head,
                                                                       uint32_t* status) {
-    fill_order_table();
+    fill_tables();
     uint32_t nvis = 0, ntri = 0;
     const uint32_t flag = any ? kAnyHit : 0u;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
@@ -992,9 +1027,6 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
         *d = mk(pd[0], pd[1], pd[2]);
         const float t = tmaxv[q];
         *tmax = t >= 0.0f ? t : -1.0f;
-        *nodes = S.nodes;
-        *tris = S.tris;
-        *shade = S.shade;
     };
     auto finish = [&](uint32_t handle, const Trav& h) {
         const uint32_t i = handle & ~kAnyHit;
@@ -1002,7 +1034,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
         if (any) occluded[i] = hit ? 1 : 0;
         else hits[i] = make_float4(hit ? h.best_t : FLT_MAX, h.bb, h.bg, __uint_as_float(h.best_id));
     };
-    ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, fetch, finish, &nvis, &ntri);
+    ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, S.nodes, S.tris, fetch, finish, &nvis, &ntri);
 }
 
 // Whether the chunk's loop stops before iteration `it` and leaves its queues
@@ -1021,7 +1053,7 @@ __device__ __forceinline__ bool left_to_finish(const Frame& F, const RenderParam
 // to go on, so the loop ends with one iteration on empty queues.
 // STACK: traversal stack entries; BT: threads per block (the register budget
 // is that of GB_TRAV_MIN_BLOCKS blocks of 128 threads).
-template <bool INSTR, int MODE, int STACK, int BT>
+template <bool INSTR, int MODE, int STACK, int BT, bool MULTI>
 __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Frame F, RenderParams P,
                                                                             unsigned long long cond, int has_cond) {
     const int it = F.iter[0];
@@ -1046,7 +1078,7 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
         if (has_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, work && it < P.max_iters ? 1u : 0u);
     }
     if (leave) return;
-    fill_order_table();
+    fill_tables();
     const uint32_t *qe = F.q[it & 1], *qs = F.q[2];
     uint32_t nvis = 0, ntri = 0, nvis_any = 0, ntri_any = 0;
     auto fetch = [&](uint32_t q, uint32_t* handle, v3* o, v3* d, float* tmax, const float4** nodes,
@@ -1058,7 +1090,7 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
             *handle = slot;
             r = rec_ld(&F.ray[slot]);
             *tmax = FLT_MAX;
-            sc = scene_of(F, r.w[7]);
+            sc = MULTI ? scene_of(F, r.w[7]) : 0u;
         } else {
             const uint32_t slot = qs[q - next];
             *handle = slot | kAnyHit;
@@ -1066,10 +1098,12 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
             *tmax = __uint_as_float(r.w[6]);
             sc = r.w[7];
         }
-        const SceneRec& R = F.scenes[sc];
-        *nodes = R.S.nodes;
-        *tris = R.S.tris;
-        *shade = R.S.shade;
+        if (MULTI) {
+            const SceneRec& R = F.scenes[sc];
+            *nodes = R.S.nodes;
+            *tris = R.S.tris;
+            *shade = R.S.shade;
+        }
         *o = sec3(r, 0);
         *d = sec3(r, 3);
     };
@@ -1084,7 +1118,8 @@ __global__ void __launch_bounds__(BT, GB_TRAV_MIN_BLOCKS * 128 / BT) k_rays(Fram
             ntri = 0;
         }
     };
-    ray_loop<INSTR, MODE, STACK, BT>(next + nsh, cs + CTR_HEAD, P.refill, F.status, fetch, finish, &nvis, &ntri);
+    ray_loop<INSTR, MODE, STACK, BT>(next + nsh, cs + CTR_HEAD, P.refill, F.status, MULTI ? nullptr : P.nodes,
+                                     MULTI ? nullptr : P.tris, fetch, finish, &nvis, &ntri);
     if (INSTR) {
         add_stats(&F.stats[5], nvis_any);
         add_stats(&F.stats[6], ntri_any);
@@ -1517,7 +1552,7 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
 
 template <bool TEX>
 __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P, const MrgPowers J) {
-    fill_order_table();
+    fill_tables();
     const uint32_t l = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
     const bool alive = l < P.chunk_paths;
     const PathStart ps = path_start(F, P, alive ? l : 0u, &J);
@@ -1537,7 +1572,7 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F
     const uint32_t* cs = ctr_set(F, it);
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
     if (blockIdx.x * GB_PATHS_BLOCK >= count) return;
-    fill_order_table();
+    fill_tables();
     const uint32_t i = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
     if ((i & ~31u) >= count) return;
     const bool alive = i < count;
@@ -1731,7 +1766,7 @@ template <bool HYBRID>
 __global__ void __launch_bounds__(GB_DIRECT_BLOCK, GB_DIRECT_MIN) k_direct(
     DevScene S, CameraRec cam, int w, int h, int cam_samples, int light_samples, uint32_t seed, float shadow_offset,
     v3 background, float* out, uint32_t* status, const MrgSubseqTable T) {
-    fill_order_table();
+    fill_tables();
     const int g0 = blockIdx.x * GB_DIRECT_BLOCK + threadIdx.x;
     const bool mine = g0 < w * h;
     const int g = mine ? g0 : 0;  // idle threads of the last block trace nothing
@@ -2165,23 +2200,29 @@ void launch_traversal(K kernel, dim3 grid, int block, const RenderParams& P, cud
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <bool INSTR, int MODE, int STACK, int BT>
+template <bool INSTR, int MODE, int STACK, int BT, bool MULTI>
 void launch_rays_v(const Frame& F, const RenderParams& P, unsigned long long cond, bool has_cond, cudaStream_t st) {
-    static Grid g = persistent_grid(k_rays<INSTR, MODE, STACK, BT>, BT);
-    launch_traversal(k_rays<INSTR, MODE, STACK, BT>, traversal_grid(g, P.blocks_per_sm, BT), BT, P, st, F, P, cond,
+    static Grid g = persistent_grid(k_rays<INSTR, MODE, STACK, BT, MULTI>, BT);
+    launch_traversal(k_rays<INSTR, MODE, STACK, BT, MULTI>, traversal_grid(g, P.blocks_per_sm, BT), BT, P, st, F, P, cond,
                      has_cond ? 1 : 0);
 }
 
 // The default triangle policy has variants for two stack depths and two
-// block shapes (RenderParams::trav_variant), the other policies one each.
+// block shapes (RenderParams::trav_variant) and for frames of one scene, whose
+// tree is a kernel parameter (four registers less); the other policies have
+// one each.
+template <bool INSTR, bool MULTI>
+void launch_rays_0(const Frame& F, const RenderParams& P, unsigned long long c, bool h, cudaStream_t st) {
+    if (P.trav_variant == 1) launch_rays_v<INSTR, 0, 24, 128, MULTI>(F, P, c, h, st);
+    else if (P.trav_variant == 2) launch_rays_v<INSTR, 0, 32, 64, MULTI>(F, P, c, h, st);
+    else if (P.trav_variant == 3) launch_rays_v<INSTR, 0, 24, 64, MULTI>(F, P, c, h, st);
+    else launch_rays_v<INSTR, 0, kStack, kBlock, MULTI>(F, P, c, h, st);
+}
 template <bool INSTR, int MODE>
 void launch_rays_t(const Frame& F, const RenderParams& P, unsigned long long c, bool h, cudaStream_t st) {
-    if constexpr (MODE == 0) {
-        if (P.trav_variant == 1) return launch_rays_v<INSTR, MODE, 24, 128>(F, P, c, h, st);
-        if (P.trav_variant == 2) return launch_rays_v<INSTR, MODE, 32, 64>(F, P, c, h, st);
-        if (P.trav_variant == 3) return launch_rays_v<INSTR, MODE, 24, 64>(F, P, c, h, st);
-    }
-    launch_rays_v<INSTR, MODE, kStack, kBlock>(F, P, c, h, st);
+    if constexpr (MODE != 0) launch_rays_v<INSTR, MODE, kStack, kBlock, true>(F, P, c, h, st);
+    else if (P.nodes) launch_rays_0<INSTR, false>(F, P, c, h, st);
+    else launch_rays_0<INSTR, true>(F, P, c, h, st);
 }
 
 cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument, unsigned long long c, bool h,

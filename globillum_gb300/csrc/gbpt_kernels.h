@@ -215,6 +215,8 @@ struct RenderParams {
     int pad_;
     int max_iters;     // iteration bound of the chunk's loop
     int finish_max;    // the loop leaves the chunk's last paths to k_finish once at most this many are alive (0: never)
+    const float4* nodes;  // the tree of a frame of one scene (null: every lane has its own scene's)
+    const float4* tris;
     // L2 window of the traversal launches (GB_NODE_L2_PERSIST, frames of one
     // scene): the scene's node array, accessed as persisting
     const void* l2_nodes;

@@ -192,6 +192,8 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     P.refill = 16;
     P.tri_mode = 0;
     P.blocks_per_sm = 0;
+    P.nodes = R.S.nodes;
+    P.tris = R.S.tris;
     P.rounds = 1;
     P.pool_round = 1;
     P.round_start[0] = 0;

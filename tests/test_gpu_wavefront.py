@@ -163,3 +163,31 @@ def test_direct_light_sample_groups(gpu_ctx, w, h, cams, lights, sky):
     assert np.array_equal(s.render_hybrid_direct(sc.camera, rd, cams, lights),
                           orc.render_hybrid_direct(sc.camera, rd, cams, lights, pool))
     s.close()
+
+
+@pytest.mark.parametrize("builder", ["host", "device"])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 9, 24, 25, 77])
+def test_small_trees_under_every_policy(gpu_ctx, builder, n):
+    """Trees of one node and of a few, with leaves of one to three triangles in
+    any slot: the leaf bits of a node name the right triangles for the voting
+    policy, the postponing ones (groups on the stack) and the cooperative one."""
+    from oracle import oracle
+    rng = np.random.default_rng(n)
+    c = rng.uniform(-2, 2, (n, 1, 3))
+    pos = (c + rng.uniform(-1, 1, (n, 3, 3))).astype(np.float32).reshape(n, 9)
+    base = scenes.cornell(width=24, height=20, spp=2, max_bounces=3)
+    sc = scenes.SceneData(pos, None, np.zeros(n, np.int32), base.materials, [],
+                          [dict(base.lights[0], center=(0.0, 5.0, 0.0), wh=(2.0, 2.0))],
+                          dict(base.camera, pos=(0.0, 0.0, -6.0)), dict(base.render, rng_mode=gbpt.GB_RNG_MRG32K3A_POOL))
+    s = gpu_ctx.scene(sc, builder=builder)
+    pool = gpu_ctx.mrg_pool(24 * 20, 2 * 3)
+    ref = oracle.OracleScene(sc, use_bvh=False).render(sc.camera, sc.render, pool).astype(np.float32)
+    old = gpu_ctx.get_tuning()
+    try:
+        for mode in (1, 2, 3, 4):
+            for graph in (1, 2):
+                gpu_ctx.set_tuning(tri_mode=mode, graph=graph)
+                assert np.array_equal(s.render(sc.camera, sc.render), ref), (mode, graph)
+    finally:
+        gpu_ctx.set_tuning(tri_mode=old["tri_mode"], graph=old["graph"])
+        s.close()
