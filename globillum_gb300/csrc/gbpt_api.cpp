@@ -30,7 +30,7 @@ static const size_t kMaxGraphs = 16, kStatWords = 16;
 
 // Chunks of at most kPathsMax paths run in k_paths, the last kFinishMax paths of
 // larger ones in k_finish (measured at follow_paths).
-static const int kPathsMax = 1 << 18, kFinishMax = 1 << 16;
+static const int kPathsMax = 3 << 16, kFinishMax = 1 << 16;
 
 // One scene of a frame as the host sees it.
 struct BatchScene {

@@ -1447,11 +1447,12 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 // A queue that does not fill the chip is bound by latency: each bounce costs
 // the loop two launches, a tail of long rays and a round trip of the path
 // state, whatever the work: 250 us for the 64x64 room at 1 and at 4 spp.
-// Wall time of a frame, loop against k_paths (us, paths in thousands):
-//   room      4K 249 / 153   48K 269 / 169   128K 312 / 267   256K 393 / 368   512K 569 / 628
-//   64 K tri  6K 393 / 215   48K 434 / 247   144K 493 / 336   250K 539 / 431
-//   512 K tri               48K 485 / 287   144K 536 / 440   225K 618 / 526
-// hence k_paths up to 2^18 paths.  The last paths of a chunk at 0 / 2^14 /
+// Wall time of a frame, the loop with k_finish for its last paths against
+// k_paths (us, paths in thousands):
+//   room      4K 140 / 117   48K 157 / 130   128K 241 / 229   256K 328 / 341   512K 478 / 624
+//   64 K tri  6K 181 / 164   48K 221 / 201   144K 319 / 283   250K 350 / 376
+//   512 K tri               48K 254 / 231   144K 355 / 378   225K 403 / 448
+// hence k_paths up to 3 * 2^16 paths.  The last paths of a chunk at 0 / 2^14 /
 // 2^15 / 2^16 / 2^17 / 2^18 alive: 1 spp of the 1M-triangle frame 1303 / 1187
 // / 1187 / 1097 / 1149 / 1146, textured sky 1231 / 1195 / 1113 / 1140 / 1131 /
 // 1151, 12 mixed scenes 3692 / 3635 / 3628 / 3632 / 3634 / 3594: 2^16.

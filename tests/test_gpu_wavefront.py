@@ -43,10 +43,11 @@ def test_path_counts_and_pools(gpu_ctx, w, h, spp, slots, bounces, graph):
         gpu_ctx.set_tuning(slots=old["slots"], graph=old["graph"])
 
 
-@pytest.mark.parametrize("w,h,spp,slots", [(512, 512, 1, 0), (513, 512, 1, 0), (300, 310, 3, 5000), (257, 129, 16, 0)])
+@pytest.mark.parametrize("w,h,spp,slots", [(512, 384, 1, 0), (513, 384, 1, 0), (512, 512, 1, 0), (513, 512, 1, 0),
+                                           (300, 310, 3, 5000), (257, 129, 16, 0)])
 @pytest.mark.parametrize("kind", ["room", "textured"])
 def test_finish_of_a_chunk(gpu_ctx, w, h, spp, slots, kind):
-    """Chunks at and above the 2^18 paths of k_paths: the graph's loop leaves
+    """Chunks at and above the 3 * 2^16 paths of k_paths: the graph's loop leaves
     its last paths to k_finish; the host-driven loop does not.  Same frames,
     same ray counts."""
     if kind == "room":
