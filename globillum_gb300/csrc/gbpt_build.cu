@@ -67,7 +67,7 @@ __global__ void k_check_finite(const float* __restrict__ v, size_t n, int* bad) 
 // its material index) and the three normals (the face normal without any).
 // Nothing is written when a vertex was not finite.  On the host this loop and
 // the copy of its 96 B per triangle took most of a refit (205 K triangles:
-// refit and a 2-spp frame 5.4 ms; 0.86 ms here, 0.28 ms of it the refit).
+// refit and a 2-spp frame 5.4 ms; 0.86 ms with this kernel, 10 us of it here).
 __global__ void k_shade_records(const float* __restrict__ pos, const float* __restrict__ nrm, int n, float4* shade,
                                 const int* __restrict__ bad) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -261,10 +261,9 @@ __global__ void k_ploc_compact(const int* __restrict__ nn, int n, int inner_base
 // ------------------------------------------------------------ bottom-up pass
 // One thread per leaf climbs towards the root; the second thread to reach a
 // node combines its children (Karras, "Maximizing Parallelism in the
-// Construction of BVHs, Octrees, and k-d Trees", HPG 2012).  Build mode:
-// subtree triangle counts and the leaf rule of the host builder (a node of
-// at most kLeafMax triangles is stored as one leaf when count <= 0.5 +
-// (A_l c_l + A_r c_r) / A).  Refit mode: boxes from the moved vertices.
+// Construction of BVHs, Octrees, and k-d Trees", HPG 2012): subtree triangle
+// counts and the leaf rule of the host builder (a node of at most kLeafMax
+// triangles is stored as one leaf when count <= 0.5 + (A_l c_l + A_r c_r) / A).
 // bad = 2 if a parent chain is longer than the tree.
 // SAH-optimal 8-wide grouping (WideDp of gbpt_bvh.cpp), when dcost is
 // given: dcost[8v + i-1] = least cost of v's subtree as at most i slots of
@@ -302,26 +301,19 @@ __device__ void wide_dp_node(int v, int l, int r, int cnt, float area, float pri
     }
 }
 
-__global__ void k_bottom_up(int n, const int* __restrict__ bparent, const int2* __restrict__ bchild, float4* blo,
-                            float4* bhi, int* bcount, uint8_t* bleaf, unsigned* visit, const float* __restrict__ pos,
-                            int refit, int* bad, float* dcost, int8_t* dhow, int8_t* dsplit, float prim_cost) {
+__global__ void k_bottom_up(int n, const int* __restrict__ bparent, const int2* __restrict__ bchild,
+                            const float4* __restrict__ blo, const float4* __restrict__ bhi, int* bcount,
+                            uint8_t* bleaf, unsigned* visit, int* bad, float* dcost, int8_t* dhow, int8_t* dsplit,
+                            float prim_cost) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (refit) {
-        if (bad[1]) return;  // a vertex is not finite: the tree stays as it is
-        float4 lo, hi;
-        tri_box(pos, ~bchild[i].x, &lo, &hi);
-        blo[i] = lo;
-        bhi[i] = hi;
-    } else {
-        bcount[i] = 1;
-        bleaf[i] = 1;
-        if (dcost) {
-            const float c = box_area(blo[i], bhi[i]) * prim_cost;
-            for (int k = 0; k < 8; ++k) {
-                dcost[8 * (size_t)i + k] = c;
-                dhow[8 * (size_t)i + k] = k == 0 ? 1 : 0;
-            }
+    bcount[i] = 1;
+    bleaf[i] = 1;
+    if (dcost) {
+        const float c = box_area(blo[i], bhi[i]) * prim_cost;
+        for (int k = 0; k < 8; ++k) {
+            dcost[8 * (size_t)i + k] = c;
+            dhow[8 * (size_t)i + k] = k == 0 ? 1 : 0;
         }
     }
     int node = bparent[i];
@@ -334,22 +326,15 @@ __global__ void k_bottom_up(int n, const int* __restrict__ bparent, const int2* 
         if (atomicAdd(&visit[node], 1u) == 0u) return;  // the sibling's thread continues
         __threadfence();
         int2 c = bchild[node];
-        float4 llo = __ldcg(&blo[c.x]), lhi = __ldcg(&bhi[c.x]);
-        float4 rlo = __ldcg(&blo[c.y]), rhi = __ldcg(&bhi[c.y]);
-        if (refit) {
-            blo[node] = vmin(llo, rlo);
-            bhi[node] = vmax(lhi, rhi);
-        } else {
-            int cl = __ldcg(&bcount[c.x]), cr = __ldcg(&bcount[c.y]);
-            int cnt = cl + cr;
-            bcount[node] = cnt;
-            float pa = box_area(blo[node], bhi[node]);
-            float best = box_area(llo, lhi) * (float)cl + box_area(rlo, rhi) * (float)cr;
-            float split = 0.5f + (pa > 0.0f ? best / pa : 0.0f);
-            bleaf[node] = (cnt <= kLeafMax && (float)cnt <= split) ? 1 : 0;
-            if (dcost) wide_dp_node(node, c.x, c.y, cnt, pa, prim_cost, dcost, dhow, dsplit, bleaf);
-            __threadfence();
-        }
+        int cl = __ldcg(&bcount[c.x]), cr = __ldcg(&bcount[c.y]);
+        int cnt = cl + cr;
+        bcount[node] = cnt;
+        float pa = box_area(blo[node], bhi[node]);
+        float best = box_area(blo[c.x], bhi[c.x]) * (float)cl + box_area(blo[c.y], bhi[c.y]) * (float)cr;
+        float split = 0.5f + (pa > 0.0f ? best / pa : 0.0f);
+        bleaf[node] = (cnt <= kLeafMax && (float)cnt <= split) ? 1 : 0;
+        if (dcost) wide_dp_node(node, c.x, c.y, cnt, pa, prim_cost, dcost, dhow, dsplit, bleaf);
+        __threadfence();
         node = bparent[node];
     }
 }
@@ -464,7 +449,7 @@ __global__ void k_collapse_plan(const int* __restrict__ q, int m, int node_base,
     unsigned long long n_inner = 0, n_tri = 0;
     for (int s = 0; s < 8; ++s) {
         int c = slot_child[s];
-        plan[(size_t)(node_base + k) * 8 + s] = c;
+        plan[(size_t)k * 8 + s] = c;
         if (c < 0) continue;
         if (bleaf[c]) n_tri += (unsigned long long)bcount[c];
         else ++n_inner;
@@ -473,15 +458,30 @@ __global__ void k_collapse_plan(const int* __restrict__ q, int m, int node_base,
 }
 
 // Smallest e >= -100 with 255 * 2^e >= ext (the exponent rule of the host
-// collapse), from the binary exponent of ext / 255.
-__device__ int plane_exponent(float ext) {
+// collapse), from the bits of ext: 255 is 0x1.fep7.  ext = inf (boxes of
+// vertices near the type's largest value) gives the rule's 1017.
+__device__ __forceinline__ int plane_exponent(float ext) {
     if (!(ext > 0.0f)) return -100;
-    int k;
-    double mant = frexp((double)ext / 255.0, &k);
-    int e = mant == 0.5 ? k - 1 : k;
-    while (ldexp(255.0, e) < (double)ext) ++e;
-    while (e > -100 && ldexp(255.0, e - 1) >= (double)ext) --e;
-    return max(e, -100);
+    const uint32_t u = __float_as_uint(ext);
+    if (u == 0x7f800000u) return 1017;
+    return max((int)(u >> 23) - 134 + ((u & 0x7fffffu) > 0x7f0000u ? 1 : 0), -100);
+}
+
+// floor (UP: ceil) of (v - o) / 2^e in double, within [0, 255].  The float
+// difference rounds monotonically, so it can be on another side of a multiple
+// of 2^e than the exact one only where it is that multiple; there (or where
+// the quotient underflowed or is no number) the double operations decide.
+// A multiprocessor does 2 of them a clock, and 128 float ones.
+template <bool UP>
+__device__ __forceinline__ int plane_quantise(float v, float o, float rsc) {
+    const float d = v - o, t = d * rsc;
+    const float bb = d - v, err = (v - (d - bb)) + (-o - bb);  // Knuth's two-sum: d + err = v - o
+    float q = UP ? ceilf(t) : floorf(t);
+    if (!(t <= 255.0f) || (t == q && (err != 0.0f || (t == 0.0f && d != 0.0f)))) {
+        const double x = ((double)v - (double)o) * (double)rsc;
+        return (int)fmax(0.0, fmin(255.0, UP ? ceil(x) : floor(x)));
+    }
+    return (int)fmaxf(0.0f, q);
 }
 
 __device__ __forceinline__ uint32_t pack4(const uint8_t* b) {
@@ -489,36 +489,29 @@ __device__ __forceinline__ uint32_t pack4(const uint8_t* b) {
 }
 
 // Writes the 8-wide node of each planned item and the triangle records of
-// its leaf children.  Build mode: child and triangle bases from the scan
-// of the plan's counts, inner children queued for the next level, the last
-// item writing (inner children, triangles) of the level to totals.  Refit
-// mode (q unused, item = node index): bases from the node being rewritten.
-// bad = 3 if an index would leave its buffer (nothing is written there).
+// its leaf children: child and triangle bases from the scan of the plan's
+// counts, inner children queued for the next level with the node as their
+// parent, the last item writing (inner children, triangles) of the level to
+// totals.  bad = 3 if an index would leave its buffer (nothing is written
+// there).
 __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_base, int next_base, int tri_base,
                                 const unsigned long long* __restrict__ offs,
                                 const unsigned long long* __restrict__ flags, const float4* __restrict__ blo,
                                 const float4* __restrict__ bhi, const int2* __restrict__ bchild,
                                 const uint8_t* __restrict__ bleaf, int n, const float* __restrict__ pos,
-                                uint4* nodes, float4* tris, int* q_next, int node_cap, int2* totals, int refit,
+                                uint4* nodes, float4* tris, int* parent, int* q_next, int node_cap, int2* totals,
                                 int* bad) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m || (refit && bad[1])) return;
+    if (k >= m) return;
     int cw = node_base + k;
     if (cw >= node_cap) { atomicExch(bad, 3); return; }
-    int base_child, base_tri;
-    if (refit) {
-        uint4 w4 = nodes[(size_t)cw * 5 + 1];
-        base_child = (int)w4.x;
-        base_tri = (int)w4.y;
-    } else {
-        base_child = next_base + (int)(offs[k] >> 32);
-        base_tri = tri_base + (int)(offs[k] & 0xffffffffull);
-    }
+    const int base_child = next_base + (int)(offs[k] >> 32);
+    const int base_tri = tri_base + (int)(offs[k] & 0xffffffffull);
     int slot[8];
     float4 clo[8], chi[8];
     float4 nlo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f), nhi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
     for (int s = 0; s < 8; ++s) {
-        slot[s] = plan[(size_t)cw * 8 + s];
+        slot[s] = plan[(size_t)k * 8 + s];
         if (slot[s] < 0) continue;
         clo[s] = blo[slot[s]];
         chi[s] = bhi[slot[s]];
@@ -527,12 +520,11 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
         nhi = vmax(nhi, chi[s]);
     }
     int ex[3];
-    float sc[3];
-    double rsc[3];  // 1 / sc, exact: a double division costs some 20 operations of a pipe that does 2 a clock per SM
+    float sc[3], rsc[3];  // rsc = 1 / sc, exact
     for (int a = 0; a < 3; ++a) {
         ex[a] = plane_exponent(comp(nhi, a) - comp(nlo, a));
         sc[a] = ldexpf(1.0f, ex[a]);
-        rsc[a] = 1.0 / (double)sc[a];
+        rsc[a] = ldexpf(1.0f, -ex[a]);
     }
     uint32_t leaves = 0;  // 3 bits per slot: a leaf's triangles in unary
     uint8_t qv[6][8];
@@ -544,10 +536,8 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
         if (c < 0) continue;
         for (int a = 0; a < 3; ++a) {
             float o = comp(nlo, a), l = comp(clo[s], a), h = comp(chi[s], a);
-            double dl = ((double)l - (double)o) * rsc[a];
-            double dh = ((double)h - (double)o) * rsc[a];
-            int ql = (int)fmax(0.0, fmin(255.0, floor(dl)));
-            int qh = (int)fmax(0.0, fmin(255.0, ceil(dh)));
+            int ql = plane_quantise<false>(l, o, rsc[a]);
+            int qh = plane_quantise<true>(h, o, rsc[a]);
             while (ql > 0 && o + (float)ql * sc[a] > l) --ql;
             while (qh < 255 && o + (float)qh * sc[a] < h) ++qh;
             qv[a][s] = (uint8_t)ql;
@@ -557,7 +547,8 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
             imask |= 1u << s;
             int child = base_child + k_inner;
             if (child >= node_cap) { atomicExch(bad, 3); return; }
-            if (!refit) q_next[child - next_base] = c;
+            q_next[child - next_base] = c;
+            parent[child] = cw;
             ++k_inner;
             continue;
         }
@@ -601,9 +592,148 @@ __global__ void k_collapse_emit(const int* __restrict__ plan, int m, int node_ba
     }
     for (int j = 0; j < 5; ++j)
         nodes[(size_t)cw * 5 + j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-    if (!refit && k == m - 1) {
+    if (k == m - 1) {
         unsigned long long f = flags[k], o = offs[k];
         *totals = make_int2((int)(o >> 32) + (int)(f >> 32), (int)(o & 0xffffffffull) + (int)(f & 0xffffffffull));
+    }
+}
+
+// Least and greatest of a float over the 8 lanes of a group.
+__device__ __forceinline__ float min8(unsigned gm, float v) {
+    for (int o = 4; o; o >>= 1) v = fminf(v, __shfl_xor_sync(gm, v, o));
+    return v;
+}
+__device__ __forceinline__ float max8(unsigned gm, float v) {
+    for (int o = 4; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(gm, v, o));
+    return v;
+}
+
+// Boxes, planes and triangle records of a built tree for moved vertices, with
+// its child and triangle bases, slots and leaves: what k_collapse_emit would
+// write for the same grouping.  A group of 8 lanes per 8-wide node, a lane per
+// slot.  Groups of nodes without inner children start; the group that brings a
+// node its last inner child goes on with that node, so a climb is as long as
+// the 8-wide tree is deep.  box: each node's own box (no padding), for its
+// parent; arrived: inner children done.  Every min and max is exact, so the
+// boxes are those of the binary tree, which need not be kept.
+// Bound by instruction issue (groups of a warp diverge as they climb) and the
+// latency of the climb.  205 K triangles: 59 us, against 72 + 63 us for a
+// climb of the binary tree and a thread per 8-wide node after it (50 us of that
+// in double operations); refit and a 2-spp frame 725 -> 650 us.  Kept for a
+// refit: 4 B per 8-wide node, where the binary tree took 90 B per triangle.
+// bad[0] = 2: a parent that does not come before its child; 3: an index
+// outside its buffer.
+__global__ void __launch_bounds__(kBuildBlock) k_refit(const float* __restrict__ pos, int n, int n_nodes,
+                                                       const int* __restrict__ parent, uint4* nodes, float4* tris,
+                                                       float4* box, unsigned* arrived, int* bad) {
+    const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
+    const int s = threadIdx.x & 7;
+    const unsigned gm = 0xffu << (threadIdx.x & 24);
+    if (g >= n_nodes || bad[1]) return;  // a vertex is not finite: the tree stays as it is
+    int cw = (int)g;
+    uint32_t imask = nodes[(size_t)cw * 5].w >> 24;
+    if (imask) return;
+    for (;;) {
+        const uint4 w1 = nodes[(size_t)cw * 5 + 1];
+        int up = parent[cw];
+        if (up >= cw) {
+            atomicExch(bad, 2);
+            up = -1;
+        }
+        const uint32_t up_mask = up >= 0 ? nodes[(size_t)up * 5].w >> 24 : 0u;
+        const int cnt = __popc((w1.z >> (3 * s)) & 7u);
+        const bool inner = (imask >> s) & 1u;
+        float4 lo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f), hi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
+        bool used = false;
+        if (inner) {
+            const uint32_t child = w1.x + __popc(imask & ((1u << s) - 1u));
+            if (child < (uint32_t)n_nodes) {
+                lo = __ldcg(&box[2 * (size_t)child]);
+                hi = __ldcg(&box[2 * (size_t)child + 1]);
+                used = true;
+            } else {
+                atomicExch(bad, 3);
+            }
+        } else {
+            const uint32_t first = w1.y + __popc(w1.z & ((1u << (3 * s)) - 1u));
+            // all loads before the first store, so that their latencies overlap
+            uint32_t id[kLeafMax];
+            float v[kLeafMax][9];
+#pragma unroll
+            for (int j = 0; j < kLeafMax; ++j)
+                id[j] = j < cnt && first + j < (uint32_t)n ? __float_as_uint(tris[3 * (size_t)(first + j)].w) : 0xffffffffu;
+#pragma unroll
+            for (int j = 0; j < kLeafMax; ++j)
+                if (id[j] < (uint32_t)n)
+                    for (int e = 0; e < 9; ++e) v[j][e] = pos[9 * (size_t)id[j] + e];
+#pragma unroll
+            for (int j = 0; j < kLeafMax; ++j) {
+                if (j >= cnt) continue;
+                if (id[j] >= (uint32_t)n) { atomicExch(bad, 3); continue; }
+                const size_t at = 3 * (size_t)(first + j);
+                const float4 a = make_float4(v[j][0], v[j][1], v[j][2], __uint_as_float(id[j]));
+                const float4 b = make_float4(v[j][3], v[j][4], v[j][5], 0.0f);
+                const float4 c = make_float4(v[j][6], v[j][7], v[j][8], 0.0f);
+                tris[at] = a;
+                tris[at + 1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, 0.0f);
+                tris[at + 2] = make_float4(c.x - a.x, c.y - a.y, c.z - a.z, 0.0f);
+                const float4 l = vmin(vmin(a, b), c), h = vmax(vmax(a, b), c);
+                lo = used ? vmin(lo, l) : l;
+                hi = used ? vmax(hi, h) : h;
+                used = true;
+            }
+        }
+        const float4 blo = make_float4(min8(gm, lo.x), min8(gm, lo.y), min8(gm, lo.z), 0.0f);
+        const float4 bhi = make_float4(max8(gm, hi.x), max8(gm, hi.y), max8(gm, hi.z), 0.0f);
+        if (used) pad_box_d(&lo, &hi);
+        uint32_t plane[6];  // the slot's byte of each plane, then the plane's four bytes of the half group
+        float org[3];
+        uint32_t exw = imask << 24;
+        for (int a = 0; a < 3; ++a) {
+            const float l = comp(lo, a), h = comp(hi, a);
+            const float o = min8(gm, l), e = max8(gm, h) - o;
+            const int ex = plane_exponent(e);
+            const float sc = ldexpf(1.0f, ex);
+            int ql = 0, qh = 0;
+            if (used) {
+                const float rsc = ldexpf(1.0f, -ex);
+                ql = plane_quantise<false>(l, o, rsc);
+                qh = plane_quantise<true>(h, o, rsc);
+                while (ql > 0 && o + (float)ql * sc > l) --ql;
+                while (qh < 255 && o + (float)qh * sc < h) ++qh;
+            }
+            org[a] = o;
+            exw |= (uint32_t)(ex + 127) << (8 * a);
+            plane[a] = (uint32_t)ql << (8 * (s & 3));
+            plane[3 + a] = (uint32_t)qh << (8 * (s & 3));
+        }
+        uint32_t other[6];
+        for (int a = 0; a < 6; ++a) {
+            plane[a] |= __shfl_xor_sync(gm, plane[a], 1);
+            plane[a] |= __shfl_xor_sync(gm, plane[a], 2);
+            other[a] = __shfl_xor_sync(gm, plane[a], 4);
+        }
+        // lanes 0, 2, 3 and 4 hold words 0-3, 8-11, 12-15 and 16-19; word 4-7 stays
+        uint4* w = nodes + (size_t)cw * 5;
+        if (s == 0) {
+            w[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]), exw);
+            box[2 * (size_t)cw] = blo;
+            box[2 * (size_t)cw + 1] = bhi;
+        }
+        if (s == 2) w[2] = make_uint4(plane[0], other[0], plane[1], other[1]);
+        if (s == 3) w[3] = make_uint4(plane[2], other[2], plane[3], other[3]);
+        if (s == 4) w[4] = make_uint4(other[4], plane[4], other[5], plane[5]);
+        // the node's parent, if this was the last of its inner children
+        if (s == 0 && up >= 0) {
+            __threadfence();
+            if (atomicAdd(&arrived[up], 1u) + 1u != (uint32_t)__popc(up_mask)) up = -1;
+            __threadfence();
+        }
+        __syncwarp(gm);
+        up = __shfl_sync(gm, up, threadIdx.x & 24);
+        if (up < 0) return;
+        imask = up_mask;
+        cw = up;
     }
 }
 
@@ -636,15 +766,21 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
     GpuBvh& B = *out;
     B.n = n;
     // kept
-    GB_TRY(A.alloc((void**)&B.blo, sizeof(float4) * N2, true));
-    GB_TRY(A.alloc((void**)&B.bhi, sizeof(float4) * N2, true));
-    GB_TRY(A.alloc((void**)&B.bchild, sizeof(int2) * N2, true));
-    GB_TRY(A.alloc((void**)&B.bparent, sizeof(int) * N2, true));
-    GB_TRY(A.alloc((void**)&B.bleaf, N2, true));
     GB_TRY(A.alloc((void**)&B.tris, sizeof(float4) * 3 * (size_t)n, true));
-    // temporaries
+    // temporaries; binary nodes: leaves 0 .. n-1 in Morton order, inner ones
+    // with (left, right) children, leaves with (~triangle, -1), the root's
+    // parent -1, bleaf 1 where a node is stored as one leaf
+    float4 *blo, *bhi;
+    int2* bchild;
+    int* bparent;
+    uint8_t* bleaf;
+    GB_TRY(A.alloc((void**)&blo, sizeof(float4) * N2, false));
+    GB_TRY(A.alloc((void**)&bhi, sizeof(float4) * N2, false));
+    GB_TRY(A.alloc((void**)&bchild, sizeof(int2) * N2, false));
+    GB_TRY(A.alloc((void**)&bparent, sizeof(int) * N2, false));
+    GB_TRY(A.alloc((void**)&bleaf, N2, false));
     float4 *tlo, *thi, *clo[2], *chi[2];
-    int *vals[2], *cnode[2], *nn, *bcount, *q[2], *plan_tmp, *bad;
+    int *vals[2], *cnode[2], *nn, *bcount, *q[2], *plan, *parent_tmp, *bad;
     uint64_t* keys[2];
     unsigned *cb, *visit;
     unsigned long long *flags, *offs;
@@ -665,7 +801,8 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
     GB_TRY(A.alloc((void**)&offs, sizeof(unsigned long long) * n, false));
     GB_TRY(A.alloc((void**)&bcount, sizeof(int) * N2, false));
     GB_TRY(A.alloc((void**)&visit, sizeof(unsigned) * N2, false));
-    GB_TRY(A.alloc((void**)&plan_tmp, sizeof(int) * 8 * (size_t)cap, false));
+    GB_TRY(A.alloc((void**)&plan, sizeof(int) * 8 * (size_t)cap, false));
+    GB_TRY(A.alloc((void**)&parent_tmp, sizeof(int) * (size_t)cap, false));
     GB_TRY(A.alloc((void**)&nodes_tmp, sizeof(uint4) * 5 * (size_t)cap, false));
     GB_TRY(A.alloc((void**)&cb, sizeof(unsigned) * 8, false));
     GB_TRY(A.alloc((void**)&bad, sizeof(int) * 2, false));
@@ -690,7 +827,7 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
     k_morton<<<blocks_of(n, T), T, 0, st>>>(tlo, thi, n, cb, keys[0], vals[0]);
     GB_TRY(cudaGetLastError());
     GB_TRY(cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys[0], keys[1], vals[0], vals[1], n, 0, 63, st));
-    k_leaves<<<blocks_of(n, T), T, 0, st>>>(vals[1], tlo, thi, n, B.blo, B.bhi, B.bchild, B.bparent, clo[0], chi[0],
+    k_leaves<<<blocks_of(n, T), T, 0, st>>>(vals[1], tlo, thi, n, blo, bhi, bchild, bparent, clo[0], chi[0],
                                            cnode[0]);
     GB_TRY(cudaGetLastError());
 
@@ -704,8 +841,8 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
         GB_TRY(cudaGetLastError());
         GB_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, flags, offs, m, st));
         k_ploc_compact<<<blocks_of(m, T), T, 0, st>>>(nn, m, next_inner, offs, clo[cur], chi[cur], cnode[cur],
-                                                     clo[cur ^ 1], chi[cur ^ 1], cnode[cur ^ 1], B.blo, B.bhi,
-                                                     B.bchild, B.bparent, totals);
+                                                     clo[cur ^ 1], chi[cur ^ 1], cnode[cur ^ 1], blo, bhi,
+                                                     bchild, bparent, totals);
         GB_TRY(cudaGetLastError());
         GB_TRY(cudaMemcpyAsync(&h_tot, totals, sizeof(int2), cudaMemcpyDeviceToHost, st));
         GB_TRY(cudaStreamSynchronize(st));
@@ -727,25 +864,26 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
         GB_TRY(A.alloc((void**)&dhow, 8 * N2, false));
         GB_TRY(A.alloc((void**)&dsplit, N2, false));
     }
-    k_bottom_up<<<blocks_of(n, T), T, 0, st>>>(n, B.bparent, B.bchild, B.blo, B.bhi, bcount, B.bleaf, visit, d_pos, 0,
-                                               bad, dcost, dhow, dsplit, prim_cost);
+    k_bottom_up<<<blocks_of(n, T), T, 0, st>>>(n, bparent, bchild, blo, bhi, bcount, bleaf, visit, bad,
+                                               dcost, dhow, dsplit, prim_cost);
     GB_TRY(cudaGetLastError());
 
     // collapse, one level of 8-wide nodes per pass
     int node_base = 0, tri_base = 0, level = 1;
     cur = 0;
     GB_TRY(cudaMemcpyAsync(q[0], &root, sizeof(int), cudaMemcpyHostToDevice, st));
+    GB_TRY(cudaMemsetAsync(parent_tmp, 0xff, sizeof(int), st));  // the root's: -1
     m = 1;
     while (m > 0) {
         int next_base = node_base + m;
         if (next_base > cap) { *err = "8-wide node count out of range"; return cudaErrorInvalidValue; }
-        k_collapse_plan<<<blocks_of(m, T), T, 0, st>>>(q[cur], m, node_base, B.blo, B.bhi, B.bchild, B.bleaf, bcount,
-                                                      plan_tmp, flags, dhow, dsplit, n);
+        k_collapse_plan<<<blocks_of(m, T), T, 0, st>>>(q[cur], m, node_base, blo, bhi, bchild, bleaf, bcount,
+                                                      plan, flags, dhow, dsplit, n);
         GB_TRY(cudaGetLastError());
         GB_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, flags, offs, m, st));
-        k_collapse_emit<<<blocks_of(m, T), T, 0, st>>>(plan_tmp, m, node_base, next_base, tri_base, offs, flags, B.blo,
-                                                      B.bhi, B.bchild, B.bleaf, n, d_pos, nodes_tmp, B.tris,
-                                                      q[cur ^ 1], cap, totals, 0, bad);
+        k_collapse_emit<<<blocks_of(m, T), T, 0, st>>>(plan, m, node_base, next_base, tri_base, offs, flags, blo,
+                                                      bhi, bchild, bleaf, n, d_pos, nodes_tmp, B.tris,
+                                                      parent_tmp, q[cur ^ 1], cap, totals, bad);
         GB_TRY(cudaGetLastError());
         int hb[2] = {0, 0};
         GB_TRY(cudaMemcpyAsync(&h_tot, totals, sizeof(int2), cudaMemcpyDeviceToHost, st));
@@ -764,9 +902,9 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
     B.n_nodes = node_base;
     B.n_tris = n;
     GB_TRY(A.alloc((void**)&B.nodes, sizeof(uint4) * 5 * (size_t)B.n_nodes, true));
-    GB_TRY(A.alloc((void**)&B.plan, sizeof(int) * 8 * (size_t)B.n_nodes, true));
+    GB_TRY(A.alloc((void**)&B.parent, sizeof(int) * (size_t)B.n_nodes, true));
     GB_TRY(cudaMemcpyAsync(B.nodes, nodes_tmp, sizeof(uint4) * 5 * (size_t)B.n_nodes, cudaMemcpyDeviceToDevice, st));
-    GB_TRY(cudaMemcpyAsync(B.plan, plan_tmp, sizeof(int) * 8 * (size_t)B.n_nodes, cudaMemcpyDeviceToDevice, st));
+    GB_TRY(cudaMemcpyAsync(B.parent, parent_tmp, sizeof(int) * (size_t)B.n_nodes, cudaMemcpyDeviceToDevice, st));
     // the structure is checked on the host before any traversal reads it
     CwBvh chk;
     chk.n_nodes = B.n_nodes;
@@ -775,34 +913,33 @@ cudaError_t gpu_build_cwbvh(const float* d_pos, int n, int radius, DevAllocator&
     GB_TRY(cudaMemcpyAsync(chk.nodes.data(), B.nodes, sizeof(uint32_t) * chk.nodes.size(), cudaMemcpyDeviceToHost, st));
     GB_TRY(cudaStreamSynchronize(st));
     if (!validate_cwbvh(chk, err)) return cudaErrorInvalidValue;
-    B.device_bytes = (sizeof(float4) * 2 + sizeof(int2) + sizeof(int) + 1) * N2 + sizeof(float4) * 3 * (size_t)n +
-                     (sizeof(uint4) * 5 + sizeof(int) * 8) * (size_t)B.n_nodes;
+    B.device_bytes = sizeof(float4) * 3 * (size_t)n + (sizeof(uint4) * 5 + sizeof(int)) * (size_t)B.n_nodes;
     return cudaSuccess;
 }
 
-size_t refit_scratch_bytes(const GpuBvh& B) { return sizeof(unsigned) * (2 * (size_t)B.n + 1); }
+// Node boxes, arrival counters, then the two words of `bad`.
+size_t refit_scratch_bytes(const GpuBvh& B) {
+    return (sizeof(float4) * 2 + sizeof(unsigned)) * (size_t)B.n_nodes + sizeof(int) * 2;
+}
 
 // Bound by the passes over the vertices and the tree (205 K triangles:
-// about 0.17 ms, 0.1 ms of copies); everything is enqueued at once, with the verdict on the
+// 0.08 ms of kernels, 0.1 ms of copies); everything is enqueued at once, with the verdict on the
 // vertices left in a device word that the writing kernels test, so that the
 // host waits once.
 cudaError_t gpu_refit_cwbvh(const float* d_pos, const float* d_nrm, float4* d_shade, void* scratch, GpuBvh* bvh,
                             std::string* err, cudaStream_t st) {
     GpuBvh& B = *bvh;
     const int n = B.n;
-    if (n <= 0 || !B.nodes || !B.plan) { *err = "no device-built tree to refit"; return cudaErrorInvalidValue; }
-    const size_t N2 = 2 * (size_t)n - 1;
-    int* bad = (int*)scratch;  // [0] index out of range or a cycle, [1] non-finite vertex
-    unsigned* visit = (unsigned*)scratch + 2;
+    if (n <= 0 || !B.nodes || !B.parent) { *err = "no device-built tree to refit"; return cudaErrorInvalidValue; }
+    float4* box = (float4*)scratch;
+    unsigned* arrived = (unsigned*)(box + 2 * (size_t)B.n_nodes);
+    int* bad = (int*)(arrived + B.n_nodes);  // [0] index out of range or a cycle, [1] non-finite vertex
     const int T = kBuildBlock;
-    GB_TRY(cudaMemsetAsync(scratch, 0, sizeof(unsigned) * (N2 + 2), st));
+    GB_TRY(cudaMemsetAsync(arrived, 0, sizeof(unsigned) * (size_t)B.n_nodes + sizeof(int) * 2, st));
     k_check_finite<<<(int)std::min<long long>(((long long)9 * n + T - 1) / T, 152 * 8), T, 0, st>>>(d_pos, 9 * (size_t)n,
                                                                                                 bad + 1);
-    k_bottom_up<<<blocks_of(n, T), T, 0, st>>>(n, B.bparent, B.bchild, B.blo, B.bhi, nullptr, nullptr, visit, d_pos, 1,
-                                               bad, nullptr, nullptr, nullptr, 0.0f);
-    k_collapse_emit<<<blocks_of(B.n_nodes, T), T, 0, st>>>(B.plan, B.n_nodes, 0, 0, 0, nullptr, nullptr, B.blo, B.bhi,
-                                                          B.bchild, B.bleaf, n, d_pos, (uint4*)B.nodes, B.tris,
-                                                          nullptr, B.n_nodes, nullptr, 1, bad);
+    k_refit<<<blocks_of(8 * (long long)B.n_nodes, T), T, 0, st>>>(d_pos, n, B.n_nodes, B.parent, (uint4*)B.nodes, B.tris,
+                                                                  box, arrived, bad);
     k_shade_records<<<(int)((6 * (long long)n + T - 1) / T), T, 0, st>>>(d_pos, d_nrm, n, d_shade, bad + 1);
     GB_TRY(cudaGetLastError());
     int h_bad[2] = {0, 0};
@@ -810,7 +947,7 @@ cudaError_t gpu_refit_cwbvh(const float* d_pos, const float* d_nrm, float4* d_sh
     GB_TRY(cudaStreamSynchronize(st));
     if (h_bad[1]) { *err = "non-finite vertex"; return cudaErrorInvalidValue; }
     if (h_bad[0]) {
-        *err = h_bad[0] == 2 ? "cycle in the binary tree" : "refit index out of range";
+        *err = h_bad[0] == 2 ? "cycle in the tree" : "refit index out of range";
         return cudaErrorInvalidValue;
     }
     return cudaSuccess;

@@ -13,9 +13,9 @@
 // binary tree it writes the nodes the host collapse would write; only the
 // node numbering differs (level order).
 //
-// The binary tree and the 8-wide grouping are kept, so a scene whose
-// vertices move can be refitted: boxes are recomputed bottom-up and the
-// nodes re-quantised in place, with no change of topology.
+// Each 8-wide node's parent is kept, so a scene whose vertices move can be
+// refitted: boxes are recomputed bottom-up and the nodes re-quantised in
+// place, with no change of topology.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -42,12 +42,7 @@ struct GpuBvh {
     int iterations = 0;            // clustering passes
     // kept for refits
     int n = 0;                     // triangles
-    float4* blo = nullptr;         // binary node boxes (2n - 1); leaves 0 .. n-1 in Morton order
-    float4* bhi = nullptr;
-    int2* bchild = nullptr;        // inner: (left, right); leaf: (~triangle, -1)
-    int* bparent = nullptr;        // -1 at the root
-    uint8_t* bleaf = nullptr;      // 1 where a binary node is stored as one leaf
-    int* plan = nullptr;           // 8 binary nodes per 8-wide node, in slot order (-1 = empty)
+    int* parent = nullptr;         // of each 8-wide node, -1 at the root; parents come first
     size_t device_bytes = 0;       // bytes of the kept buffers
 };
 

@@ -192,3 +192,65 @@ def test_small_trees_under_every_policy(gpu_ctx, builder, n):
     finally:
         gpu_ctx.set_tuning(tri_mode=old["tri_mode"], graph=old["graph"])
         s.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 9, 65, 700, 5000])
+@pytest.mark.parametrize("kind", ["soup", "grid", "far", "flat"])
+def test_refit_small_and_odd_trees(gpu_ctx, n, kind):
+    """Refits of trees of one leaf, one node and many levels: after a refit to
+    the vertices it was built from a tree costs the same node visits
+    (the nodes are the same; counted under the policy that tests pending
+    triangles before each node, since with the others a ray's visits depend on
+    the rays that share its warp); after a refit to others the hits
+    are the oracle's, and moving back restores the costs."""
+    from oracle import oracle
+    rng = np.random.default_rng(n)
+    c = rng.uniform(-4.0, 4.0, (n, 1, 3))
+    p = (c + rng.uniform(-0.4, 0.4, (n, 3, 3))).astype(np.float32)
+    q = (c[::-1] * 0.8 + rng.uniform(-0.6, 0.6, (n, 3, 3))).astype(np.float32)
+    if kind == "grid":  # box sides that are whole multiples of the planes' steps
+        p, q = np.round(p * 4) / 4, np.round(q * 2) / 2
+    elif kind == "far":
+        p, q = p + np.float32(3.0e4), q + np.float32(3.0e4)
+    elif kind == "flat":
+        p[..., 1] = q[..., 1] = 0.5
+    p, q = (np.ascontiguousarray(v.reshape(n, 9), dtype=np.float32) for v in (p, q))
+    base = scenes.cornell()
+    desc = {**base.__dict__, "normals": None, "texcoords": None, "material_index": np.zeros(n, np.int32)}
+    sp, sq = (scenes.SceneData(**{**desc, "positions": v}) for v in (p, q))
+    cam = dict(base.camera)
+    mid = p.reshape(-1, 3).mean(0)
+    cam.update(pos=(float(mid[0]), float(mid[1]) + 2.0, float(mid[2]) + 11.0), dir=(0.0, -0.15, -1.0), up=(0.0, 1.0, 0.0))
+    rd = {**base.render, "width": 24, "height": 20, "spp": 2, "max_bounces": 2}
+    s = gpu_ctx.scene(sp, builder="device")
+
+    def cost():
+        s.render(cam, rd, instrumented=True)
+        st = gpu_ctx.stats()
+        return st["closest_node_visits"], st["shadow_node_visits"]
+
+    old = gpu_ctx.get_tuning()["tri_mode"]
+    gpu_ctx.set_tuning(tri_mode=4)
+    try:
+        built = cost()
+        assert cost() == built
+        s.refit(p)
+        assert cost() == built
+    finally:
+        gpu_ctx.set_tuning(tri_mode=old)
+    s.refit(q)
+    o, d = scenes.random_rays(sq, 4000, seed=n)
+    tmax = np.full(o.shape[0], 3.4e38, np.float32)
+    got = s.trace_closest(o, d, tmax)
+    ref = oracle.OracleScene(sq, use_bvh=False).trace_closest(o, d, tmax)
+    assert np.array_equal(got["ref"], ref["ref"])
+    hit = ref["ref"] != 0xFFFFFFFF
+    for k in ("t", "beta", "gamma"):
+        assert np.array_equal(got[k][hit].view(np.uint32), ref[k][hit].view(np.uint32)), k
+    s.refit(p)
+    gpu_ctx.set_tuning(tri_mode=4)
+    try:
+        assert cost() == built
+    finally:
+        gpu_ctx.set_tuning(tri_mode=old)
+        s.close()
