@@ -1441,8 +1441,9 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 // slot-pool loop in the same order per path: k_paths takes a small chunk from
 // the camera on, k_finish the paths a chunk has left when few are alive.
 // After a vertex the warp traces the lanes' shadow rays and next extension
-// rays together (a lane goes on to its extension ray as soon as its shadow ray
-// is done) and meets again to shade.
+// rays together and meets again to shade: a lane goes on to its extension ray
+// as soon as its shadow ray is done, or, in warps of at most 16 paths, leaves
+// it to the lane 16 further on.
 //
 // A queue that does not fill the chip is bound by latency: each bounce costs
 // the loop two launches, a tail of long rays and a round trip of the path
@@ -1464,6 +1465,12 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 #ifndef GB_PATHS_MIN
 #define GB_PATHS_MIN 10
 #endif
+#ifndef GB_PATHS_WARPS8
+#define GB_PATHS_WARPS8 1216
+#endif
+#ifndef GB_PATHS_WARPS
+#define GB_PATHS_WARPS 3040
+#endif
 struct PathState {
     v3 o, d, tp, acc, pend;  // extension ray, throughput, accumulation, pending light sample
     v3 so, sd;               // shadow ray of the pending light sample
@@ -1474,20 +1481,39 @@ struct PathState {
     MrgState st;
 };
 
+__device__ __forceinline__ v3 shfl3(v3 v, uint32_t lane) {
+    return mk(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
+              __shfl_sync(0xffffffffu, v.z, lane));
+}
+
 // All 32 lanes call this; `alive` lanes have a path.  The sample goes to
-// *sample.
+// *sample.  helpers: paths are in lanes 0 .. 15 at most, and lane l + 16 traces
+// the extension ray of lane l's path while lane l traces its shadow ray.
 template <bool TEX>
 __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, bool alive, PathState& p, RayDiff& df,
-                                             float4* sample) {
+                                             float4* sample, bool helpers) {
     uint32_t n_ext = 0, n_shadow = 0, n_hit = 0, nvis = 0, ntri = 0;
     uint2 deep[kStack];
     const StackRef stack{deep, deep, 1};
     RayInv r;
     Trav s;
+    // a helper traces in its path's scene, which need not be this lane's
+    const float4 *nodes = R.S.nodes, *tris = R.S.tris;
+    if (helpers) {
+        nodes = (const float4*)__shfl_sync(0xffffffffu, (unsigned long long)nodes, lane_id() & 15u);
+        tris = (const float4*)__shfl_sync(0xffffffffu, (unsigned long long)tris, lane_id() & 15u);
+    }
     while (__any_sync(0xffffffffu, alive)) {
         bool any = alive && p.shadow, occl = false;
-        if (alive) {
-            r = any ? make_ray(p.so, p.sd) : make_ray(p.o, p.d);
+        bool ext = alive && p.ext;  // an extension ray this lane traces
+        v3 eo = p.o, ed = p.d;
+        if (helpers) {
+            eo = shfl3(eo, lane_id() & 15u);
+            ed = shfl3(ed, lane_id() & 15u);
+            ext = __shfl_sync(0xffffffffu, (int)ext, lane_id() & 15u) != 0 && lane_id() >= 16u;
+        }
+        if (any || ext) {
+            r = any ? make_ray(p.so, p.sd) : make_ray(eo, ed);
             trav_init(s, r, any ? p.smax : FLT_MAX);
         }
         else trav_stop(s);
@@ -1498,8 +1524,8 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
             if (any && !tri && !node) {  // the shadow ray is done
                 occl = s.best_id != 0xffffffffu;
                 any = false;
-                if (p.ext) {
-                    r = make_ray(p.o, p.d);
+                if (ext) {
+                    r = make_ray(eo, ed);
                     trav_init(s, r, FLT_MAX);
                     node = true;
                 }
@@ -1512,7 +1538,12 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
                 trav_stop(s);
                 continue;
             }
-            warp_step<false, kStack>(tri, node, mt, mn, R.S.nodes, R.S.tris, r, any, s, stack, F.status, &nvis, &ntri);
+            warp_step<false, kStack>(tri, node, mt, mn, nodes, tris, r, any, s, stack, F.status, &nvis, &ntri);
+        }
+        if (helpers) {
+            s.best_id = __shfl_sync(0xffffffffu, s.best_id, lane_id() | 16u);
+            s.bb = __shfl_sync(0xffffffffu, s.bb, lane_id() | 16u);
+            s.bg = __shfl_sync(0xffffffffu, s.bg, lane_id() | 16u);
         }
         if (alive) {
             if (p.shadow && !occl) p.acc = p.acc + p.pend;
@@ -1551,11 +1582,25 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
     add_stats(&F.stats[8], n_hit);
 }
 
+// Paths a warp follows when there are n: 16 while all their warps are resident
+// together (10 blocks of 2 on 152 SMs), 8 up to two warps per scheduler, else
+// 32.  The chip is then far from full whatever the split; fewer paths make
+// fewer turns of the vote between nodes and triangles, fewer lobes one after
+// the other, and leave lanes for the second ray.  32 always / this rule (us,
+// paths in thousands): room 1K 115 / 100, 16K 120 / 109, 36K 130 / 125; 64 K
+// triangles 6K 166 / 149, 32K 179 / 161; 512 K triangles 32K 216 / 197; last
+// paths of 225K there 412 / 383.  8 paths up to 3040 warps: room 16K 125; 16 up
+// to 4096 (more than resident): room 48K 131 / 158.
+__host__ __device__ __forceinline__ uint32_t paths_per_warp(uint32_t n) {
+    return n <= 8u * GB_PATHS_WARPS8 ? 8u : n <= 16u * GB_PATHS_WARPS ? 16u : 32u;
+}
+
 template <bool TEX>
 __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P, const MrgPowers J) {
     fill_tables();
-    const uint32_t l = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
-    const bool alive = l < P.chunk_paths;
+    const uint32_t lanes = paths_per_warp(P.chunk_paths);
+    const uint32_t l = (blockIdx.x * GB_PATHS_BLOCK + threadIdx.x) / 32u * lanes + lane_id();
+    const bool alive = lane_id() < lanes && l < P.chunk_paths;
     const PathStart ps = path_start(F, P, alive ? l : 0u, &J);
     const SceneRec& R = F.scenes[ps.sc];
     const v3 z = mk(0.0f, 0.0f, 0.0f);
@@ -1564,7 +1609,7 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F,
     RayDiff df;
     if (TEX && R.S.texcoord) df = camera_diff(R.cam, ps.x, ps.y);
     add_stats(&F.stats[0], alive ? 1u : 0u);
-    follow_paths<TEX>(F, R, alive, p, df, F.samples + l);
+    follow_paths<TEX>(F, R, alive, p, df, F.samples + (alive ? l : 0u), lanes <= 16u);
 }
 
 template <bool TEX>
@@ -1572,11 +1617,12 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F
     const int it = F.iter[0];
     const uint32_t* cs = ctr_set(F, it);
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
-    if (blockIdx.x * GB_PATHS_BLOCK >= count) return;
+    const uint32_t lanes = paths_per_warp(count);
+    if (blockIdx.x * (GB_PATHS_BLOCK / 32) * lanes >= count) return;
     fill_tables();
-    const uint32_t i = blockIdx.x * GB_PATHS_BLOCK + threadIdx.x;
-    if ((i & ~31u) >= count) return;
-    const bool alive = i < count;
+    const uint32_t first = (blockIdx.x * GB_PATHS_BLOCK + threadIdx.x) / 32u * lanes, i = first + lane_id();
+    if (first >= count) return;
+    const bool alive = lane_id() < lanes && i < count;
     const uint32_t k = alive ? i : 0u;
     const uint32_t slot = k < ne ? F.q[it & 1][k] : F.q[3 + (it & 1)][k - ne];
     const Sector rs = rec_ld(&F.ray[slot]), ps = rec_ld(&F.path[slot]), ss = rec_ld(&F.strm[slot]);
@@ -1601,7 +1647,7 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F
     }
     RayDiff df;
     if (TEX && R.S.texcoord) df = ld_rdiff(F, slot);
-    follow_paths<TEX>(F, R, alive, p, df, F.samples + P.round_start[p.path - (uint32_t)P.p0] + p.pix);
+    follow_paths<TEX>(F, R, alive, p, df, F.samples + P.round_start[p.path - (uint32_t)P.p0] + p.pix, lanes <= 16u);
 }
 
 // Path-replay adjoint of every path that finished this iteration (done queue,
@@ -2340,7 +2386,8 @@ cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t s
 }
 
 cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    const unsigned grid = (P.chunk_paths + GB_PATHS_BLOCK - 1) / GB_PATHS_BLOCK;
+    const unsigned per_block = GB_PATHS_BLOCK / 32 * paths_per_warp(P.chunk_paths);
+    const unsigned grid = (P.chunk_paths + per_block - 1) / per_block;
     if (P.textured) k_paths<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
     else k_paths<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
     return cudaGetLastError();
@@ -2348,7 +2395,10 @@ cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t s
 
 cudaError_t k_launch_finish(const Frame& F, const RenderParams& P, cudaStream_t st) {
     if (P.finish_max <= 0) return cudaSuccess;
-    const unsigned grid = ((unsigned)std::min(P.finish_max, F.nslots) + GB_PATHS_BLOCK - 1) / GB_PATHS_BLOCK;
+    // the blocks of the most paths and, for fewer at 8 or 16 a warp, of at most GB_PATHS_WARPS warps
+    const unsigned most = (unsigned)std::min(P.finish_max, F.nslots), per_block = GB_PATHS_BLOCK / 32;
+    const unsigned warps = std::max((most + 31) / 32, std::min((most + 7) / 8, (unsigned)std::max(GB_PATHS_WARPS, GB_PATHS_WARPS8)));
+    const unsigned grid = (warps + per_block - 1) / per_block;
     if (P.textured) k_finish<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
     else k_finish<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
     return cudaGetLastError();

@@ -254,3 +254,29 @@ def test_refit_small_and_odd_trees(gpu_ctx, n, kind):
     finally:
         gpu_ctx.set_tuning(tri_mode=old)
         s.close()
+
+
+@pytest.mark.parametrize("wa,wb", [(40, 7), (5000, 4728), (5001, 4728), (20000, 28640), (20001, 28640)])
+@pytest.mark.parametrize("spp", [1, 9])
+def test_paths_per_warp(gpu_ctx, wa, wb, spp):
+    """Chunks whose warps follow 8, 16 or 32 paths, at the edges between them
+    (8 * 1216 and 16 * 3040 paths) and, with more samples, for the last paths of
+    larger chunks: lanes without a path trace for a path of another scene.
+    Same images and ray counts as the host-driven loop."""
+    sa = scenes.principled_room(width=wa, height=1, spp=spp, max_bounces=5, rr_start=1)
+    sb = scenes.with_textures(scenes.icospheres(n_spheres=30, level=2, box=12.0, width=wb, height=1, spp=spp,
+                                                max_bounces=4, n_lights=2), scale=0.2)
+    handles = [gpu_ctx.scene(sa), gpu_ctx.scene(sb)]
+    jobs = [(h, sc.camera, sc.render) for h, sc in zip(handles, (sa, sb))]
+    out = []
+    try:
+        for graph in (False, True):
+            imgs = gpu_ctx.render_batch(jobs, graph=graph)
+            st = gpu_ctx.stats()
+            out.append((imgs, [st[k] for k in ("camera_rays", "extension_rays", "shadow_rays", "light_samples")]))
+    finally:
+        for h in handles:
+            h.close()
+    for a, b in zip(out[0][0], out[1][0]):
+        assert np.array_equal(a, b)
+    assert out[0][1] == out[1][1] and out[0][1][0] == (wa + wb) * spp
