@@ -45,9 +45,9 @@ constexpr int kBlock = 128;
 #endif
 constexpr int kStack = 32;
 constexpr int kIterLimit = 1 << 22;
-// Experimental build options, each off by default (measured in the design
-// notes): traversal stack entries kept in shared memory, L2 prefetch of hit
-// child nodes, register budgets.
+// Experimental build options, each off by default (both slower: the L1 serves
+// the stack and the nodes are L2 hits): traversal stack entries kept in shared
+// memory, L2 prefetch of hit child nodes.
 #ifndef GB_SMEM_STACK
 #define GB_SMEM_STACK 0
 #endif
@@ -1193,7 +1193,10 @@ __device__ __forceinline__ LightSample light_sample(const Frame& F, const SceneR
 // hits, handle_no_hit for the misses).  A block takes tiles of kShadeTile queue
 // entries, sorts each into hits and paths that end here (misses, and ended
 // paths whose last shadow ray has now been traced) and works on them in rounds
-// of 32 of one kind, one round per warp at a time.  The outcome is gathered in
+// of 32 of one kind, which warps take as they get to them, the hits' first (hits
+// cost several times what ends do; every fourth round a warp instead: 35.3
+// against 34.8 ms on the 1M-triangle 64-spp frame, 3.15 against 3.10 ms on 12
+// mixed scenes, 684 against 664 us on a textured frame).  The outcome is gathered in
 // lists in shared memory, which take their places in the global queues with
 // one atomic per list.  A path that ends stores its sample and restarts on its
 // slot with the chunk's next path; in MODE_ADJOINT it goes to the done queue
@@ -1257,11 +1260,11 @@ __device__ __forceinline__ Vertex make_vertex(const Frame& F, const SceneRec& R,
 #define GB_SHADE_TILE 512
 #endif
 constexpr uint32_t kShadeTile = GB_SHADE_TILE;
-enum { L_CONT = 0, L_SHADOW = 1, L_ENDED = 2, L_FIN = 3, L_HIT = 4, L_END = 5 };
+enum { L_CONT = 0, L_SHADOW = 1, L_ENDED = 2, L_FIN = 3, L_HIT = 4, L_END = 5, L_ROUND = 6 };
 struct ShadeTile {
     float4 entry[kShadeTile];  // beta, gamma, triangle id, slot: hits from the front, the others from the back
     uint32_t list[4][kShadeTile];
-    uint32_t n[6];             // entries of the lists, hits, others
+    uint32_t n[7];             // entries of the lists, hits, others; rounds taken
     uint32_t base[4];          // places taken in the global queues
 };
 
@@ -1294,7 +1297,7 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
     if (F.iter[2]) return;  // the loop is over: k_finish takes the queues
     if (blockIdx.x == 0 && tid == 0) F.iter[0] = it + 1;
     for (uint32_t base = blockIdx.x * tile; base < count; base += gridDim.x * tile) {
-        if (tid < 6) T.n[tid] = 0;
+        if (tid < 7) T.n[tid] = 0;
         __syncthreads();
         const uint32_t n = min(count - base, tile);
         for (uint32_t k = tid & ~31u; k < n; k += kBlock) {
@@ -1320,7 +1323,11 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
         }
         __syncthreads();
         const uint32_t nh = T.n[L_HIT], rounds = ((nh + 31u) >> 5) + ((n - nh + 31u) >> 5);
-        for (uint32_t round = tid >> 5; round < rounds; round += kBlock / 32) {
+        while (true) {  // warps take rounds as they get to them, the hits' first
+            uint32_t round = 0;
+            if (lane == 0) round = atomicAdd(&T.n[L_ROUND], 1u);
+            round = __shfl_sync(0xffffffffu, round, 0);
+            if (round >= rounds) break;
             const bool hits = round < ((nh + 31u) >> 5);  // this round shades hits
             const uint32_t e = (hits ? 0u : nh) + (round - (hits ? 0u : (nh + 31u) >> 5)) * 32u + lane;
             const bool valid = e < (hits ? nh : n);
@@ -2288,14 +2295,12 @@ cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument
 }
 
 // Grid of the streaming per-path kernels (k_shade, k_regen): persistent for
-// pools of up to 2^20 slots, one thread per four slots above that (or
-// always, with GB_WIDE_STREAM_GRIDS), each thread taking every
-// (grid size)-th queue entry.  On the 1M-triangle frame with 2^21 slots a
-// thread per slot shades in 7.0 ms against 8.0 for the persistent grid; with
-// 2^24 slots a quarter of that grid (an iteration shades ~3 M hits) in
-// 4.8 ms against 6.2 for a thread per slot (1071 against 1058 Mpaths/s); on
-// the 256x256 16-spp Cornell frame (2^20 slots) the persistent grid in
-// 0.39 ms against 0.47.
+// pools of up to 2^20 slots, one thread per four slots above that, with a loop
+// over what is left.  A block per 512 slots gives a full queue's blocks
+// one whole tile each; a thread per slot makes the tiles of 128, fewer blocks
+// leave a long last wave.  nslots / 1 / 4 / 16 / 64 threads: 1M-triangle 64-spp
+// frame 38.1 / 34.8 / 35.2 / 35.6 ms, 12 mixed scenes 3.51 / 3.10 / 3.15 /
+// 3.43 ms.
 #ifndef GB_WIDE_GRID_DIV
 #define GB_WIDE_GRID_DIV 4  // the wide grid has nslots / GB_WIDE_GRID_DIV threads
 #endif
