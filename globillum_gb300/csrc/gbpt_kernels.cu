@@ -1268,11 +1268,17 @@ struct ShadeTile {
     uint32_t base[4];          // places taken in the global queues
 };
 
-// Tile of a launch with `count` entries: whole kShadeTile entries, or as few
-// as give every block one (at least one per thread).
+// Tile of a launch with `count` entries: as few entries as give every block
+// one tile (at least one per thread), or, where that is more than kShadeTile,
+// each block's share in equal tiles, so that no wave of tiles is nearly empty
+// (whole tiles of 512 instead: 256x256 16-spp room 866 against 838 us, textured
+// frame 664 against 647; equal tiles in steps of 32 for single tiles as well:
+// 12 mixed scenes 3.10 against 3.15 ms).
 __device__ __forceinline__ uint32_t shade_tile(uint32_t count) {
-    const uint32_t per = (count / gridDim.x + 127u) & ~127u;
-    return min(max(per, (uint32_t)kBlock), kShadeTile);
+    const uint32_t per = count / gridDim.x;
+    if (count <= gridDim.x * kShadeTile) return min(max((per + 127u) & ~127u, (uint32_t)kBlock), kShadeTile);
+    const uint32_t tiles = (per + kShadeTile) / kShadeTile;
+    return min((per / tiles + 32u) & ~31u, kShadeTile);
 }
 
 // Appends `v` of the flagged lanes to a list of the block.

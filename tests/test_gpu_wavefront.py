@@ -44,12 +44,14 @@ def test_path_counts_and_pools(gpu_ctx, w, h, spp, slots, bounces, graph):
 
 
 @pytest.mark.parametrize("w,h,spp,slots", [(512, 384, 1, 0), (513, 384, 1, 0), (512, 512, 1, 0), (513, 512, 1, 0),
-                                           (300, 310, 3, 5000), (257, 129, 16, 0)])
+                                           (300, 310, 3, 5000), (257, 129, 16, 0),
+                                           (681, 800, 1, 0), (681, 801, 1, 0), (1024, 1023, 1, 0)])
 @pytest.mark.parametrize("kind", ["room", "textured"])
 def test_finish_of_a_chunk(gpu_ctx, w, h, spp, slots, kind):
     """Chunks at and above the 3 * 2^16 paths of k_paths: the graph's loop leaves
-    its last paths to k_finish; the host-driven loop does not.  Same frames,
-    same ray counts."""
+    its last paths to k_finish; the host-driven loop does not.  And queues at
+    and above one shading tile of 512 per block (7 blocks on 152 SMs).  Same
+    frames, same ray counts."""
     if kind == "room":
         sc = scenes.principled_room(width=w, height=h, spp=spp, max_bounces=5, rr_start=1)
     else:
