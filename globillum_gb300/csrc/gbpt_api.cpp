@@ -1616,8 +1616,8 @@ int gb_backward(gb_ctx* ctx, gb_scene* scene, const gb_camera* cam, const gb_ren
 
 namespace {
 
-// Device buffers and launch knobs a fitting graph was captured with; a
-// change (another render grew the frame, a new tuning) means a new graph.
+// Device buffers, layout and launch knobs a fitting graph was captured with; a
+// change (another render, a new tuning) means a new graph.
 std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     const Frame& F = ctx->F;
     std::vector<uint64_t> k;
@@ -1632,6 +1632,9 @@ std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     k.push_back((uint64_t)ctx->sampling_terms);
     for (const gb_fit_item& u : ctx->fit.user)
         k.push_back((uint64_t)(uintptr_t)u.scene->S.mats ^ ((uint64_t)(uintptr_t)u.scene->S.lights << 1));
+    // the layout whose RNG states and pixel scenes the buffers hold: another
+    // frame may have replaced them without moving anything
+    k.insert(k.end(), ctx->pristine_key.begin(), ctx->pristine_key.end());
     return k;
 }
 

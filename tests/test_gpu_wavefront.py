@@ -282,3 +282,30 @@ def test_paths_per_warp(gpu_ctx, wa, wb, spp):
     for a, b in zip(out[0][0], out[1][0]):
         assert np.array_equal(a, b)
     assert out[0][1] == out[1][1] and out[0][1][0] == (wa + wb) * spp
+
+
+def test_fit_step_after_a_frame_of_another_layout(gpu_ctx):
+    """A fitting step after a render that used the same buffers for other
+    pixels: the step's frame is again that of the batch, whatever the other
+    frame left in them."""
+    import torch
+    big = scenes.cornell(width=160, height=120, spp=4, max_bounces=3)
+    big.render["seed"] = 5
+    small = scenes.principled_room(width=24, height=20, spp=2, max_bounces=3)
+    small.render["rng_mode"] = gbpt.GB_RNG_MRG32K3A_POOL
+    hb, hs = gpu_ctx.scene(big), gpu_ctx.scene(small)
+    try:
+        hb.render(big.camera, big.render)  # the buffers are large enough for both from here on
+        x = hs.get_params()
+        target = torch.zeros(20, 24, 3, device="cuda")
+        image = torch.empty_like(target)
+        gpu_ctx.fit_prepare([(hs, small.camera, small.render)], [target.data_ptr()], [image.data_ptr()])
+        gpu_ctx.fit_step([x])
+        first = image.cpu().numpy()
+        hb.render(big.camera, big.render)
+        gpu_ctx.fit_step([x])
+        assert np.array_equal(image.cpu().numpy(), first)
+        assert np.array_equal(hs.render(small.camera, small.render), first)
+    finally:
+        hb.close()
+        hs.close()
