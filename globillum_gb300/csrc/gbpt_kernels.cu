@@ -23,7 +23,7 @@
 //
 // Traversal: compressed 8-wide BVH (80 B nodes, 8-bit quantised child
 // boxes), node-group stack of 32 entries, octant-ordered child visits,
-// conservative slab tests (relative slack 1e-5 on top of outward-rounded
+// conservative slab tests (relative slack 2e-5 on top of outward-rounded
 // boxes), so the result equals the (t, id)-minimum over all triangles.
 #include "gbpt_kernels.h"
 
@@ -205,7 +205,8 @@ __device__ __forceinline__ void fill_tables() {
 // neither a node nor a triangle.
 //
 // The ALU pipe (byte permutes, min/max, compares, selects; half rate) bounds
-// this function, not FMA: 65-70 % against 17 % busy.  So
+// this function, not FMA: 65-70 % against 17 % busy before, 64-69 % against
+// 30 % with what follows.
 //  - one PRMT places two plane bytes in the mantissas of two FP16 subnormals
 //    (q 2^-24, exact), which the FMA pipe widens to FP32 (cvt.f32.f16), so
 //    distances are in units of 2^24 (exact, and no plane step overflows that

@@ -440,8 +440,8 @@ typedef struct {
 } gb_stats;
 
 /* Knobs of the wavefront (chosen by the autotuner); 0 keeps a value:
- *   refill    idle lanes (1..32) at which a closest-hit traversal warp
- *             fetches new rays, default 20 (any-hit warps refill at 12)
+ *   refill    idle lanes (1..32) at which a traversal warp fetches new
+ *             rays, default 20 (ray queries refill at 12)
  *   slots     paths in flight (queue capacity), default 2^24 (a frame
  *             allocates min(its paths, slots); 169 B of path state and queues per slot;
  *             the adjoint replay uses at most 2^22)
