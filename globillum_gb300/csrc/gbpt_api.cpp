@@ -77,6 +77,7 @@ struct FitState {
     double* h_out = nullptr;            // gradient sums (stride), then one loss per scene
     double* d_loss = nullptr;           // one loss per scene, then kLossBlocks partial sums per scene
     FitLossItem* d_items = nullptr;
+    bool ordered = false;               // images written by copies, scene after scene (fit_images_ordered)
     int stride = 0, replicas = 0;
     size_t mats_total = 0, lights_total = 0;
 };
@@ -1671,7 +1672,7 @@ std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     std::vector<uint64_t> k;
     const void* ptrs[] = {ctx->d_scenes, F.ray, F.halton, F.out, F.pristine,
                           F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr, F.iter, F.stats,
-                          F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->fit.d_loss};
+                          F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->fit.d_loss, ctx->fit.ordered ? ctx->d_rgb : nullptr};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
     k.push_back(((uint64_t)ctx->slot_cap << 32) ^ (uint64_t)ctx->sample_cap);
     k.push_back(((uint64_t)(uint32_t)ctx->slots << 32) | (uint32_t)ctx->sample_mb);
@@ -1694,6 +1695,35 @@ cudaError_t host_buf(void** p, size_t* cap, size_t bytes) {
     cudaError_t e = cudaHostAlloc(p, std::max<size_t>(bytes, 16), cudaHostAllocDefault);
     if (e == cudaSuccess) *cap = bytes;
     return e;
+}
+
+// Whether the scenes' losses have to follow one another with each scene's image
+// copied out after its loss: when only a copy can write an image, or when an
+// image shares memory with a target or another image, so that the order decides
+// what a loss reads and which image stays.  Otherwise one launch takes every
+// loss and writes every image (an image in its own scene's target is written
+// behind each pixel's read).  GB_ERR_CUDA for an allocation shorter than its image.
+int fit_images_ordered(gb_ctx* ctx, const std::vector<BatchScene>& items, bool* ordered) {
+    *ordered = false;
+    auto overlap = [](const void* a, size_t na, const void* b, size_t nb) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+        return x < y + nb && y < x + na;
+    };
+    for (size_t i = 0; i < items.size(); ++i) {
+        const float* img = items[i].image;
+        if (!img) continue;
+        const size_t bytes = sizeof(float) * 3 * (size_t)items[i].n;
+        const int route = write_route(ctx, img, bytes);
+        if (route == WRITE_NONE) return cuda_fail(ctx, cudaErrorInvalidValue, "output smaller than the image");
+        bool apart = route == WRITE_KERNEL;
+        for (size_t j = 0; j < items.size() && apart; ++j) {
+            const size_t nb = sizeof(float) * 3 * (size_t)items[j].n;
+            if (overlap(img, bytes, items[j].target, nb) && !(i == j && img == items[j].target)) apart = false;
+            if (j != i && items[j].image && overlap(img, bytes, items[j].image, nb)) apart = false;
+        }
+        if (!apart) *ordered = true;
+    }
+    return GB_OK;
 }
 
 // Lays the fitting frame out (an ordinary start of the forward frame: scene
@@ -1737,13 +1767,17 @@ int fit_build(gb_ctx* ctx) {
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fitting buffers");
     if (f.d_loss) { cudaFree(f.d_loss); f.d_loss = nullptr; }
     if (f.d_items) { cudaFree(f.d_items); f.d_items = nullptr; }
+    rc = fit_images_ordered(ctx, f.items, &f.ordered);
+    if (rc == GB_OK && f.ordered) rc = ensure_rgb(ctx);
+    if (rc != GB_OK) return rc;
     std::vector<void*> tmp;
     CK(dalloc(tmp, (void**)&f.d_loss, sizeof(double) * ns * (1 + kLossBlocks)));
     CK(dalloc(tmp, (void**)&f.d_items, sizeof(FitLossItem) * ns));
     std::vector<FitLossItem> loss_items(ns);
     for (size_t k = 0; k < ns; ++k) {
         const BatchScene& it = f.items[k];
-        loss_items[k] = FitLossItem{it.target, it.image, it.base, it.n, 1.0f / (float)it.desc.spp};
+        loss_items[k] = FitLossItem{it.target, f.ordered ? nullptr : it.image, it.base, it.n,
+                                    1.0f / (float)it.desc.spp};
     }
     CK(cudaMemcpy(f.d_items, loss_items.data(), sizeof(FitLossItem) * ns, cudaMemcpyHostToDevice));
     f.mat_off.assign(ns, 0);
@@ -1801,7 +1835,16 @@ int fit_build(gb_ctx* ctx) {
             p0 = p1;
         }
         if (rc != GB_OK) break;
-        if (pass == 0) {
+        if (pass == 0 && f.ordered) {
+            e = k_launch_pack_rgb(F.out, F.ntot, ctx->d_rgb, a);
+            for (size_t k = 0; k < ns && e == cudaSuccess; ++k) {
+                const BatchScene& it = f.items[k];
+                e = k_launch_l2_loss(f.d_items + k, 1, F.out, F.dimg, f.d_loss + ns + kLossBlocks * k, f.d_loss + k, a);
+                if (e == cudaSuccess && it.image)
+                    e = cudaMemcpyAsync(it.image, ctx->d_rgb + 3 * (size_t)it.base, sizeof(float) * 3 * (size_t)it.n,
+                                        cudaMemcpyDeviceToDevice, a);
+            }
+        } else if (pass == 0) {
             e = k_launch_l2_loss(f.d_items, (int)ns, F.out, F.dimg, f.d_loss + ns, f.d_loss, a);
         } else {
             e = k_launch_grad_reduce(F.grad, f.replicas, f.stride, ctx->d_gsum, a);

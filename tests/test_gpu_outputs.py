@@ -87,3 +87,77 @@ def test_allocation_that_ends_before_the_image(gpu_ctx, memory, size, offset):
         assert np.array_equal(out, ref)
     finally:
         s.close()
+
+
+def _fit_jobs(ctx, n, w=24, h=20):
+    data = [scenes.cornell(width=w, height=h + k, spp=2, max_bounces=3, seed=k) for k in range(n)]
+    for sc in data:
+        sc.render["rng_mode"] = gbpt.GB_RNG_MRG32K3A_POOL
+    hs = [ctx.scene(sc) for sc in data]
+    jobs = [(s, sc.camera, sc.render) for s, sc in zip(hs, data)]
+    return hs, jobs, [s.render(sc.camera, sc.render) for s, sc in zip(hs, data)]
+
+
+def _loss(img, target):
+    d = (img - target).astype(np.float64)  # float differences, squared and summed in double
+    return float((d * d).sum())
+
+
+@pytest.mark.parametrize("share", ["none", "own", "earlier", "later", "ring", "one image"])
+def test_fit_images_that_share_memory(gpu_ctx, share):
+    """A fitting step takes the scenes in their order: each loss reads its target
+    as the images of the scenes before it have left it, and of images in the same
+    place the last one stays.  Two steps, since a later scene's image is
+    an earlier one's target only from the second step on.  A sum of 1,500 squares
+    in double in another order differs by less than 1500 * 2^-53 of itself."""
+    import torch
+    hs, jobs, imgs = _fit_jobs(gpu_ctx, 3, h=20)
+    n = [im.size for im in imgs]
+    buf = torch.full((6, max(n)), 0.25, dtype=torch.float32, device="cuda")
+    target, image = [0, 1, 2], [3, 4, 5]  # rows of buf
+    if share == "own":
+        image = target
+    elif share == "earlier":
+        target[1] = image[0]
+    elif share == "later":
+        target[0] = image[2]
+    elif share == "ring":
+        target = [image[2], image[0], image[1]]
+    elif share == "one image":
+        image = [3, 3, 3]
+    try:
+        gpu_ctx.fit_prepare(jobs, [buf[k].data_ptr() for k in target], [buf[k].data_ptr() for k in image])
+        xs = [s.get_params() for s in hs]
+        model = [np.full(max(n), 0.25, np.float32) for _ in range(6)]
+        for step in range(2):
+            _, loss = gpu_ctx.fit_step(xs)
+            for k in range(3):
+                want = _loss(imgs[k].reshape(-1), model[target[k]][: n[k]])
+                assert abs(loss[k] - want) <= 1500 * 2.0 ** -53 * want, (step, k)
+                model[image[k]][: n[k]] = imgs[k].reshape(-1)
+            assert np.array_equal(buf.cpu().numpy(), np.stack(model)), step
+    finally:
+        for s in hs:
+            s.close()
+
+
+@pytest.mark.parametrize("offset", [0, 4, 2])
+@pytest.mark.parametrize("managed", [False, True])
+def test_fit_image_anywhere_in_an_allocation(gpu_ctx, memory, offset, managed):
+    import torch
+    hs, jobs, imgs = _fit_jobs(gpu_ctx, 1)
+    target = torch.zeros(imgs[0].size, device="cuda")
+    try:
+        p = memory.device(imgs[0].nbytes + offset, managed)
+        gpu_ctx.fit_prepare(jobs, [target.data_ptr()], [p + offset])
+        gpu_ctx.fit_step([hs[0].get_params()])
+        got = memory.read(p, imgs[0].nbytes + offset)
+        assert np.array_equal(got[offset:], imgs[0].view(np.uint8).reshape(-1))
+        assert (got[:offset] == 0xAB).all()
+        short = memory.device(imgs[0].nbytes // 2)
+        with pytest.raises(gbpt.GBError):
+            gpu_ctx.fit_prepare(jobs, [target.data_ptr()], [short])
+        assert (memory.read(short, imgs[0].nbytes // 2) == 0xAB).all()
+    finally:
+        for s in hs:
+            s.close()
