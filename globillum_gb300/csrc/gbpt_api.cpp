@@ -133,8 +133,10 @@ struct gb_ctx {
     std::vector<int> ev_stage;          // stage of each recorded pair
     size_t ev_used = 0;
     // layout (pixels and seed of each scene, in order) whose initial RNG
-    // states F.pristine and scene map F.pscene hold
-    std::vector<uint64_t> pristine_key;
+    // states F.pristine and scene map F.pscene hold, and the one whose light
+    // draws d_halton holds (kept apart, so that frames with and without Halton
+    // draws of one layout can follow one another without a new start of either)
+    std::vector<uint64_t> pristine_key, halton_key;
     // scratch for API calls with host pointers
     DevBuf scratch[4];
     float* d_rgb = nullptr;
@@ -820,12 +822,13 @@ int enqueue_frame_setup(gb_ctx* ctx, cudaStream_t st, const SceneRec* recs, bool
     // their order and the seeds only
     std::vector<uint64_t> key;
     key.push_back((uint64_t)F.ntot);
-    key.push_back((uint64_t)(uintptr_t)F.halton);
     for (const BatchScene& b : ctx->items) key.push_back(((uint64_t)b.desc.seed << 32) | (uint32_t)b.n);
-    if (key != ctx->pristine_key) {
-        CK(k_launch_frame_init(F, true, st));
-        ctx->launches += 2;
-        ctx->pristine_key = key;
+    const bool rng = key != ctx->pristine_key, draws = F.halton && key != ctx->halton_key;
+    if (rng || draws) {
+        CK(k_launch_frame_init(F, rng, st));
+        ctx->launches += rng ? 2 : 1;
+        if (F.halton) ctx->halton_key = key;
+        ctx->pristine_key.swap(key);
     }
     return GB_OK;
 }
@@ -858,6 +861,7 @@ int begin_frame(gb_ctx* ctx, std::vector<BatchScene>& items) {
     ctx->F.halton = nullptr;
     for (const BatchScene& b : items)
         if (b.desc.rng_mode == GB_RNG_HALTON_LIGHT) {
+            if (sizeof(float2) * (size_t)ntot > ctx->halton_cap) ctx->halton_key.clear();
             CK(ensure_buf(ctx, (void**)&ctx->d_halton, &ctx->halton_cap, sizeof(float2) * (size_t)ntot));
             ctx->F.halton = ctx->d_halton;
             break;
@@ -1670,7 +1674,7 @@ namespace {
 std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     const Frame& F = ctx->F;
     std::vector<uint64_t> k;
-    const void* ptrs[] = {ctx->d_scenes, F.ray, F.halton, F.out, F.pristine,
+    const void* ptrs[] = {ctx->d_scenes, F.ray, ctx->d_halton, F.out, F.pristine,
                           F.cursor, F.jcursor, F.pscene, F.samples, F.jpool, F.spool, F.ctr, F.path_ctr, F.iter, F.stats,
                           F.status, F.adj, F.dimg, F.grad, ctx->d_gsum, ctx->fit.d_loss, ctx->fit.ordered ? ctx->d_rgb : nullptr};
     for (const void* p : ptrs) k.push_back((uint64_t)(uintptr_t)p);
@@ -1684,6 +1688,11 @@ std::vector<uint64_t> fit_key(const gb_ctx* ctx) {
     // the layout whose RNG states and pixel scenes the buffers hold: another
     // frame may have replaced them without moving anything
     k.insert(k.end(), ctx->pristine_key.begin(), ctx->pristine_key.end());
+    for (const gb_fit_item& u : ctx->fit.user)
+        if (u.desc.rng_mode == GB_RNG_HALTON_LIGHT) {
+            k.insert(k.end(), ctx->halton_key.begin(), ctx->halton_key.end());
+            break;
+        }
     return k;
 }
 

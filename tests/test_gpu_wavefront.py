@@ -309,3 +309,34 @@ def test_fit_step_after_a_frame_of_another_layout(gpu_ctx):
     finally:
         hb.close()
         hs.close()
+
+
+@pytest.mark.parametrize("other", [(40, 30, 0), (40, 30, 3), (30, 40, 0), (64, 48, 0)])
+def test_light_draws_of_a_layout_are_kept(gpu_ctx, other):
+    """Frames with Halton and with MRG32k3a light draws in turns: of one layout
+    they need no other launches than the same frame again does, and of several
+    (another seed, size or order of sizes) every frame stays the same."""
+    w, h, seed = other
+    a = scenes.cornell(width=40, height=30, spp=2, max_bounces=4)
+    s = gpu_ctx.scene(a)
+    halton, mrg = (dict(a.render, rng_mode=m) for m in (gbpt.GB_RNG_HALTON_LIGHT, gbpt.GB_RNG_MRG32K3A_POOL))
+    mixed = dict(a.render, width=w, height=h, seed=seed, rng_mode=gbpt.GB_RNG_HALTON_LIGHT)
+
+    def render(rd):
+        img = s.render(a.camera, rd)
+        return img, gpu_ctx.stats()["kernel_launches"]
+
+    try:
+        ref = []
+        for rd in (halton, mrg, mixed):
+            render(rd)
+            ref.append(render(rd))
+        render(halton)
+        for _ in range(2):  # one layout: nothing is started anew
+            for rd, (img, n) in ((mrg, ref[1]), (halton, ref[0])):
+                got, m = render(rd)
+                assert np.array_equal(got, img) and m == n
+        for rd, k in ((mixed, 2), (mrg, 1), (halton, 0), (mixed, 2), (halton, 0), (mrg, 1)):
+            assert np.array_equal(render(rd)[0], ref[k][0])
+    finally:
+        s.close()
