@@ -340,3 +340,46 @@ def test_light_draws_of_a_layout_are_kept(gpu_ctx, other):
             assert np.array_equal(render(rd)[0], ref[k][0])
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("fit_mode,view_mode", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_fit_steps_between_views(gpu_ctx, fit_mode, view_mode):
+    """Fitting steps with a view of another layout between them: the step keeps
+    its graph (it allocates nothing, so an allocation set to fail does not
+    matter) and its frames, losses and the view stay what they were."""
+    import torch
+    a = scenes.principled_room(width=24, height=20, spp=2, max_bounces=3)
+    b = scenes.cornell(width=31, height=9, spp=3, max_bounces=2, seed=4)
+    for sc in (a, b):
+        sc.render["rng_mode"] = fit_mode
+    hs = [gpu_ctx.scene(sc) for sc in (a, b)]
+    view = dict(a.render, width=33, height=17, spp=1, rng_mode=view_mode, seed=9)
+    lib = gpu_ctx.lib
+    try:
+        targets = [torch.zeros(20, 24, 3, device="cuda"), torch.zeros(9, 31, 3, device="cuda")]
+        images = [torch.empty_like(t) for t in targets]
+        xs = [h.get_params() for h in hs]
+        seen = hs[0].render(a.camera, view)
+        gpu_ctx.fit_prepare([(h, sc.camera, sc.render) for h, sc in zip(hs, (a, b))],
+                            [t.data_ptr() for t in targets], [t.data_ptr() for t in images])
+        _, loss = gpu_ctx.fit_step(xs)
+        first = [t.cpu().numpy() for t in images]
+        for h, sc, im in zip(hs, (a, b), first):
+            assert np.array_equal(h.render(sc.camera, sc.render), im)
+        gpu_ctx.fit_step(xs)
+        for _ in range(2):
+            assert np.array_equal(hs[0].render(a.camera, view), seen)
+            for t in images:
+                t.zero_()
+            torch.cuda.synchronize()
+            lib.gb_set_fault_injection(0)
+            try:
+                _, again = gpu_ctx.fit_step(xs)
+            finally:
+                lib.gb_set_fault_injection(-1)
+            assert np.array_equal(again, loss)
+            for t, im in zip(images, first):
+                assert np.array_equal(t.cpu().numpy(), im)
+    finally:
+        for h in hs:
+            h.close()
