@@ -1599,7 +1599,7 @@ int gb_backward_batch(gb_ctx* ctx, int n, const gb_adjoint_item* items, int dimg
     if (rc != GB_OK) return rc;
     Frame& F = ctx->F;
     const int stride = (int)std::max<uint32_t>(1, gtot);
-    const int replicas = k_adjoint_replicas(stride);
+    const int replicas = k_adjoint_grid();
     cudaError_t e = ensure_buf(ctx, (void**)&F.adj, &ctx->adj_cap,
                                sizeof(float4) * kAdjPlanes * (size_t)ctx->max_L *
                                    std::min(ctx->slot_cap, (size_t)kAdjMaxSlots));
@@ -1758,7 +1758,7 @@ int fit_build(gb_ctx* ctx) {
     f.items = ctx->items;
     Frame& F = ctx->F;
     f.stride = (int)std::max<uint32_t>(1, gtot);
-    f.replicas = k_adjoint_replicas(f.stride);
+    f.replicas = k_adjoint_grid();
     const size_t ns = f.items.size();
     cudaError_t e = ensure_buf(ctx, (void**)&F.adj, &ctx->adj_cap,
                                sizeof(float4) * kAdjPlanes * (size_t)ctx->max_L *

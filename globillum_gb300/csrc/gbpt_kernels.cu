@@ -1683,7 +1683,13 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F
 // values; the reverse sweep k = K-1 .. 0 carries a = dLoss/dT_{k+1} and adds
 // the BRDF vector-Jacobian products and the emission gradient to this
 // block's gradient replica.  g = dLoss/dI(pixel) / spp.
-__global__ void __launch_bounds__(kBlock) k_adjoint(Frame F, RenderParams P) {
+// A copy per block keeps a float sum to the terms of one block (they are summed
+// in double), whatever the number of parameters.  A fifth of the copies would
+// cost less to clear and sum (8 scenes of 3.6 K floats: 3.71 against 3.75 ms a
+// fitting step), but each sum would take five times as many terms: a step's
+// gradient moved by 2e-7 with them, where two runs differ by 1e-8.  5 blocks per
+// SM (96 registers; 104 and 4 blocks without the bound) for the same reason.
+__global__ void __launch_bounds__(kBlock, 5) k_adjoint(Frame F, RenderParams P) {
     const uint32_t count = ctr_set(F, F.iter[1] + 1)[CTR_DONE];
     float* grad = F.grad + (size_t)(blockIdx.x % (uint32_t)F.grad_replicas) * (size_t)F.grad_stride;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -2342,17 +2348,10 @@ cudaError_t k_launch_shade(const Frame& F, const RenderParams& P, cudaStream_t s
     return cudaGetLastError();
 }
 
+// The adjoint's blocks, each with a gradient copy of its own.
 int k_adjoint_grid() {
     static int g = persistent_blocks(k_adjoint);
     return g;
-}
-// A copy per block while they take no more than 16 MB, else fewer, down to one
-// for five blocks: clearing and summing them costs more than the contention
-// then (8 scenes of 3.6 K floats: 4.15 -> 4.09 ms per fitting step with a fifth
-// of the copies; one scene's gradient 2.94 -> 3.03 ms).
-int k_adjoint_replicas(int stride) {
-    const int g = k_adjoint_grid();
-    return std::max(std::max(1, g / 5), std::min(g, (4 << 20) / std::max(1, stride)));
 }
 
 cudaError_t k_launch_adjoint(const Frame& F, const RenderParams& P, cudaStream_t st) {

@@ -246,7 +246,7 @@ cudaError_t k_launch_direct(const DevScene& S, const CameraRec& cam, int w, int 
 cudaError_t k_launch_direct_hybrid(const DevScene& S, const CameraRec& cam, int w, int h, int cam_samples,
                                    int light_samples, uint32_t seed, float shadow_offset, v3 background, float* out,
                                    uint32_t* status, cudaStream_t st);
-int k_adjoint_replicas(int stride);  // gradient copies the adjoint's blocks add into
+int k_adjoint_grid();  // blocks of the adjoint, as many as gradient copies
 cudaError_t k_launch_dimg_pack(const float* src, int n, float scale, float4* dst, cudaStream_t st);
 cudaError_t k_launch_grad_reduce(const float* grad, int replicas, int stride, double* out, cudaStream_t st);
 // One scene of a fitting step's loss: its pixels are base .. base + n - 1 of the

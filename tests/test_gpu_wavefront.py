@@ -383,3 +383,37 @@ def test_fit_steps_between_views(gpu_ctx, fit_mode, view_mode):
     finally:
         for h in hs:
             h.close()
+
+
+@pytest.mark.parametrize("materials", [6, 3000])
+def test_gradient_copies(gpu_ctx, materials):
+    """A float sum of the gradient holds the terms of one block of the adjoint,
+    however many parameters there are.  Terms of 2^-27 are lost where they follow
+    one of 1 in the same sum: 152 large pixels among 2^18, in tiles of 128 that
+    760 blocks (5 on each SM) take two or three of each, can lose the terms of at
+    most 152 * 3 tiles of 2048, 22 % (25 % with the spread of the terms' sizes);
+    a fifth of the sums loses about twice as much."""
+    sc = scenes.cornell(width=512, height=512, spp=1, max_bounces=1)
+    sc.render["rng_mode"] = gbpt.GB_RNG_MRG32K3A_POOL
+    sc.materials += [dict(sc.materials[0]) for _ in range(materials - len(sc.materials))]
+    s = gpu_ctx.scene(sc)
+    img = s.render(sc.camera, sc.render)[..., 1].reshape(-1)
+    lit = np.flatnonzero((img > np.median(img[img > 0])) & (img < 0.99))
+    big = np.random.default_rng(1).choice(lit, 152, replace=False)
+    small = np.full(512 * 512, 2.0 ** -27, np.float32)
+    small[big] = 0.0
+    large = np.zeros(512 * 512, np.float32)
+    large[big] = 1.0
+
+    def light_gradient(g):  # the light's green emission
+        full = s.backward(sc.camera, sc.render, np.repeat(g[:, None], 3, 1).reshape(512, 512, 3))
+        return float(full[5 * len(sc.materials) + 1])
+
+    try:
+        a, b, both = light_gradient(small), light_gradient(large), light_gradient(small + large)
+        assert a > 0 and b > 100 * a
+        lost = (a + b - both) / a
+        print("lost", lost)
+        assert -0.02 < lost < 0.25
+    finally:
+        s.close()
