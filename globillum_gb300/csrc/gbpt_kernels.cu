@@ -81,19 +81,13 @@ struct RayInv {
     uint32_t oxor;
 };
 
-__device__ __forceinline__ float fast_rcp(float x) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ RayInv make_ray(v3 o, v3 d) {
     RayInv r;
     r.o = o; r.d = d;
     const float ooeps = 8.271806125530277e-25f;  // 2^-80 (tracers.cu:48-51)
-    // one ulp off at most: only the slab tests use it, whose slack is 2e-5
-    r.idir.x = fast_rcp(fabsf(d.x) > ooeps ? d.x : copysignf(ooeps, d.x));
-    r.idir.y = fast_rcp(fabsf(d.y) > ooeps ? d.y : copysignf(ooeps, d.y));
-    r.idir.z = fast_rcp(fabsf(d.z) > ooeps ? d.z : copysignf(ooeps, d.z));
+    r.idir.x = 1.0f / (fabsf(d.x) > ooeps ? d.x : copysignf(ooeps, d.x));
+    r.idir.y = 1.0f / (fabsf(d.y) > ooeps ? d.y : copysignf(ooeps, d.y));
+    r.idir.z = 1.0f / (fabsf(d.z) > ooeps ? d.z : copysignf(ooeps, d.z));
     uint32_t oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
     r.oxor = oct ^ 7u;
     return r;
