@@ -1032,6 +1032,45 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
     ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, S.nodes, S.tris, fetch, finish, &nvis, &ntri);
 }
 
+// The same with every lane on its own: all pending triangles, then a node, with no
+// vote.  A vote pays where other rays refill the lanes that have finished; a
+// warp that gets no more rays only becomes as slow as its slowest lane at every
+// step instead of at the end, and in a tree of a few levels there is little to
+// vote on.  At most two waves of blocks, since each fills the tables (2 M rays, 3.8 K
+// triangles: 95 against 108 us with a block per 128 rays).
+__global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace_alone(DevScene S, uint32_t n,
+                                                                            const float* __restrict__ orig,
+                                                                            const float* __restrict__ dir,
+                                                                            const float* __restrict__ tmaxv,
+                                                                            float4* hits, uint8_t* occluded, int any,
+                                                                            uint32_t* status) {
+    fill_tables();
+    uint32_t nvis = 0, ntri = 0;
+    uint2 deep[kStack];
+    const StackRef stack{deep, deep, 1};
+    for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+        const float *po = orig + 3 * (size_t)i, *pd = dir + 3 * (size_t)i;
+        const RayInv r = make_ray(mk(po[0], po[1], po[2]), mk(pd[0], pd[1], pd[2]));
+        const float t = tmaxv[i];
+        Trav s;
+        trav_init(s, r, t >= 0.0f ? t : -1.0f);
+        for (int steps = 0;; ++steps) {
+            bool done = false;
+            while (s.tg.y != 0u && !done) done = tri_step<false>(S.tris, r, any != 0, s, &ntri);
+            if (done) break;
+            if (s.ng.y <= 0x00ffffffu) {
+                if (s.sp == 0) break;
+                s.ng = stack_get(stack, --s.sp);
+            }
+            if (steps > kIterLimit) { atomicOr(status, (uint32_t)ST_ITER_LIMIT); break; }
+            if (visit_node<false>(S.nodes, r, s, stack, status, &nvis, &s.tg, &s.tv)) break;
+        }
+        const bool hit = s.best_id != 0xffffffffu;
+        if (any) occluded[i] = hit ? 1 : 0;
+        else hits[i] = make_float4(hit ? s.best_t : FLT_MAX, s.bb, s.bg, __uint_as_float(s.best_id));
+    }
+}
+
 // Whether the chunk's loop stops before iteration `it` and leaves its queues
 // to k_finish: every path has started and few are alive.  k_rays decides and
 // notes it in F.iter[2]: path_ctr moves while k_shade runs.
@@ -2190,11 +2229,32 @@ inline int traversal_grid(const Grid& g, int blocks_per_sm, int bt = kBlock) {
 
 }  // namespace
 
+// Whether n rays go through k_trace_alone instead of k_trace, whose grid has
+// `lanes` lanes (136 K on 152 SMs).  k_trace / k_trace_alone, us a call, warm and
+// after a flush of the L2:
+//   no more rays than lanes   1 M triangles, 16 K and 131 K shadow rays 52 57 / 44 55, 74 79 / 68 68, closest 59 71 /
+//                             57 71, 84 92 / 80 90; 64 K triangles, 131 K closest 60 58 / 55 57
+//   up to two rays a lane     13 K triangles, 262 K closest 62 58 / 57 53, any 61 58 / 56 53; 23 K any 57 55 / 49 53;
+//                             but 64 K, 262 K any 63 60 / 63 64, 13 K, 400 K closest 64 62 / 69 65
+//   more                      1.3 K triangles, 2 M closest 101 98 / 83 80; 3.8 K closest 110 105 / 96 98; 2.6 K, 450 K
+//                             any 59 55 / 50 52; but 5.1 K, 2 M closest 112 108 / 122 126, 3.8 K any 123 119 / 169 176
+inline bool trace_alone(int n, int lanes, int tris, bool any) {
+    if (n <= lanes) return true;
+    if (n <= 2ll * lanes) return tris <= 3 << 13;
+    return tris <= (any ? 2560 : 4096);
+}
+
 cudaError_t k_launch_trace(const DevScene& S, int n, const float* orig, const float* dir, const float* tmax,
                            float4* hits, uint8_t* occluded, bool any, uint32_t* head, uint32_t* status,
                            cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     static int g = persistent_blocks(k_trace);
+    if (trace_alone(n, g * kBlock, S.n_tris, any)) {
+        static int ga = persistent_blocks(k_trace_alone);
+        k_trace_alone<<<std::min(2 * ga, blocks_for(n)), kBlock, 0, st>>>(S, (uint32_t)n, orig, dir, tmax, hits, occluded,
+                                                                          any ? 1 : 0, status);
+        return cudaGetLastError();
+    }
     if (n > g * kBlock) {
         cudaError_t e = cudaMemsetAsync(head, 0, sizeof(uint32_t), st);
         if (e != cudaSuccess) return e;
