@@ -25,6 +25,11 @@ ORACLE_SRC = ROOT / "oracle" / "gbpt_oracle.cpp"
 ORACLE_F64_SRC = ROOT / "oracle" / "fp64_render.cpp"
 ORACLE_LIB = ROOT / "oracle" / "_build" / "libgbpt_oracle.so"
 
+# experimental compile options (GBPT_<name> in the environment -> -DGB_<name>):
+# the defines that the sources give a default
+KNOBS = ("TRAV_MIN_BLOCKS", "PREFETCH", "SHADE_MIN_BLOCKS", "TRI_NOALLOC", "NODE_L2_128", "REC_EVICT_FIRST",
+         "NODE_L2_PERSIST", "TREE_WINDOW", "WIDE_GRID_DIV", "TRI_RATIO")
+
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -70,9 +75,7 @@ def build_lib(force: bool = False, verbose_ptxas: bool = False) -> Path:
     cpp = [CSRC / "gbpt_api.cpp", CSRC / "gbpt_bvh.cpp", CSRC / "gbpt_ingest.cpp"]
     deps = cu + cpp + _sources()
     # the library records the build-time defines it was made with
-    # experimental compile options (GBPT_<name> in the environment -> -DGB_<name>)
-    knobs = ("TRAV_MIN_BLOCKS", "SMEM_STACK", "PREFETCH", "SHADE_MIN_BLOCKS", "TRI_NOALLOC", "NODE_L2_128",
-             "REC_EVICT_FIRST", "NODE_L2_PERSIST", "TREE_WINDOW", "WIDE_GRID_DIV", "TRI_RATIO")
+    knobs = KNOBS
     flags = " ".join(f"GB_{k}={os.environ.get('GBPT_' + k, '')}" for k in knobs)
     stamp = LIB.with_suffix(".flags")
     if not stamp.exists() or stamp.read_text() != flags:

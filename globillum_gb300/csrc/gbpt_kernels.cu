@@ -45,34 +45,14 @@ constexpr int kBlock = 128;
 #endif
 constexpr int kStack = 32;
 constexpr int kIterLimit = 1 << 22;
-// Experimental build options, each off by default (both slower: the L1 serves
-// the stack and the nodes are L2 hits): traversal stack entries kept in shared
-// memory, L2 prefetch of hit child nodes.
-#ifndef GB_SMEM_STACK
-#define GB_SMEM_STACK 0
-#endif
+// Experimental build option, off by default (slower: the nodes are L2 hits): L2
+// prefetch of hit child nodes.
 #ifndef GB_PREFETCH
 #define GB_PREFETCH 0
 #endif
 #ifndef GB_SHADE_MIN_BLOCKS
 #define GB_SHADE_MIN_BLOCKS 7  // resident k_shade blocks per SM (72 registers)
 #endif
-constexpr int kSmemStack = GB_SMEM_STACK;
-
-// A thread's traversal stack: entry e < kSmemStack at top[e * stride]
-// (a column of a shared-memory array), deeper entries in deep[e - kSmemStack].
-struct StackRef {
-    uint2* top;
-    uint2* deep;
-    int stride;
-};
-__device__ __forceinline__ void stack_put(const StackRef& k, int e, uint2 v) {
-    if (e < kSmemStack) k.top[e * k.stride] = v;
-    else k.deep[e - kSmemStack] = v;
-}
-__device__ __forceinline__ uint2 stack_get(const StackRef& k, int e) {
-    return e < kSmemStack ? k.top[e * k.stride] : k.deep[e - kSmemStack];
-}
 
 __device__ __forceinline__ v3 ld3(const float4 a) { return mk(a.x, a.y, a.z); }
 
@@ -345,7 +325,7 @@ __device__ __forceinline__ bool tri_step(const float4* __restrict__ tris, const 
 // true when the stack overflows.
 template <bool INSTR, int STACK = kStack>
 __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
-                                           const StackRef& stack, uint32_t* status, uint32_t* nvis, uint2* tg,
+                                           uint2* stack, uint32_t* status, uint32_t* nvis, uint2* tg,
                                            uint32_t* tv) {
     const uint32_t k = 31u - (uint32_t)__clz(s.ng.y);
     s.ng.y &= ~(1u << k);
@@ -354,7 +334,7 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
     const uint32_t child = s.ng.x + (uint32_t)__popc(imask & ((1u << slot) - 1u));
     if (s.ng.y > 0x00ffffffu) {
         if (s.sp >= STACK) { atomicOr(status, ST_STACK_OVERFLOW); return true; }
-        stack_put(stack, s.sp++, s.ng);
+        stack[s.sp++] = s.ng;
     }
     if (INSTR) ++*nvis;
     intersect_node(nodes, child, r, s.best_t, &s.ng, tg, tv);
@@ -366,7 +346,7 @@ __device__ __forceinline__ bool visit_node(const float4* __restrict__ nodes, con
 // is the (t, id)-minimum in s (any-hit: best_id != none when found).
 template <bool INSTR, int STACK = kStack>
 __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, const RayInv& r, Trav& s,
-                                          const StackRef& stack, uint32_t* status, uint32_t* nvis) {
+                                          uint2* stack, uint32_t* status, uint32_t* nvis) {
     if (s.ng.y > 0x00ffffffu) {
         const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &s.tg, &s.tv);
         // these policies stack groups and hand them to other lanes: bits without gaps, for any tv
@@ -377,7 +357,7 @@ __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, cons
         return over;
     }
     if (s.sp > 0) {
-        uint2 g = stack_get(stack, --s.sp);
+        uint2 g = stack[--s.sp];
         if (g.y > 0x00ffffffu) s.ng = g;
         else s.tg = g;
         return false;
@@ -412,7 +392,7 @@ __device__ __forceinline__ void trav_stop(Trav& s) {
 template <bool INSTR, int STACK>
 __device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint32_t mn,
                                           const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                          const RayInv& r, bool any, Trav& s, const StackRef& stack,
+                                          const RayInv& r, bool any, Trav& s, uint2* stack,
                                           uint32_t* status, uint32_t* nvis, uint32_t* ntri) {
     if (__popc(mt) * GB_TRI_RATIO >= __popc(mn)) {
         if (tri) {
@@ -425,7 +405,7 @@ __device__ __forceinline__ void warp_step(bool tri, bool node, uint32_t mt, uint
             if (found) trav_stop(s);
         }
     } else if (node) {
-        if (s.ng.y <= 0x00ffffffu) s.ng = stack_get(stack, --s.sp);
+        if (s.ng.y <= 0x00ffffffu) s.ng = stack[--s.sp];
         uint2 tg = make_uint2(0u, 0u);
         uint32_t tv = 0u;
         const bool over = visit_node<INSTR, STACK>(nodes, r, s, stack, status, nvis, &tg, &tv);
@@ -896,9 +876,7 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
     RayInv r;
     Trav s;
     trav_stop(s);
-    __shared__ uint2 s_stack[kSmemStack > 0 ? kSmemStack * BT : 1];
-    uint2 deep[STACK - kSmemStack];
-    const StackRef stack{s_stack + threadIdx.x, deep, BT};
+    uint2 stack[STACK];
     const float4* nodes = nodes0;
     const float4* tris = tris0;
     const float4* shade = nullptr;
@@ -974,7 +952,7 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
                 const uint32_t ma = __ballot_sync(0xffffffffu, act);
                 bool do_tri = want_tri;
                 if (want_tri && 5u * (uint32_t)__popc(mt) < (uint32_t)__popc(ma) && s.sp < STACK) {
-                    stack_put(stack, s.sp++, s.tg);
+                    stack[s.sp++] = s.tg;
                     s.tg.y = 0u;
                     do_tri = false;
                 }
@@ -1002,9 +980,7 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
 // gb_trace_closest / gb_trace_any: the caller's rays through the persistent
 // ray loop.  head: the queue head (zero), read only when there are more rays
 // than lanes in the grid.  A negative or NaN max_t traces nothing.
-#ifndef GB_TRACE_REFILL
-#define GB_TRACE_REFILL 12
-#endif
+constexpr int kTraceRefill = 12;
 __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S, uint32_t n,
                                                                       const float* __restrict__ orig,
                                                                       const float* __restrict__ dir,
@@ -1029,7 +1005,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S
         if (any) occluded[i] = hit ? 1 : 0;
         else hits[i] = make_float4(hit ? h.best_t : FLT_MAX, h.bb, h.bg, __uint_as_float(h.best_id));
     };
-    ray_loop<false, 0, kStack, kBlock>(n, head, GB_TRACE_REFILL, status, S.nodes, S.tris, fetch, finish, &nvis, &ntri);
+    ray_loop<false, 0, kStack, kBlock>(n, head, kTraceRefill, status, S.nodes, S.tris, fetch, finish, &nvis, &ntri);
 }
 
 // The same with every lane on its own: all pending triangles, then a node, with no
@@ -1046,8 +1022,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace_alone(DevS
                                                                             uint32_t* status) {
     fill_tables();
     uint32_t nvis = 0, ntri = 0;
-    uint2 deep[kStack];
-    const StackRef stack{deep, deep, 1};
+    uint2 stack[kStack];
     for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
         const float *po = orig + 3 * (size_t)i, *pd = dir + 3 * (size_t)i;
         const RayInv r = make_ray(mk(po[0], po[1], po[2]), mk(pd[0], pd[1], pd[2]));
@@ -1060,7 +1035,7 @@ __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace_alone(DevS
             if (done) break;
             if (s.ng.y <= 0x00ffffffu) {
                 if (s.sp == 0) break;
-                s.ng = stack_get(stack, --s.sp);
+                s.ng = stack[--s.sp];
             }
             if (steps > kIterLimit) { atomicOr(status, (uint32_t)ST_ITER_LIMIT); break; }
             if (visit_node<false>(S.nodes, r, s, stack, status, &nvis, &s.tg, &s.tv)) break;
@@ -1305,10 +1280,7 @@ __device__ __forceinline__ float4* adj_tail(const Frame& F, int bounce, uint32_t
 
 // Shared memory of a shading block: the tile's entries and what became of
 // them.
-#ifndef GB_SHADE_TILE
-#define GB_SHADE_TILE 512
-#endif
-constexpr uint32_t kShadeTile = GB_SHADE_TILE;
+constexpr uint32_t kShadeTile = 512;
 enum { L_CONT = 0, L_SHADOW = 1, L_ENDED = 2, L_FIN = 3, L_HIT = 4, L_END = 5, L_ROUND = 6 };
 struct ShadeTile {
     float4 entry[kShadeTile];  // beta, gamma, triangle id, slot: hits from the front, the others from the back
@@ -1518,18 +1490,10 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 // 1151, 12 mixed scenes 3692 / 3635 / 3628 / 3632 / 3634 / 3594: 2^16.
 // 10 blocks of 64 per SM (102 registers): 1-3 % slower than with as many
 // registers as it likes below 64 K paths, up to 20 % faster above.
-#ifndef GB_PATHS_BLOCK
-#define GB_PATHS_BLOCK 64
-#endif
-#ifndef GB_PATHS_MIN
-#define GB_PATHS_MIN 10
-#endif
-#ifndef GB_PATHS_WARPS8
-#define GB_PATHS_WARPS8 1216
-#endif
-#ifndef GB_PATHS_WARPS
-#define GB_PATHS_WARPS 3040
-#endif
+constexpr int kPathsBlock = 64;
+constexpr int kPathsMinBlocks = 10;
+constexpr uint32_t kPathsWarps8 = 1216;
+constexpr uint32_t kPathsWarps16 = 3040;
 struct PathState {
     v3 o, d, tp, acc, pend;  // extension ray, throughput, accumulation, pending light sample
     v3 so, sd;               // shadow ray of the pending light sample
@@ -1552,8 +1516,7 @@ template <bool TEX>
 __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, bool alive, PathState& p, RayDiff& df,
                                              float4* sample, bool helpers) {
     uint32_t n_ext = 0, n_shadow = 0, n_hit = 0, nvis = 0, ntri = 0;
-    uint2 deep[kStack];
-    const StackRef stack{deep, deep, 1};
+    uint2 stack[kStack];
     RayInv r;
     Trav s;
     // a helper traces in its path's scene, which need not be this lane's
@@ -1651,14 +1614,14 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
 // paths of 225K there 412 / 383.  8 paths up to 3040 warps: room 16K 125; 16 up
 // to 4096 (more than resident): room 48K 131 / 158.
 __host__ __device__ __forceinline__ uint32_t paths_per_warp(uint32_t n) {
-    return n <= 8u * GB_PATHS_WARPS8 ? 8u : n <= 16u * GB_PATHS_WARPS ? 16u : 32u;
+    return n <= 8u * kPathsWarps8 ? 8u : n <= 16u * kPathsWarps16 ? 16u : 32u;
 }
 
 template <bool TEX>
-__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F, RenderParams P, const MrgPowers J) {
+__global__ void __launch_bounds__(kPathsBlock, kPathsMinBlocks) k_paths(Frame F, RenderParams P, const MrgPowers J) {
     fill_tables();
     const uint32_t lanes = paths_per_warp(P.chunk_paths);
-    const uint32_t l = (blockIdx.x * GB_PATHS_BLOCK + threadIdx.x) / 32u * lanes + lane_id();
+    const uint32_t l = (blockIdx.x * kPathsBlock + threadIdx.x) / 32u * lanes + lane_id();
     const bool alive = lane_id() < lanes && l < P.chunk_paths;
     const PathStart ps = path_start(F, P, alive ? l : 0u, &J);
     const SceneRec& R = F.scenes[ps.sc];
@@ -1672,14 +1635,14 @@ __global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_paths(Frame F,
 }
 
 template <bool TEX>
-__global__ void __launch_bounds__(GB_PATHS_BLOCK, GB_PATHS_MIN) k_finish(Frame F, RenderParams P) {
+__global__ void __launch_bounds__(kPathsBlock, kPathsMinBlocks) k_finish(Frame F, RenderParams P) {
     const int it = F.iter[0];
     const uint32_t* cs = ctr_set(F, it);
     const uint32_t ne = cs[CTR_EXT], count = ne + cs[CTR_ENDED];
     const uint32_t lanes = paths_per_warp(count);
-    if (blockIdx.x * (GB_PATHS_BLOCK / 32) * lanes >= count) return;
+    if (blockIdx.x * (kPathsBlock / 32) * lanes >= count) return;
     fill_tables();
-    const uint32_t first = (blockIdx.x * GB_PATHS_BLOCK + threadIdx.x) / 32u * lanes, i = first + lane_id();
+    const uint32_t first = (blockIdx.x * kPathsBlock + threadIdx.x) / 32u * lanes, i = first + lane_id();
     if (first >= count) return;
     const bool alive = lane_id() < lanes && i < count;
     const uint32_t k = alive ? i : 0u;
@@ -1863,22 +1826,15 @@ __global__ void __launch_bounds__(kBlock, 5) k_adjoint(Frame F, RenderParams P) 
 // 471 3267 / 923 470 3275 / 906 468 3210, but 200x150 frames 172 / 161 / 173.
 // The loops over a group stay rolled: unrolled, the code leaves the
 // instruction cache (1190 us).
-#ifndef GB_DIRECT_GROUP
-#define GB_DIRECT_GROUP 8
-#endif
-#ifndef GB_DIRECT_BLOCK
-#define GB_DIRECT_BLOCK 64
-#endif
-#ifndef GB_DIRECT_MIN
-#define GB_DIRECT_MIN 14
-#endif
-constexpr int kDirectGroup = GB_DIRECT_GROUP;
+constexpr int kDirectGroup = 8;
+constexpr int kDirectBlock = 64;
+constexpr int kDirectMinBlocks = 14;
 template <bool HYBRID>
-__global__ void __launch_bounds__(GB_DIRECT_BLOCK, GB_DIRECT_MIN) k_direct(
+__global__ void __launch_bounds__(kDirectBlock, kDirectMinBlocks) k_direct(
     DevScene S, CameraRec cam, int w, int h, int cam_samples, int light_samples, uint32_t seed, float shadow_offset,
     v3 background, float* out, uint32_t* status, const MrgSubseqTable T) {
     fill_tables();
-    const int g0 = blockIdx.x * GB_DIRECT_BLOCK + threadIdx.x;
+    const int g0 = blockIdx.x * kDirectBlock + threadIdx.x;
     const bool mine = g0 < w * h;
     const int g = mine ? g0 : 0;  // idle threads of the last block trace nothing
     const int px = g % w, py = g / w;
@@ -1886,8 +1842,7 @@ __global__ void __launch_bounds__(GB_DIRECT_BLOCK, GB_DIRECT_MIN) k_direct(
     const bool aperture = HYBRID && cam.aperture != 0.0f;
     if (aperture) lens = mrg_stream(T, seed, (uint32_t)((g + 17) % (w * h)));
     const int L = light_samples;
-    uint2 deep[kStack];
-    const StackRef stack{deep, deep, 1};
+    uint2 stack[kStack];
     Trav t;
     RayInv r;
     uint32_t nvis = 0, ntri = 0;
@@ -2290,14 +2245,12 @@ const MrgPowers& jitter_powers() {
     return T;
 }
 
-#ifndef GB_START_THREADS
-#define GB_START_THREADS (1 << 17)
-#endif
+constexpr int kStartThreads = 1 << 17;
 cudaError_t k_launch_start(const Frame& F, const RenderParams& P, int nstart, cudaStream_t st) {
     // enough threads to fill the chip, at most 8 paths each (12 mixed scenes 3.43 ms with the pool for every path,
     // 3.52 with a thread per path, 3.25 so; 256x256 room 0.935 / 0.921 / 0.907); rounds beyond the first nstart
     // paths have no blocks
-    const int group = std::min(8, std::max(1, nstart / GB_START_THREADS));
+    const int group = std::min(8, std::max(1, nstart / kStartThreads));
     int rounds = 1;
     while (rounds < P.rounds && P.round_start[rounds] < (uint32_t)nstart) ++rounds;
     const dim3 grid((unsigned)blocks_for(F.ntot), (unsigned)((rounds + group - 1) / group));
@@ -2416,7 +2369,7 @@ cudaError_t k_launch_adjoint(const Frame& F, const RenderParams& P, cudaStream_t
 cudaError_t k_launch_direct(const DevScene& S, const CameraRec& cam, int w, int h, int samples, uint32_t seed,
                             float shadow_offset, v3 background, float* out, uint32_t* status, cudaStream_t st) {
     if (w * h <= 0) return cudaSuccess;
-    k_direct<false><<<(w * h + GB_DIRECT_BLOCK - 1) / GB_DIRECT_BLOCK, GB_DIRECT_BLOCK, 0, st>>>(
+    k_direct<false><<<(w * h + kDirectBlock - 1) / kDirectBlock, kDirectBlock, 0, st>>>(
         S, cam, w, h, 1, samples, seed, shadow_offset, background, out, status, subseq_table());
     return cudaGetLastError();
 }
@@ -2425,7 +2378,7 @@ cudaError_t k_launch_direct_hybrid(const DevScene& S, const CameraRec& cam, int 
                                    int light_samples, uint32_t seed, float shadow_offset, v3 background, float* out,
                                    uint32_t* status, cudaStream_t st) {
     if (w * h <= 0) return cudaSuccess;
-    k_direct<true><<<(w * h + GB_DIRECT_BLOCK - 1) / GB_DIRECT_BLOCK, GB_DIRECT_BLOCK, 0, st>>>(
+    k_direct<true><<<(w * h + kDirectBlock - 1) / kDirectBlock, kDirectBlock, 0, st>>>(
         S, cam, w, h, cam_samples, light_samples, seed, shadow_offset, background, out, status, subseq_table());
     return cudaGetLastError();
 }
@@ -2462,21 +2415,21 @@ cudaError_t k_launch_regen(const Frame& F, const RenderParams& P, cudaStream_t s
 }
 
 cudaError_t k_launch_paths(const Frame& F, const RenderParams& P, cudaStream_t st) {
-    const unsigned per_block = GB_PATHS_BLOCK / 32 * paths_per_warp(P.chunk_paths);
+    const unsigned per_block = kPathsBlock / 32 * paths_per_warp(P.chunk_paths);
     const unsigned grid = (P.chunk_paths + per_block - 1) / per_block;
-    if (P.textured) k_paths<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
-    else k_paths<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P, jitter_powers());
+    if (P.textured) k_paths<true><<<grid, kPathsBlock, 0, st>>>(F, P, jitter_powers());
+    else k_paths<false><<<grid, kPathsBlock, 0, st>>>(F, P, jitter_powers());
     return cudaGetLastError();
 }
 
 cudaError_t k_launch_finish(const Frame& F, const RenderParams& P, cudaStream_t st) {
     if (P.finish_max <= 0) return cudaSuccess;
-    // the blocks of the most paths and, for fewer at 8 or 16 a warp, of at most GB_PATHS_WARPS warps
-    const unsigned most = (unsigned)std::min(P.finish_max, F.nslots), per_block = GB_PATHS_BLOCK / 32;
-    const unsigned warps = std::max((most + 31) / 32, std::min((most + 7) / 8, (unsigned)std::max(GB_PATHS_WARPS, GB_PATHS_WARPS8)));
+    // the blocks of the most paths and, for fewer at 8 or 16 a warp, of at most kPathsWarps16 warps
+    const unsigned most = (unsigned)std::min(P.finish_max, F.nslots), per_block = kPathsBlock / 32;
+    const unsigned warps = std::max((most + 31) / 32, std::min((most + 7) / 8, std::max(kPathsWarps16, kPathsWarps8)));
     const unsigned grid = (warps + per_block - 1) / per_block;
-    if (P.textured) k_finish<true><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
-    else k_finish<false><<<grid, GB_PATHS_BLOCK, 0, st>>>(F, P);
+    if (P.textured) k_finish<true><<<grid, kPathsBlock, 0, st>>>(F, P);
+    else k_finish<false><<<grid, kPathsBlock, 0, st>>>(F, P);
     return cudaGetLastError();
 }
 

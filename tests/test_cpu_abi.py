@@ -103,3 +103,14 @@ def test_struct_layouts_match_the_header(tmp_path):
     for name, fields in c_fields.items():
         for f in fields:
             assert int(got[f"{name}.{f}"]) == getattr(pairs[name], f).offset, f"{name}.{f}"
+
+
+def test_build_options_are_the_sources_defaults():
+    """Every build option names a define that the sources give a default, and
+    every such define is an option: none is taken and then ignored."""
+    from globillum_gb300 import build
+    found = set()
+    for f in build.CSRC.iterdir():
+        if f.suffix in (".cu", ".cpp", ".h"):
+            found |= set(re.findall(r"^#ifndef GB_(\w+)\n#define GB_", f.read_text(), flags=re.M))
+    assert found == set(build.KNOBS)
