@@ -235,19 +235,16 @@ def _f3(v) -> F3:
 
 
 def make_camera(cam: dict) -> Camera:
-    get = cam.get
-    return Camera(F3(*cam["pos"]), F3(*cam["dir"]), F3(*cam["up"]), cam["fovy_deg"], get("aperture", 0.0),
-                  get("focus_distance", 970.0), get("eye_to_lens", 5.0))
-
-
-_WHITE = (1.0, 1.0, 1.0)
+    return Camera(_f3(cam["pos"]), _f3(cam["dir"]), _f3(cam["up"]), float(cam["fovy_deg"]),
+                  float(cam.get("aperture", 0.0)), float(cam.get("focus_distance", 970.0)),
+                  float(cam.get("eye_to_lens", 5.0)))
 
 
 def make_render_desc(r: dict) -> RenderDesc:
-    get = r.get
     return RenderDesc(int(r["width"]), int(r["height"]), int(r["spp"]), int(r["max_bounces"]),
-                      int(get("rng_mode", GB_RNG_MRG32K3A_POOL)), int(get("seed", 0)), get("ray_offset", 0.3),
-                      get("shadow_offset", 0.9), F3(*get("background", _WHITE)), int(get("rr_start", -1)))
+                      int(r.get("rng_mode", GB_RNG_MRG32K3A_POOL)), int(r.get("seed", 0)),
+                      float(r.get("ray_offset", 0.3)), float(r.get("shadow_offset", 0.9)),
+                      _f3(r.get("background", (1.0, 1.0, 1.0))), int(r.get("rr_start", -1)))
 
 
 def make_scene_desc(scene) -> tuple[SceneDesc, list]:

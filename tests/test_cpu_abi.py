@@ -4,6 +4,7 @@ import ctypes as C
 import re
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -114,3 +115,23 @@ def test_build_options_are_the_sources_defaults():
         if f.suffix in (".cu", ".cpp", ".h"):
             found |= set(re.findall(r"^#ifndef GB_(\w+)\n#define GB_", f.read_text(), flags=re.M))
     assert found == set(build.KNOBS)
+
+
+@pytest.mark.parametrize("number", [float, int, str, lambda x: str(x).encode(), np.float32, np.int64])
+def test_descriptors_take_what_float_takes(number):
+    from globillum_gb300 import gbpt
+    v = [number(k) for k in (1, 2, 3)]
+    cam = gbpt.make_camera({"pos": v, "dir": tuple(v), "up": v, "fovy_deg": number(45), "aperture": number(2)})
+    assert (tuple(cam.pos), tuple(cam.dir), cam.fovy_deg, cam.aperture) == ((1.0, 2.0, 3.0), (1.0, 2.0, 3.0), 45.0, 2.0)
+    rd = gbpt.make_render_desc({"width": 4, "height": 5, "spp": 6, "max_bounces": 7, "ray_offset": number(8),
+                                "background": v})
+    assert (rd.width, rd.ray_offset, tuple(rd.background), rd.rr_start) == (4, 8.0, (1.0, 2.0, 3.0), -1)
+
+
+@pytest.mark.parametrize("bad", [None, "x", [1.0], {}])
+def test_descriptors_refuse_what_is_no_number(bad):
+    from globillum_gb300 import gbpt
+    with pytest.raises((TypeError, ValueError)):
+        gbpt.make_camera({"pos": (0, 0, 0), "dir": (0, 0, 1), "up": (0, 1, 0), "fovy_deg": bad})
+    with pytest.raises((TypeError, ValueError)):
+        gbpt.make_render_desc({"width": 4, "height": 5, "spp": 6, "max_bounces": 7, "shadow_offset": bad})
