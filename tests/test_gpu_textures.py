@@ -85,3 +85,44 @@ def test_texture_errors(gpu_ctx):
     rc = gpu_ctx.lib.gb_render_noalloc(s.h, C.byref(cam), C.byref(desc), C.c_void_p(16), None)
     assert rc == gbpt.GB_ERR_UNSUPPORTED
     s.close()
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_colours_of_textured_materials(gpu_ctx, seed):
+    """x^2.2 of a textured material's colours on the device (float pairs, with
+    doubles to decide) against the oracle's doubles: a wall of 256 x 64 cells of
+    a material each under a white texture, colours of every size from 2^-30 to 2^30,
+    zero, one, and the ends of the range of the float pairs."""
+    from oracle import oracle
+    w, h = 256, 64
+    r = np.random.default_rng(seed)
+    n = w * h
+    colour = np.exp2(r.uniform(-30.0, 30.0, (n, 3))).astype(np.float32)
+    colour[: n // 2] = r.uniform(0.0, 1.0, (n // 2, 3)).astype(np.float32)
+    ends = np.array([2.0 ** -20, 2.0 ** 20, 0.0, 1.0, 0.5, 1e-38], np.float32)
+    edge = np.concatenate([ends, np.nextafter(ends, np.float32(0)), np.nextafter(ends, np.float32(np.inf))])
+    colour.reshape(-1)[r.integers(0, 3 * n, 6000)] = edge[r.integers(0, edge.size, 6000)]
+    x, y = np.meshgrid(np.arange(w + 1.0), np.arange(h + 1.0))
+    p = np.stack([x / w * 4.0 - 2.0, y / h - 0.5, np.zeros_like(x)], -1)  # 4 x 1 at z = 0, seen from z = -2
+    a, b, c, d = p[:-1, :-1], p[:-1, 1:], p[1:, 1:], p[1:, :-1]
+    tri = np.stack([np.stack([a, b, c], 2), np.stack([a, c, d], 2)], 2).reshape(2 * n, 3, 3)
+    tc = np.stack([tri[..., 0] * 0.1 + 0.5, tri[..., 1] * 0.1 + 0.5], -1)
+    base = scenes.cornell()
+    params = [dict(color=tuple(map(float, k)), roughness=0.6, metallic=float(m), specular=0.5)
+              for k, m in zip(colour, r.choice([0.0, 0.5, 1.0], n))]
+    sc = scenes.SceneData(
+        tri.reshape(2 * n, 9).astype(np.float32), np.tile(np.float32([0, 0, -1]), (2 * n, 3)),
+        np.repeat(np.arange(n), 2).astype(np.int32),
+        [{"diffuse": (0.5, 0.5, 0.5), "principled": i, "diffuse_texture": 0} for i in range(n)], params,
+        [dict(base.lights[0], center=(0.0, 0.0, -3.0), dir=(0.0, 0.0, 1.0), up=(0.0, 1.0, 0.0), wh=(1.0, 1.0))],
+        dict(base.camera, pos=(0.0, 0.0, -2.0), dir=(0.0, 0.0, 1.0), up=(0.0, 1.0, 0.0), fovy_deg=27.0, aperture=0.0),
+        dict(base.render, width=2 * w, height=2 * h, spp=2, max_bounces=1, rng_mode=gbpt.GB_RNG_MRG32K3A_POOL, ray_offset=1e-3,
+             shadow_offset=1e-3),
+        textures=[np.full((64, 64, 4), 255, np.uint8)], texcoords=tc.reshape(2 * n, 6).astype(np.float32))
+    s = gpu_ctx.scene(sc)
+    img = s.render(sc.camera, sc.render)
+    s.close()
+    pool = gpu_ctx.mrg_pool(4 * n, 2)
+    ref = oracle.OracleScene(sc, use_bvh=True).render(sc.camera, sc.render, pool).astype(np.float32)
+    assert len(np.unique(ref)) > 0.4 * ref.size  # most pixels show a colour of their own
+    assert np.array_equal(img, ref, equal_nan=True)

@@ -417,3 +417,56 @@ def test_gradient_copies(gpu_ctx, materials):
         assert -0.02 < lost < 0.25
     finally:
         s.close()
+
+
+def _three_scenes():
+    """A room with Halton light draws, a textured soup under a sky through a lens,
+    and a plain soup with two lights: 200x150 at 7 spp, 300x250 at 5 and
+    31x23 at 6."""
+    room = scenes.principled_room(width=200, height=150, spp=7, max_bounces=5, rr_start=2)
+    soup = scenes.with_textures(scenes.icospheres(n_spheres=30, level=2, box=12.0, width=300, height=250, spp=5,
+                                                  max_bounces=4, n_lights=1), scale=0.2)
+    soup.lights.append({"type": gbpt.GB_LIGHT_SKY, "map": scenes.procedural_sky(32, 16), "scale": 0.5, "diameter": 30.0,
+                        "power": -1.0})
+    soup.camera.update(aperture=0.2, focus_distance=8.0)
+    plain = scenes.icospheres(n_spheres=9, level=2, box=9.0, width=31, height=23, spp=6, max_bounces=6, n_lights=2)
+    return [room, soup, plain]
+
+
+@pytest.fixture(scope="module")
+def three_references(gpu_ctx):
+    from oracle import oracle
+    out = []
+    for sc in _three_scenes():
+        rd = sc.render
+        pool = gpu_ctx.mrg_pool(rd["width"] * rd["height"], rd["spp"] * rd["max_bounces"], seed=rd.get("seed", 0))
+        out.append(oracle.OracleScene(sc, use_bvh=True).render(sc.camera, rd, pool).astype(np.float32))
+    return out
+
+
+@pytest.mark.parametrize("sample_mb,slots,graph", [(1024, 4099, True), (1024, 4099, False), (4, 4099, True), (4, 1 << 24, True),
+                                                   (4, 70000, True), (4, 70000, False), (2, 333, True), (2, 333, False)])
+def test_large_frames_with_small_pools(gpu_ctx, three_references, sample_mb, slots, graph):
+    """Frames beyond the chunks that follow whole paths, with pools far smaller
+    than they are: paths restart on used slots inside the captured loop (textured,
+    under a sky, through a lens, of several scenes), k_finish takes what is
+    left, and chunks of both kinds follow one another (4 MB of samples: two
+    rounds of 105,713 pixels through the loop, the last 167,000 paths whole).
+    Every image equals the oracle's."""
+    data = _three_scenes()
+    hs = [gpu_ctx.scene(sc) for sc in data]
+    old = gpu_ctx.get_tuning()
+    try:
+        gpu_ctx.set_tuning(slots=slots, sample_mb=sample_mb)
+        got = gpu_ctx.render_batch([(h, sc.camera, sc.render) for h, sc in zip(hs, data)], graph=graph)
+        for g, ref in zip(got, three_references):
+            assert np.array_equal(g, ref), np.abs(g - ref).max()
+        st = gpu_ctx.stats()
+        assert st["camera_rays"] == sum(sc.render["width"] * sc.render["height"] * sc.render["spp"] for sc in data)
+        for h, sc, ref in zip(hs[:2], data, three_references):
+            gpu_ctx.set_tuning(graph=2 if graph else 1)
+            assert np.array_equal(h.render(sc.camera, sc.render), ref)
+    finally:
+        gpu_ctx.set_tuning(slots=old["slots"], sample_mb=old["sample_mb"], graph=old["graph"])
+        for h in hs:
+            h.close()
