@@ -254,13 +254,6 @@ static inline CameraRec make_camera(const gb_camera& c, int w, int h) {
     return r;
 }
 
-// Jump matrices for `steps` MRG32k3a steps (mrg_power of the one-step
-// matrices, gbpt_math.h).
-static inline void mrg_jump_matrices(uint64_t steps, uint32_t J1[9], uint32_t J2[9]) {
-    mrg_power(kMrgA1, steps, J1, 209u, kMrgM1);
-    mrg_power(kMrgA2, steps, J2, 22853u, kMrgM2);
-}
-
 static inline ShadeParams make_shade_params(const gb_render_desc& d) {
     ShadeParams s;
     s.ray_offset = d.ray_offset;

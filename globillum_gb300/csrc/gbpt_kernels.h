@@ -183,8 +183,8 @@ struct Frame {
 
 // Counter set of an iteration: extension rays, shadow rays and pending ended
 // paths queued for it, head of its ray queue, finished paths of the adjoint,
-// closest hits found, paths started.
-enum { CTR_EXT = 0, CTR_SHADOW = 1, CTR_ENDED = 2, CTR_HEAD = 3, CTR_DONE = 4, CTR_HITS = 5, CTR_STARTED = 6 };
+// paths started.
+enum { CTR_EXT = 0, CTR_SHADOW = 1, CTR_ENDED = 2, CTR_HEAD = 3, CTR_DONE = 4, CTR_STARTED = 5 };
 
 // Points the per-slot arrays of F at `base` (kSlotBytes * cap bytes, cap a
 // multiple of kSlotAlign).
@@ -212,7 +212,7 @@ struct RenderParams {
     int p0, rounds;    // path samples p0 .. p0+rounds-1
     int pool_round;    // first round of the chunk that k_start does not start whole (rounds: none)
     int more;          // chunks of the frame follow: the pixels' stream cursors move on
-    int pad_;
+    int pad_;          // no hidden padding before the pointers: the words are a graph's key
     int max_iters;     // iteration bound of the chunk's loop
     int finish_max;    // the loop leaves the chunk's last paths to k_finish once at most this many are alive (0: never)
     const float4* nodes;  // the tree of a frame of one scene (null: every lane has its own scene's)

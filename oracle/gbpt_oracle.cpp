@@ -1062,12 +1062,24 @@ int orc_sincos_2pi(int n, const float* u, float* s, float* c) {
     return 0;
 }
 
-// MRG32k3a jump of `steps` generator steps (mrg_jump_matrices + mrg_jump of
-// the library's shared headers) applied to s1[3], s2[3] in place.
-int orc_mrg_jump(unsigned long long steps, uint32_t* s1, uint32_t* s2) {
-    uint32_t J1[9], J2[9];
-    mrg_jump_matrices(steps, J1, J2);
-    mrg_jump(s1, s2, J1, J2);
+// MRG32k3a jump of `steps` generator steps (mrg_powers + mrg_jump of the
+// library's shared headers) applied to s1[3], s2[3] in place; power k: of
+// steps * 2^k steps.
+int orc_mrg_jump(unsigned long long steps, int power, uint32_t* s1, uint32_t* s2) {
+    if (power < 0 || power > 6) return 1;
+    MrgPowers T;
+    mrg_powers(steps, &T);
+    mrg_jump(s1, s2, T.j1[power], T.j2[power]);
+    return 0;
+}
+
+// n draws of the shared integer generator (mrg_next, mrg_uniform) from s1[3],
+// s2[3], which move on.
+int orc_mrg_draws(int n, uint32_t* s1, uint32_t* s2, uint32_t* z, float* u) {
+    for (int i = 0; i < n; ++i) {
+        z[i] = mrg_next(s1, s2);
+        u[i] = mrg_uniform(z[i]);
+    }
     return 0;
 }
 

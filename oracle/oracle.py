@@ -45,7 +45,8 @@ def load() -> C.CDLL:
         lib.orc_material_sample_eval.argtypes = [vp] * 12
         lib.orc_sincos_2pi.argtypes = [ip, vp, vp, vp]
         lib.orc_shade_eval.argtypes = [vp] * 7
-        lib.orc_mrg_jump.argtypes = [C.c_ulonglong, vp, vp]
+        lib.orc_mrg_jump.argtypes = [C.c_ulonglong, C.c_int, vp, vp]
+        lib.orc_mrg_draws.argtypes = [C.c_int, vp, vp, vp, vp]
         lib.orc_atan2_acos.argtypes = [ip, vp, vp, vp, vp]
         lib.orc_dist1d.argtypes = [ip, vp, ip, vp, vp, vp]
         lib.orc64_scene_create.restype = vp
@@ -291,12 +292,23 @@ def shade_eval(diffuse, principled: bool, params18, n_raw, ray_dir, rnd, to_ligh
     return out
 
 
-def mrg_jump(steps: int, s1, s2):
-    """Library jump-ahead of an MRG32k3a state by `steps` generator steps."""
+def mrg_jump(steps: int, s1, s2, power: int = 0):
+    """Library jump-ahead of an MRG32k3a state by steps * 2^power generator
+    steps (power 0 .. 6)."""
     a = np.ascontiguousarray(s1, np.uint32).copy()
     b = np.ascontiguousarray(s2, np.uint32).copy()
-    load().orc_mrg_jump(int(steps), _p(a), _p(b))
+    if load().orc_mrg_jump(int(steps), int(power), _p(a), _p(b)):
+        raise ValueError("power must be 0 .. 6")
     return a, b
+
+
+def mrg_draws(n: int, s1, s2):
+    """n draws of the library's integer generator: (z, uniforms, s1, s2)."""
+    a = np.ascontiguousarray(s1, np.uint32).copy()
+    b = np.ascontiguousarray(s2, np.uint32).copy()
+    z, u = np.empty(n, np.uint32), np.empty(n, np.float32)
+    load().orc_mrg_draws(n, _p(a), _p(b), _p(z), _p(u))
+    return z, u, a, b
 
 
 def atan2_acos(y, x):
