@@ -620,7 +620,10 @@ __device__ __forceinline__ float max8(unsigned gm, float v) {
 // latency of the climb.  205 K triangles: 59 us, against 72 + 63 us for a
 // climb of the binary tree and a thread per 8-wide node after it (50 us of that
 // in double operations); refit and a 2-spp frame 725 -> 650 us.  Kept for a
-// refit: 4 B per 8-wide node, where the binary tree took 90 B per triangle.
+// refit: 4 B per 8-wide node of each scene, where the binary tree took 90 B per
+// triangle, and in the context's scratch, until the context is destroyed, the
+// vertices and normals as copied (72 B per triangle of the largest scene
+// refitted) and 36 B per node.
 // bad[0] = 2: a parent that does not come before its child; 3: an index
 // outside its buffer.
 __global__ void __launch_bounds__(kBuildBlock) k_refit(const float* __restrict__ pos, int n, int n_nodes,

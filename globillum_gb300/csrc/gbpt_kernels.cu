@@ -37,9 +37,10 @@ namespace {
 
 constexpr int kBlock = 128;
 // Resident 128-thread blocks per SM the traversal kernels are compiled for: 7
-// (72 registers, no spills).  1M-triangle frame, 64 spp, at 6 / 7 / 8 blocks:
-// 36.7 / 35.3 / 35.2 ms; 12 mixed scenes 3.26 / 3.17 / 3.22 ms; 262 K closest
-// hits 95 / 96 / 102 us; 2 M shadow rays 320 / 306 / 304 us.
+// (72 registers; 8 B of spills in the variants for several scenes, none in those
+// for one).  1M-triangle frame, 64 spp, at 6 / 7 / 8 blocks: 35.7 / 34.0 / 33.9
+// ms; 12 mixed scenes 3.19 / 3.09 / 3.01 ms; 262 K closest hits in 64 K triangles
+// 95 / 94 / 96 us; 2 M shadow rays 319 / 297 / 290 us.
 #ifndef GB_TRAV_MIN_BLOCKS
 #define GB_TRAV_MIN_BLOCKS 7
 #endif
@@ -374,11 +375,12 @@ __device__ __forceinline__ bool node_step(const float4* __restrict__ nodes, cons
 // second one (nt), which it cannot store further.  A pop and the visit it
 // leads to are one step, and a lane whose last group is empty is finished at
 // the end of the step.  GB_TRI_RATIO (triangle lanes times this >= node lanes
-// tests triangles) on the 1M-triangle 64-spp frame: 51.0 / 50.0 / 50.0 /
-// 50.1 / 50.5 ms for 1 / 2 / 3 / 4 / 6, 1.84 / 1.82 / 1.84 / 1.85 / 1.89 ms
-// at 1 spp; every pending triangle after each visit, with pops as steps of
-// their own: 55.4 and 2.05 ms.  A lane is finished when it has neither, so the
-// two votes of the step also tell which lanes are idle.
+// tests triangles) on the 1M-triangle frame at 64 spp / 1 spp / the 256x256
+// 16-spp room: 34.3 34.0 34.1 34.3 ms / 896 893 904 909 us / 822 833 847 848 us
+// for 1 / 2 / 3 / 4; every pending triangle after each visit, with pops as steps
+// of their own, was slower by a tenth when the vote was introduced.  A lane is
+// finished when it has neither, so the two votes of the step also tell which
+// lanes are idle.
 #ifndef GB_TRI_RATIO
 #define GB_TRI_RATIO 2
 #endif
@@ -979,7 +981,9 @@ __device__ __forceinline__ void ray_loop(uint32_t count, uint32_t* head, int ref
 
 // gb_trace_closest / gb_trace_any: the caller's rays through the persistent
 // ray loop.  head: the queue head (zero), read only when there are more rays
-// than lanes in the grid.  A negative or NaN max_t traces nothing.
+// than lanes in the grid.  A negative or NaN max_t traces nothing.  Refilled at
+// 4 / 8 / 12 / 16 / 20 idle lanes: 2 M shadow rays 342 / 306 / 297 / 298 / 307 us,
+// 262 K closest hits 96 / 93 / 94 / 94 / 93.
 constexpr int kTraceRefill = 12;
 __global__ void __launch_bounds__(kBlock, GB_TRAV_MIN_BLOCKS) k_trace(DevScene S, uint32_t n,
                                                                       const float* __restrict__ orig,
@@ -1211,17 +1215,17 @@ __device__ __forceinline__ LightSample light_sample(const Frame& F, const SceneR
 // slot with the chunk's next path; in MODE_ADJOINT it goes to the done queue
 // instead, for k_adjoint and k_regen.
 //
-// What bounds it: latency of the scattered sector, triangle and material loads
-// and of the ~1100 dependent instructions of a hit, at 28 warps per SM.
-// Measured on the 1M-triangle 64-spp frame / 1 spp / 256x256 room: tiles of one
-// entry per thread sorted by a block scan 45.8 / 1.37 / 1.02 ms; a warp on its
-// own with tiles of 128 44.6 / 1.39 / 1.05; of 32..64 49.6 / 1.41 / 1.05
-// (rounds half empty); this form with tiles of 256 / 512 / 1024 at 5 blocks per
-// SM 44.8 / 43.3 / 43.5; 512 at 6 / 7 / 8 / 10 blocks (80 / 72 / 64 / 48
-// registers) 43.0 / 42.3 / 42.6 / 43.9, 1.36 / 1.34 / 1.35 / 1.39 and 1.05 /
-// 1.01 / 1.02 / 1.08: more warps are worth the spills up to 7 blocks.  Fetching
-// a tile's sectors to L2 ahead changes nothing, triangles as well slows small
-// scenes by a quarter.
+// What bounds it: latency of the scattered sector, triangle and material loads,
+// of the ~1100 dependent instructions of a hit and of fetching them (the code is
+// larger than the instruction cache), at 28 warps per SM.  Tiles of one entry per
+// thread sorted by a block scan, and a warp on its own with tiles of 128, were
+// slower by 3 to 6 % when rounds of one kind were introduced.  1M-triangle 64-spp frame
+// / 1 spp / 256x256 room: tiles of 256 / 384 / 512 / 640 / 768 36.7 35.4 34.0
+// 34.0 34.3 ms (room 856 849 831 834 846 us); 5 / 6 / 7 / 8 / 10 blocks per SM
+// (96 / 80 / 72 / 64 / 48 registers) 34.7 34.1 34.0 34.2 35.4 ms, 917 896 890
+// 900 925 us and 862 842 831 884 945 us, spills of 110 to 230 B at 7 among them.
+// Fetching a tile's sectors to L2 ahead changes nothing, triangles as well slows
+// small scenes by a quarter.
 //
 // A vertex's light sample adds bl * (tp * psc) to the accumulation if its
 // shadow ray is free.  The contribution is formed here and kept pending; the
@@ -1478,18 +1482,20 @@ __global__ void __launch_bounds__(kBlock, GB_SHADE_MIN_BLOCKS) k_shade(Frame F, 
 //
 // A queue that does not fill the chip is bound by latency: each bounce costs
 // the loop two launches, a tail of long rays and a round trip of the path
-// state, whatever the work: 250 us for the 64x64 room at 1 and at 4 spp.
-// Wall time of a frame, the loop with k_finish for its last paths against
-// k_paths (us, paths in thousands):
-//   room      4K 140 / 117   48K 157 / 130   128K 241 / 229   256K 328 / 341   512K 478 / 624
-//   64 K tri  6K 181 / 164   48K 221 / 201   144K 319 / 283   250K 350 / 376
-//   512 K tri               48K 254 / 231   144K 355 / 378   225K 403 / 448
-// hence k_paths up to 3 * 2^16 paths.  The last paths of a chunk at 0 / 2^14 /
-// 2^15 / 2^16 / 2^17 / 2^18 alive: 1 spp of the 1M-triangle frame 1303 / 1187
-// / 1187 / 1097 / 1149 / 1146, textured sky 1231 / 1195 / 1113 / 1140 / 1131 /
-// 1151, 12 mixed scenes 3692 / 3635 / 3628 / 3632 / 3634 / 3594: 2^16.
-// 10 blocks of 64 per SM (102 registers): 1-3 % slower than with as many
-// registers as it likes below 64 K paths, up to 20 % faster above.
+// state, whatever the work.  Wall time of a frame, the loop with k_finish for its
+// last paths against k_paths (us, paths in thousands):
+//   room      4K 122 / 102   48K 156 / 131   128K 232 / 225   196K 282 / 263   256K 320 / 341   512K 478 / 633
+//   64 K tri  6K 169 / 150   48K 213 / 189   144K 301 / 258   192K 312 / 323   250K 327 / 351
+//   512 K tri               48K 228 / 200   144K 335 / 364   192K 378 / 426   225K 390 / 478
+// hence k_paths up to 3 * 2^16 paths: past the crossing of the largest trees, short
+// of that of small ones.  The last paths of a chunk at 0 / 2^14 /
+// 2^15 / 2^16 / 2^17 / 2^18 alive: 1 spp of the 1M-triangle frame 1090 / 935 /
+// 938 / 887 / 965 / 966, textured sky 712 / 651 / 628 / 642 / 639 / 641, 12 mixed
+// scenes 3160 / 3086 / 3088 / 3086 / 3086 / 3089: 2^16.
+// 10 blocks of 64 per SM (96 registers, 270 to 310 B of spills) against as many
+// registers as it likes: room 1K 102 / 99, 128K 225 / 212, 196K 263 / 280; 64 K
+// triangles 48K 189 / 181, 192K 323 / 311; 512 K triangles 48K 200 / 227, 225K
+// 387 / 376: neither is better everywhere.
 constexpr int kPathsBlock = 64;
 constexpr int kPathsMinBlocks = 10;
 constexpr uint32_t kPathsWarps8 = 1216;
@@ -1609,10 +1615,9 @@ __device__ __forceinline__ void follow_paths(const Frame& F, const SceneRec& R, 
 // 32.  The chip is then far from full whatever the split; fewer paths make
 // fewer turns of the vote between nodes and triangles, fewer lobes one after
 // the other, and leave lanes for the second ray.  32 always / this rule (us,
-// paths in thousands): room 1K 115 / 100, 16K 120 / 109, 36K 130 / 125; 64 K
-// triangles 6K 166 / 149, 32K 179 / 161; 512 K triangles 32K 216 / 197; last
-// paths of 225K there 412 / 383.  8 paths up to 3040 warps: room 16K 125; 16 up
-// to 4096 (more than resident): room 48K 131 / 158.
+// paths in thousands): room 1K 115 / 102, 16K 117 / 106, 48K 129 / 131; 64 K
+// triangles 6K 175 / 150, 48K 199 / 189; 512 K triangles 48K 224 / 200; last
+// paths of 225K there 416 / 387.
 __host__ __device__ __forceinline__ uint32_t paths_per_warp(uint32_t n) {
     return n <= 8u * kPathsWarps8 ? 8u : n <= 16u * kPathsWarps16 ? 16u : 32u;
 }
@@ -1819,11 +1824,13 @@ __global__ void __launch_bounds__(kBlock, 5) k_adjoint(Frame F, RenderParams P) 
 // (warp_step), and the samples are then averaged in order, so that the warp
 // waits for its slowest lane once a group and not once a ray.  A sample whose
 // weight is exactly zero traces nothing (its term is zero either way while the
-// colour is finite).  641x359, 64 K triangles, hybrid 2 x 8 / 2 x 2; 1280x720,
-// 384 K triangles, 16 samples (us with the image to the host): a ray at a time
-// per thread 1446 / 642 / 4594; groups of 4 / 8 / 16 at 10 blocks of 64 per SM
-// 962 476 3522 / 952 482 3470 / 950 479 5225; of 8 at 12 / 14 / 16 blocks 926
-// 471 3267 / 923 470 3275 / 906 468 3210, but 200x150 frames 172 / 161 / 173.
+// colour is finite).  64 K triangles, 641x359 hybrid 2 x 8, the same 2 x 2,
+// 384 K triangles 1280x720 with 16 samples, and 64 K 200x150 hybrid 2 x 8 (us with
+// the image to the host):
+//   groups of 4 / 8 / 16 at 14 blocks of 64 per SM   904 471 3192 497 / 893 469 3163 480 / 896 471 3150 483
+//   of 8 at 10 / 12 / 16 blocks                      902 471 3198 446 / 893 469 3086 459 / 908 469 3193 493
+// (14 blocks spill 290 to 430 B).  A ray at a time per thread: 641x359 1266 against
+// 863, 200x150 631 against 480, 500x400 2 x 2 630 against 447.
 // The loops over a group stay rolled: unrolled, the code leaves the
 // instruction cache (1190 us).
 constexpr int kDirectGroup = 8;
@@ -2330,8 +2337,8 @@ cudaError_t k_launch_rays(const Frame& F, const RenderParams& P, bool instrument
 // over what is left.  A block per 512 slots gives a full queue's blocks
 // one whole tile each; a thread per slot makes the tiles of 128, fewer blocks
 // leave a long last wave.  nslots / 1 / 4 / 16 / 64 threads: 1M-triangle 64-spp
-// frame 38.1 / 34.8 / 35.2 / 35.6 ms, 12 mixed scenes 3.51 / 3.10 / 3.15 /
-// 3.43 ms.
+// frame 37.2 / 34.0 / 34.8 / 34.7 ms, 12 mixed scenes 3.49 / 3.08 / 3.19 /
+// 3.42 ms.
 #ifndef GB_WIDE_GRID_DIV
 #define GB_WIDE_GRID_DIV 4  // the wide grid has nslots / GB_WIDE_GRID_DIV threads
 #endif

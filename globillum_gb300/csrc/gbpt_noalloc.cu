@@ -206,9 +206,9 @@ int render_noalloc(const gb_scene* scene, const gb_camera* cam, const gb_render_
     // one path sample of every pixel per pass, one slot per pixel: a path
     // has at most max_bounces segments and its last light sample is settled
     // one iteration later, so the queues are empty after max_bounces + 1
-    // iterations; the host checks the queue counts every 8 iterations and the
-    // device flags queues still non-empty after max_bounces + 2 iterations
-    // (ST_ITER_LIMIT)
+    // iterations; the host checks the queue counts every 8 iterations and after
+    // max_bounces + 2, the last it launches, where queues that are still not empty
+    // end the call with an error
     const int max_iters = d->max_bounces + 2;
     P.max_iters = max_iters;
     uint32_t left = 0;

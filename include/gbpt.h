@@ -432,7 +432,10 @@ typedef struct {
     /* per-stage device time when stage timing is on (gb_ctx_set_stage_timing):
      * 0 path start, 1 traversal (closest-hit and any-hit rays together),
      * 2 unused, 3 shade + light sample + restart, 4 adjoint sweep + its
-     * restarts, 5 moving average                                               */
+     * restarts, 5 moving average.  Frames of up to 3 * 2^16 paths, which
+     * otherwise follow whole paths in one launch, run these stages as well
+     * then (and under gb_render_instrumented): their times are not those of
+     * the untimed frame                                                        */
     double stage_ms[6];
     uint64_t stage_launches[6];
     int paths_done;
@@ -523,7 +526,11 @@ typedef struct {
  * gb_backward_batch apply).  The targets and images must stay valid and the
  * scenes must not be used by other calls while steps run.  Renders on the
  * same context in between may grow its buffers; the next step then
- * captures the graph again by itself. */
+ * captures the graph again by itself.  Losses are taken and images written
+ * scene after scene (by spp, the most first, else as given): a target that
+ * shares memory with another scene's image is read as the scenes before have
+ * left it.  An image may lie anywhere a device copy can write; an allocation
+ * shorter than its image is refused (GB_ERR_CUDA). */
 int gb_fit_prepare(gb_ctx* ctx, int n, const gb_fit_item* items);
 /* One step: params[i] (host, gb_scene_param_count floats) become item i's
  * scene parameters, as gb_scene_set_params sets them; dL_dparams[i] (host)
